@@ -40,11 +40,15 @@ int current_sm_count() {
 }
 
 // conv_generic.cu
-int conv_gather_generic(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr,
-                        int64_t n_out, int kv, int K, int N, int flip_k, const float* scale, const float* bias,
-                        int relu, void* out, int out_dtype, int* status, cudaStream_t st);
-int conv_wgrad_generic(const void* rows, const void* dout, int dtype, int64_t n_rows, const int* nbr,
-                       int64_t n_out, int kv, int K, int N, float* dw, int* status, cudaStream_t st);
+int conv_gather_generic(const void* rows, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out, int kv,
+                        int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                        int out_dtype, int* status, cudaStream_t st);
+// conv_ffma.cu
+int conv_gather_ffma(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
+                     int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                     int out_dtype, int* status, cudaStream_t st);
+int conv_wgrad_ffma(const void* rows, const void* dout, int dtype, int64_t n_rows, const int* nbr, int64_t n_out, int kv,
+                    int K, int N, float* dw, int* status, cudaStream_t st);
 // conv_tc.cu
 int conv_gather_tc(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
                    int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
@@ -140,8 +144,11 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
     return conv_gather_sparse(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias,
                               relu, d_out, out_dtype, d_status, st);
   }
-  return conv_gather_generic(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias,
-                             relu, d_out, out_dtype, d_status, st);
+  if (dtype == SPH_I8)
+    return conv_gather_generic(d_rows, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias, relu,
+                               d_out, out_dtype, d_status, st);
+  return conv_gather_ffma(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias, relu,
+                          d_out, out_dtype, d_status, st);
 }
 
 extern "C" int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype, int64_t n_rows,
@@ -158,5 +165,5 @@ extern "C" int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype,
   // narrow rows the tensor-core kernel does not take and small fp32 layers: the pair-compacting walk
   if (conv_wgrad_pairs_supported(dtype, kv, k_ch, n_ch) && ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0))
     return conv_wgrad_pairs(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
-  return conv_wgrad_generic(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
+  return conv_wgrad_ffma(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
 }

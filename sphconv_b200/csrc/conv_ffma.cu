@@ -1,0 +1,492 @@
+// fp32 arithmetic (FFMA) kernels of the rule-driven convolution: float32 rows (the 1e-4 tolerance rules out single-pass
+// TF32) and 16-bit rows of channel counts the tensor-core kernels do not take.
+//
+// Both kernels work on the PRESENT pairs only - the FMA pipe is what bounds a float32 layer, so a slot without a
+// neighbour must cost nothing - and both are register-blocked outer products over rows staged in shared memory.
+#include "common.cuh"
+#include "tc_common.cuh"
+
+namespace sph {
+
+namespace {
+
+using tc::cp_async_16;
+using tc::cp_async_commit;
+using tc::cp_async_wait_pending;
+using tc::smem_u32;
+
+__device__ __forceinline__ float widen(float v) { return v; }
+__device__ __forceinline__ float widen(__half v) { return __half2float(v); }
+__device__ __forceinline__ float widen(__nv_bfloat16 v) { return __bfloat162float(v); }
+
+__device__ __forceinline__ void store_one(void* out, int out_dtype, int64_t idx, float v) {
+  switch (out_dtype) {
+    case SPH_F32: ((float*)out)[idx] = v; break;
+    case SPH_F16: ((__half*)out)[idx] = __float2half_rn(v); break;
+    default: ((__nv_bfloat16*)out)[idx] = __float2bfloat16_rn(v);
+  }
+}
+
+constexpr int kRows = 128;            // output rows of a tile
+constexpr int kItem = 64;             // pairs of a step
+constexpr int kKC = 32;               // input channels of a step
+constexpr int kAStride = kKC + 4;     // floats; consecutive rows start 4 banks apart: 16-byte reads of 8 rows do not conflict
+constexpr int kBatch = 9;             // kernel offsets whose pair lists are held at a time
+
+struct FfmaParams {
+  const void* rows;
+  const void* weight;                 // [KV, K, N]
+  const int* nbr;                     // [KV, n_out]
+  int64_t n_rows, n_out;
+  int kv, K, N, flip_k, relu, out_dtype;
+  const float* scale;
+  const float* bias;
+  void* out;
+  int* status;
+};
+
+template <int CG> struct FfmaShape {
+  static constexpr int NP = CG * 8;                  // output channels of a CTA, padded
+  static constexpr int T = CG == 8 ? 128 : 64;       // threads of a CTA
+  static constexpr int RL = T / CG;                  // row lanes
+  static constexpr int RP = kItem / RL;              // rows per thread at most
+  static constexpr int ACC = kRows * (NP + 4);       // floats
+  static constexpr int A = kItem * kAStride;
+  static constexpr int W = kKC * NP;
+  static constexpr int BYTES = (ACC + 2 * A + 2 * W) * 4 + kBatch * kRows * 5 + kBatch * 4;
+};
+
+// One step (offset, 32 input channels) of RP rows x 8 output channels per thread.  The two 4-channel groups of a thread are
+// NP/2 apart, so the lanes of a row read consecutive 16-byte pieces of the filter row.
+template <int CG, int RP>
+__device__ __forceinline__ void ffma_step(const float* __restrict__ a, const float* __restrict__ w, int rl, int cg,
+                                          float (&acc)[FfmaShape<CG>::RP][8]) {
+  using S = FfmaShape<CG>;
+#pragma unroll 2
+  for (int k4 = 0; k4 < kKC; k4 += 4) {
+    float av[RP][4];
+#pragma unroll
+    for (int j = 0; j < RP; ++j) {
+      const float4 t = *(const float4*)(a + (rl + j * S::RL) * kAStride + k4);
+      av[j][0] = t.x; av[j][1] = t.y; av[j][2] = t.z; av[j][3] = t.w;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 w0 = *(const float4*)(w + (k4 + q) * S::NP + cg * 4);
+      const float4 w1 = *(const float4*)(w + (k4 + q) * S::NP + S::NP / 2 + cg * 4);
+#pragma unroll
+      for (int j = 0; j < RP; ++j) {
+        acc[j][0] = fmaf(av[j][q], w0.x, acc[j][0]); acc[j][1] = fmaf(av[j][q], w0.y, acc[j][1]);
+        acc[j][2] = fmaf(av[j][q], w0.z, acc[j][2]); acc[j][3] = fmaf(av[j][q], w0.w, acc[j][3]);
+        acc[j][4] = fmaf(av[j][q], w1.x, acc[j][4]); acc[j][5] = fmaf(av[j][q], w1.y, acc[j][5]);
+        acc[j][6] = fmaf(av[j][q], w1.z, acc[j][6]); acc[j][7] = fmaf(av[j][q], w1.w, acc[j][7]);
+      }
+    }
+  }
+}
+
+// A CTA owns 128 consecutive output rows x up to 64 output channels.  Per offset k the rows of the tile that have a
+// neighbour are compacted into a list; up to 64 of their input rows and W[k] are staged (32 input channels a step, the next
+// step's copies in flight), every thread multiplies ceil(pairs / row lanes) listed rows by 8 channels in registers, on top
+// of the tile's fp32 accumulator in shared memory.  An output row occurs once per offset, so no two threads of a step hold the
+// same accumulator.
+// The CTA is small (64 or 128 threads) so that a thread has up to four rows: with one row per thread (256 threads a tile)
+// the shared-memory reads of the filter, not the FMAs, set the pace; with eight rows too few warps fit on an SM.
+// Bound by the issue slots (67 % busy, two thirds of them FMAs) and the shared-memory reads (60 %).  Measured: 64 -> 64 on
+// 170 k rows of 22 neighbours 3.2 -> 0.94 ms, 32 -> 32 on 390 k rows of 12 neighbours 1.9 -> 0.5 ms against the kernel it
+// replaced (one thread group per row walking every slot of the table).
+// VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by element.
+template <typename T, int CG, bool VEC>
+__global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams p) {
+  using S = FfmaShape<CG>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* s_acc = (float*)smem;                       // [kRows][NP + 4]
+  float* s_a = s_acc + S::ACC;                       // [2][kItem][kAStride]
+  float* s_w = s_a + 2 * S::A;                       // [2][kKC][NP]
+  int* s_in = (int*)(s_w + 2 * S::W);                // [kBatch][kRows] input row
+  int* s_m = s_in + kBatch * kRows;                  // [kBatch] pairs
+  unsigned char* s_out = (unsigned char*)(s_m + kBatch);   // [kBatch][kRows] row in the tile
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t r0 = (int64_t)blockIdx.x * kRows;
+  const int n0 = blockIdx.y * S::NP;                 // first output channel of this CTA
+  const int nc = min(S::NP, p.N - n0);
+  const int rl = tid / CG, cg = tid % CG;
+  const T* rows = (const T*)p.rows;
+  const T* weight = (const T*)p.weight;
+  const int k_chunks = (p.K + kKC - 1) / kKC;
+
+  for (int e = tid; e < S::ACC; e += S::T) s_acc[e] = 0.f;
+
+  auto stage = [&](int buf, int kb, int kk, int p0, int kc) {
+    const int m = min(kItem, s_m[kk] - p0);
+    const int* in = s_in + kk * kRows + p0;
+    float* a = s_a + buf * S::A;
+    float* w = s_w + buf * S::W;
+    const T* wk = weight + ((int64_t)(kb + kk) * p.K + kc * kKC) * p.N + n0;
+    const int kn = min(kKC, p.K - kc * kKC);
+    if constexpr (VEC) {
+      const int c = tid % (kKC / 4) * 4;
+      const bool ok = c < kn;
+      for (int r = tid / (kKC / 4); r < m; r += S::T / (kKC / 4)) {
+        cp_async_16(smem_u32(a + r * kAStride + c), ok ? rows + (int64_t)in[r] * p.K + kc * kKC + c : rows, ok ? 16u : 0u);
+      }
+      const int wc = tid % (S::NP / 4) * 4;
+      const T* src = wk + (int64_t)(tid / (S::NP / 4)) * p.N + wc;
+#pragma unroll 4
+      for (int r = tid / (S::NP / 4); r < kKC; r += S::T / (S::NP / 4)) {
+        const bool ok = r < kn && wc < nc;
+        cp_async_16(smem_u32(w + r * S::NP + wc), ok ? src : weight, ok ? 16u : 0u);
+        src += (S::T / (S::NP / 4)) * p.N;
+      }
+    } else {
+      for (int e = tid; e < m * kKC; e += S::T) {
+        const int r = e / kKC, c = e % kKC;
+        a[r * kAStride + c] = c < kn ? widen(rows[(int64_t)in[r] * p.K + kc * kKC + c]) : 0.f;
+      }
+      for (int e = tid; e < kKC * S::NP; e += S::T) {
+        const int r = e / S::NP, c = e % S::NP;
+        w[e] = (r < kn && c < nc) ? widen(wk[(int64_t)r * p.N + c]) : 0.f;
+      }
+    }
+  };
+
+  for (int kb = 0; kb < p.kv; kb += kBatch) {
+    const int nk = min(kBatch, p.kv - kb);
+    __syncthreads();                                  // the previous batch's lists are done with
+    for (int kk = warp; kk < nk; kk += S::T / 32) {
+      const int* col = p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - (kb + kk) : kb + kk) * p.n_out + r0;
+      int v[kRows / 32];
+#pragma unroll
+      for (int h = 0; h < kRows / 32; ++h) v[h] = r0 + h * 32 + lane < p.n_out ? __ldg(col + h * 32 + lane) : -1;
+      int n = 0;
+#pragma unroll
+      for (int h = 0; h < kRows / 32; ++h) {
+        if (v[h] >= p.n_rows) {
+          if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
+          v[h] = -1;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, v[h] >= 0);
+        if (v[h] >= 0) {
+          const int pos = n + __popc(m & ((1u << lane) - 1u));
+          s_in[kk * kRows + pos] = v[h];
+          s_out[kk * kRows + pos] = (unsigned char)(h * 32 + lane);
+        }
+        n += __popc(m);
+      }
+      if (lane == 0) s_m[kk] = n;
+    }
+    __syncthreads();
+    int kk = 0, p0 = 0, kc = 0;
+    while (kk < nk && s_m[kk] == 0) ++kk;
+    if (kk < nk) stage(0, kb, kk, 0, 0);
+    cp_async_commit();
+    float acc[S::RP][8];
+    for (int buf = 0; kk < nk; buf ^= 1) {
+      int nkk = kk, np0 = p0, nkc = kc + 1;
+      if (nkc == k_chunks) {
+        nkc = 0;
+        np0 += kItem;
+        if (np0 >= s_m[kk]) {
+          np0 = 0;
+          do { ++nkk; } while (nkk < nk && s_m[nkk] == 0);
+        }
+      }
+      cp_async_wait_pending(0);
+      __syncthreads();       // the step's operands are there, everybody has left the other buffer and the accumulator
+      if (nkk < nk) stage(buf ^ 1, kb, nkk, np0, nkc);
+      cp_async_commit();
+      const int m = min(kItem, s_m[kk] - p0);
+      // the accumulator tile is read before an item and written behind it: an output is ONE chain of fused multiply-adds
+      // over the offsets and input channels in ascending order, whatever the tiling
+      auto tile_row = [&](int r) { return s_acc + (int)s_out[kk * kRows + p0 + r] * (S::NP + 4) + cg * 4; };
+      if (kc == 0) {
+#pragma unroll
+        for (int j = 0; j < S::RP; ++j) {
+          if (rl + j * S::RL < m) {
+            const float* d = tile_row(rl + j * S::RL);
+            const float4 t0 = *(const float4*)d, t1 = *(const float4*)(d + S::NP / 2);
+            acc[j][0] = t0.x; acc[j][1] = t0.y; acc[j][2] = t0.z; acc[j][3] = t0.w;
+            acc[j][4] = t1.x; acc[j][5] = t1.y; acc[j][6] = t1.z; acc[j][7] = t1.w;
+          }
+        }
+      }
+      const float* a = s_a + buf * S::A;
+      const float* w = s_w + buf * S::W;
+      // rows beyond m are staged rows of an earlier step: multiplied, never added
+      const int rp = (m + S::RL - 1) / S::RL;
+      switch (rp) {
+        case 1: ffma_step<CG, 1>(a, w, rl, cg, acc); break;
+        case 2: ffma_step<CG, (S::RP < 2 ? 1 : 2)>(a, w, rl, cg, acc); break;
+        case 3: ffma_step<CG, (S::RP < 3 ? 1 : 3)>(a, w, rl, cg, acc); break;
+        default: ffma_step<CG, (S::RP < 4 ? 1 : 4)>(a, w, rl, cg, acc);
+      }
+      if (kc == k_chunks - 1) {
+#pragma unroll
+        for (int j = 0; j < S::RP; ++j) {
+          if (rl + j * S::RL < m) {
+            float* d = tile_row(rl + j * S::RL);
+            *(float4*)d = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+            *(float4*)(d + S::NP / 2) = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
+          }
+        }
+      }
+      kk = nkk; p0 = np0; kc = nkc;
+    }
+  }
+  __syncthreads();
+  const int rows_here = (int)min((int64_t)kRows, p.n_out - r0);
+  for (int e = tid; e < rows_here * nc; e += S::T) {
+    const int r = e / nc, c = e % nc;
+    float v = s_acc[r * (S::NP + 4) + c];
+    if (p.scale) v *= __ldg(p.scale + n0 + c);
+    if (p.bias) v += __ldg(p.bias + n0 + c);
+    store_one(p.out, p.out_dtype, (r0 + r) * p.N + n0 + c, p.relu ? fmaxf(v, 0.f) : v);
+  }
+}
+
+// ---- weight gradient: dW[k] += X_i^T dY_o over the pairs of offset k ------------------------------------------------
+// grid (row slices, KV).  A CTA compacts the pairs of its slice, then stages kWgPairs of them at a time (the next ones'
+// copies in flight); a thread owns 8 input x 8 output channels of the product, the threads are as many copies of the
+// K x N tile as fit, and each copy takes its share of the staged pairs.  The copies are summed in shared memory and added
+// to the gradient once per CTA.
+constexpr int kThreads = 256;
+constexpr int kWgSlice = 2048;
+constexpr int kWgPairs = 32;
+constexpr int kWgMaxCh = 64;
+
+struct FfmaWgradParams {
+  const void* rows;                   // [n_rows, K]
+  const void* dout;                   // [n_out, N]
+  const int* nbr;                     // [KV, n_out]
+  int64_t n_rows, n_out;
+  int K, N;
+  float* dw;                          // [KV, K, N], accumulated into
+  int* status;
+};
+
+// KG / NG: groups of 8 channels on either side.
+template <int KG, int NG> struct WgShape {
+  static constexpr int XS = KG * 8 + 4, DS = NG * 8 + 4;     // staged row strides in floats
+  static constexpr int COPIES = kThreads / (KG * NG);
+  static constexpr int STAGE = kWgPairs * (XS + DS);         // floats
+  static constexpr int RED = KG * NG * 64;                   // floats of the product
+  static constexpr int BYTES = (2 * STAGE > RED ? 2 * STAGE : RED) * 4 + kWgSlice * 8 + 64;
+};
+
+template <typename T, int KG, int NG, bool VEC>
+__global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradParams p) {
+  using S = WgShape<KG, NG>;
+  extern __shared__ __align__(16) unsigned char smem[];
+  float* s_st = (float*)smem;                                // [2]{x [kWgPairs][XS], dy [kWgPairs][DS]}, later the sum
+  int* s_in = (int*)(smem + (2 * S::STAGE > S::RED ? 2 * S::STAGE : S::RED) * 4);
+  int* s_out = s_in + kWgSlice;
+  int* s_cnt = s_out + kWgSlice;                             // [8] hits per warp
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int k = blockIdx.y;
+  const int64_t r0 = (int64_t)blockIdx.x * kWgSlice;
+  const int nr = (int)min((int64_t)kWgSlice, p.n_out - r0);
+  const T* rows = (const T*)p.rows;
+  const T* dout = (const T*)p.dout + r0 * p.N;
+
+  // compaction in ascending row order: a warp's eighth of the slice stays in registers between the count and the write
+  constexpr int kPer = kWgSlice / kThreads;                  // 32-row chunks per warp
+  const int* col = p.nbr + (int64_t)k * p.n_out + r0 + warp * (kPer * 32);
+  int v[kPer], cnt = 0;
+#pragma unroll
+  for (int h = 0; h < kPer; ++h) v[h] = warp * (kPer * 32) + h * 32 + lane < nr ? __ldg(col + h * 32 + lane) : -1;
+#pragma unroll
+  for (int h = 0; h < kPer; ++h) {
+    if (v[h] >= p.n_rows) {
+      if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
+      v[h] = -1;
+    }
+    cnt += __popc(__ballot_sync(0xffffffffu, v[h] >= 0));
+  }
+  if (lane == 0) s_cnt[warp] = cnt;
+  __syncthreads();
+  int at = 0, n = 0;
+  for (int w = 0; w < kThreads / 32; ++w) {
+    if (w < warp) at += s_cnt[w];
+    n += s_cnt[w];
+  }
+  if (n == 0) return;
+#pragma unroll
+  for (int h = 0; h < kPer; ++h) {
+    const unsigned m = __ballot_sync(0xffffffffu, v[h] >= 0);
+    if (v[h] >= 0) {
+      const int pos = at + __popc(m & ((1u << lane) - 1u));
+      s_in[pos] = v[h];
+      s_out[pos] = warp * (kPer * 32) + h * 32 + lane;
+    }
+    at += __popc(m);
+  }
+  __syncthreads();
+
+  auto stage = [&](int buf, int p0) {
+    float* x = s_st + buf * S::STAGE;
+    float* d = x + kWgPairs * S::XS;
+    const int np = min(kWgPairs, n - p0);
+    if constexpr (VEC) {
+      for (int e = tid; e < kWgPairs * KG * 2; e += kThreads) {
+        const int r = e / (KG * 2), c = (e % (KG * 2)) * 4;
+        const bool ok = r < np && c < p.K;
+        cp_async_16(smem_u32(x + r * S::XS + c), ok ? rows + (int64_t)s_in[p0 + r] * p.K + c : rows, ok ? 16u : 0u);
+      }
+      for (int e = tid; e < kWgPairs * NG * 2; e += kThreads) {
+        const int r = e / (NG * 2), c = (e % (NG * 2)) * 4;
+        const bool ok = r < np && c < p.N;
+        cp_async_16(smem_u32(d + r * S::DS + c), ok ? dout + (int64_t)s_out[p0 + r] * p.N + c : dout, ok ? 16u : 0u);
+      }
+    } else {
+      for (int e = tid; e < kWgPairs * KG * 8; e += kThreads) {
+        const int r = e / (KG * 8), c = e % (KG * 8);
+        x[r * S::XS + c] = (r < np && c < p.K) ? widen(rows[(int64_t)s_in[p0 + r] * p.K + c]) : 0.f;
+      }
+      for (int e = tid; e < kWgPairs * NG * 8; e += kThreads) {
+        const int r = e / (NG * 8), c = e % (NG * 8);
+        d[r * S::DS + c] = (r < np && c < p.N) ? widen(dout[(int64_t)s_out[p0 + r] * p.N + c]) : 0.f;
+      }
+    }
+  };
+
+  const int copy = tid / (KG * NG), in_copy = tid % (KG * NG);
+  const int ig = in_copy / NG, og = in_copy % NG;
+  float acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  stage(0, 0);
+  cp_async_commit();
+  int buf = 0;
+  for (int p0 = 0; p0 < n; p0 += kWgPairs, buf ^= 1) {
+    cp_async_wait_pending(0);
+    __syncthreads();
+    if (p0 + kWgPairs < n) stage(buf ^ 1, p0 + kWgPairs);
+    cp_async_commit();
+    const float* x = s_st + buf * S::STAGE + ig * 8;
+    const float* d = s_st + buf * S::STAGE + kWgPairs * S::XS + og * 4;
+    const int np = min(kWgPairs, n - p0);
+#pragma unroll 2
+    for (int r = copy; r < np; r += S::COPIES) {
+      const float4 x0 = *(const float4*)(x + r * S::XS), x1 = *(const float4*)(x + r * S::XS + 4);
+      // the thread's output channels: 4 og .. 4 og + 3 of either half, so that the lanes read consecutive pieces
+      const float4 d0 = *(const float4*)(d + r * S::DS), d1 = *(const float4*)(d + r * S::DS + NG * 4);
+      const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+      const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(xv[i], dv[j], acc[i][j]);
+    }
+  }
+  // sum of the copies, one after the other
+  float* red = s_st;
+  for (int c = 0; c < S::COPIES; ++c) {
+    __syncthreads();
+    if (copy == c) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float* t = red + (ig * 8 + i) * (NG * 8) + (j < 4 ? 0 : NG * 4) + og * 4 + (j & 3);
+          *t = c == 0 ? acc[i][j] : *t + acc[i][j];
+        }
+    }
+  }
+  __syncthreads();
+  float* dw = p.dw + (int64_t)k * p.K * p.N;
+  for (int e = tid; e < p.K * p.N; e += kThreads) atomicAdd(dw + e, red[(e / p.N) * (NG * 8) + e % p.N]);
+}
+
+template <typename T, int CG, bool VEC>
+int launch_ffma(const FfmaParams& p, cudaStream_t st) {
+  using S = FfmaShape<CG>;
+  auto kern = conv_ffma_kernel<T, CG, VEC>;
+  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
+  const dim3 grid((unsigned)div_up64(p.n_out, kRows), (unsigned)div_up(p.N, S::NP));
+  kern<<<grid, S::T, S::BYTES, st>>>(p);
+  SPH_LAUNCH_CHECK();
+  return SPH_OK;
+}
+
+template <typename T, bool VEC>
+int launch_ffma_cg(const FfmaParams& p, cudaStream_t st) {
+  // the narrowest tile that holds the output channels; beyond 64 of them the grid repeats the rows per 64
+  if (p.N <= 8) return launch_ffma<T, 1, VEC>(p, st);
+  if (p.N <= 16) return launch_ffma<T, 2, VEC>(p, st);
+  if (p.N <= 32) return launch_ffma<T, 4, VEC>(p, st);
+  return launch_ffma<T, 8, VEC>(p, st);
+}
+
+template <typename T, int KG, int NG, bool VEC>
+int launch_wg(const FfmaWgradParams& p, int kv, cudaStream_t st) {
+  using S = WgShape<KG, NG>;
+  auto kern = conv_wgrad_ffma_kernel<T, KG, NG, VEC>;
+  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
+  kern<<<dim3((unsigned)div_up64(p.n_out, kWgSlice), (unsigned)kv), kThreads, S::BYTES, st>>>(p);
+  SPH_LAUNCH_CHECK();
+  return SPH_OK;
+}
+
+template <typename T, int KG, bool VEC>
+int launch_wg_n(const FfmaWgradParams& p, int kv, cudaStream_t st) {
+  if (p.N <= 8) return launch_wg<T, KG, 1, VEC>(p, kv, st);
+  if (p.N <= 16) return launch_wg<T, KG, 2, VEC>(p, kv, st);
+  if (p.N <= 32) return launch_wg<T, KG, 4, VEC>(p, kv, st);
+  return launch_wg<T, KG, 8, VEC>(p, kv, st);
+}
+
+template <typename T, bool VEC>
+int launch_wg_k(const FfmaWgradParams& p, int kv, cudaStream_t st) {
+  if (p.K <= 8) return launch_wg_n<T, 1, VEC>(p, kv, st);
+  if (p.K <= 16) return launch_wg_n<T, 2, VEC>(p, kv, st);
+  if (p.K <= 32) return launch_wg_n<T, 4, VEC>(p, kv, st);
+  return launch_wg_n<T, 8, VEC>(p, kv, st);
+}
+
+}  // namespace
+
+int conv_gather_ffma(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
+                     int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                     int out_dtype, int* status, cudaStream_t st) {
+  FfmaParams p;
+  p.rows = rows; p.weight = weight; p.nbr = nbr;
+  p.n_rows = n_rows; p.n_out = n_out;
+  p.kv = kv; p.K = K; p.N = N; p.flip_k = flip_k; p.relu = relu; p.out_dtype = out_dtype;
+  p.scale = scale; p.bias = bias; p.out = out; p.status = status;
+  switch (dtype) {
+    case SPH_F32:
+      if (K % 4 == 0 && N % 4 == 0 && (((uintptr_t)rows | (uintptr_t)weight) & 15u) == 0)
+        return launch_ffma_cg<float, true>(p, st);
+      return launch_ffma_cg<float, false>(p, st);
+    case SPH_F16: return launch_ffma_cg<__half, false>(p, st);
+    case SPH_BF16: return launch_ffma_cg<__nv_bfloat16, false>(p, st);
+  }
+  set_error("unknown dtype %d", dtype);
+  return SPH_ERR_INVALID;
+}
+
+int conv_wgrad_ffma(const void* rows, const void* dout, int dtype, int64_t n_rows, const int* nbr, int64_t n_out, int kv,
+                    int K, int N, float* dw, int* status, cudaStream_t st) {
+  if (K > kWgMaxCh || N > kWgMaxCh) {
+    set_error("weight gradient supports up to %d channels (got %d x %d)", kWgMaxCh, K, N);
+    return SPH_ERR_LIMIT;
+  }
+  FfmaWgradParams p;
+  p.rows = rows; p.dout = dout; p.nbr = nbr;
+  p.n_rows = n_rows; p.n_out = n_out;
+  p.K = K; p.N = N; p.dw = dw; p.status = status;
+  switch (dtype) {
+    case SPH_F32:
+      if (K % 4 == 0 && N % 4 == 0 && (((uintptr_t)rows | (uintptr_t)dout) & 15u) == 0)
+        return launch_wg_k<float, true>(p, kv, st);
+      return launch_wg_k<float, false>(p, kv, st);
+    case SPH_F16: return launch_wg_k<__half, false>(p, kv, st);
+    case SPH_BF16: return launch_wg_k<__nv_bfloat16, false>(p, kv, st);
+  }
+  set_error("weight gradient is not defined for dtype %d", dtype);
+  return SPH_ERR_UNSUPPORTED;
+}
+
+}  // namespace sph

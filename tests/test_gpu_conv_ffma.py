@@ -1,0 +1,29 @@
+"""The fp32-arithmetic kernels (float32 layers of any width, 16-bit layers of odd widths) at the edges of their tiles:
+channel counts around the column groups of 8 / 16 / 32 / 64 and the steps of 32 input channels, output channels beyond one
+tile of 64, kernel volumes beyond one batch of lists, full tiles (more than 64 pairs per offset) and nearly empty ones."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import conv_np
+from sphconv_b200 import sphconv_cuda as ops
+from test_gpu_conv import TOL, _close, _setup
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("iC,oC", [(1, 1), (33, 9), (36, 17), (31, 33), (40, 64), (64, 32), (65, 68), (20, 130)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("dens,ks", [(1.0, (3, 3, 3)), (0.01, (3, 3, 3)), (0.4, (5, 3, 3))])
+def test_forward_and_gradients(iC, oC, dtype, dens, ks):
+    rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(1, [9, 13, 12], True, dens, 11, iC, oC, dtype, ks)
+    f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
+    _close(ops.rule_conv(feat, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[dtype])
+    g = torch.as_tensor(rng.standard_normal((n_out, oC)), dtype=torch.float32).to(dtype).cuda()
+    g64 = g.double().cpu().numpy()
+    dx = ops.rule_conv_d_feature(g, w.permute(0, 2, 1).contiguous(), rules, rule_size, [5, 7], n_in)
+    _close(dx, conv_np.conv_dgrad(g64, w64, pairs, n_in), TOL[dtype])
+    if iC <= 64 and oC <= 64:
+        dw = ops.rule_conv_d_weight(feat, g, rules, rule_size)
+        ref = conv_np.conv_wgrad(f64, g64, pairs, int(np.prod(ks)))
+        _close(dw, ref, 1e-4 if dtype == torch.float32 else 1e-3)
