@@ -221,7 +221,9 @@ int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype, int64_t n_
  *                  gather = 0 is the forward reorder d_dst[permutation[n]] = d_src[n].
  * sph_to_dense     ref: to_dense / to_dense_backward, tensor.cu:222-309.  d_dense is [B,s0,s1,s2,row_bytes]; backward = 0
  *                  copies every row to its voxel (the other voxels of d_dense are left as they are, as in the
- *                  reference: the caller zero-fills), backward = 1 copies the voxels' values back into d_rows. */
+ *                  reference: the caller zero-fills), backward = 1 copies the voxels' values back into d_rows.
+ * sph_dense_channels_first  the same between rows [nnz, channels] of elem_bytes-byte elements and a channels-first dense
+ *                  tensor [B,channels,s0,s1,s2] (s2 <= 2048), which backward = 0 writes in full, zeros included. */
 int64_t sph_init_tensor_scratch_bytes(int32_t B, const int32_t shape[3]);
 int sph_init_tensor(const void* d_feature, int32_t row_bytes, int64_t nnz, const int32_t* d_indices, int32_t B,
                     const int32_t shape[3], void* d_scratch, void* d_out_feature, int32_t* d_z_idx,
@@ -230,6 +232,9 @@ int sph_permute_rows(const void* d_src, int32_t row_bytes, int64_t n_rows, const
                      void* d_dst, void* stream);
 int sph_to_dense(void* d_rows, int32_t row_bytes, int64_t nnz, const int32_t* d_z_idx, const int32_t* d_z_ptr,
                  int32_t B, const int32_t shape[3], void* d_dense, int backward, int32_t* d_status, void* stream);
+int sph_dense_channels_first(void* d_rows, int32_t elem_bytes, int32_t channels, int64_t nnz, const int32_t* d_z_idx,
+                             const int32_t* d_z_ptr, int32_t B, const int32_t shape[3], void* d_dense, int backward,
+                             int32_t* d_status, void* stream);
 
 /* Backward of the fused epilogue relu(acc + bias) of sph_conv_gather (an extension: the reference applies no bias or
  * activation).  d_dpre[r][c] = d_out[r][c] > 0 ? d_dout[r][c] : 0 (relu != 0; else a copy) and

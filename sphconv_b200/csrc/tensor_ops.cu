@@ -96,6 +96,164 @@ dense_rows_kernel(V* __restrict__ rows, const int* __restrict__ z_idx, const int
   else dense[off] = rows[n * pieces + c];
 }
 
+// Rows <-> dense [B,C,H,W,D], channels first: what a convolution head reads.  A block takes whole columns (consecutive
+// columns are consecutive rows AND consecutive dense cells of every channel), stages their rows in shared memory with a
+// cell -> row map, and moves every channel's cells in vectors of V elements; cells without a row are zeros.  The dense
+// tensor is written once; a fill, a channels-last scatter and a permuting copy moved its bytes four times.  [8,64,16,128,64]
+// fp16 (134 MB) with 30 % of the cells occupied: 58 us to dense and 53 us back against 350 and 325 us, half the copy rate
+// (the per-element reads of the staged rows).
+constexpr int kDenseCells = 256;         // cells of a block, when columns are shorter
+constexpr int kDenseMaxCells = 2048;     // columns up to this deep are staged
+
+// Rows of `words` pieces between memory (pitch words apart) and shared memory (s_pitch), a power of two of lanes per row.
+template <typename P, bool TO_SMEM>
+__device__ __forceinline__ void move_rows(P* mem, P* sm, int n_rows, int words, int64_t pitch, int s_pitch) {
+  int sh = 0;
+  while ((1 << sh) < words && sh < 5) ++sh;
+  const int lane = threadIdx.x & ((1 << sh) - 1);
+  for (int r = threadIdx.x >> sh; r < n_rows; r += kOpsThreads >> sh)
+    for (int w = lane; w < words; w += 1 << sh) {
+      if (TO_SMEM) sm[r * s_pitch + w] = mem[r * pitch + w];
+      else mem[r * pitch + w] = sm[r * s_pitch + w];
+    }
+}
+
+template <typename E, bool TO_SMEM>
+__device__ __forceinline__ void move_rows_of(E* mem, E* sm, int n_rows, int cn, int C, int stride) {
+  constexpr int PER = sizeof(E) < 4 ? 4 / (int)sizeof(E) : 1;
+  if (PER > 1 && cn % PER == 0 && C % PER == 0 && ((uintptr_t)mem & 3) == 0)
+    move_rows<uint32_t, TO_SMEM>((uint32_t*)mem, (uint32_t*)sm, n_rows, cn / PER, C / PER, stride / PER);
+  else
+    move_rows<E, TO_SMEM>(mem, sm, n_rows, cn, C, stride);
+}
+
+template <typename E, int V, bool BACK>
+__global__ void __launch_bounds__(kOpsThreads)
+dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx, const int* __restrict__ z_ptr,
+                            int64_t nnz, int64_t cols_per_b, int cols_per_block, int D, int C, int chunk, int stride,
+                            E* __restrict__ dense, int* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  int* s_map = (int*)smem;                                        // [cells] staged row of the cell or -1
+  E* s_rows = (E*)(smem + ((size_t)cols_per_block * D * sizeof(int) + 15) / 16 * 16);   // [rows][stride]
+  const int tid = threadIdx.x;
+  const int64_t col0 = (int64_t)blockIdx.x * cols_per_block;
+  const int nc = (int)min((int64_t)cols_per_block, cols_per_b - col0);
+  const int64_t gcol0 = (int64_t)blockIdx.y * cols_per_b + col0;
+  const int cells = nc * D;
+  const int64_t r0 = min((int64_t)col_begin(z_ptr, gcol0), nnz);
+  const int n_rows = (int)(min((int64_t)__ldg(z_ptr + gcol0 + nc - 1), nnz) - r0);
+  for (int i = tid; i < cells; i += kOpsThreads) s_map[i] = -1;
+  __syncthreads();
+  for (int i = tid; i < n_rows; i += kOpsThreads) {
+    int lo = 0, hi = nc - 1;               // first column of the block whose inclusive prefix exceeds the row
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (__ldg(z_ptr + gcol0 + mid) > r0 + i) hi = mid; else lo = mid + 1;
+    }
+    const int z = __ldg(z_idx + r0 + i);
+    if ((unsigned)z < (unsigned)D) s_map[lo * D + z] = i;
+    else if (status) atomicOr(status, SPH_STATUS_BAD_INDEX);
+  }
+  const int64_t vol = cols_per_b * D;
+  E* plane0 = dense + (int64_t)blockIdx.y * C * vol + col0 * D;
+  struct alignas(V * sizeof(E)) Vec { E e[V]; };
+  constexpr int PAIR = sizeof(E) == 2 && V > 1 ? 2 : 1;
+  for (int c0 = 0; c0 < C; c0 += chunk) {
+    const int cn = min(chunk, C - c0);
+    E* mem = rows + r0 * C + c0;
+    if (!BACK) move_rows_of<E, true>(mem, s_rows, n_rows, cn, C, stride);
+    __syncthreads();
+    // a thread keeps the staged rows of its V cells in registers and walks channels, two at a time for 2-byte elements
+    // (one 4-byte access to shared memory per cell and pair)
+    const int groups = cells / V;
+    const int lanes = groups < kOpsThreads ? kOpsThreads / groups : 1;
+    for (int t = tid; t < groups * lanes; t += kOpsThreads) {
+      const int g = t % groups;
+      int at[V];
+#pragma unroll
+      for (int j = 0; j < V; ++j) {
+        const int r = s_map[g * V + j];
+        at[j] = r < 0 ? -1 : r * stride;
+      }
+      Vec* cell = (Vec*)(plane0 + (int64_t)c0 * vol) + g;
+      const int64_t plane = vol / V;
+      int c = t / groups * PAIR;
+      for (; c + PAIR <= cn; c += lanes * PAIR) {
+        Vec v[PAIR];
+        if (BACK) {
+#pragma unroll
+          for (int q = 0; q < PAIR; ++q) v[q] = cell[(c + q) * plane];
+#pragma unroll
+          for (int j = 0; j < V; ++j)
+            if (at[j] >= 0) {
+              if constexpr (PAIR == 2) *(uint32_t*)(s_rows + at[j] + c) = (uint32_t)v[0].e[j] | (uint32_t)v[1].e[j] << 16;
+              else s_rows[at[j] + c] = v[0].e[j];
+            }
+        } else {
+#pragma unroll
+          for (int j = 0; j < V; ++j) {
+            if constexpr (PAIR == 2) {
+              const uint32_t w = at[j] >= 0 ? *(const uint32_t*)(s_rows + at[j] + c) : 0u;
+              v[0].e[j] = (E)w;
+              v[1].e[j] = (E)(w >> 16);
+            } else {
+              v[0].e[j] = at[j] >= 0 ? s_rows[at[j] + c] : E(0);
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < PAIR; ++q) cell[(c + q) * plane] = v[q];
+        }
+      }
+      if (PAIR == 2 && c < cn) {          // the last of an odd number of channels
+        Vec v;
+        if (BACK) v = cell[c * plane];
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+          if (!BACK) v.e[j] = at[j] >= 0 ? s_rows[at[j] + c] : E(0);
+          else if (at[j] >= 0) s_rows[at[j] + c] = v.e[j];
+        }
+        if (!BACK) cell[c * plane] = v;
+      }
+    }
+    __syncthreads();
+    if (BACK) {
+      move_rows_of<E, false>(mem, s_rows, n_rows, cn, C, stride);
+      __syncthreads();
+    }
+  }
+}
+
+template <typename E, int V>
+int launch_dense_cf(void* rows, const int* z_idx, const int* z_ptr, int64_t nnz, int B, int64_t cols_per_b, int D, int C,
+                    void* dense, int backward, int* status, cudaStream_t st) {
+  int cols = D >= kDenseCells ? 1 : kDenseCells / D;
+  while (cols > 1 && (int64_t)cols * D % V) --cols;
+  const int cells = cols * D;
+  // as many channels at a time as fit in 64 KB when every cell holds a row; an odd number of 4-byte words per row, so that
+  // consecutive rows start on other banks
+  int chunk = (int)(65536 / ((int64_t)cells * sizeof(E)));
+  chunk = chunk > C ? C : chunk < 1 ? 1 : chunk;
+  constexpr int per = sizeof(E) < 4 ? 4 / (int)sizeof(E) : 1;
+  const int stride = (div_up(chunk, per) | 1) * per;
+  const int smem = (cells * (int)sizeof(int) + 15) / 16 * 16 + cells * stride * (int)sizeof(E);
+  auto kern = backward ? dense_channels_first_kernel<E, V, true> : dense_channels_first_kernel<E, V, false>;
+  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  kern<<<dim3((unsigned)div_up64(cols_per_b, cols), (unsigned)B), kOpsThreads, smem, st>>>(
+      (E*)rows, z_idx, z_ptr, nnz, cols_per_b, cols, D, C, chunk, stride, (E*)dense, status);
+  SPH_LAUNCH_CHECK();
+  return SPH_OK;
+}
+
+template <typename E>
+int dense_cf(void* rows, const int* z_idx, const int* z_ptr, int64_t nnz, int B, int64_t cols_per_b, int D, int C,
+             void* dense, int backward, int* status, cudaStream_t st) {
+  // 16-byte vectors where every channel plane and every block of columns starts on one
+  constexpr int V = 16 / (int)sizeof(E);
+  if (cols_per_b * D % V == 0 && D % V == 0 && ((uintptr_t)dense & 15) == 0)
+    return launch_dense_cf<E, V>(rows, z_idx, z_ptr, nnz, B, cols_per_b, D, C, dense, backward, status, st);
+  return launch_dense_cf<E, 1>(rows, z_idx, z_ptr, nnz, B, cols_per_b, D, C, dense, backward, status, st);
+}
+
 int piece_bytes(int row_bytes, const void* a, const void* b) {
   const uintptr_t bits = (uintptr_t)a | (uintptr_t)b | (uintptr_t)row_bytes;
   if ((bits & 15) == 0) return 16;
@@ -207,6 +365,29 @@ extern "C" int sph_to_dense(void* d_rows, int32_t row_bytes, int64_t nnz, const 
   }
   SPH_LAUNCH_CHECK();
   return SPH_OK;
+}
+
+extern "C" int sph_dense_channels_first(void* d_rows, int32_t elem_bytes, int32_t channels, int64_t nnz,
+                                        const int32_t* d_z_idx, const int32_t* d_z_ptr, int32_t B, const int32_t shape[3],
+                                        void* d_dense, int backward, int32_t* d_status, void* stream) {
+  SPH_CHECK_ARG(B > 0 && B <= 65535 && shape && shape[0] > 0 && shape[1] > 0 && shape[2] > 0,
+                "batch and shape must be positive");
+  SPH_CHECK_ARG(nnz >= 0 && channels > 0, "bad sizes");
+  SPH_CHECK_ARG(d_z_ptr && d_dense && (nnz == 0 || (d_rows && d_z_idx)), "null pointer");
+  if (shape[2] > kDenseMaxCells) {
+    set_error("sph_dense_channels_first: columns of more than %d cells are not supported", kDenseMaxCells);
+    return SPH_ERR_LIMIT;
+  }
+  const int64_t cols = (int64_t)shape[0] * shape[1];
+  cudaStream_t st = (cudaStream_t)stream;
+  switch (elem_bytes) {
+    case 1: return dense_cf<uint8_t>(d_rows, d_z_idx, d_z_ptr, nnz, B, cols, shape[2], channels, d_dense, backward, d_status, st);
+    case 2: return dense_cf<uint16_t>(d_rows, d_z_idx, d_z_ptr, nnz, B, cols, shape[2], channels, d_dense, backward, d_status, st);
+    case 4: return dense_cf<uint32_t>(d_rows, d_z_idx, d_z_ptr, nnz, B, cols, shape[2], channels, d_dense, backward, d_status, st);
+    case 8: return dense_cf<uint64_t>(d_rows, d_z_idx, d_z_ptr, nnz, B, cols, shape[2], channels, d_dense, backward, d_status, st);
+  }
+  set_error("sph_dense_channels_first: elements of %d bytes", elem_bytes);
+  return SPH_ERR_UNSUPPORTED;
 }
 
 // ---- backward of the fused epilogue relu(acc + bias): gradient mask and bias gradient in one pass ---------------

@@ -4,8 +4,9 @@ from typing import List
 import torch
 
 from . import profiling
-from .sphconv_cuda import (epilogue_backward, init_tensor, init_tensor_backward, rule_conv, rule_conv_d_feature,
-                           rule_conv_d_weight, to_dense, to_dense_backward)
+from .sphconv_cuda import (dense_channels_first, dense_channels_first_backward, dense_in_one_pass, epilogue_backward,
+                           init_tensor, init_tensor_backward, rule_conv, rule_conv_d_feature, rule_conv_d_weight, to_dense,
+                           to_dense_backward)
 
 
 class ConvFunction(torch.autograd.Function):
@@ -86,6 +87,8 @@ class ToDenseFunction(torch.autograd.Function):
     def forward(ctx, feature: torch.Tensor, z_idx: torch.Tensor, z_ptr: torch.Tensor, shape: List[int]):
         ctx.save_for_backward(z_idx, z_ptr)
         B, C, D, H, W = shape  # the reference's names; the dense layout is [B, s0, s1, s2, C]
+        if dense_in_one_pass(feature, B, C, H):
+            return dense_channels_first(feature.contiguous(), z_idx.contiguous(), z_ptr.contiguous(), [B, C, D, W, H])
         res = torch.zeros((B, D, W, H, C), device=feature.device, dtype=feature.dtype)
         to_dense(feature, z_idx, z_ptr, D, res)
         return res.permute((0, 4, 1, 2, 3)).contiguous()
@@ -93,6 +96,9 @@ class ToDenseFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, d_featureOut):
         z_idx, z_ptr = ctx.saved_tensors
+        if dense_in_one_pass(d_featureOut, d_featureOut.shape[0], d_featureOut.shape[1], d_featureOut.shape[4]):
+            return dense_channels_first_backward(d_featureOut.contiguous(), z_idx.contiguous(), z_ptr.contiguous()), \
+                None, None, None
         d_feature = to_dense_backward(d_featureOut.permute((0, 2, 3, 4, 1)).contiguous(), z_idx, z_ptr)
         return d_feature, None, None, None
 

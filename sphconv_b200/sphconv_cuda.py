@@ -462,6 +462,36 @@ def to_dense_backward(d_featureOut: torch.Tensor, zIndices: torch.Tensor, zPtr: 
     return out
 
 
+def dense_in_one_pass(t: torch.Tensor, batch: int, channels: int, depth: int) -> bool:
+    """Whether dense_channels_first takes these sizes (elements of 1 to 8 bytes, columns of up to 2048 cells)."""
+    return depth <= 2048 and 0 < batch <= 65535 and channels > 0 and t.element_size() <= 8
+
+
+def dense_channels_first(feature: torch.Tensor, zIndices: torch.Tensor, zPtr: torch.Tensor, shape: List[int]):
+    """Rows [NNZ,C] -> dense [B,C,s0,s1,s2], written in one pass (extension; the reference scatters channels-last and
+    permutes, sphconv/functional.py:81-106).  shape = [B, C, s0, s1, s2]."""
+    C.require_cuda(feature, zIndices, zPtr)
+    B, ch, s0, s1, s2 = [int(v) for v in shape]
+    out = torch.empty((B, ch, s0, s1, s2), dtype=feature.dtype, device=feature.device)
+    with torch.cuda.device(feature.device):
+        C.check(C.lib().sph_dense_channels_first(C.ptr(feature), feature.element_size(), ch, feature.shape[0],
+                                                 C.ptr(zIndices), C.ptr(zPtr), B, _shape3([s0, s1, s2]), C.ptr(out), 0,
+                                                 C.ptr(C.status_tensor(feature.device)), C.stream_ptr(feature.device)))
+    return out
+
+
+def dense_channels_first_backward(d_dense: torch.Tensor, zIndices: torch.Tensor, zPtr: torch.Tensor):
+    """Dense gradient [B,C,s0,s1,s2] -> rows [NNZ,C]."""
+    C.require_cuda(d_dense, zIndices, zPtr)
+    B, ch, s0, s1, s2 = d_dense.shape
+    out = torch.empty((zIndices.shape[0], ch), dtype=d_dense.dtype, device=d_dense.device)
+    with torch.cuda.device(d_dense.device):
+        C.check(C.lib().sph_dense_channels_first(C.ptr(out), out.element_size(), ch, out.shape[0], C.ptr(zIndices),
+                                                 C.ptr(zPtr), B, _shape3([s0, s1, s2]), C.ptr(d_dense), 1,
+                                                 C.ptr(C.status_tensor(d_dense.device)), C.stream_ptr(d_dense.device)))
+    return out
+
+
 def epilogue_backward(d_out: torch.Tensor, out: Optional[torch.Tensor], relu: bool, need_bias: bool):
     """Backward of the fused epilogue relu(acc + bias) (extension, no reference counterpart): returns
     (d_pre, d_bias fp32 [C] or None) with d_pre = d_out masked by (out > 0) when `relu`."""

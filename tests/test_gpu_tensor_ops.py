@@ -77,3 +77,21 @@ def test_epilogue_backward(dtype, C, n):
         assert torch.allclose(d_bias.double(), ref, rtol=1e-4, atol=1e-3 * max(1.0, float(ref.abs().max())))
     d_pre, d_bias = ops.epilogue_backward(d_out, out, True, False)
     assert d_bias is None and torch.equal(d_pre, torch.where(out > 0, d_out, torch.zeros((), dtype=dtype, device=DEV)))
+
+
+@pytest.mark.parametrize("dtype,C", [(torch.float16, 64), (torch.float16, 3), (torch.float32, 5), (torch.int8, 6), (torch.float64, 2),
+                                     (torch.bfloat16, 130)])
+@pytest.mark.parametrize("shape,dens", [([5, 7, 16], 0.3), ([3, 9, 13], 1.0), ([2, 3, 300], 0.1), ([1, 2, 2048], 0.5), ([4, 4, 1], 0.5)])
+def test_dense_channels_first_matches_two_step(dtype, C, shape, dens):
+    """The one-pass channels-first dense tensor and its gradient against the channels-last operator and torch's permute, at
+    depths on either side of the block size, odd volumes (no 16-byte vectors) and rows wider than one chunk."""
+    rng = np.random.default_rng(C)
+    idx = torch.as_tensor(_coo(rng, 2, shape, dens), device=DEV)
+    feat = torch.as_tensor(rng.integers(-100, 100, (idx.shape[0], C)), device=DEV).to(dtype)
+    f, z_idx, z_ptr, _ = ops.init_tensor(feat, idx, 2, shape)
+    want = torch.zeros((2, *shape, C), dtype=dtype, device=DEV)
+    ops.to_dense(f, z_idx, z_ptr, shape[2], want)
+    got = ops.dense_channels_first(f, z_idx, z_ptr, [2, C, *shape])
+    assert torch.equal(got, want.permute(0, 4, 1, 2, 3))
+    assert torch.equal(ops.dense_channels_first_backward(got, z_idx, z_ptr), f)
+    assert check_status() == 0
