@@ -69,8 +69,12 @@ struct Geom {
 // Validates and converts; returns SPH_OK or an error code (message set).
 int make_geom(const sph_geom* g, Geom* out);
 
-// rules.cu: inclusive prefix over columns of the popcounts of per-column bit masks.
-int column_prefix_from_masks(const uint32_t* mask, int words, int64_t ncols, const int* zero_flag, int* prefix,
-                             int* blocksum, int* total_dev, cudaStream_t st);
+// rules.cu: inclusive prefix over columns of the popcounts of per-column bit masks; the total also goes to a word of mapped
+// host memory when total_host is not null.
+int column_prefix_from_masks(const uint32_t* mask, int words, int64_t ncols, int* prefix, int* blocksum, int* total_dev,
+                             int* total_host, cudaStream_t st);
+
+// rules.cu: the next word of the current device's ring of mapped pinned host words (see there).
+int count_slot(int32_t** host_word, int32_t** dev_word);
 
 }  // namespace sph

@@ -31,42 +31,26 @@ __device__ __forceinline__ int col_start(const int* __restrict__ zp, int64_t c) 
   return c == 0 ? 0 : __ldg(zp + c - 1);
 }
 
-// Per-column depth bitmask of the INPUT tensor, used when columns are long: word w of column c holds
-// {bits of depths [32w, 32w+32), number of set bits in the words before w}.  "Is depth iz active, and which
-// row is it" is then one 8-byte load plus the column start - valid only when every column is stored in
-// ascending depth order, which the table's builder checks (flag != 0 means some column is not).
-struct ColMask {
-  const uint2* table;  // null: not built (short columns), scan the column instead
-  int words;
-  const int* unsorted;  // device flag written by the builder
-};
+// Per-column depth bitmask of the INPUT tensor: word w of column c holds {bits of depths [32w, 32w+32), number of set bits
+// in the words before w}.  "Is depth iz active, and which row is it" is then one 8-byte load plus the column start - valid
+// only when the column is stored in ascending depth order; the builder sets kUnsorted in every second half-word of a column
+// that is not, and its rows are then searched one by one.  (A flag per column instead of one for the tensor: no word to
+// clear before the builder, no fallback kernels behind it.)
+constexpr uint32_t kUnsorted = 0x80000000u;
 
-// Row id of input voxel (b,ix,iy,iz) or -1.
-__device__ __forceinline__ int find_row(const int* __restrict__ zi, const int* __restrict__ zp, const Geom& g,
-                                        const ColMask& cm, bool use_mask, int b, int ix, int iy, int iz) {
-  int64_t c = ((int64_t)b * g.H + ix) * g.W + iy;
-  if (use_mask) {
-    uint2 e = __ldg(cm.table + c * cm.words + (iz >> 5));
-    uint32_t bit = 1u << (iz & 31);
-    if (!(e.x & bit)) return -1;
-    return col_start(zp, c) + (int)e.y + __popc(e.x & (bit - 1u));
-  }
-  int s = col_start(zp, c);
-  int e = __ldg(zp + c);
-  for (int r = s; r < e; ++r) {
-    if (__ldg(zi + r) == iz) return r;
-  }
-  return -1;
-}
+struct ColMask {
+  const uint2* table;  // null: not built (nearly empty grids), search the columns instead
+  int words;
+};
 
 // One thread per (input column, 32-bin word): the thread walks the column's rows (a handful; the threads of one
 // column read the same addresses, one transaction per warp), keeps the bits of its word and the number of rows below
 // its word, and writes its {bits, prefix} entry: every entry of the table is written exactly once, coalesced, so the
-// table needs no clearing beforehand.  The thread of word 0 also checks the depth order and parks the column id of
-// every row in row_col (optional).
+// table needs no clearing beforehand.  Every thread of a column sees all of its rows, so each can tell whether they are in
+// order; the thread of word 0 also parks the column id of every row in row_col (optional).
 __global__ void __launch_bounds__(256)
 build_colmask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, int64_t ncols, int words, int D,
-                     uint2* __restrict__ table, int* __restrict__ unsorted, int* __restrict__ row_col) {
+                     uint2* __restrict__ table, int* __restrict__ row_col) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncols * words) return;
   const int64_t c = t / words;
@@ -77,19 +61,16 @@ build_colmask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, int
   bool bad = false;
   for (int r = s; r < e; ++r) {
     const int z = __ldg(zi + r);
-    if (w == 0) {
-      if (z <= prev || z >= D) bad = true;
-      prev = z;
-      if (row_col) row_col[r] = (int)c;
-    }
+    if (z <= prev || z >= D) bad = true;
+    prev = z;
+    if (w == 0 && row_col) row_col[r] = (int)c;
     if (z >= 0 && z < D) {
       const int zw = z >> 5;
       if (zw == w) bits |= 1u << (z & 31);
       else if (zw < w) ++below;
     }
   }
-  if (bad) *unsorted = 1;
-  table[t] = make_uint2(bits, (uint32_t)below);
+  table[t] = make_uint2(bits, (uint32_t)below | (bad ? kUnsorted : 0u));
 }
 
 // The same index with one thread per COLUMN for columns of up to 8 words (depth <= 256): the column's rows are read
@@ -98,7 +79,7 @@ build_colmask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, int
 template <int WORDS>
 __global__ void __launch_bounds__(256)
 build_colmask_cols_kernel(const int* __restrict__ zi, const int* __restrict__ zp, int64_t ncols, int D,
-                          uint2* __restrict__ table, int* __restrict__ unsorted, int* __restrict__ row_col) {
+                          uint2* __restrict__ table, int* __restrict__ row_col) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncols) return;
   const int s = col_start(zp, c), e = __ldg(zp + c);
@@ -120,11 +101,10 @@ build_colmask_cols_kernel(const int* __restrict__ zi, const int* __restrict__ zp
         if (zw == w) bits[w] |= bit;
     }
   }
-  if (bad) *unsorted = 1;
-  uint32_t below = 0u;
+  uint32_t below = bad ? kUnsorted : 0u;
   uint2* dst = table + c * WORDS;
   if constexpr (WORDS == 1) {
-    dst[0] = make_uint2(bits[0], 0u);
+    dst[0] = make_uint2(bits[0], below);
   } else {
 #pragma unroll
     for (int w = 0; w < WORDS; w += 2) {
@@ -135,16 +115,21 @@ build_colmask_cols_kernel(const int* __restrict__ zi, const int* __restrict__ zp
   }
 }
 
-// One CTA per output tile.  in_* describe the input tensor, out_* the output tensor (the same
+// Column id of every row, for grids without the index.
+__global__ void __launch_bounds__(256)
+park_columns_kernel(const int* __restrict__ zp, int64_t ncols, int* __restrict__ row_col) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncols) return;
+  const int e = __ldg(zp + c);
+  for (int r = col_start(zp, c); r < e; ++r) row_col[r] = (int)c;
+}
+
+// One CTA per output tile, for callers that want no neighbour table.  in_* describe the input tensor, out_* the output tensor (the same
 // arrays for a submanifold layer).
 __global__ void __launch_bounds__(kEmitThreads)
 emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
-                  const int* __restrict__ out_zp, Geom g, int64_t in_nnz, int64_t out_nnz, int tile_n_max,
-                  int* __restrict__ rules, int* __restrict__ rule_size, int* __restrict__ nbr,
-                  int* __restrict__ nbr_t, ColMask cm, int* __restrict__ status, int fast_done) {
-  // fast_done: the row-parallel kernels below were launched for this call; they did the work unless
-  // they found a column stored out of depth order
-  if (fast_done && *cm.unsorted == 0) return;
+                  const int* __restrict__ out_zp, Geom g, int64_t in_nnz, int tile_n_max, int* __restrict__ rules,
+                  int* __restrict__ rule_size, int* __restrict__ nbr_t, int* __restrict__ status) {
   __shared__ int s_cnt[kMaxKV];
   __shared__ int s_rstart[kEmitMaxRanges];
   __shared__ int s_roff[kEmitMaxRanges + 1];
@@ -162,7 +147,6 @@ emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
   const int tHe = min(g.tH, g.oH - ox0);
   const int tWe = min(g.tW, g.oW - oy0);
   const int R = g.B * tHe;  // (batch, tile row) ranges; each is one contiguous run of output rows
-  const bool use_mask = cm.table != nullptr && *cm.unsorted == 0;
 
   for (int k = tid; k < g.KV; k += kEmitThreads) s_cnt[k] = 0;
   __syncthreads();
@@ -232,33 +216,12 @@ emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
             const int iz0 = s_voz[v] * g.sD - g.pD;   // input depth for kd = 0; kd = j reads iz0 + j * dD
             if (ix >= 0 && ix < g.H && iy >= 0 && iy < g.W) {
               const int64_t ci = ((int64_t)b * g.H + ix) * g.W + iy;
-              if (use_mask) {
-                int cur_w = -1;
-                uint2 e = make_uint2(0u, 0u);
-                int cstart = -1;
+              const int cs = col_start(in_zp, ci), ce = __ldg(in_zp + ci);
+              for (int r = cs; r < ce; ++r) {
+                const int d = __ldg(in_zi + r) - iz0;
 #pragma unroll
-                for (int j = 0; j < kMaxKD; ++j) {
-                  const int iz = iz0 + j * g.dD;
-                  if (j < g.KD && iz >= 0 && iz < g.D) {
-                    if ((iz >> 5) != cur_w) {
-                      cur_w = iz >> 5;
-                      e = __ldg(cm.table + ci * cm.words + cur_w);
-                    }
-                    const uint32_t bit = 1u << (iz & 31);
-                    if (e.x & bit) {
-                      if (cstart < 0) cstart = col_start(in_zp, ci);
-                      found[j] = cstart + (int)e.y + __popc(e.x & (bit - 1u));
-                    }
-                  }
-                }
-              } else {
-                const int cs = col_start(in_zp, ci), ce = __ldg(in_zp + ci);
-                for (int r = cs; r < ce; ++r) {
-                  const int d = __ldg(in_zi + r) - iz0;
-#pragma unroll
-                  for (int j = 0; j < kMaxKD; ++j)
-                    if (d == j * g.dD && j < g.KD && found[j] < 0) found[j] = r;
-                }
+                for (int j = 0; j < kMaxKD; ++j)
+                  if (d == j * g.dD && j < g.KD && found[j] < 0) found[j] = r;
               }
             }
           }
@@ -267,7 +230,6 @@ emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
             if (j < g.KD) {   // uniform across the warp
               const int k = k0 + j;
               const int in_row = found[j];
-              if (v < np && nbr) nbr[(int64_t)k * out_nnz + out_row] = in_row;
               const unsigned m = __ballot_sync(0xffffffffu, in_row >= 0);
               if (in_row >= 0) {
                 const int slot = base[j] + __popc(m & ((1u << lane) - 1u));
@@ -302,22 +264,22 @@ emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
 
 
 // ---------------------------------------------------------------------------------------------
-// Row-parallel path (needs the input column masks and the neighbour table as an output).
+// Row-parallel path (needs the neighbour table as an output).
 //  1. nbr_rows_kernel: one thread per OUTPUT row looks its KH*KW input columns up in the mask table and
 //     writes the KV entries nbr[k][row] (coalesced over rows) and, if asked, nbr_t[k][in] = row.
 //     The row's column id was parked in the last plane of nbr by the kernel that enumerated the rows
 //     (build_colmask_kernel for a submanifold layer, write_oz_idx_kernel for a strided one); the thread reads
-//     it first and overwrites it last.
+//     it first and overwrites it last.  A column that is out of depth order, or every column of a grid without the
+//     index, is searched row by row.
 //  2. rule_lists_kernel: one warp per (tile, group of offsets) walks the tile's row ranges in list order
 //     (batch, tile row, row), reads nbr[k][row] and ballot-compacts the hits into rules[tile][k].
-// Both do nothing when a column was found out of depth order; emit_rules_kernel then does the work.
 // ---------------------------------------------------------------------------------------------
 // KD_CT = 3: the filter is 3 wide and 3 deep (those two loops are unrolled), 0 = extents read from the geometry.
 template <int KD_CT, bool HAS_T>
 __global__ void __launch_bounds__(256)
-nbr_rows_kernel(const int* __restrict__ in_zp, const int* __restrict__ out_zi, Geom g, int64_t in_nnz,
-                int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, ColMask cm, int* __restrict__ status) {
-  if (*cm.unsorted) return;
+nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi, Geom g,
+                int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, ColMask cm,
+                int* __restrict__ status) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= out_nnz) return;
   const int c = nbr[(int64_t)(g.KV - 1) * out_nnz + r];
@@ -343,9 +305,10 @@ nbr_rows_kernel(const int* __restrict__ in_zp, const int* __restrict__ out_zi, G
       const int iy = oy * g.sW - g.pW + kw * g.dW;
       const bool col_ok = ix >= 0 && ix < g.H && iy >= 0 && iy < g.W;
       int cstart = 0;
+      int64_t ci = 0;
       const uint2* row = cm.table;
       if (col_ok) {
-        const int64_t ci = ((int64_t)b * g.H + ix) * g.W + iy;
+        ci = ((int64_t)b * g.H + ix) * g.W + iy;
         cstart = col_start(in_zp, ci);
         row = cm.table + ci * cm.words;
       }
@@ -359,10 +322,18 @@ nbr_rows_kernel(const int* __restrict__ in_zp, const int* __restrict__ out_zi, G
         if (col_ok && iz >= 0 && iz < g.D) {
           if ((iz >> 5) != cur_w) {
             cur_w = iz >> 5;
-            e = __ldg(row + cur_w);
+            e = cm.table ? __ldg(row + cur_w) : make_uint2(~0u, kUnsorted);
           }
           const uint32_t bit = 1u << (iz & 31);
-          if (e.x & bit) found = cstart + (int)e.y + __popc(e.x & (bit - 1u));
+          if (e.x & bit) {
+            if (e.y & kUnsorted) {
+              const int end = __ldg(in_zp + ci);
+              for (int q = cstart; q < end && found < 0; ++q)
+                if (__ldg(in_zi + q) == iz) found = q;
+            } else {
+              found = cstart + (int)e.y + __popc(e.x & (bit - 1u));
+            }
+          }
         }
         *dst = found;
         dst += out_nnz;
@@ -424,10 +395,9 @@ template <int NK, int CH>
 __global__ void __launch_bounds__(kFixWarps * 32)
 rule_lists_fixed_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int tile_n_max, int n_kg,
                         const int* __restrict__ nbr, int* __restrict__ rules, int* __restrict__ rule_size,
-                        const int* __restrict__ unsorted, int* __restrict__ status) {
+                        int* __restrict__ status) {
   __shared__ int s_rs[kFixWarps][kListRanges];
   __shared__ int s_off[kFixWarps][kListRanges + 1];
-  if (unsorted && *unsorted) return;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int64_t item = (int64_t)blockIdx.x * kFixWarps + wib;
@@ -525,10 +495,9 @@ template <int kListChunks>
 __global__ void __launch_bounds__(kListWarps * 32)
 rule_lists_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int tile_n_max, int kg, int n_kg,
                   const int* __restrict__ nbr, int* __restrict__ rules, int* __restrict__ rule_size,
-                  const int* __restrict__ unsorted, int* __restrict__ status) {
+                  int* __restrict__ status) {
   __shared__ int s_rs[kListWarps][kListRanges];
   __shared__ int s_off[kListWarps][kListRanges + 1];
-  if (unsorted && *unsorted) return;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   const int64_t item = (int64_t)blockIdx.x * kListWarps + wib;
@@ -657,12 +626,9 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int* s_warp /*[8]*/, 
 
 __global__ void __launch_bounds__(kScanThreads)
 strided_mask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, Geom g, int words, int64_t ncols,
-                    ColMask cm, uint32_t* __restrict__ mask, int* __restrict__ counts, int* __restrict__ blocksum,
-                    int fast_done) {
-  if (fast_done && *cm.unsorted == 0) return;   // strided_bits_kernel + count_columns_kernel do the work
+                    ColMask cm, uint32_t* __restrict__ mask, int* __restrict__ counts, int* __restrict__ blocksum) {
   __shared__ int s_warp[kScanThreads / 32];
   const int64_t c = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
-  const bool use_mask = cm.table != nullptr && *cm.unsorted == 0;
   int count = 0;
   if (c < ncols) {
     const int oy = (int)(c % g.oW);
@@ -694,7 +660,7 @@ strided_mask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, Geom
           int iy = oy * g.sW - g.pW + kw * g.dW;
           if (iy < 0 || iy >= g.W) continue;
           int64_t ci = ((int64_t)b * g.H + ix) * g.W + iy;
-          if (use_mask) {
+          if (cm.table != nullptr) {
             for (int w = 0; w < cm.words; ++w) {
               uint32_t bits = __ldg(cm.table + ci * cm.words + w).x;
               while (bits) {
@@ -734,12 +700,16 @@ __host__ __device__ inline bool strided_bits_ok(const Geom& g) {
 }
 
 __global__ void __launch_bounds__(256)
-strided_bits_kernel(Geom g, int words_out, int64_t ncols_out, ColMask cm, uint32_t* __restrict__ mask) {
-  if (*cm.unsorted) return;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ncols_out * words_out) return;
-  const int w = (int)(t % words_out);
-  const int64_t c = t / words_out;
+strided_bits_kernel(Geom g, int words_out, int cols_per_block, int64_t ncols_out, ColMask cm, uint32_t* __restrict__ mask,
+                    int* __restrict__ counts, int* __restrict__ blocksum) {
+  __shared__ int s_pop[256];
+  __shared__ int s_warp[kScanThreads / 32];
+  const int64_t c0 = (int64_t)blockIdx.x * cols_per_block;
+  const int tid = threadIdx.x;
+  const int w = tid % words_out;
+  const int64_t c = c0 + tid / words_out;
+  uint32_t out = 0;
+  if (tid < cols_per_block * words_out && c < ncols_out) {
   const int oy = (int)(c % g.oW);
   const int ox = (int)((c / g.oW) % g.oH);
   const int b = (int)(c / ((int64_t)g.oW * g.oH));
@@ -747,7 +717,6 @@ strided_bits_kernel(Geom g, int words_out, int64_t ncols_out, ColMask cm, uint32
   const int n_bits = min(g.oD - oz_lo, 32);
   const int iz_lo = max(0, oz_lo * g.sD - g.pD);
   const int iz_hi = min(g.D - 1, (oz_lo + n_bits - 1) * g.sD - g.pD + (g.KD - 1) * g.dD);
-  uint32_t out = 0;
   if (iz_lo <= iz_hi) {
     const int w_lo = iz_lo >> 5;
     const int nw = (iz_hi >> 5) - w_lo + 1;
@@ -803,14 +772,25 @@ strided_bits_kernel(Geom g, int words_out, int64_t ncols_out, ColMask cm, uint32
       out |= hit << bit;
     }
   }
-  mask[t] = out;
+  mask[c * words_out + w] = out;
+  }
+  // bin counts of the block's columns and their sum, for the scan
+  s_pop[tid] = __popc(out);
+  __syncthreads();
+  int count = 0;
+  if (tid < cols_per_block && c0 + tid < ncols_out) {
+    for (int j = 0; j < words_out; ++j) count += s_pop[tid * words_out + j];
+    counts[c0 + tid] = count;
+  }
+  int total;
+  block_inclusive_scan(count, s_warp, &total);
+  if (tid == 0) blocksum[blockIdx.x] = total;
 }
 
-// One thread per output column: bin count of the column, block-level sums for the scan.
+// One thread per column: bin count of the column, block-level sums for the scan.
 __global__ void __launch_bounds__(kScanThreads)
-count_columns_kernel(const uint32_t* __restrict__ mask, int words, int64_t ncols, const int* __restrict__ unsorted,
-                     int* __restrict__ counts, int* __restrict__ blocksum) {
-  if (*unsorted) return;
+count_columns_kernel(const uint32_t* __restrict__ mask, int words, int64_t ncols, int* __restrict__ counts,
+                     int* __restrict__ blocksum) {
   __shared__ int s_warp[kScanThreads / 32];
   const int64_t c = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
   int count = 0;
@@ -823,36 +803,41 @@ count_columns_kernel(const uint32_t* __restrict__ mask, int words, int64_t ncols
   if (threadIdx.x == 0) blocksum[blockIdx.x] = total;
 }
 
-// Single CTA: exclusive scan of the block sums in place, grand total to *out_total.
+// counts -> inclusive prefix (in place).  A block takes kScanCols columns and adds up the block sums in front of them by
+// itself (a few KB of L2 reads), so no kernel is needed to scan those; `per` = block sums per kScanCols columns.  The last
+// block hands over the grand total.
+constexpr int kScanCols = 4 * kScanThreads;
+
 __global__ void __launch_bounds__(kScanThreads)
-scan_blocksums_kernel(int* __restrict__ blocksum, int n, int* __restrict__ out_total, int* out_total_host) {
+scan_columns_kernel(int* __restrict__ counts, int64_t ncols, const int* __restrict__ blocksum, int per,
+                    int* __restrict__ out_total, int* out_total_host) {
   __shared__ int s_warp[kScanThreads / 32];
-  int carry = 0;
-  for (int base = 0; base < n; base += kScanThreads) {
-    int i = base + threadIdx.x;
-    int v = i < n ? blocksum[i] : 0;
-    int total;
-    int inc = block_inclusive_scan(v, s_warp, &total);
-    if (i < n) blocksum[i] = carry + inc - v;
-    carry += total;
+  const int tid = threadIdx.x;
+  int before = 0;
+  for (int i = tid; i < (int)blockIdx.x * per; i += kScanThreads) before += __ldg(blocksum + i);
+  int base;
+  block_inclusive_scan(before, s_warp, &base);
+  const int64_t c0 = (int64_t)blockIdx.x * kScanCols + tid * 4;
+  int v[4], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = c0 + j < ncols ? counts[c0 + j] : 0;
+    sum += v[j];
   }
-  if (threadIdx.x == 0) {
-    *out_total = carry;
+  int total;
+  int at = base + block_inclusive_scan(sum, s_warp, &total) - sum;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    at += v[j];
+    if (c0 + j < ncols) counts[c0 + j] = at;
+  }
+  if (tid == 0 && blockIdx.x == gridDim.x - 1) {
+    *out_total = base + total;
     if (out_total_host) {          // mapped pinned host word: the host reads it after synchronising the stream
-      *(volatile int*)out_total_host = carry;
+      *(volatile int*)out_total_host = base + total;
       __threadfence_system();
     }
   }
-}
-
-// counts -> inclusive prefix (in place) using the scanned block sums.
-__global__ void __launch_bounds__(kScanThreads)
-scan_columns_kernel(int* __restrict__ counts, int64_t ncols, const int* __restrict__ blocksum) {
-  __shared__ int s_warp[kScanThreads / 32];
-  const int64_t c = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
-  int v = c < ncols ? counts[c] : 0;
-  int inc = block_inclusive_scan(v, s_warp, nullptr);
-  if (c < ncols) counts[c] = inc + blocksum[blockIdx.x];
 }
 
 __global__ void __launch_bounds__(kScanThreads)
@@ -909,35 +894,38 @@ bool want_colmask(const Geom& g, int64_t in_nnz) {
 
 size_t colmask_bytes(const Geom& g, int64_t in_nnz) {
   if (!want_colmask(g, in_nnz)) return 0;
-  size_t b = 256 + (size_t)g.B * g.H * g.W * div_up(g.D, 32) * sizeof(uint2);
+  const size_t b = (size_t)g.B * g.H * g.W * div_up(g.D, 32) * sizeof(uint2);
   return (b + 255) & ~(size_t)255;
 }
 
-// Builds the table at `scratch` (layout: 256-byte header holding the unsorted flag, then the table).
+// Builds the table at `scratch` and parks the rows' column ids; without a table (nearly empty grid, no scratch) only the
+// latter.
 int build_colmask(const int* zi, const int* zp, const Geom& g, int64_t in_nnz, void* scratch, ColMask* cm,
                   cudaStream_t st, int* row_col = nullptr) {
   cm->table = nullptr;
   cm->words = 0;
-  cm->unsorted = nullptr;
-  if (!want_colmask(g, in_nnz) || scratch == nullptr) return SPH_OK;
   const int64_t ncols = (int64_t)g.B * g.H * g.W;
+  if (!want_colmask(g, in_nnz) || scratch == nullptr) {
+    if (row_col == nullptr || in_nnz == 0) return SPH_OK;
+    park_columns_kernel<<<(unsigned)div_up64(ncols, 256), 256, 0, st>>>(zp, ncols, row_col);
+    SPH_LAUNCH_CHECK();
+    return SPH_OK;
+  }
   const int words = div_up(g.D, 32);
-  SPH_CUDA(cudaMemsetAsync(scratch, 0, 256, st));      // the header (flag); the kernel writes every table entry
-  cm->unsorted = (const int*)scratch;
   cm->words = words;
-  cm->table = (const uint2*)((char*)scratch + 256);
-  uint2* table = (uint2*)((char*)scratch + 256);
+  cm->table = (const uint2*)scratch;
+  uint2* table = (uint2*)scratch;
   const unsigned col_grid = (unsigned)div_up64(ncols, 256);
   // one thread per column pays off on large grids; a small grid (a few hundred CTAs of the other form) is launch-bound
   // either way and has more threads in flight with one thread per column and word
   switch (ncols >= 100000 ? words : 0) {
-    case 1: build_colmask_cols_kernel<1><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, (int*)scratch, row_col); break;
-    case 2: build_colmask_cols_kernel<2><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, (int*)scratch, row_col); break;
-    case 4: build_colmask_cols_kernel<4><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, (int*)scratch, row_col); break;
-    case 8: build_colmask_cols_kernel<8><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, (int*)scratch, row_col); break;
+    case 1: build_colmask_cols_kernel<1><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
+    case 2: build_colmask_cols_kernel<2><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
+    case 4: build_colmask_cols_kernel<4><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
+    case 8: build_colmask_cols_kernel<8><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
     default:
       build_colmask_kernel<<<(unsigned)div_up64(ncols * words, 256), 256, 0, st>>>(zi, zp, ncols, words, g.D, table,
-                                                                            (int*)scratch, row_col);
+                                                                                            row_col);
   }
   SPH_LAUNCH_CHECK();
   return SPH_OK;
@@ -950,7 +938,7 @@ int* parked_columns(const Geom& g, int* nbr, int64_t out_nnz) {
 
 // Pair lists of every (tile, offset) from a finished neighbour table.
 int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm, const int* nbr, int* rules,
-                      int* rule_size, const int* unsorted, int* status, cudaStream_t st) {
+                      int* rule_size, int* status, cudaStream_t st) {
   if (g.KV == 27) {
     // the usual 3 x 3 x 3 filter: the kernel with the offsets' running counts in registers
     // nine offsets per warp where that gives the machine enough warps, else three (small tile grids have long tiles:
@@ -959,7 +947,7 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
     // convolution CTA), and 27 offsets per warp leaves too few warps.
 #define SPH_LISTS_FIXED(NK)                                                                                           \
   rule_lists_fixed_kernel<NK, 1><<<(unsigned)div_up64((int64_t)g.nTile * (27 / NK), kFixWarps), kFixWarps * 32, 0,     \
-                                   st>>>(out_zp, g, out_nnz, tnm, 27 / NK, nbr, rules, rule_size, unsorted, status)
+                                   st>>>(out_zp, g, out_nnz, tnm, 27 / NK, nbr, rules, rule_size, status)
     if ((int64_t)g.nTile * 3 >= 6000) SPH_LISTS_FIXED(9);
     else SPH_LISTS_FIXED(3);
 #undef SPH_LISTS_FIXED
@@ -978,7 +966,7 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
   const int64_t want = (out_nnz / (g.nTile > 0 ? g.nTile : 1)) * 5 / 4;
 #define SPH_LISTS(CH)                                                                                             \
   rule_lists_kernel<CH><<<grid, kListWarps * 32, 0, st>>>(out_zp, g, out_nnz, tnm, kg, n_kg, nbr, rules, rule_size, \
-                                                          unsorted, status)
+                                                          status)
   if (want <= 32) SPH_LISTS(1);
   else if (want <= 64) SPH_LISTS(2);
   else if (want <= 128) SPH_LISTS(4);
@@ -988,53 +976,50 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
   return SPH_OK;
 }
 
-// rows_parked: the column ids of the output rows are in parked_columns() (row-parallel path possible).
+// With a neighbour table: the row-parallel path (the column ids of the output rows are in parked_columns()), then the lists
+// from the table.  Without one: the tile kernel.
 int launch_emit(const int* in_zi, const int* in_zp, const int* out_zi, const int* out_zp, const Geom& g,
                 int64_t in_nnz, int64_t out_nnz, int tnm, int* rules, int* rule_size, int* nbr, int* nbr_t,
-                const ColMask& cm, bool rows_parked, int fill_unused, int* status, cudaStream_t st) {
+                const ColMask& cm, int fill_unused, int* status, cudaStream_t st) {
   if (rules && fill_unused) {
     SPH_CUDA(cudaMemsetAsync(rules, 0xFF, (size_t)g.nTile * g.KV * 2 * (size_t)tnm * sizeof(int), st));
   }
   if (nbr_t && in_nnz > 0) {
     SPH_CUDA(cudaMemsetAsync(nbr_t, 0xFF, (size_t)g.KV * (size_t)in_nnz * sizeof(int), st));
   }
-  const bool fast = rows_parked && cm.table != nullptr && nbr != nullptr;
-  if (fast) {
-    if (out_nnz > 0) {
-      const unsigned grid = (unsigned)div_up64(out_nnz, 256);
-#define SPH_NBR_ROWS(KD, T) nbr_rows_kernel<KD, T><<<grid, 256, 0, st>>>(in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, cm, status)
-      if (g.KD == 3 && g.KW == 3) {
-        if (nbr_t) SPH_NBR_ROWS(3, true); else SPH_NBR_ROWS(3, false);
-      } else {
-        if (nbr_t) SPH_NBR_ROWS(0, true); else SPH_NBR_ROWS(0, false);
-      }
-#undef SPH_NBR_ROWS
-      SPH_LAUNCH_CHECK();
-    }
-    if (rule_size) {
-      const int rc = launch_rule_lists(out_zp, g, out_nnz, tnm, nbr, rules, rule_size, cm.unsorted, status, st);
-      if (rc != SPH_OK) return rc;
-    }
+  if (nbr == nullptr && out_nnz > 0) {
+    emit_rules_kernel<<<g.nTile, kEmitThreads, 0, st>>>(in_zi, in_zp, out_zi, out_zp, g, in_nnz, tnm, rules, rule_size,
+                                                        nbr_t, status);
+    SPH_LAUNCH_CHECK();
+    return SPH_OK;
   }
-  emit_rules_kernel<<<g.nTile, kEmitThreads, 0, st>>>(in_zi, in_zp, out_zi, out_zp, g, in_nnz, out_nnz, tnm, rules,
-                                                      rule_size, nbr, nbr_t, cm, status, fast ? 1 : 0);
-  SPH_LAUNCH_CHECK();
+  if (out_nnz > 0) {
+    const unsigned grid = (unsigned)div_up64(out_nnz, 256);
+#define SPH_NBR_ROWS(KD, T) \
+  nbr_rows_kernel<KD, T><<<grid, 256, 0, st>>>(in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, cm, status)
+    if (g.KD == 3 && g.KW == 3) {
+      if (nbr_t) SPH_NBR_ROWS(3, true); else SPH_NBR_ROWS(3, false);
+    } else {
+      if (nbr_t) SPH_NBR_ROWS(0, true); else SPH_NBR_ROWS(0, false);
+    }
+#undef SPH_NBR_ROWS
+    SPH_LAUNCH_CHECK();
+  }
+  if (rule_size) return launch_rule_lists(out_zp, g, out_nnz, tnm, nbr, rules, rule_size, status, st);
   return SPH_OK;
 }
 
 }  // namespace
 
 // Inclusive prefix over columns of the popcounts of per-column bit masks (shared with the tensor ops):
-// prefix[c] = number of set bits in columns 0..c; *total_dev = the grand total.  `zero_flag` points to a device int
-// that holds 0; `blocksum` needs ceil(ncols / 256) ints.
-int column_prefix_from_masks(const uint32_t* mask, int words, int64_t ncols, const int* zero_flag, int* prefix,
-                             int* blocksum, int* total_dev, cudaStream_t st) {
-  const int nblk = (int)div_up64(ncols, kScanThreads);
-  count_columns_kernel<<<nblk, kScanThreads, 0, st>>>(mask, words, ncols, zero_flag, prefix, blocksum);
+// prefix[c] = number of set bits in columns 0..c; *total_dev (and the host word, if any) = the grand total; `blocksum`
+// needs ceil(ncols / 256) ints.
+int column_prefix_from_masks(const uint32_t* mask, int words, int64_t ncols, int* prefix, int* blocksum, int* total_dev,
+                             int* total_host, cudaStream_t st) {
+  count_columns_kernel<<<(unsigned)div_up64(ncols, kScanThreads), kScanThreads, 0, st>>>(mask, words, ncols, prefix, blocksum);
   SPH_LAUNCH_CHECK();
-  scan_blocksums_kernel<<<1, kScanThreads, 0, st>>>(blocksum, nblk, total_dev, nullptr);
-  SPH_LAUNCH_CHECK();
-  scan_columns_kernel<<<nblk, kScanThreads, 0, st>>>(prefix, ncols, blocksum);
+  scan_columns_kernel<<<(unsigned)div_up64(ncols, kScanCols), kScanThreads, 0, st>>>(
+      prefix, ncols, blocksum, kScanCols / kScanThreads, total_dev, total_host);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -1142,7 +1127,7 @@ extern "C" int sph_rules_subm(const int32_t* d_z_idx, const int32_t* d_z_ptr, in
   rc = build_colmask(d_z_idx, d_z_ptr, g, nnz, d_scratch, &cm, (cudaStream_t)stream, parked_columns(g, d_nbr, nnz));
   if (rc != SPH_OK) return rc;
   return launch_emit(d_z_idx, d_z_ptr, d_z_idx, d_z_ptr, g, nnz, nnz, tile_n_max, d_rules, d_rule_size, d_nbr,
-                     nullptr, cm, /*rows_parked=*/d_nbr != nullptr, fill_unused, d_status, (cudaStream_t)stream);
+                     nullptr, cm, fill_unused, d_status, (cudaStream_t)stream);
 }
 
 extern "C" int sph_rule_lists(const int32_t* d_oz_ptr, const sph_geom* s, int64_t out_nnz, const int32_t* d_nbr,
@@ -1157,7 +1142,7 @@ extern "C" int sph_rule_lists(const int32_t* d_oz_ptr, const sph_geom* s, int64_
   if (d_rules && fill_unused)
     SPH_CUDA(cudaMemsetAsync(d_rules, 0xFF, (size_t)g.nTile * g.KV * 2 * (size_t)tile_n_max * sizeof(int), st));
   // without d_rules the kernel only counts: d_rule_size gets the exact list lengths
-  return launch_rule_lists(d_oz_ptr, g, out_nnz, tile_n_max, d_nbr, d_rules, d_rule_size, nullptr, d_status, st);
+  return launch_rule_lists(d_oz_ptr, g, out_nnz, tile_n_max, d_nbr, d_rules, d_rule_size, d_status, st);
 }
 
 // ---- allocation-free variant of sph_rules_subm ---------------------------------------------------
@@ -1205,6 +1190,7 @@ namespace {
 struct StridedScratch {
   int words;
   int64_t ncols;
+  int cols_per_block;      // columns per block sum (a power of two)
   int nblk;
   size_t mask_bytes, blocksum_bytes, colmask_bytes;
 };
@@ -1212,9 +1198,13 @@ StridedScratch strided_layout(const Geom& g, int64_t nnz) {
   StridedScratch s;
   s.words = div_up(g.oD, 32);
   s.ncols = (int64_t)g.B * g.oH * g.oW;
-  s.nblk = (int)div_up64(s.ncols, kScanThreads);
+  // strided_bits_kernel takes one thread per word of a column; columns too deep for that are counted by a kernel of their own
+  s.cols_per_block = kScanThreads;
+  if (s.words <= 64)
+    while (s.cols_per_block * s.words > kScanThreads) s.cols_per_block >>= 1;
+  s.nblk = (int)div_up64(s.ncols, s.cols_per_block);
   s.mask_bytes = ((size_t)s.ncols * s.words * sizeof(uint32_t) + 255) & ~(size_t)255;
-  s.blocksum_bytes = ((size_t)s.nblk * sizeof(int) + 255) & ~(size_t)255;
+  s.blocksum_bytes = ((size_t)s.nblk * sizeof(int) + 255) & ~(size_t)255;     // >= ceil(ncols / 256) ints
   s.colmask_bytes = colmask_bytes(g, nnz);
   return s;
 }
@@ -1223,12 +1213,9 @@ ColMask strided_colmask(const Geom& g, int64_t nnz, const StridedScratch& l, con
   ColMask cm;
   cm.table = nullptr;
   cm.words = 0;
-  cm.unsorted = nullptr;
   if (l.colmask_bytes) {
-    const char* base = (const char*)scratch + l.mask_bytes + l.blocksum_bytes;
-    cm.unsorted = (const int*)base;
     cm.words = div_up(g.D, 32);
-    cm.table = (const uint2*)(base + 256);
+    cm.table = (const uint2*)((const char*)scratch + l.mask_bytes + l.blocksum_bytes);
   }
   return cm;
 }
@@ -1246,6 +1233,8 @@ struct CountRing {
   int32_t* dev = nullptr;
   unsigned next = 0;          // per device: a word is reused only after kCountSlots - 1 further calls on ITS device
 };
+}  // namespace
+namespace sph {
 int count_slot(int32_t** host_word, int32_t** dev_word) {
   constexpr int kMaxDevices = 64;
   static CountRing rings[kMaxDevices];
@@ -1271,7 +1260,7 @@ int count_slot(int32_t** host_word, int32_t** dev_word) {
   *dev_word = r.dev + slot;
   return SPH_OK;
 }
-}  // namespace
+}  // namespace sph
 
 extern "C" int64_t sph_rules_strided_scratch_bytes(const sph_geom* s, int64_t nnz) {
   Geom g;
@@ -1299,16 +1288,14 @@ int strided_count_impl(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t n
   rc = build_colmask(d_z_idx, d_z_ptr, g, nnz, l.colmask_bytes ? (char*)d_scratch + l.mask_bytes + l.blocksum_bytes : nullptr,
                      &cm, st);
   if (rc != SPH_OK) return rc;
-  const bool fast = cm.table != nullptr && strided_bits_ok(g);
-  if (fast) {
-    strided_bits_kernel<<<(unsigned)div_up64(l.ncols * l.words, 256), 256, 0, st>>>(g, l.words, l.ncols, cm, mask);
+  int per = kScanCols / kScanThreads;              // block sums per kScanCols columns
+  if (cm.table != nullptr && strided_bits_ok(g) && l.words <= 64) {
+    strided_bits_kernel<<<l.nblk, 256, 0, st>>>(g, l.words, l.cols_per_block, l.ncols, cm, mask, d_oz_ptr, blocksum);
     SPH_LAUNCH_CHECK();
-  }
-  strided_mask_kernel<<<l.nblk, kScanThreads, 0, st>>>(d_z_idx, d_z_ptr, g, l.words, l.ncols, cm, mask, d_oz_ptr,
-                                                       blocksum, fast ? 1 : 0);
-  SPH_LAUNCH_CHECK();
-  if (fast) {
-    count_columns_kernel<<<l.nblk, kScanThreads, 0, st>>>(mask, l.words, l.ncols, cm.unsorted, d_oz_ptr, blocksum);
+    per = kScanCols / l.cols_per_block;
+  } else {
+    strided_mask_kernel<<<(unsigned)div_up64(l.ncols, kScanThreads), kScanThreads, 0, st>>>(
+        d_z_idx, d_z_ptr, g, l.words, l.ncols, cm, mask, d_oz_ptr, blocksum);
     SPH_LAUNCH_CHECK();
   }
   int32_t* host_word = nullptr;
@@ -1317,9 +1304,8 @@ int strided_count_impl(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t n
     rc = count_slot(&host_word, &dev_word);
     if (rc != SPH_OK) return rc;
   }
-  scan_blocksums_kernel<<<1, kScanThreads, 0, st>>>(blocksum, l.nblk, d_out_nnz, dev_word);
-  SPH_LAUNCH_CHECK();
-  scan_columns_kernel<<<l.nblk, kScanThreads, 0, st>>>(d_oz_ptr, l.ncols, blocksum);
+  scan_columns_kernel<<<(unsigned)div_up64(l.ncols, kScanCols), kScanThreads, 0, st>>>(d_oz_ptr, l.ncols, blocksum, per,
+                                                                                       d_out_nnz, dev_word);
   SPH_LAUNCH_CHECK();
   if (host_word_out) *host_word_out = host_word;
   return SPH_OK;
@@ -1375,8 +1361,7 @@ extern "C" int sph_rules_strided_fill(const int32_t* d_z_idx, const int32_t* d_z
     SPH_LAUNCH_CHECK();
   }
   return launch_emit(d_z_idx, d_z_ptr, d_oz_idx, d_oz_ptr, g, nnz, out_nnz, tile_n_max, d_rules, d_rule_size,
-                     d_nbr, d_nbr_t, strided_colmask(g, nnz, l, d_scratch), /*rows_parked=*/d_nbr != nullptr,
-                     fill_unused, d_status, st);
+                     d_nbr, d_nbr_t, strided_colmask(g, nnz, l, d_scratch), fill_unused, d_status, st);
 }
 
 extern "C" int sph_rules_to_nbr(const int32_t* d_rules, const int32_t* d_rule_size, int32_t n_tile, int32_t kv,

@@ -301,7 +301,7 @@ extern "C" int sph_init_tensor(const void* d_feature, int32_t row_bytes, int64_t
   const InitScratch l = init_layout(B, shape);
   SPH_CHECK_ARG(l.ncols <= 0x7fffffffLL, "more than 2^31 columns");
   cudaStream_t st = (cudaStream_t)stream;
-  int* header = (int*)d_scratch;                           // [0] = 0 (flag for the scan), [1] = total
+  int* header = (int*)d_scratch;                           // [0] = total
   uint32_t* mask = (uint32_t*)((char*)d_scratch + 256);
   int* blocksum = (int*)((char*)d_scratch + 256 + l.mask_bytes);
   SPH_CUDA(cudaMemsetAsync(d_scratch, 0, 256 + l.mask_bytes, st));
@@ -311,7 +311,7 @@ extern "C" int sph_init_tensor(const void* d_feature, int32_t row_bytes, int64_t
                                                                                       mask, d_status);
     SPH_LAUNCH_CHECK();
   }
-  int rc = column_prefix_from_masks(mask, l.words, l.ncols, header, d_z_ptr, blocksum, header + 1, st);
+  int rc = column_prefix_from_masks(mask, l.words, l.ncols, d_z_ptr, blocksum, header, nullptr, st);
   if (rc != SPH_OK) return rc;
   if (nnz > 0) {
     place_voxels_kernel<<<(unsigned)div_up64(nnz, kOpsThreads), kOpsThreads, 0, st>>>(d_indices, nnz, B, H, W, D, l.words,

@@ -248,7 +248,7 @@ voxel_mean_kernel(const float* __restrict__ pts, int stride, const float4* __res
 
 int run_passes(const float4* sys, const int* scan_ptr, int64_t n, const VoxGrid& g, const VoxScratch& l, char* scratch,
                int* z_ptr, bool with_cut_search, cudaStream_t st) {
-  int* header = (int*)(scratch + l.header);            // [0] = 0 (flag for the scan), [1] = rows, [2] = a scan was cut
+  int* header = (int*)(scratch + l.header);            // [1] = rows, [2] = a scan was cut
   int* cut = (int*)(scratch + l.cut);
   uint32_t* mask = (uint32_t*)(scratch + l.mask);
   int* blocksum = (int*)(scratch + l.blocksum);
@@ -263,7 +263,7 @@ int run_passes(const float4* sys, const int* scan_ptr, int64_t n, const VoxGrid&
     voxel_bin_kernel<<<blocks, kVoxThreads, 0, st>>>(sys, n, scan_ptr, g, cut, mask, cell);
     SPH_LAUNCH_CHECK();
   }
-  int rc = column_prefix_from_masks(mask, g.words, g.ncols, header, z_ptr, blocksum, header + 1, st);
+  int rc = column_prefix_from_masks(mask, g.words, g.ncols, z_ptr, blocksum, header + 1, nullptr, st);
   if (rc != SPH_OK) return rc;
   if (n > 0) {
     voxel_rows_kernel<<<blocks, kVoxThreads, 0, st>>>(cell, n, g.words, mask, z_ptr, row, sel);
