@@ -2,15 +2,18 @@
 
 The shared library is built in-tree by ``python -m sphconv_b200.build`` (or ``__graft_entry__.build()``)
 into ``sphconv_b200/_lib/libsphconv_b200.so``.  There is no fallback: if the library is missing, every op
-raises.  torch is used only for device memory and the current stream.
+raises.  torch is used only for device memory and the current stream.  The operators go through ``host()``,
+which calls the same entry points natively.
 """
 import ctypes
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "_lib", "libsphconv_b200.so")
+HOST_PATH = os.path.join(_HERE, "_lib", "sph_host.so")
 
 SPH_F32, SPH_F16, SPH_BF16, SPH_I8 = 0, 1, 2, 3
 STATUS_RULE_OVERFLOW, STATUS_BAD_INDEX, STATUS_TIMEOUT = 1, 2, 4
@@ -95,6 +98,25 @@ def lib():
     return _lib
 
 
+_host = None
+
+
+def host():
+    """The native host side of the operators (csrc/host.cpp); raises RuntimeError when it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError("sphconv_b200: host module %s is missing - build it with `python -m sphconv_b200.build`; "
+                               "there is no CPU or PyTorch fallback" % HOST_PATH)
+        spec = importlib.util.spec_from_file_location("sph_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        module.load(LIB_PATH)
+        _host = module
+    return _host
+
+
 def check(rc):
     if rc < 0:
         raise RuntimeError("sphconv_b200: %s (code %d)" % (lib().sph_last_error().decode(), rc))
@@ -133,17 +155,10 @@ def require_cuda(*tensors):
             raise RuntimeError("sphconv_b200 ops need contiguous tensors")
 
 
-_status = {}
-
-
 def status_tensor(device):
     """Per-device int32 status word the kernels OR error bits into."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
-    t = _status.get(key)
-    if t is None:
-        t = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
-        _status[key] = t
-    return t
+    index = torch.device(device).index
+    return host().status_tensor(torch.cuda.current_device() if index is None else index)
 
 
 def check_status(device=None, reset=True, ignore_overflow=True):

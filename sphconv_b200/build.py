@@ -1,4 +1,5 @@
-"""Builds the C-ABI CUDA library in-tree: sphconv_b200/_lib/libsphconv_b200.so (sm_100a only).
+"""Builds the C-ABI CUDA library in-tree, sphconv_b200/_lib/libsphconv_b200.so (sm_100a only), and the host module that
+drives it from torch, sphconv_b200/_lib/sph_host.so.
 
     python -m sphconv_b200.build [--force] [--verbose]
 """
@@ -17,17 +18,36 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", 
               "-Xcompiler", "-fPIC", "--use_fast_math=false"]
 
 
+HOST_LIB = os.path.join(LIBDIR, "sph_host.so")
+
+
 def _nvcc():
     cand = os.environ.get("NVCC") or "/usr/local/cuda/bin/nvcc"
     return cand if os.path.exists(cand) else "nvcc"
 
 
 def _stale():
-    if not os.path.exists(LIB):
+    if not os.path.exists(LIB) or not os.path.exists(HOST_LIB):
         return True
-    t = os.path.getmtime(LIB)
+    t = min(os.path.getmtime(LIB), os.path.getmtime(HOST_LIB))
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(ROOT, "include", "sphconv_b200.h")]
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def _host_command():
+    """g++ command of the torch-facing host module (csrc/host.cpp)."""
+    import sysconfig
+
+    import torch
+    t = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(_nvcc())) if os.path.sep in _nvcc() else "/usr/local/cuda"
+    includes = [os.path.join(ROOT, "include"), os.path.join(t, "include"),
+                os.path.join(t, "include", "torch", "csrc", "api", "include"), os.path.join(cuda, "include"),
+                sysconfig.get_paths()["include"]]
+    return (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=sph_host",
+             "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + ["-isystem" + i for i in includes] +
+            [os.path.join(CSRC, "host.cpp"), "-o", HOST_LIB, "-L" + os.path.join(t, "lib"), "-L" + os.path.join(cuda, "lib64")] +
+            ["-l" + n for n in ("c10", "c10_cuda", "torch", "torch_cpu", "torch_cuda", "torch_python", "cudart", "dl")])
 
 
 HOOKS_LIB = os.path.join(LIBDIR, "libsphconv_b200_hooks.so")
@@ -51,7 +71,7 @@ def build_test_hooks(force=False):
 
 
 def build(force=False, verbose=False):
-    """Compile every .cu into one shared library; returns its path."""
+    """Compile every .cu into one shared library and host.cpp into the host module; returns the library's path."""
     if not force and not _stale():
         return LIB
     os.makedirs(LIBDIR, exist_ok=True)
@@ -65,6 +85,7 @@ def build(force=False, verbose=False):
         cmd = [_nvcc(), *flags, "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c", os.path.join(CSRC, src), "-o", obj]
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
         objs.append(obj)
+    procs.append(("host.cpp", subprocess.Popen(_host_command(), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, pr in procs:
         out, _ = pr.communicate()
@@ -72,7 +93,7 @@ def build(force=False, verbose=False):
             sys.stderr.write("[%s]\n%s\n" % (src, out))
         failed |= pr.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed")
+        raise RuntimeError("the compiler failed")
     subprocess.check_call([_nvcc(), "-shared", "-o", LIB, *objs, "-lcudart"])
     return LIB
 

@@ -102,6 +102,15 @@ class Conv3d(Convolution):
                     out_shape=list(out_shape), n_tile=tg[0] * tg[1],
                     kv=self.kernel_size[0] * self.kernel_size[1] * self.kernel_size[2])
 
+    def _timed_rules(self, name, tag, input, in_shape, out_shape):
+        """profiling.section of the rule generation of this layer (free of cost while profiling is off)."""
+        if not profiling.is_active():
+            return profiling.NO_SECTION
+        return profiling.section(name + tag, **self._rule_meta(input, in_shape, out_shape))
+
+    def _out_shape(self, in_shape):
+        return in_shape if self.subm else out_spatial(in_shape, self.kernel_size, self.stride, self.padding, self.dilation)
+
     def begin_rules(self, input: SparseConvTensor):
         """Extension used by Sequential: enqueue the first step of this (strided) layer's rule generation on a tensor
         that has the geometry this layer will see - the input of the submanifold layer in front of it - so that
@@ -110,70 +119,83 @@ class Conv3d(Convolution):
         if self.subm or (self.indice_key is not None and input.find_rule(self.indice_key) is not None):
             return
         in_shape = [input.D, input.W, input.H]
-        out_shape = out_spatial(in_shape, self.kernel_size, self.stride, self.padding, self.dilation)
+        out_shape = self._out_shape(in_shape)
         tag = self.name or "conv{}_{}".format(self.in_channels, self.weight.shape[4])
-        with profiling.section("rules:" + tag, **self._rule_meta(input, in_shape, out_shape)):
+        with self._timed_rules("rules:", tag, input, in_shape, out_shape):
             input.rule_cache[("pending", id(self))] = ops.get_rules_begin(
                 input.z_idx, input.z_ptr, input.B, in_shape, out_shape, self.kernel_size, self.stride, self.padding,
                 self.dilation, self.tile_size)
 
-    def forward(self, input: SparseConvTensor):
-        batch_size, in_channels = input.B, input.C
-        out_channels = self.weight.shape[4]
-        assert self.in_channels == in_channels, \
-            "input channel does not match Expect: {}, got {}".format(self.in_channels, in_channels)
+    def find_or_make_rules(self, input: SparseConvTensor, tag: str):
+        """(output shape, rule set) of this layer on `input`: from the tensor's rule cache, or generated and cached."""
         in_shape = [input.D, input.W, input.H]
-        out_shape = in_shape
-        if not self.subm:
-            out_shape = out_spatial(in_shape, self.kernel_size, self.stride, self.padding, self.dilation)
-
-        tag = self.name or "{}{}_{}".format("subm" if self.subm else "conv", in_channels, out_channels)
+        out_shape = self._out_shape(in_shape)
         datas = input.find_rule(self.indice_key) if self.indice_key is not None else None
         if datas is None:
             profiling.current_rule_tag = tag
-            with profiling.section("rules:" + tag, **self._rule_meta(input, in_shape, out_shape)):
+            with self._timed_rules("rules:", tag, input, in_shape, out_shape):
                 datas = self._rules(input, in_shape, out_shape)
             if self.indice_key is not None:
                 input.rule_cache[self.indice_key] = datas
-        oz_idx, oz_ptr, rules, rule_size, tile_grid_shape = datas
+        return out_shape, datas
+
+    def forward(self, input: SparseConvTensor):
+        batch_size, in_channels = input.B, input.C
+        weight = self.weight
+        out_channels = weight.shape[4]
+        assert self.in_channels == in_channels, \
+            "input channel does not match Expect: {}, got {}".format(self.in_channels, in_channels)
+        tag = self.name or "{}{}_{}".format("subm" if self.subm else "conv", in_channels, out_channels)
+        out_shape, (oz_idx, oz_ptr, rules, rule_size, tile_grid_shape) = self.find_or_make_rules(input, tag)
         self.rule_size = rule_size
 
-        weight = self.weight.view((-1, in_channels, out_channels))
-        if weight.dtype != input.feature.dtype and input.feature.dtype != torch.int8:
-            weight = weight.to(input.feature.dtype)
-        bias = self.bias if (self.apply_bias and self.bias is not None) else None
-        needs_grad = torch.is_grad_enabled() and (input.feature.requires_grad or self.weight.requires_grad)
+        feature = input.feature
+        bias = self.bias if self.apply_bias else None
+        needs_grad = torch.is_grad_enabled() and (feature.requires_grad or weight.requires_grad)
         if needs_grad:
             profiling.current_tag = tag
+            w = weight.view((-1, in_channels, out_channels))
+            if w.dtype != feature.dtype and feature.dtype != torch.int8:
+                w = w.to(feature.dtype)
             # bias and activation run in the kernel's epilogue in training too (extension arguments of ConvFunction)
-            mw = getattr(self.weight, "_sph_master_grad", None)      # slices of a sharding.GradBuffer, if attached
+            mw = getattr(weight, "_sph_master_grad", None)           # slices of a sharding.GradBuffer, if attached
             mb = getattr(bias, "_sph_master_grad", None) if bias is not None else None
             master = None if mw is None and mb is None else \
                 (None if mw is None else mw.view(-1, in_channels, out_channels), mb)
-            out_feature = ConvFunction.apply(input.feature, weight, rules, rule_size, tile_grid_shape,
+            out_feature = ConvFunction.apply(feature, w, rules, rule_size, tile_grid_shape,
                                              oz_idx.shape[0], bias, self.activation == 'relu', master)
         else:
-            weight = self._cached_packed(weight)
-            with profiling.section("conv:" + tag, iC=in_channels, oC=out_channels, n_in=input.feature.shape[0],
-                                   n_out=oz_idx.shape[0], esize=input.feature.element_size()):
-                profiling.count_pairs("conv:" + tag, rules)
-                out_feature = ops.rule_conv(input.feature, weight, rules, rule_size, oz_idx.shape[0],
-                                            bias=None if bias is None else bias.detach().float(),
+            w, b = self._inference_weights(feature.dtype, bias)
+            if profiling.is_active() or profiling.pair_counts is not None:
+                with profiling.section("conv:" + tag, iC=in_channels, oC=out_channels, n_in=feature.shape[0],
+                                       n_out=oz_idx.shape[0], esize=feature.element_size()):
+                    profiling.count_pairs("conv:" + tag, rules)
+                    out_feature = ops.rule_conv(feature, w, rules, rule_size, oz_idx.shape[0], bias=b,
+                                                relu=self.activation == 'relu')
+            else:
+                out_feature = ops.rule_conv(feature, w, rules, rule_size, oz_idx.shape[0], bias=b,
                                             relu=self.activation == 'relu')
         out_tensor = SparseConvTensor(out_feature, out_shape, batch_size, z_ptr=oz_ptr, z_idx=oz_idx)
         out_tensor.rule_cache = input.rule_cache
         return out_tensor
 
-    def _cached_packed(self, weight):
-        """Inference: keep the tensor-core weight image across calls while the parameter is unchanged."""
-        key = (self.weight._version, self.weight.data_ptr(), weight.dtype)
+    def _inference_weights(self, dtype, bias):
+        """Inference: the weight in the features' dtype (with its tensor-core image attached) and the float32 bias, kept
+        across calls while the parameters are unchanged."""
+        weight = self.weight
+        key = (weight._version, weight.data_ptr(), weight.dtype, dtype, None if bias is None else bias._version,
+               None if bias is None else bias.data_ptr())
         cached = getattr(self, "_w_cache", None)
         if cached is not None and cached[0] == key:
-            return cached[1]
-        w = weight.detach().contiguous()
+            return cached[1], cached[2]
+        w = weight.detach().view((-1, self.in_channels, weight.shape[4]))
+        if w.dtype != dtype and dtype != torch.int8:
+            w = w.to(dtype)
+        w = w.contiguous()
         ops._packed_weight(w)
-        self._w_cache = (key, w)
-        return w
+        b = None if bias is None else bias.detach().float()
+        self._w_cache = (key, w, b)
+        return w, b
 
 
 SparseConv3d = Conv3d

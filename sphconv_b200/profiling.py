@@ -9,6 +9,9 @@ current_tag = ""          # name of the layer whose ops are being issued (set by
 _records = []   # (name, start_event, stop_event, meta)
 
 
+NO_SECTION = contextlib.nullcontext()
+
+
 def enable(flag=True):
     global _active
     _active = bool(flag)

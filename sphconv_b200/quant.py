@@ -13,10 +13,9 @@ import torch
 
 from . import profiling
 from . import sphconv_cuda as ops
-from .conv import Conv3d, get_tile_grid_shape
+from .conv import Conv3d
 from .modules import Sequential
 from .tensor import SparseConvTensor
-from .utils import out_spatial
 
 QMAX = 127.0
 
@@ -37,19 +36,11 @@ class QuantConv:
 
     def __call__(self, x: SparseConvTensor) -> SparseConvTensor:
         c = self.conv
-        in_shape = [x.D, x.W, x.H]
-        out_shape = in_shape if c.subm else out_spatial(in_shape, c.kernel_size, c.stride, c.padding, c.dilation)
         tag = c.name or "{}{}_{}".format("subm" if c.subm else "conv", c.in_channels, c.out_channels)
-        datas = x.find_rule(c.indice_key) if c.indice_key is not None else None
-        if datas is None:
-            profiling.current_rule_tag = tag
-            with profiling.section("rules:" + tag, **c._rule_meta(x, in_shape, out_shape)):
-                datas = c._rules(x, in_shape, out_shape)
-            if c.indice_key is not None:
-                x.rule_cache[c.indice_key] = datas
-        oz_idx, oz_ptr, rules, rule_size, _ = datas
-        with profiling.section("conv:" + tag, iC=c.in_channels, oC=c.out_channels, n_in=x.feature.shape[0],
-                               n_out=oz_idx.shape[0], esize=1, k_ch=self.weight_q.shape[1], n_ch=self.weight_q.shape[2]):
+        out_shape, (oz_idx, oz_ptr, rules, rule_size, _) = c.find_or_make_rules(x, tag)
+        with (profiling.section("conv:" + tag, iC=c.in_channels, oC=c.out_channels, n_in=x.feature.shape[0],
+                                n_out=oz_idx.shape[0], esize=1, k_ch=self.weight_q.shape[1], n_ch=self.weight_q.shape[2])
+              if profiling.is_active() else profiling.NO_SECTION):
             profiling.count_pairs("conv:" + tag, rules)
             y = ops.rule_conv(x.feature, self.weight_q, rules, rule_size, oz_idx.shape[0], scale=self.scale,
                               bias=self.bias, relu=self.relu, out_dtype=self.out_dtype)

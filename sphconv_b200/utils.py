@@ -11,7 +11,7 @@ from torch.nn.init import calculate_gain
 def out_spatial(in_spatial: List[int], kernel_size: List[int], stride: List[int], padding: List[int],
                 dilation: List[int] = [1, 1, 1]) -> List[int]:
     """floor((i + 2p - d(k-1) - 1)/s + 1) per axis (sphconv/utils/__init__.py:27-44)."""
-    return [math.floor((i + 2 * p - d * (k - 1) - 1) / s + 1)
+    return [(i + 2 * p - d * (k - 1) - 1) // s + 1
             for i, k, s, p, d in zip(in_spatial, kernel_size, stride, padding, dilation)]
 
 

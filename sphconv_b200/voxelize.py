@@ -11,7 +11,6 @@ Differences from the reference, all on purpose: the points are a CUDA tensor (a 
 per-voxel point lists (``voxels`` [V, max_points, C]) are not materialised, only their mean is.  Which points a
 voxel keeps, which voxels survive ``max_voxels`` and every cell index are the reference's.
 """
-import ctypes
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -53,6 +52,7 @@ class VoxelGenerator:
         self.max_voxels = int(max_voxels)
         self.append_mode = int(append_mode)
         self.system_range = system_range(point_cloud_range, point_cloud_sphere_range, coord_system)
+        self._range = [float(v) for v in self.system_range]
 
     @property
     def spatial_shape(self) -> List[int]:
@@ -60,66 +60,22 @@ class VoxelGenerator:
         g = self.grid_size
         return [g[2], g[1], g[0]]
 
-    def _grid(self, B: int) -> C.VoxelGrid:
-        g = C.VoxelGrid()
-        g.B = B
-        for i in range(3):
-            g.cells[i] = self.grid_size[i]
-        for i in range(6):
-            g.range[i] = float(self.system_range[i])
-        g.max_points, g.max_voxels, g.append_mode = self.max_num_points, self.max_voxels, self.append_mode
-        return g
-
     def transform(self, points: torch.Tensor) -> torch.Tensor:
         """[N,4] system coordinates + intensity of the points (coord_transform.py of the reference)."""
-        C.require_cuda(points)
-        if points.dtype != torch.float32 or points.dim() != 2 or points.shape[1] < 4:
-            raise RuntimeError("points must be a float32 tensor [N, >=4]")
-        sys_pts = torch.empty((points.shape[0], 4), dtype=torch.float32, device=points.device)
-        with torch.cuda.device(points.device):
-            C.check(C.lib().sph_voxel_transform(C.ptr(points), points.shape[1], points.shape[0],
-                                                SYSTEMS[self.coord_system], C.ptr(sys_pts),
-                                                C.stream_ptr(points.device)))
-        return sys_pts
+        return C.host().voxel_transform(points, SYSTEMS[self.coord_system])
 
     def generate(self, points: torch.Tensor, scan_ptr: Optional[torch.Tensor] = None,
                  system_points: Optional[torch.Tensor] = None, with_coordinates: bool = True) -> dict:
         """points float32 [N, F] on the device; scan_ptr int32 [B+1] (device or host; None = one scan).
         Returns feature [NNZ, C], z_idx, z_ptr [B, s0, s1], coordinates int32 [NNZ,4] = (b, c0, c1, c2),
         num_points_per_voxel int32 [NNZ], voxel_num, batch_size, spatial_shape."""
-        C.require_cuda(points)
-        dev = points.device
-        n = points.shape[0]
-        if scan_ptr is None:
-            scan_ptr = torch.tensor([0, n], dtype=torch.int32)
-        B = scan_ptr.shape[0] - 1
-        scan_dev = scan_ptr.to(device=dev, dtype=torch.int32).contiguous()
         sys_pts = self.transform(points) if system_points is None else system_points
-        C.require_cuda(sys_pts)
-        if sys_pts.dtype != torch.float32 or tuple(sys_pts.shape) != (n, 4):
-            raise RuntimeError("system_points must be float32 [N, 4]")
-        lib = C.lib()
-        grid = self._grid(B)
-        s = self.spatial_shape
-        nbytes = C.check(lib.sph_voxelize_scratch_bytes(ctypes.byref(grid), n))
-        scratch = torch.empty((nbytes,), dtype=torch.uint8, device=dev)
-        z_ptr = torch.empty((B, s[0], s[1]), dtype=torch.int32, device=dev)
-        nnz = ctypes.c_int32(0)
-        with torch.cuda.device(dev):
-            st = C.stream_ptr(dev)
-            C.check(lib.sph_voxelize_count(C.ptr(sys_pts), C.ptr(scan_dev), n, ctypes.byref(grid), C.ptr(scratch),
-                                           C.ptr(z_ptr), ctypes.byref(nnz), st))
-            nnz = int(nnz.value)
-            n_feat = C.check(lib.sph_voxel_feature_count(points.shape[1], self.append_mode))
-            feature = torch.empty((nnz, n_feat), dtype=torch.float32, device=dev)
-            z_idx = torch.empty((nnz,), dtype=torch.int32, device=dev)
-            coords = torch.empty((nnz, 4), dtype=torch.int32, device=dev) if with_coordinates else None
-            num = torch.empty((nnz,), dtype=torch.int32, device=dev) if with_coordinates else None
-            C.check(lib.sph_voxelize_fill(C.ptr(points), points.shape[1], C.ptr(sys_pts), C.ptr(scan_dev), n,
-                                          ctypes.byref(grid), C.ptr(scratch), nnz, C.ptr(feature), C.ptr(z_idx),
-                                          C.ptr(coords), C.ptr(num), st))
+        feature, z_idx, z_ptr, coords, num = C.host().voxelize(
+            points, scan_ptr, sys_pts, self.grid_size, self._range, self.max_num_points, self.max_voxels, self.append_mode,
+            with_coordinates)
         return {"feature": feature, "z_idx": z_idx, "z_ptr": z_ptr, "coordinates": coords,
-                "num_points_per_voxel": num, "voxel_num": nnz, "batch_size": B, "spatial_shape": s}
+                "num_points_per_voxel": num, "voxel_num": feature.shape[0], "batch_size": z_ptr.shape[0],
+                "spatial_shape": self.spatial_shape}
 
     def to_tensor(self, points: torch.Tensor, scan_ptr: Optional[torch.Tensor] = None,
                   dtype: Optional[torch.dtype] = None) -> SparseConvTensor:
