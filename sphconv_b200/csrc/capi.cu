@@ -61,6 +61,13 @@ bool conv_tc_rows_supported(int dtype, int kv, int K, int N);
 int conv_gather_tc_rows(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
                         int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
                         int out_dtype, int* status, cudaStream_t st);
+// conv_strip.cu
+bool conv_strip_supported(int dtype, int kv, int K, int N);
+int64_t strip_filter_bytes(int dtype, int kv, int K, int N);
+int pack_strip_filter(const void* w, int dtype, int kv, int K, int N, void* packed, cudaStream_t st);
+int conv_gather_strip(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out, int kv,
+                    int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out, int out_dtype,
+                    int* status, cudaStream_t st);
 // conv_sparse.cu
 bool conv_sparse_supported(int dtype, int kv, int K, int N);
 int conv_gather_sparse(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
@@ -84,7 +91,17 @@ extern "C" const char* sph_last_error(void) { return g_err; }
 extern "C" int sph_version(void) { return 100; }
 extern "C" int64_t sph_kernel_launches(void) { return (int64_t)g_launches.load(std::memory_order_relaxed); }
 
+// Whether a shape runs the strip kernel (conv_strip.cuh) when the caller passes a packed filter: everything the tcgen05
+// kernels do not take, but for rows of 4 or 8 channels (sparse first layers: the pair kernel); of what they do take, 16
+// channels to at most 16 (1.1 to 1.4 times faster at 1.5 to 12 neighbours per row; from 32 output channels on it loses).
+static bool runs_strip(int dtype, int kv, int K, int N) {
+  if (!conv_strip_supported(dtype, kv, K, N)) return false;
+  if (conv_tc_supported(dtype, kv, K, N)) return dtype != SPH_I8 && K == 16 && N <= 16;
+  return !((K == 4 || K == 8) && conv_sparse_supported(dtype, kv, K, N));
+}
+
 extern "C" int64_t sph_packed_weight_bytes(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch) {
+  if (runs_strip(dtype, kv, k_ch, n_ch)) return strip_filter_bytes(dtype, kv, k_ch, n_ch);
   if (!conv_tc_supported(dtype, kv, k_ch, n_ch)) return 0;
   return packed_weight_bytes(dtype, kv, k_ch, n_ch);
 }
@@ -92,6 +109,7 @@ extern "C" int64_t sph_packed_weight_bytes(int dtype, int32_t kv, int32_t k_ch, 
 extern "C" int sph_pack_weight(const void* d_weight, int dtype, int32_t kv, int32_t k_ch, int32_t n_ch,
                                void* d_packed, void* stream) {
   SPH_CHECK_ARG(d_weight && d_packed, "null pointer");
+  if (runs_strip(dtype, kv, k_ch, n_ch)) return pack_strip_filter(d_weight, dtype, kv, k_ch, n_ch, d_packed, (cudaStream_t)stream);
   return pack_weight(d_weight, dtype, kv, k_ch, n_ch, d_packed, (cudaStream_t)stream);
 }
 
@@ -126,6 +144,12 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
   SPH_CHECK_ARG(n_rows == 0 || d_rows, "null rows");
   SPH_CHECK_ARG(n_rows < 0x7fffffffLL && n_out < 0x7fffffffLL, "row ids are 32-bit");
   cudaStream_t st = (cudaStream_t)stream;
+  if (d_packed && runs_strip(dtype, kv, k_ch, n_ch)) {
+    if ((((uintptr_t)d_rows | (uintptr_t)d_out) & 15u) == 0)
+      return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias, relu,
+                             d_out, out_dtype, d_status, st);
+    d_packed = nullptr;      // its image is not the one the other tensor-core kernels read
+  }
   // 64-byte rows: the form with the output row on the TMEM lane (absent neighbours masked, not copied) is the faster
   // of the two; wider rows are dense deep layers, where the transposed form issues half as many instructions
   if (d_packed && k_ch * dtype_bytes(dtype) == 64 && conv_tc_rows_supported(dtype, kv, k_ch, n_ch)) {
