@@ -170,15 +170,19 @@ int64_t sph_packed_weight_bytes(int dtype, int32_t kv, int32_t k_ch, int32_t n_c
 int sph_pack_weight(const void* d_weight, int dtype, int32_t kv, int32_t k_ch, int32_t n_ch, void* d_packed,
                     void* stream);
 
-/* 1 when sph_conv_gather runs the tcgen05 kernel for this combination, 0 when it runs a CUDA-core kernel. */
+/* 1 when rows of this combination are wide and regular enough for the tensor-core kernels proper (tcgen05; 16 -> at most 16
+ * channels the strip kernel), 0 for the widths that the other kernels take. */
 int sph_conv_uses_tensor_cores(int dtype, int32_t k_ch, int32_t n_ch);
-/* Which CUDA-core kernel runs when the tensor-core kernels do not take the combination (27 offsets assumed, operands
- * 16-byte aligned): 1 = the pair-compacting kernel for sparse levels (rows of 4 / 8 / 16 / 32 channels in and out, the
- * fp32 filter within its shared-memory limit), 0 = the row-walking kernel (any shape).  No reference counterpart. */
-int sph_conv_uses_pair_kernel(int dtype, int32_t k_ch, int32_t n_ch);
-/* Which kernel sph_conv_wgrad runs for the combination (27 offsets assumed, operands 16-byte aligned): 1 = tcgen05,
- * 2 = the pair-compacting CUDA-core kernel (narrow rows, small fp32 layers), 0 = the general CUDA-core kernel.
+/* The widths beyond those (27 offsets assumed, operands 16-byte aligned): 1 = narrow rows, which a sparse first level can
+ * keep (4 / 8 / 16 / 32 channels in and out, the fp32 filter within the pair-compacting kernel's shared memory; int8 rows of
+ * 16 channels run the strip kernel when the packed filter is passed), 0 = any other width: the strip kernel for 16-bit and
+ * int8 rows of up to 128 bytes with a packed filter, else the FFMA kernel (int8: the row-walking one).
  * No reference counterpart. */
+int sph_conv_uses_pair_kernel(int dtype, int32_t k_ch, int32_t n_ch);
+/* The class of a combination's weight gradient (27 offsets assumed, operands 16-byte aligned): 1 = 16-bit rows of 16 / 32 /
+ * 64 / 128 channels (tcgen05 from 64 x 64 on, below that the pairs' kernel on mma.sync), 2 = narrow rows (16-bit: the pairs'
+ * kernel; fp32: the pair-compacting CUDA-core kernel), 0 = other widths (16-bit: the pairs' kernel up to 64 channels; fp32:
+ * the FFMA kernel).  No reference counterpart. */
 int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch);
 
 /* out[r,:] = epilogue( sum_k rows[ nbr[k][r], : ] @ weight[k] )   for r in [0, n_out)

@@ -15,9 +15,12 @@ using tc::cp_async_commit;
 using tc::cp_async_wait_pending;
 using tc::smem_u32;
 
-__device__ __forceinline__ float widen(float v) { return v; }
-__device__ __forceinline__ float widen(__half v) { return __half2float(v); }
-__device__ __forceinline__ float widen(__nv_bfloat16 v) { return __bfloat162float(v); }
+// One element global -> shared as a float; float32 elements asynchronously.
+__device__ __forceinline__ void stage_one(float* dst, const float* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(ok ? 4u : 0u));
+}
+__device__ __forceinline__ void stage_one(float* dst, const __half* src, bool ok) { *dst = ok ? __half2float(*src) : 0.f; }
+__device__ __forceinline__ void stage_one(float* dst, const __nv_bfloat16* src, bool ok) { *dst = ok ? __bfloat162float(*src) : 0.f; }
 
 __device__ __forceinline__ void store_one(void* out, int out_dtype, int64_t idx, float v) {
   switch (out_dtype) {
@@ -95,7 +98,8 @@ __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const flo
 // Bound by the issue slots (67 % busy, two thirds of them FMAs) and the shared-memory reads (60 %).  Measured: 64 -> 64 on
 // 170 k rows of 22 neighbours 3.2 -> 0.94 ms, 32 -> 32 on 390 k rows of 12 neighbours 1.9 -> 0.5 ms against the kernel it
 // replaced (one thread group per row walking every slot of the table).
-// VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by element.
+// VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by
+// element.
 template <typename T, int CG, bool VEC>
 __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams p) {
   using S = FfmaShape<CG>;
@@ -141,11 +145,12 @@ __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams 
     } else {
       for (int e = tid; e < m * kKC; e += S::T) {
         const int r = e / kKC, c = e % kKC;
-        a[r * kAStride + c] = c < kn ? widen(rows[(int64_t)in[r] * p.K + kc * kKC + c]) : 0.f;
+        stage_one(a + r * kAStride + c, c < kn ? rows + (int64_t)in[r] * p.K + kc * kKC + c : rows, c < kn);
       }
       for (int e = tid; e < kKC * S::NP; e += S::T) {
         const int r = e / S::NP, c = e % S::NP;
-        w[e] = (r < kn && c < nc) ? widen(wk[(int64_t)r * p.N + c]) : 0.f;
+        const bool ok = r < kn && c < nc;
+        stage_one(w + e, ok ? wk + (int64_t)r * p.N + c : weight, ok);
       }
     }
   };
@@ -340,11 +345,13 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
     } else {
       for (int e = tid; e < kWgPairs * KG * 8; e += kThreads) {
         const int r = e / (KG * 8), c = e % (KG * 8);
-        x[r * S::XS + c] = (r < np && c < p.K) ? widen(rows[(int64_t)s_in[p0 + r] * p.K + c]) : 0.f;
+        const bool ok = r < np && c < p.K;
+        stage_one(x + r * S::XS + c, ok ? rows + (int64_t)s_in[p0 + r] * p.K + c : rows, ok);
       }
       for (int e = tid; e < kWgPairs * NG * 8; e += kThreads) {
         const int r = e / (NG * 8), c = e % (NG * 8);
-        d[r * S::DS + c] = (r < np && c < p.N) ? widen(dout[(int64_t)s_out[p0 + r] * p.N + c]) : 0.f;
+        const bool ok = r < np && c < p.N;
+        stage_one(d + r * S::DS + c, ok ? dout + (int64_t)s_out[p0 + r] * p.N + c : dout, ok);
       }
     }
   };

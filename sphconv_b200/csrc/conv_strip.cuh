@@ -25,43 +25,17 @@
 //   16 -> 32 int8  60 -> 41 / 244 -> 74 (pair kernel)       32 -> 32 fp16   63 -> 63 /   97 -> 107 (tcgen05: kept there)
 #include "common.cuh"
 #include "conv_strip.h"
-#include "tc_common.cuh"
+#include "strip_common.cuh"
 
 namespace sph {
 
 namespace {
 
-using tc::cp_async_16;
-using tc::cp_async_wait_all;
-using tc::smem_u32;
+using namespace strip;
 
 constexpr int kWarps = kStripThreads / 32;
 constexpr int kGroup = 9;                 // offsets of a group: the 3 x 3 of one kernel height
 constexpr int MT = 2;                     // 16-row tiles of a warp
-constexpr int kZeroUnits = 8;             // the row of zeros, 16-byte units
-
-template <int DT>
-__device__ __forceinline__ void mma_step(uint32_t (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  if constexpr (DT == SPH_I8) {
-    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  } else if constexpr (DT == SPH_BF16) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  } else {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
-                 : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
-                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-  }
-}
-
-// Four 8 x 16-byte matrices: rows 0-7 and 8-15 of a 16-row tile, first and second half of a 32-byte step.
-__device__ __forceinline__ void ldmatrix4(uint32_t (&a)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(addr));
-}
 
 __device__ __forceinline__ uint32_t pack16(float a, float b, int out_dtype) {
   if (out_dtype == SPH_F16) {
@@ -84,69 +58,6 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int t) {
       const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j | s], s);
       if (up) v[j] = got; else v[j | s] = got;
     }
-  }
-}
-
-// Two windows of consecutive input rows, held one behind the other in a buffer.
-struct Windows {
-  int base1, len1, base2, len2;
-  bool fit;
-};
-
-// Merges the warps' runs (lo, hi of either part; lo > hi: empty); called by whole warps.
-__device__ __forceinline__ Windows merge_runs(const int4* runs, int cap) {
-  const int4 mine = runs[threadIdx.x % kWarps];
-  const int all_lo = __reduce_min_sync(0xffffffffu, mine.x);
-  const int all_hi = __reduce_max_sync(0xffffffffu, max(mine.y, mine.w));
-  Windows o;
-  o.base1 = all_hi < 0 ? 0 : all_lo;
-  o.len1 = all_hi < 0 ? 0 : all_hi - all_lo + 1;
-  o.base2 = o.len2 = 0;
-  o.fit = true;
-  if (o.len1 <= cap) return o;
-  // the end of a line of columns lies inside the tile: two windows
-  int lo1 = INT_MAX, hi1 = -1, lo2 = INT_MAX, hi2 = -1;
-  bool fit = true;
-  const int slack = cap / 4;
-  auto add = [&](int lo, int hi) {
-    if (lo > hi) return;
-    if (hi1 < 0 || (lo <= hi1 + slack && hi >= lo1 - slack)) {
-      lo1 = min(lo1, lo);
-      hi1 = max(hi1, hi);
-    } else if (hi2 < 0 || (lo <= hi2 + slack && hi >= lo2 - slack)) {
-      lo2 = min(lo2, lo);
-      hi2 = max(hi2, hi);
-    } else {
-      fit = false;
-    }
-  };
-#pragma unroll 1
-  for (int w = 0; w < kWarps; ++w) {
-    const int4 r = runs[w];
-    add(r.x, r.y);
-    add(r.z, r.w);
-  }
-  o.base1 = lo1;
-  o.len1 = hi1 - lo1 + 1;
-  o.base2 = hi2 < 0 ? 0 : lo2;
-  o.len2 = hi2 < 0 ? 0 : hi2 - lo2 + 1;
-  o.fit = fit && (int64_t)o.len1 + o.len2 <= cap;
-  return o;
-}
-
-// Rows of a width that is no multiple of 16 bytes -> rows `pitch` units apart, in the widest pieces that keep both sides
-// aligned (8 or 4 bytes by cp.async, 2 or 1 by way of a register).
-__device__ __forceinline__ void copy_ragged_rows(const uint8_t* rows, int base, int len, int row_bytes, int pitch, uint32_t to) {
-  const int piece = row_bytes & 1 ? 1 : row_bytes & 2 ? 2 : row_bytes & 4 ? 4 : 8;
-  const unsigned per = row_bytes / piece, n = per * len;
-  for (unsigned u = threadIdx.x; u < n; u += kStripThreads) {
-    const unsigned r = u / per, b = u % per * piece;
-    const uint8_t* src = rows + (int64_t)(base + (int)r) * row_bytes + b;
-    const uint32_t dst = to + r * pitch * 16 + b;
-    if (piece == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src));
-    else if (piece == 4) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src));
-    else if (piece == 2) asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst), "h"(__ldg((const uint16_t*)src)) : "memory");
-    else asm volatile("{.reg .b16 t; cvt.u16.u32 t, %1; st.shared.u8 [%0], t;}" ::"r"(dst), "r"((uint32_t)__ldg(src)) : "memory");
   }
 }
 
@@ -247,7 +158,7 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
     const uint32_t dst = smem0 + (kZeroUnits + slot * buf_units) * 16;
     auto copy = [&](int base, int len, uint32_t to) {
       if (!WHOLE && (p.row_bytes & 15)) {
-        copy_ragged_rows(p.rows, base, len, p.row_bytes, pitch, to);
+        copy_ragged_rows<kStripThreads>(p.rows, p.n_rows, base, len, p.row_bytes, pitch, to);
         return;
       }
       const unsigned n = len * rb16;
@@ -318,7 +229,7 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
   load_entries(here);
   post_run(0);
   __syncthreads();
-  wn = merge_runs(s_runs, p.cap);
+  wn = merge_runs<kWarps>(s_runs, p.cap);
   stage(wn, 0);
   pack(wn, 0, cur);
   cur_fit = wn.fit;
@@ -329,7 +240,7 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
 
   for (int j = 0; j < total; ++j) {
     // the next group's rows start moving, the entries of the one behind it are requested
-    wn = merge_runs(s_runs + ((j + 1) & 1) * kWarps, p.cap);
+    wn = merge_runs<kWarps>(s_runs + ((j + 1) & 1) * kWarps, p.cap);
     stage(wn, (j + 1) & 1);
     pack(wn, (j + 1) & 1, nxt);
     const Place behind = after(there);

@@ -274,22 +274,58 @@ emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
 //  2. rule_lists_kernel: one warp per (tile, group of offsets) walks the tile's row ranges in list order
 //     (batch, tile row, row), reads nbr[k][row] and ballot-compacts the hits into rules[tile][k].
 // ---------------------------------------------------------------------------------------------
+// The table entries of output row r by searching the input columns row by row: for columns out of depth order and grids
+// without the index.  Not inlined: the registers of the path that every row takes are worth more.
+__device__ __noinline__ void search_row(const int* __restrict__ in_zi, const int* __restrict__ in_zp, int oz, const Geom& g,
+                                        int64_t in_nnz, int64_t out_nnz, int64_t r, int c, int* nbr, int* nbr_t) {
+  const int oy = c % g.oW, ox = c / g.oW % g.oH, b = c / g.oW / g.oH;
+  for (int k = 0; k < g.KV; ++k) {
+    const int ix = ox * g.sH - g.pH + k / (g.KW * g.KD) * g.dH;
+    const int iy = oy * g.sW - g.pW + k / g.KD % g.KW * g.dW;
+    const int iz = oz * g.sD - g.pD + k % g.KD * g.dD;
+    int found = -1;
+    if (ix >= 0 && ix < g.H && iy >= 0 && iy < g.W && iz >= 0 && iz < g.D) {
+      const int64_t ci = ((int64_t)b * g.H + ix) * g.W + iy;
+      const int end = __ldg(in_zp + ci);
+      for (int q = col_start(in_zp, ci); q < end && found < 0; ++q)
+        if (__ldg(in_zi + q) == iz) found = q;
+    }
+    nbr[(int64_t)k * out_nnz + r] = found;
+    if (nbr_t && found >= 0) nbr_t[(int64_t)k * in_nnz + found] = (int)r;
+  }
+}
+
+// Column id parked for row r, or -1 (with no neighbours and the status bit written) for a row nobody parked one for: the
+// caller's row count exceeds the prefix total, and the buffer holds whatever it held.
+__device__ __forceinline__ int parked_column(const Geom& g, int64_t out_nnz, int64_t r, int* nbr, int* status) {
+  const int c = nbr[(int64_t)(g.KV - 1) * out_nnz + r];
+  if ((unsigned)c < (unsigned)(g.B * g.oH * g.oW)) return c;
+  for (int k = 0; k < g.KV; ++k) nbr[(int64_t)k * out_nnz + r] = -1;
+  if (status) atomicOr(status, SPH_STATUS_BAD_INDEX);
+  return -1;
+}
+
+__global__ void __launch_bounds__(256)
+nbr_search_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
+                  const __grid_constant__ Geom g,
+                  int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, int* __restrict__ status) {
+  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= out_nnz) return;
+  const int c = parked_column(g, out_nnz, r, nbr, status);
+  if (c >= 0) search_row(in_zi, in_zp, __ldg(out_zi + r), g, in_nnz, out_nnz, r, c, nbr, nbr_t);
+}
+
 // KD_CT = 3: the filter is 3 wide and 3 deep (those two loops are unrolled), 0 = extents read from the geometry.
 template <int KD_CT, bool HAS_T>
 __global__ void __launch_bounds__(256)
-nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi, Geom g,
+nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
+                const __grid_constant__ Geom g,
                 int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, ColMask cm,
                 int* __restrict__ status) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= out_nnz) return;
-  const int c = nbr[(int64_t)(g.KV - 1) * out_nnz + r];
-  // A row nobody parked a column id for (the caller's row count exceeds the prefix total) holds whatever the buffer
-  // held: it gets no neighbours and the status bit, instead of reads outside the index.
-  if ((unsigned)c >= (unsigned)(g.B * g.oH * g.oW)) {
-    for (int k = 0; k < g.KV; ++k) nbr[(int64_t)k * out_nnz + r] = -1;
-    if (status) atomicOr(status, SPH_STATUS_BAD_INDEX);
-    return;
-  }
+  const int c = parked_column(g, out_nnz, r, nbr, status);
+  if (c < 0) return;
   const int oy = c % g.oW;
   const int t2 = c / g.oW;
   const int ox = t2 % g.oH;
@@ -297,6 +333,7 @@ nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, co
   const int iz0 = __ldg(out_zi + r) * g.sD - g.pD;
   int* dst = nbr + r;
   int* dst_t = nbr_t;
+  uint32_t order = 0u;                       // the second half-words read: kUnsorted of any column
   for (int kh = 0; kh < g.KH; ++kh) {
     const int ix = ox * g.sH - g.pH + kh * g.dH;
     const int KW = KD_CT ? KD_CT : g.KW;   // the unrolled form is the cubic 3 x 3 x 3 filter
@@ -305,10 +342,9 @@ nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, co
       const int iy = oy * g.sW - g.pW + kw * g.dW;
       const bool col_ok = ix >= 0 && ix < g.H && iy >= 0 && iy < g.W;
       int cstart = 0;
-      int64_t ci = 0;
       const uint2* row = cm.table;
       if (col_ok) {
-        ci = ((int64_t)b * g.H + ix) * g.W + iy;
+        const int64_t ci = ((int64_t)b * g.H + ix) * g.W + iy;
         cstart = col_start(in_zp, ci);
         row = cm.table + ci * cm.words;
       }
@@ -322,28 +358,23 @@ nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, co
         if (col_ok && iz >= 0 && iz < g.D) {
           if ((iz >> 5) != cur_w) {
             cur_w = iz >> 5;
-            e = cm.table ? __ldg(row + cur_w) : make_uint2(~0u, kUnsorted);
+            e = __ldg(row + cur_w);
+            order |= e.y;
+            e.y &= ~kUnsorted;
           }
           const uint32_t bit = 1u << (iz & 31);
-          if (e.x & bit) {
-            if (e.y & kUnsorted) {
-              const int end = __ldg(in_zp + ci);
-              for (int q = cstart; q < end && found < 0; ++q)
-                if (__ldg(in_zi + q) == iz) found = q;
-            } else {
-              found = cstart + (int)e.y + __popc(e.x & (bit - 1u));
-            }
-          }
+          if (e.x & bit) found = cstart + (int)e.y + __popc(e.x & (bit - 1u));
         }
         *dst = found;
         dst += out_nnz;
         if (HAS_T) {
-          if (found >= 0) dst_t[found] = (int)r;
+          if (found >= 0 && !(order & kUnsorted)) dst_t[found] = (int)r;
           dst_t += in_nnz;
         }
       }
     }
   }
+  if (order & kUnsorted) search_row(in_zi, in_zp, __ldg(out_zi + r), g, in_nnz, out_nnz, r, c, nbr, HAS_T ? nbr_t : nullptr);
 }
 
 constexpr int kListWarps = 8;
@@ -997,7 +1028,9 @@ int launch_emit(const int* in_zi, const int* in_zp, const int* out_zi, const int
     const unsigned grid = (unsigned)div_up64(out_nnz, 256);
 #define SPH_NBR_ROWS(KD, T) \
   nbr_rows_kernel<KD, T><<<grid, 256, 0, st>>>(in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, cm, status)
-    if (g.KD == 3 && g.KW == 3) {
+    if (cm.table == nullptr) {
+      nbr_search_kernel<<<grid, 256, 0, st>>>(in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, status);
+    } else if (g.KD == 3 && g.KW == 3) {
       if (nbr_t) SPH_NBR_ROWS(3, true); else SPH_NBR_ROWS(3, false);
     } else {
       if (nbr_t) SPH_NBR_ROWS(0, true); else SPH_NBR_ROWS(0, false);

@@ -64,6 +64,25 @@ def test_two_windows_and_groups(kv, jump):
     _check(x, w, torch.as_tensor(nbr.astype(np.int32), device=DEV))
 
 
+@pytest.mark.parametrize("K,N", [(16, 16), (4, 16), (37, 11), (64, 24), (45, 51), (33, 64), (32, 64)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n_out,spread,kv", [(1, 1, 27), (257, 40, 27), (1500, 100000, 10), (3000, 30, 45)])
+def test_weight_gradient_tables(K, N, dtype, n_out, spread, kv):
+    """The pairs' weight gradient on the same kinds of table; one offset has every row, as the centre of a layer does."""
+    rng = np.random.default_rng(K + N)
+    n_in = n_out + spread
+    nbr = np.arange(n_out)[None, :] + rng.integers(0, spread + 1, (kv, n_out))
+    nbr[rng.random((kv, n_out)) < 0.8] = -1
+    nbr[kv // 2] = np.arange(n_out)
+    t = torch.as_tensor(nbr.astype(np.int32), device=DEV)
+    x, _ = _operands(rng, n_in, 1, K, N, dtype)
+    g, _ = _operands(rng, n_out, 1, N, K, dtype)
+    dw = C.host().conv_wgrad(x, g, t, None, False)
+    want = torch.stack([x.double()[t[k][t[k] >= 0].long()].T @ g.double()[t[k] >= 0] for k in range(kv)])
+    assert float((dw.double() - want).abs().max()) <= 1e-4 * max(1.0, float(want.abs().max()))
+    assert check_status() == 0
+
+
 def test_entries_that_are_no_rows():
     rng = np.random.default_rng(3)
     x, w = _operands(rng, 300, 27, 16, 16, torch.float16)
