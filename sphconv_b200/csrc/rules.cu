@@ -276,7 +276,7 @@ emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
 // ---------------------------------------------------------------------------------------------
 // The table entries of output row r by searching the input columns row by row: for columns out of depth order and grids
 // without the index.  Not inlined: the registers of the path that every row takes are worth more.
-__device__ __noinline__ void search_row(const int* __restrict__ in_zi, const int* __restrict__ in_zp, int oz, const Geom& g,
+__device__ __noinline__ void search_row(const int* __restrict__ in_zi, const int* __restrict__ in_zp, int oz, Geom g,
                                         int64_t in_nnz, int64_t out_nnz, int64_t r, int c, int* nbr, int* nbr_t) {
   const int oy = c % g.oW, ox = c / g.oW % g.oH, b = c / g.oW / g.oH;
   for (int k = 0; k < g.KV; ++k) {
@@ -307,7 +307,7 @@ __device__ __forceinline__ int parked_column(const Geom& g, int64_t out_nnz, int
 
 __global__ void __launch_bounds__(256)
 nbr_search_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
-                  const __grid_constant__ Geom g,
+                  Geom g,
                   int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, int* __restrict__ status) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= out_nnz) return;
@@ -316,10 +316,11 @@ nbr_search_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, 
 }
 
 // KD_CT = 3: the filter is 3 wide and 3 deep (those two loops are unrolled), 0 = extents read from the geometry.
+// Six blocks an SM (40 registers): the call of search_row, which no ordinary row makes, must not cost the others theirs.
 template <int KD_CT, bool HAS_T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 6)
 nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
-                const __grid_constant__ Geom g,
+                Geom g,
                 int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, ColMask cm,
                 int* __restrict__ status) {
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -445,7 +446,7 @@ rule_lists_fixed_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz,
   int* off = s_off[wib];
   const int* plane0 = nbr + (int64_t)k_lo * out_nnz;
   int* lst0 = rules ? rules + ((int64_t)t * g.KV + k_lo) * 2 * tile_n_max : nullptr;
-  const int64_t lst_stride = 2 * (int64_t)tile_n_max;
+  const unsigned lst_stride = 2u * (unsigned)tile_n_max;      // a tile's lists: KV x 2 x capacity < 2^32 (the launcher checks)
   int base[NK];
 #pragma unroll
   for (int j = 0; j < NK; ++j) base[j] = 0;
@@ -482,18 +483,24 @@ rule_lists_fixed_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz,
       if (more) fetch(p0 + 32 * CH, nrow, nv);
 #pragma unroll
       for (int j = 0; j < NK; ++j) {
-        int* lst = lst0 + j * lst_stride;
 #pragma unroll
         for (int u = 0; u < CH; ++u) {
           const unsigned m = __ballot_sync(0xffffffffu, v[u][j] >= 0);
           if (m == 0u) continue;
-          if (v[u][j] >= 0 && lst0) {
-            const int slot = base[j] + __popc(m & lt);
-            if (slot < tile_n_max) {
-              lst[slot] = v[u][j];
-              lst[tile_n_max + slot] = row[u];
-            } else {
-              overflow = true;
+          if (lst0) {
+            const unsigned slot = base[j] + __popc(m & lt), at = j * lst_stride + slot;
+            if (base[j] + 32 <= tile_n_max) {             // uniform: no slot of this step is beyond the list
+              if (v[u][j] >= 0) {
+                lst0[at] = v[u][j];
+                lst0[at + tile_n_max] = row[u];
+              }
+            } else if (v[u][j] >= 0) {
+              if (slot < (unsigned)tile_n_max) {
+                lst0[at] = v[u][j];
+                lst0[at + tile_n_max] = row[u];
+              } else {
+                overflow = true;
+              }
             }
           }
           base[j] += __popc(m);
@@ -970,7 +977,7 @@ int* parked_columns(const Geom& g, int* nbr, int64_t out_nnz) {
 // Pair lists of every (tile, offset) from a finished neighbour table.
 int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm, const int* nbr, int* rules,
                       int* rule_size, int* status, cudaStream_t st) {
-  if (g.KV == 27) {
+  if (g.KV == 27 && (int64_t)tnm * 54 < (1LL << 32)) {
     // the usual 3 x 3 x 3 filter: the kernel with the offsets' running counts in registers
     // nine offsets per warp where that gives the machine enough warps, else three (small tile grids have long tiles:
     // more warps per tile also evens out their lengths).  Measured beside the convolution kernels: one chunk of 32
