@@ -162,8 +162,14 @@ class Conv3d(Convolution):
             mb = getattr(bias, "_sph_master_grad", None) if bias is not None else None
             master = None if mw is None and mb is None else \
                 (None if mw is None else mw.view(-1, in_channels, out_channels), mb)
-            out_feature = ConvFunction.apply(feature, w, rules, rule_size, tile_grid_shape,
-                                             oz_idx.shape[0], bias, self.activation == 'relu', master)
+            n_out = oz_idx.shape[0]
+            relu = self.activation == 'relu'
+            tables = None if master is not None or profiling.is_active() or profiling.pair_counts is not None else \
+                ops._tables_for(rules, rule_size, feature.shape[0], n_out, need_t=False)
+            if tables is not None and (tables.nbr_t is not None or tables.symmetric):
+                out_feature = ops.conv_layer(feature, w, bias, rules, tables, n_out, relu)
+            else:    # gradients into a caller's buffer, sections to time, or a transposed table still to be made
+                out_feature = ConvFunction.apply(feature, w, rules, rule_size, tile_grid_shape, n_out, bias, relu, master)
         else:
             w, b = self._inference_weights(feature.dtype, bias)
             if profiling.is_active() or profiling.pair_counts is not None:

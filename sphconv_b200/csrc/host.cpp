@@ -358,8 +358,7 @@ Tensor conv_wgrad(const Tensor& feature, const Tensor& d_out, const Tensor& nbr,
   return dw;
 }
 
-// -> (d_pre or None, d_bias or None)
-py::tuple epilogue_backward(const Tensor& d_out, const optional<Tensor>& out, bool relu, bool need_bias) {
+std::pair<Tensor, Tensor> epilogue_grads(const Tensor& d_out, const optional<Tensor>& out, bool relu, bool need_bias) {
   require_cuda(d_out);
   require_cuda(out);
   const int64_t n = d_out.size(0), ch = d_out.size(1);
@@ -372,7 +371,56 @@ py::tuple epilogue_backward(const Tensor& d_out, const optional<Tensor>& out, bo
     check(abi.sph_epilogue_backward(ptr(d_out), relu ? ptr(out) : nullptr, dtype_code(d_out, "gradient"), n, (int32_t)ch, relu,
                                     relu ? ptr(d_pre) : nullptr, need_bias ? static_cast<float*>(ptr(d_bias)) : nullptr,
                                     stream_of(d_out)));
-  return py::make_tuple(or_none(d_pre), or_none(d_bias));
+  return {d_pre, d_bias};
+}
+
+// -> (d_pre or None, d_bias or None)
+py::tuple epilogue_backward(const Tensor& d_out, const optional<Tensor>& out, bool relu, bool need_bias) {
+  const auto r = epilogue_grads(d_out, out, relu, need_bias);
+  return py::make_tuple(or_none(r.first), or_none(r.second));
+}
+
+// The differentiable layer: relu(conv + bias) with its gradients, as sphconv_b200.functional.ConvFunction computes them (the
+// reference's sphconv/functional.py:12-78), without a trip through Python in either direction.
+struct ConvLayer : public torch::autograd::Function<ConvLayer> {
+  static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& feature, const Tensor& weight,
+                        const optional<Tensor>& bias, const Tensor& nbr, const optional<Tensor>& nbr_t, int64_t n_out, bool relu) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    optional<Tensor> b;
+    if (bias) b = bias->detach().to(at::kFloat);
+    Tensor out = conv_gather(feature, weight, pack_weight(weight), nbr, n_out, false, std::nullopt, b, relu, std::nullopt);
+    ctx->save_for_backward({feature, weight, relu ? out : Tensor(), nbr, nbr_t.value_or(Tensor())});
+    ctx->saved_data["relu"] = relu;
+    ctx->saved_data["bias"] = bias ? (int64_t)bias->scalar_type() : (int64_t)-1;
+    return out;
+  }
+
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext* ctx, torch::autograd::variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &feature = saved[0], &weight = saved[1], &out = saved[2], &nbr = saved[3], &nbr_t = saved[4];
+    const bool relu = ctx->saved_data["relu"].toBool();
+    const int64_t bias_type = ctx->saved_data["bias"].toInt();
+    Tensor d_out = grads[0].contiguous(), d_feature, d_weight, d_bias;
+    const c10::cuda::CUDAGuard guard(d_out.device());
+    if (relu || bias_type >= 0) {        // gradient mask and bias gradient in one pass over the rows
+      auto r = epilogue_grads(d_out, relu ? optional<Tensor>(out) : std::nullopt, relu, bias_type >= 0);
+      if (relu) d_out = r.first;
+      if (bias_type >= 0) d_bias = r.second.to((at::ScalarType)bias_type);
+    }
+    if (ctx->needs_input_grad(0)) {
+      // the transposed table, or - (i,o) at k is (o,i) at KV-1-k in an odd-kernel submanifold layer - the forward one, flipped
+      const Tensor wt = weight.transpose(1, 2).contiguous();
+      d_feature = conv_gather(d_out, wt, pack_weight(wt), nbr_t.defined() ? nbr_t : nbr, feature.size(0), !nbr_t.defined(),
+                              std::nullopt, std::nullopt, false, std::nullopt);
+    }
+    if (ctx->needs_input_grad(1)) d_weight = conv_wgrad(feature, d_out, nbr, std::nullopt, false).to(feature.scalar_type());
+    return {d_feature, d_weight, d_bias, Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor conv_layer(const Tensor& feature, const Tensor& weight, const optional<Tensor>& bias, const Tensor& nbr,
+                  const optional<Tensor>& nbr_t, int64_t n_out, bool relu) {
+  return ConvLayer::apply(feature, weight, bias, nbr, nbr_t, n_out, relu);
 }
 
 // ---- tensor operations ---------------------------------------------------------------------------------------------
@@ -508,6 +556,7 @@ PYBIND11_MODULE(sph_host, m) {
   m.def("conv_gather", &conv_gather);
   m.def("conv_wgrad", &conv_wgrad);
   m.def("epilogue_backward", &epilogue_backward);
+  m.def("conv_layer", &conv_layer);
   m.def("init_tensor", &init_tensor);
   m.def("gather_rows", &gather_rows);
   m.def("dense_channels_first", &dense_channels_first);

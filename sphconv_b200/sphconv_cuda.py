@@ -216,6 +216,14 @@ def rule_conv_backward(d_featureOut: torch.Tensor, feature: torch.Tensor, weight
     return [d_feature, d_weight]
 
 
+def conv_layer(feature, weight, bias, rules, tables, n_out, relu):
+    """relu(conv + bias) as one differentiable native call (extension): what functional.ConvFunction does, for a rule set
+    whose tables serve both directions."""
+    out = C.host().conv_layer(feature, weight, bias, tables.nbr, None if tables.symmetric else tables.nbr_t, n_out, relu)
+    _join_lists(rules)
+    return out
+
+
 # ---- tensor ops on either side of the path: COO -> range-voxel, range-voxel <-> dense -----------------------
 
 def init_tensor(feature: torch.Tensor, indicesBZYX: torch.Tensor, batchSize: int, spatialShape: List[int]):
