@@ -152,3 +152,19 @@ def test_against_the_reference_module():
         np.testing.assert_array_equal(r["coordinates"].cpu().numpy()[:, 1:], coors[:nv][order])
         np.testing.assert_array_equal(r["num_points_per_voxel"].cpu().numpy(), num[:nv][order])
         np.testing.assert_array_equal(r["feature"].cpu().numpy(), mean[order])
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 4099])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_four_float_points_at_any_alignment(n, offset):
+    """Points on a 16-byte boundary take one load each, others four: the rows are the same."""
+    rng = np.random.default_rng(n)
+    pts, scan_ptr = _scans(rng, [n], degenerate=0)
+    gen = VoxelGenerator(CART_RANGE, SPH_RANGE, 2, 24000, [64, 64, 32], "spherical")
+    want = _check(gen, pts, scan_ptr, True)
+    buf = torch.zeros(4 * n + offset, device=DEV)
+    view = buf[offset:].view(n, 4)
+    view.copy_(torch.as_tensor(pts))
+    got = gen.generate(view, torch.as_tensor(scan_ptr))
+    assert torch.equal(got["feature"], want["feature"]) and torch.equal(got["z_idx"], want["z_idx"])
+    assert torch.equal(got["coordinates"], want["coordinates"])
