@@ -151,6 +151,40 @@ struct ListsReady {
   void join() { event.block(at::cuda::getCurrentCUDAStream(event.device_index())); }
 };
 
+// The -1 padding of a rule set's lists, written on the side stream from the moment the lists are allocated: the fill is
+// bound by HBM and the kernels that make the neighbour table by latency, so beside one another they cost little more than
+// the longer of the two (a submanifold and a strided rule set with 207 MB of lists: 132 -> 118 us).  A fill below kBesideBytes takes
+// about as long as the two events it would need and stays on the current stream, in front of the lists.
+class Padding {
+ public:
+  static constexpr int64_t kBesideBytes = 16 << 20;
+  Padding(const Tensor& rules, bool fill) {
+    if (!fill || !rules.defined() || (int64_t)rules.nbytes() < kBesideBytes) return;
+    const int device = rules.device().index();
+    const auto side = side_stream(device);
+    at::cuda::CUDAEvent allocated;
+    allocated.record(at::cuda::getCurrentCUDAStream(device));
+    allocated.block(side);
+    C10_CUDA_CHECK(cudaMemsetAsync(rules.data_ptr(), 0xFF, rules.nbytes(), side));
+    done_.record(side);
+    device_ = device;
+  }
+  Padding(const Padding&) = delete;
+  ~Padding() {                  // an error on the way: the lists are freed on the current stream, behind the fill
+    if (begun()) try { join(); } catch (...) {}
+  }
+  bool begun() const { return device_ >= 0; }
+  void join() {                 // the current stream continues behind the fill
+    done_.block(at::cuda::getCurrentCUDAStream(device_));
+    device_ = -1;
+  }
+  void leave() { device_ = -1; }   // the lists are written on the side stream too
+
+ private:
+  at::cuda::CUDAEvent done_;
+  int device_ = -1;
+};
+
 // The lists of a rule set whose table has been enqueued on the current stream, on the side stream.
 std::shared_ptr<ListsReady> lists_beside(const sph_geom& g, const Tensor& oz_ptr, const Tensor& nbr, int32_t tnm,
                                          const Tensor& rules, const Tensor& rule_size, bool fill) {
@@ -193,16 +227,24 @@ py::tuple rules_subm(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, const 
   const sph_geom g = geometry(B, in, out, k, s, p, d, tile);
   const int64_t nnz = z_idx.size(0), kv = k[0] * k[1] * k[2];
   Lists l = make_lists(g, nnz, z_idx, materialize);
+  Padding padding(l.rules, fill && nnz > 0);
   defer = defer && materialize && nnz > 0;
   Tensor nbr = empty({kv, nnz}, at::kInt, z_idx);
   const int64_t bytes = check(abi.sph_rules_subm_scratch_bytes(&g, nnz));
   Tensor scratch = bytes ? empty({bytes}, at::kByte, z_idx) : Tensor();
-  const bool here = materialize && !defer;
+  const bool here = materialize && !defer && !padding.begun();
   check(abi.sph_rules_subm(ints(z_idx), ints(z_ptr), nnz, &g, bytes ? ptr(scratch) : nullptr, l.tnm,
                            here ? ints(l.rules) : nullptr, here ? ints(l.rule_size) : nullptr, ints(nbr), fill,
                            status_of(z_idx), stream_of(z_idx)));
   std::shared_ptr<ListsReady> ready;
-  if (defer) ready = lists_beside(g, z_ptr, nbr, l.tnm, l.rules, l.rule_size, fill);
+  if (defer) {
+    ready = lists_beside(g, z_ptr, nbr, l.tnm, l.rules, l.rule_size, fill && !padding.begun());
+    padding.leave();
+  } else if (padding.begun()) {
+    padding.join();
+    check(abi.sph_rule_lists(ints(z_ptr), &g, nnz, ints(nbr), l.tnm, ints(l.rules), ints(l.rule_size), false, status_of(nbr),
+                             stream_of(nbr)));
+  }
   return py::make_tuple(or_none(l.rules), or_none(l.rule_size), nbr, or_none(ready));
 }
 
@@ -246,6 +288,7 @@ py::tuple strided_rules(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, con
   const int64_t nnz = z_idx.size(0), kv = k[0] * k[1] * k[2];
   // everything that does not need the row count is made before the wait for it
   Lists l = make_lists(g, nnz, z_idx, materialize);
+  Padding padding(l.rules, fill);
   Tensor nbr_t = transposed ? empty({kv, nnz}, at::kInt, z_idx) : Tensor();
   {
     py::gil_scoped_release release;
@@ -255,12 +298,19 @@ py::tuple strided_rules(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, con
   defer = defer && materialize && n_out > 0;
   Tensor oz_idx = empty({n_out}, at::kInt, z_idx);
   Tensor nbr = empty({kv, n_out}, at::kInt, z_idx);
-  const bool here = materialize && !defer;
+  const bool here = materialize && !defer && !padding.begun();
   check(abi.sph_rules_strided_fill(ints(z_idx), ints(z_ptr), nnz, &g, ptr(pending->scratch), ints(pending->oz_ptr), n_out,
                                    l.tnm, ints(oz_idx), here ? ints(l.rules) : nullptr, here ? ints(l.rule_size) : nullptr,
                                    ints(nbr), transposed ? ints(nbr_t) : nullptr, fill, status_of(z_idx), stream_of(z_idx)));
   std::shared_ptr<ListsReady> ready;
-  if (defer) ready = lists_beside(g, pending->oz_ptr, nbr, l.tnm, l.rules, l.rule_size, fill);
+  if (defer) {
+    ready = lists_beside(g, pending->oz_ptr, nbr, l.tnm, l.rules, l.rule_size, fill && !padding.begun());
+    padding.leave();
+  } else if (padding.begun()) {
+    padding.join();
+    check(abi.sph_rule_lists(ints(pending->oz_ptr), &g, n_out, ints(nbr), l.tnm, ints(l.rules), ints(l.rule_size), false,
+                             status_of(nbr), stream_of(nbr)));
+  }
   return py::make_tuple(oz_idx, pending->oz_ptr, or_none(l.rules), or_none(l.rule_size), nbr, or_none(nbr_t), or_none(ready));
 }
 

@@ -437,7 +437,7 @@ epilogue_backward_kernel(const T* __restrict__ d_out, const T* __restrict__ out,
 
 // The same with 16-byte loads and stores (channels a multiple of the V elements of one): a thread owns one vector of
 // channels, keeps V sums and has kVecRows rows in flight.  Bound by memory: 1.39 M rows of 64 bf16 channels (534 MB)
-// 194 -> %s us.
+// 194 -> 84 us.
 constexpr int kVecRows = 4;
 
 template <typename T>
