@@ -32,8 +32,6 @@ __device__ __forceinline__ void store_one(void* out, int out_dtype, int64_t idx,
 
 constexpr int kRows = 128;            // output rows of a tile
 constexpr int kItem = 64;             // pairs of a step
-constexpr int kKC = 32;               // input channels of a step
-constexpr int kAStride = kKC + 4;     // floats; consecutive rows start 4 banks apart: 16-byte reads of 8 rows do not conflict
 constexpr int kBatch = 9;             // kernel offsets whose pair lists are held at a time
 
 struct FfmaParams {
@@ -48,29 +46,31 @@ struct FfmaParams {
   int* status;
 };
 
-template <int CG> struct FfmaShape {
+// KC: input channels of a step, 32 (layers of at most 8 or 16 input channels: 8 or 16).
+template <int CG, int KC> struct FfmaShape {
   static constexpr int NP = CG * 8;                  // output channels of a CTA, padded
   static constexpr int T = CG == 8 ? 128 : 64;       // threads of a CTA
   static constexpr int RL = T / CG;                  // row lanes
   static constexpr int RP = kItem / RL;              // rows per thread at most
   static constexpr int ACC = kRows * (NP + 4);       // floats
-  static constexpr int A = kItem * kAStride;
-  static constexpr int W = kKC * NP;
+  static constexpr int AS = KC + 4;                  // floats of a staged row: 16-byte reads of 8 rows do not conflict
+  static constexpr int A = kItem * AS;
+  static constexpr int W = KC * NP;
   static constexpr int BYTES = (ACC + 2 * A + 2 * W) * 4 + kBatch * kRows * 5 + kBatch * 4;
 };
 
-// One step (offset, 32 input channels) of RP rows x 8 output channels per thread.  The two 4-channel groups of a thread are
+// One step (offset, KC input channels) of RP rows x 8 output channels per thread.  The two 4-channel groups of a thread are
 // NP/2 apart, so the lanes of a row read consecutive 16-byte pieces of the filter row.
-template <int CG, int RP>
-__device__ __forceinline__ void ffma_step(const float* __restrict__ a, const float* __restrict__ w, int rl, int cg,
-                                          float (&acc)[FfmaShape<CG>::RP][8]) {
-  using S = FfmaShape<CG>;
+template <int CG, int KC, int RP>
+__device__ __forceinline__ void ffma_step(const float* __restrict__ a, const float* __restrict__ w, int kn, int rl, int cg,
+                                          float (&acc)[FfmaShape<CG, KC>::RP][8]) {
+  using S = FfmaShape<CG, KC>;
 #pragma unroll 2
-  for (int k4 = 0; k4 < kKC; k4 += 4) {
+  for (int k4 = 0; k4 < kn; k4 += 4) {
     float av[RP][4];
 #pragma unroll
     for (int j = 0; j < RP; ++j) {
-      const float4 t = *(const float4*)(a + (rl + j * S::RL) * kAStride + k4);
+      const float4 t = *(const float4*)(a + (rl + j * S::RL) * S::AS + k4);
       av[j][0] = t.x; av[j][1] = t.y; av[j][2] = t.z; av[j][3] = t.w;
     }
 #pragma unroll
@@ -89,7 +89,7 @@ __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const flo
 }
 
 // A CTA owns 128 consecutive output rows x up to 64 output channels.  Per offset k the rows of the tile that have a
-// neighbour are compacted into a list; up to 64 of their input rows and W[k] are staged (32 input channels a step, the next
+// neighbour are compacted into a list; up to 64 of their input rows and W[k] are staged (KC input channels a step, the next
 // step's copies in flight), every thread multiplies ceil(pairs / row lanes) listed rows by 8 channels in registers, on top
 // of the tile's fp32 accumulator in shared memory.  An output row occurs once per offset, so no two threads of a step hold the
 // same accumulator.
@@ -100,13 +100,13 @@ __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const flo
 // replaced (one thread group per row walking every slot of the table).
 // VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by
 // element.
-template <typename T, int CG, bool VEC>
-__global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams p) {
-  using S = FfmaShape<CG>;
+template <typename T, int CG, int KC, bool VEC>
+__global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaParams p) {
+  using S = FfmaShape<CG, KC>;
   extern __shared__ __align__(16) unsigned char smem[];
   float* s_acc = (float*)smem;                       // [kRows][NP + 4]
-  float* s_a = s_acc + S::ACC;                       // [2][kItem][kAStride]
-  float* s_w = s_a + 2 * S::A;                       // [2][kKC][NP]
+  float* s_a = s_acc + S::ACC;                       // [2][kItem][S::AS]
+  float* s_w = s_a + 2 * S::A;                       // [2][KC][NP]
   int* s_in = (int*)(s_w + 2 * S::W);                // [kBatch][kRows] input row
   int* s_m = s_in + kBatch * kRows;                  // [kBatch] pairs
   unsigned char* s_out = (unsigned char*)(s_m + kBatch);   // [kBatch][kRows] row in the tile
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams 
   const int rl = tid / CG, cg = tid % CG;
   const T* rows = (const T*)p.rows;
   const T* weight = (const T*)p.weight;
-  const int k_chunks = (p.K + kKC - 1) / kKC;
+  const int k_chunks = (p.K + KC - 1) / KC;
 
   for (int e = tid; e < S::ACC; e += S::T) s_acc[e] = 0.f;
 
@@ -126,28 +126,28 @@ __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams 
     const int* in = s_in + kk * kRows + p0;
     float* a = s_a + buf * S::A;
     float* w = s_w + buf * S::W;
-    const T* wk = weight + ((int64_t)(kb + kk) * p.K + kc * kKC) * p.N + n0;
-    const int kn = min(kKC, p.K - kc * kKC);
+    const T* wk = weight + ((int64_t)(kb + kk) * p.K + kc * KC) * p.N + n0;
+    const int kn = min(KC, p.K - kc * KC);
     if constexpr (VEC) {
-      const int c = tid % (kKC / 4) * 4;
+      const int c = tid % (KC / 4) * 4;
       const bool ok = c < kn;
-      for (int r = tid / (kKC / 4); r < m; r += S::T / (kKC / 4)) {
-        cp_async_16(smem_u32(a + r * kAStride + c), ok ? rows + (int64_t)in[r] * p.K + kc * kKC + c : rows, ok ? 16u : 0u);
+      for (int r = tid / (KC / 4); r < m; r += S::T / (KC / 4)) {
+        cp_async_16(smem_u32(a + r * S::AS + c), ok ? rows + (int64_t)in[r] * p.K + kc * KC + c : rows, ok ? 16u : 0u);
       }
       const int wc = tid % (S::NP / 4) * 4;
       const T* src = wk + (int64_t)(tid / (S::NP / 4)) * p.N + wc;
 #pragma unroll 4
-      for (int r = tid / (S::NP / 4); r < kKC; r += S::T / (S::NP / 4)) {
+      for (int r = tid / (S::NP / 4); r < KC; r += S::T / (S::NP / 4)) {
         const bool ok = r < kn && wc < nc;
         cp_async_16(smem_u32(w + r * S::NP + wc), ok ? src : weight, ok ? 16u : 0u);
         src += (S::T / (S::NP / 4)) * p.N;
       }
     } else {
-      for (int e = tid; e < m * kKC; e += S::T) {
-        const int r = e / kKC, c = e % kKC;
-        stage_one(a + r * kAStride + c, c < kn ? rows + (int64_t)in[r] * p.K + kc * kKC + c : rows, c < kn);
+      for (int e = tid; e < m * KC; e += S::T) {
+        const int r = e / KC, c = e % KC;
+        stage_one(a + r * S::AS + c, c < kn ? rows + (int64_t)in[r] * p.K + kc * KC + c : rows, c < kn);
       }
-      for (int e = tid; e < kKC * S::NP; e += S::T) {
+      for (int e = tid; e < KC * S::NP; e += S::T) {
         const int r = e / S::NP, c = e % S::NP;
         const bool ok = r < kn && c < nc;
         stage_one(w + e, ok ? wk + (int64_t)r * p.N + c : weight, ok);
@@ -158,27 +158,39 @@ __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams 
   for (int kb = 0; kb < p.kv; kb += kBatch) {
     const int nk = min(kBatch, p.kv - kb);
     __syncthreads();                                  // the previous batch's lists are done with
-    for (int kk = warp; kk < nk; kk += S::T / 32) {
-      const int* col = p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - (kb + kk) : kb + kk) * p.n_out + r0;
-      int v[kRows / 32];
+    // kCols columns of the table at a time, all their loads in flight
+    constexpr int kCols = 3;
+    for (int k0 = warp; k0 < nk; k0 += kCols * (S::T / 32)) {
+      int v[kCols][kRows / 32];
 #pragma unroll
-      for (int h = 0; h < kRows / 32; ++h) v[h] = r0 + h * 32 + lane < p.n_out ? __ldg(col + h * 32 + lane) : -1;
-      int n = 0;
+      for (int c = 0; c < kCols; ++c) {
+        const int kk = k0 + c * (S::T / 32);
+        const int* col = p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - (kb + kk) : kb + kk) * p.n_out + r0;
 #pragma unroll
-      for (int h = 0; h < kRows / 32; ++h) {
-        if (v[h] >= p.n_rows) {
-          if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
-          v[h] = -1;
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, v[h] >= 0);
-        if (v[h] >= 0) {
-          const int pos = n + __popc(m & ((1u << lane) - 1u));
-          s_in[kk * kRows + pos] = v[h];
-          s_out[kk * kRows + pos] = (unsigned char)(h * 32 + lane);
-        }
-        n += __popc(m);
+        for (int h = 0; h < kRows / 32; ++h)
+          v[c][h] = kk < nk && r0 + h * 32 + lane < p.n_out ? __ldg(col + h * 32 + lane) : -1;
       }
-      if (lane == 0) s_m[kk] = n;
+#pragma unroll
+      for (int c = 0; c < kCols; ++c) {
+        const int kk = k0 + c * (S::T / 32);
+        if (kk >= nk) break;
+        int n = 0;
+#pragma unroll
+        for (int h = 0; h < kRows / 32; ++h) {
+          if (v[c][h] >= p.n_rows) {
+            if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
+            v[c][h] = -1;
+          }
+          const unsigned m = __ballot_sync(0xffffffffu, v[c][h] >= 0);
+          if (v[c][h] >= 0) {
+            const int pos = n + __popc(m & ((1u << lane) - 1u));
+            s_in[kk * kRows + pos] = v[c][h];
+            s_out[kk * kRows + pos] = (unsigned char)(h * 32 + lane);
+          }
+          n += __popc(m);
+        }
+        if (lane == 0) s_m[kk] = n;
+      }
     }
     __syncthreads();
     int kk = 0, p0 = 0, kc = 0;
@@ -219,11 +231,13 @@ __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams 
       const float* w = s_w + buf * S::W;
       // rows beyond m are staged rows of an earlier step: multiplied, never added
       const int rp = (m + S::RL - 1) / S::RL;
+      // what is staged beyond K is zero; a bound the compiler knows costs full steps nothing (32 -> 64: 240 against 249 us)
+      const int kn = VEC ? KC : (min(KC, p.K - kc * KC) + 7) & ~7;
       switch (rp) {
-        case 1: ffma_step<CG, 1>(a, w, rl, cg, acc); break;
-        case 2: ffma_step<CG, (S::RP < 2 ? 1 : 2)>(a, w, rl, cg, acc); break;
-        case 3: ffma_step<CG, (S::RP < 3 ? 1 : 3)>(a, w, rl, cg, acc); break;
-        default: ffma_step<CG, (S::RP < 4 ? 1 : 4)>(a, w, rl, cg, acc);
+        case 1: ffma_step<CG, KC, 1>(a, w, kn, rl, cg, acc); break;
+        case 2: ffma_step<CG, KC, (S::RP < 2 ? 1 : 2)>(a, w, kn, rl, cg, acc); break;
+        case 3: ffma_step<CG, KC, (S::RP < 3 ? 1 : 3)>(a, w, kn, rl, cg, acc); break;
+        default: ffma_step<CG, KC, (S::RP < 4 ? 1 : 4)>(a, w, kn, rl, cg, acc);
       }
       if (kc == k_chunks - 1) {
 #pragma unroll
@@ -250,13 +264,12 @@ __global__ void __launch_bounds__(FfmaShape<CG>::T) conv_ffma_kernel(FfmaParams 
 }
 
 // ---- weight gradient: dW[k] += X_i^T dY_o over the pairs of offset k ------------------------------------------------
-// grid (row slices, KV).  A CTA compacts the pairs of its slice, then stages kWgPairs of them at a time (the next ones'
+// grid (row slices, KV).  A CTA compacts the pairs of its slice, then stages PAIRS of them at a time (the next ones'
 // copies in flight); a thread owns 8 input x 8 output channels of the product, the threads are as many copies of the
 // K x N tile as fit, and each copy takes its share of the staged pairs.  The copies are summed in shared memory and added
 // to the gradient once per CTA.
 constexpr int kThreads = 256;
 constexpr int kWgSlice = 2048;
-constexpr int kWgPairs = 32;
 constexpr int kWgMaxCh = 64;
 
 struct FfmaWgradParams {
@@ -273,16 +286,35 @@ struct FfmaWgradParams {
 template <int KG, int NG> struct WgShape {
   static constexpr int XS = KG * 8 + 4, DS = NG * 8 + 4;     // staged row strides in floats
   static constexpr int COPIES = kThreads / (KG * NG);
-  static constexpr int STAGE = kWgPairs * (XS + DS);         // floats
+  static constexpr int PAIRS = COPIES > 32 ? COPIES : 32;    // staged at a time: one for every copy at least
+  static constexpr int STAGE = PAIRS * (XS + DS);            // floats
   static constexpr int RED = KG * NG * 64;                   // floats of the product
   static constexpr int BYTES = (2 * STAGE > RED ? 2 * STAGE : RED) * 4 + kWgSlice * 8 + 64;
 };
+
+// Sums LEFT products a lane over the lanes that differ in the bits O, 2 O .. 16, each exchange halving what a lane holds (it
+// keeps the half its bit names).  Returns the first product that v[0] now stands for.  A serial pass over 256 copies of a
+// 5 x 5 layer took longer than its products (78 k rows of 1.5 neighbours: 377 -> 19 us; 64 -> 7: 165 -> 74 us).
+template <int O, int LEFT>
+__device__ __forceinline__ int fold_copies(float (&v)[64], int lane) {
+  if constexpr (O < 32) {
+    const bool up = (lane & O) != 0;
+#pragma unroll
+    for (int j = 0; j < LEFT / 2; ++j) {
+      const float got = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + LEFT / 2], O);
+      v[j] = (up ? v[j + LEFT / 2] : v[j]) + got;
+    }
+    return (up ? LEFT / 2 : 0) + fold_copies<O * 2, LEFT / 2>(v, lane);
+  } else {
+    return 0;
+  }
+}
 
 template <typename T, int KG, int NG, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradParams p) {
   using S = WgShape<KG, NG>;
   extern __shared__ __align__(16) unsigned char smem[];
-  float* s_st = (float*)smem;                                // [2]{x [kWgPairs][XS], dy [kWgPairs][DS]}, later the sum
+  float* s_st = (float*)smem;                                // [2]{x [PAIRS][XS], dy [PAIRS][DS]}, later the sum
   int* s_in = (int*)(smem + (2 * S::STAGE > S::RED ? 2 * S::STAGE : S::RED) * 4);
   int* s_out = s_in + kWgSlice;
   int* s_cnt = s_out + kWgSlice;                             // [8] hits per warp
@@ -329,26 +361,26 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
 
   auto stage = [&](int buf, int p0) {
     float* x = s_st + buf * S::STAGE;
-    float* d = x + kWgPairs * S::XS;
-    const int np = min(kWgPairs, n - p0);
+    float* d = x + S::PAIRS * S::XS;
+    const int np = min(S::PAIRS, n - p0);
     if constexpr (VEC) {
-      for (int e = tid; e < kWgPairs * KG * 2; e += kThreads) {
+      for (int e = tid; e < S::PAIRS * KG * 2; e += kThreads) {
         const int r = e / (KG * 2), c = (e % (KG * 2)) * 4;
         const bool ok = r < np && c < p.K;
         cp_async_16(smem_u32(x + r * S::XS + c), ok ? rows + (int64_t)s_in[p0 + r] * p.K + c : rows, ok ? 16u : 0u);
       }
-      for (int e = tid; e < kWgPairs * NG * 2; e += kThreads) {
+      for (int e = tid; e < S::PAIRS * NG * 2; e += kThreads) {
         const int r = e / (NG * 2), c = (e % (NG * 2)) * 4;
         const bool ok = r < np && c < p.N;
         cp_async_16(smem_u32(d + r * S::DS + c), ok ? dout + (int64_t)s_out[p0 + r] * p.N + c : dout, ok ? 16u : 0u);
       }
     } else {
-      for (int e = tid; e < kWgPairs * KG * 8; e += kThreads) {
+      for (int e = tid; e < S::PAIRS * KG * 8; e += kThreads) {
         const int r = e / (KG * 8), c = e % (KG * 8);
         const bool ok = r < np && c < p.K;
         stage_one(x + r * S::XS + c, ok ? rows + (int64_t)s_in[p0 + r] * p.K + c : rows, ok);
       }
-      for (int e = tid; e < kWgPairs * NG * 8; e += kThreads) {
+      for (int e = tid; e < S::PAIRS * NG * 8; e += kThreads) {
         const int r = e / (NG * 8), c = e % (NG * 8);
         const bool ok = r < np && c < p.N;
         stage_one(d + r * S::DS + c, ok ? dout + (int64_t)s_out[p0 + r] * p.N + c : dout, ok);
@@ -358,22 +390,20 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
 
   const int copy = tid / (KG * NG), in_copy = tid % (KG * NG);
   const int ig = in_copy / NG, og = in_copy % NG;
-  float acc[8][8];
+  float acc[64];                                             // [8 input][8 output channels]
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  for (int i = 0; i < 64; ++i) acc[i] = 0.f;
   stage(0, 0);
   cp_async_commit();
   int buf = 0;
-  for (int p0 = 0; p0 < n; p0 += kWgPairs, buf ^= 1) {
+  for (int p0 = 0; p0 < n; p0 += S::PAIRS, buf ^= 1) {
     cp_async_wait_pending(0);
     __syncthreads();
-    if (p0 + kWgPairs < n) stage(buf ^ 1, p0 + kWgPairs);
+    if (p0 + S::PAIRS < n) stage(buf ^ 1, p0 + S::PAIRS);
     cp_async_commit();
     const float* x = s_st + buf * S::STAGE + ig * 8;
-    const float* d = s_st + buf * S::STAGE + kWgPairs * S::XS + og * 4;
-    const int np = min(kWgPairs, n - p0);
+    const float* d = s_st + buf * S::STAGE + S::PAIRS * S::XS + og * 4;
+    const int np = min(S::PAIRS, n - p0);
 #pragma unroll 2
     for (int r = copy; r < np; r += S::COPIES) {
       const float4 x0 = *(const float4*)(x + r * S::XS), x1 = *(const float4*)(x + r * S::XS + 4);
@@ -384,21 +414,25 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(xv[i], dv[j], acc[i][j]);
+        for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(xv[i], dv[j], acc[i * 8 + j]);
     }
   }
-  // sum of the copies, one after the other
+  // Sum of the copies: those of a warp in its registers, then the warps' (or the wider copies') one after the other.
+  constexpr int kLanes = KG * NG < 32 ? KG * NG : 32;        // lanes of a warp that hold one copy
+  constexpr int kLeft = 64 * kLanes / 32;                    // products a lane is left with: acc[0 .. kLeft) are first ..
+  const int first = fold_copies<kLanes, 64>(acc, lane);
   float* red = s_st;
-  for (int c = 0; c < S::COPIES; ++c) {
+  constexpr int kSums = KG * NG < 32 ? kThreads / 32 : S::COPIES;
+  const int mine = KG * NG < 32 ? warp : copy;
+  for (int c = 0; c < kSums; ++c) {
     __syncthreads();
-    if (copy == c) {
+    if (mine == c) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          float* t = red + (ig * 8 + i) * (NG * 8) + (j < 4 ? 0 : NG * 4) + og * 4 + (j & 3);
-          *t = c == 0 ? acc[i][j] : *t + acc[i][j];
-        }
+      for (int e = 0; e < kLeft; ++e) {
+        const int i = (first + e) / 8, j = (first + e) % 8;
+        float* t = red + (ig * 8 + i) * (NG * 8) + (j < 4 ? 0 : NG * 4) + og * 4 + (j & 3);
+        *t = c == 0 ? acc[e] : *t + acc[e];
+      }
     }
   }
   __syncthreads();
@@ -406,10 +440,10 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
   for (int e = tid; e < p.K * p.N; e += kThreads) atomicAdd(dw + e, red[(e / p.N) * (NG * 8) + e % p.N]);
 }
 
-template <typename T, int CG, bool VEC>
+template <typename T, int CG, int KC, bool VEC>
 int launch_ffma(const FfmaParams& p, cudaStream_t st) {
-  using S = FfmaShape<CG>;
-  auto kern = conv_ffma_kernel<T, CG, VEC>;
+  using S = FfmaShape<CG, KC>;
+  auto kern = conv_ffma_kernel<T, CG, KC, VEC>;
   SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
   const dim3 grid((unsigned)div_up64(p.n_out, kRows), (unsigned)div_up(p.N, S::NP));
   kern<<<grid, S::T, S::BYTES, st>>>(p);
@@ -417,13 +451,22 @@ int launch_ffma(const FfmaParams& p, cudaStream_t st) {
   return SPH_OK;
 }
 
-template <typename T, bool VEC>
+template <typename T, int KC, bool VEC>
 int launch_ffma_cg(const FfmaParams& p, cudaStream_t st) {
   // the narrowest tile that holds the output channels; beyond 64 of them the grid repeats the rows per 64
-  if (p.N <= 8) return launch_ffma<T, 1, VEC>(p, st);
-  if (p.N <= 16) return launch_ffma<T, 2, VEC>(p, st);
-  if (p.N <= 32) return launch_ffma<T, 4, VEC>(p, st);
-  return launch_ffma<T, 8, VEC>(p, st);
+  if (p.N <= 8) return launch_ffma<T, 1, KC, VEC>(p, st);
+  if (p.N <= 16) return launch_ffma<T, 2, KC, VEC>(p, st);
+  if (p.N <= 32) return launch_ffma<T, 4, KC, VEC>(p, st);
+  return launch_ffma<T, 8, KC, VEC>(p, st);
+}
+
+// Narrow float32 rows take a step as wide as they are: the zeros that would fill it to 32 channels cost as many issue slots
+// as channels do, and the smaller buffers let more CTAs reside (sparse layers are bound by the latency of their steps).  Four buffers instead of two are slower (16 -> 32, 78 k rows: 46 -> 72 us).
+template <bool VEC>
+int launch_ffma_f32(const FfmaParams& p, cudaStream_t st) {
+  if (p.K <= 8) return launch_ffma_cg<float, 8, VEC>(p, st);
+  if (p.K <= 16) return launch_ffma_cg<float, 16, VEC>(p, st);
+  return launch_ffma_cg<float, 32, VEC>(p, st);
 }
 
 template <typename T, int KG, int NG, bool VEC>
@@ -465,10 +508,10 @@ int conv_gather_ffma(const void* rows, int dtype, int64_t n_rows, const void* we
   switch (dtype) {
     case SPH_F32:
       if (K % 4 == 0 && N % 4 == 0 && (((uintptr_t)rows | (uintptr_t)weight) & 15u) == 0)
-        return launch_ffma_cg<float, true>(p, st);
-      return launch_ffma_cg<float, false>(p, st);
-    case SPH_F16: return launch_ffma_cg<__half, false>(p, st);
-    case SPH_BF16: return launch_ffma_cg<__nv_bfloat16, false>(p, st);
+        return launch_ffma_f32<true>(p, st);
+      return launch_ffma_f32<false>(p, st);
+    case SPH_F16: return launch_ffma_cg<__half, 32, false>(p, st);
+    case SPH_BF16: return launch_ffma_cg<__nv_bfloat16, 32, false>(p, st);
   }
   set_error("unknown dtype %d", dtype);
   return SPH_ERR_INVALID;

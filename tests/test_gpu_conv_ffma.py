@@ -27,3 +27,16 @@ def test_forward_and_gradients(iC, oC, dtype, dens, ks):
         dw = ops.rule_conv_d_weight(feat, g, rules, rule_size)
         ref = conv_np.conv_wgrad(f64, g64, pairs, int(np.prod(ks)))
         _close(dw, ref, 1e-4 if dtype == torch.float32 else 1e-3)
+
+
+@pytest.mark.parametrize("iC,oC", [(5, 5), (8, 8), (4, 64), (7, 64), (9, 16), (16, 8), (12, 40), (16, 17), (24, 24)])
+@pytest.mark.parametrize("dens", [1.0, 0.02])
+def test_narrow_float32_rows(iC, oC, dens):
+    """Rows of up to 8 and 16 channels take steps of that width with more of them in flight; small products have up to 256
+    copies whose sum is folded within the warps."""
+    rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(2, [9, 17, 12], True, dens, 3, iC, oC, torch.float32, (3, 3, 3))
+    f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
+    _close(ops.rule_conv(feat, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[torch.float32])
+    g = torch.as_tensor(rng.standard_normal((n_out, oC)), dtype=torch.float32).cuda()
+    dw = ops.rule_conv_d_weight(feat, g, rules, rule_size)
+    _close(dw, conv_np.conv_wgrad(f64, g.double().cpu().numpy(), pairs, 27), 1e-4)
