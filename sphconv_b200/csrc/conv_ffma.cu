@@ -40,6 +40,9 @@ struct FfmaParams {
   const int* nbr;                     // [KV, n_out]
   int64_t n_rows, n_out;
   int kv, K, N, flip_k, relu, out_dtype;
+  int few, few_first;                 // conv_few_kernel's tiles: at most so many pairs, at most so many at the first kBatch
+                                      // offsets; -1: it has none
+  int w_vec;                          // filter rows can be read 4 elements at a time
   const float* scale;
   const float* bias;
   void* out;
@@ -88,6 +91,21 @@ __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const flo
   }
 }
 
+// The calling thread's share of the tile's pairs at offsets k0 and up.  Out of line: few tiles get here, and inlined it costs
+// the kernel registers and 3 % of its time.
+__device__ __noinline__ int pairs_from(int k0, const int* __restrict__ nbr, int kv, int flip_k, int64_t n_out, int64_t n_rows,
+                                       int64_t r0, int threads) {
+  int n = 0;
+  for (int k = k0; k < kv; ++k) {
+    const int* col = nbr + (int64_t)(flip_k ? kv - 1 - k : k) * n_out + r0;
+    for (int r = threadIdx.x; r < kRows; r += threads) {
+      const int v = r0 + r < n_out ? __ldg(col + r) : -1;
+      n += v >= 0 && v < n_rows;
+    }
+  }
+  return n;
+}
+
 // A CTA owns 128 consecutive output rows x up to 64 output channels.  Per offset k the rows of the tile that have a
 // neighbour are compacted into a list; up to 64 of their input rows and W[k] are staged (KC input channels a step, the next
 // step's copies in flight), every thread multiplies ceil(pairs / row lanes) listed rows by 8 channels in registers, on top
@@ -110,6 +128,7 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
   int* s_in = (int*)(s_w + 2 * S::W);                // [kBatch][kRows] input row
   int* s_m = s_in + kBatch * kRows;                  // [kBatch] pairs
   unsigned char* s_out = (unsigned char*)(s_m + kBatch);   // [kBatch][kRows] row in the tile
+  __shared__ int s_rest[S::T / 32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * kRows;
   const int n0 = blockIdx.y * S::NP;                 // first output channel of this CTA
@@ -146,6 +165,14 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
       for (int e = tid; e < m * KC; e += S::T) {
         const int r = e / KC, c = e % KC;
         stage_one(a + r * S::AS + c, c < kn ? rows + (int64_t)in[r] * p.K + kc * KC + c : rows, c < kn);
+      }
+      if (sizeof(T) == 4 && p.w_vec) {
+        for (int e = tid; e < KC * S::NP / 4; e += S::T) {
+          const int r = e / (S::NP / 4), c = e % (S::NP / 4) * 4;
+          const bool ok = r < kn && c < nc;
+          cp_async_16(smem_u32(w + r * S::NP + c), ok ? wk + (int64_t)r * p.N + c : weight, ok ? 16u : 0u);
+        }
+        return;
       }
       for (int e = tid; e < KC * S::NP; e += S::T) {
         const int r = e / S::NP, c = e % S::NP;
@@ -193,6 +220,20 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
       }
     }
     __syncthreads();
+    if (kb == 0 && p.few >= 0) {                      // conv_few_kernel's tile?  By the same two counts, the same for all threads
+      int n = 0;
+      for (int k = 0; k < nk; ++k) n += s_m[k];
+      if (n <= p.few_first) {
+        n = pairs_from(nk, p.nbr, p.kv, p.flip_k, p.n_out, p.n_rows, r0, S::T);
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) s_rest[warp] = n;
+        __syncthreads();
+        n = 0;
+        for (int k = 0; k < nk; ++k) n += s_m[k];
+        for (int w = 0; w < S::T / 32; ++w) n += s_rest[w];
+        if (n <= p.few) return;
+      }
+    }
     int kk = 0, p0 = 0, kc = 0;
     while (kk < nk && s_m[kk] == 0) ++kk;
     if (kk < nk) stage(0, kb, kk, 0, 0);
@@ -260,6 +301,135 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
     if (p.scale) v *= __ldg(p.scale + n0 + c);
     if (p.bias) v += __ldg(p.bias + n0 + c);
     store_one(p.out, p.out_dtype, (r0 + r) * p.N + n0 + c, p.relu ? fmaxf(v, 0.f) : v);
+  }
+}
+
+// ---- tiles with few pairs ------------------------------------------------------------------------------------------
+// A staged step costs its filter slice and a barrier whether it serves 2 pairs or 64, and the tile's buffers leave room for
+// a few hundred threads on an SM.  Below some pairs a row it is faster to have every row walked by threads of its own (4
+// output channels each), straight from global memory: nothing is shared, so the machine is full of independent chains of
+// loads, which is all that bounds them.  The two launches share the tiles: each counts a tile's pairs and takes it or leaves it.
+// Rules and forward of a layer on 78 k rows of 1.5 neighbours, row walks for all tiles -> staged only -> both: 64 -> 64
+// 200 -> 220 -> 155 us, with stride 2 717 -> 537 -> 390; 37 -> 64 fp16 with stride 2 514 -> 623 -> 260.  A training step of the
+// fp32 encoder, whose deeper levels are dense, takes 11.8 ms either way.
+constexpr int kFewThreads = 512;
+constexpr int kFewWords = 11;         // 32 offsets a word
+
+__device__ __forceinline__ float load_f(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float load_f(const __half* p) { return __half2float(__ldg(p)); }
+__device__ __forceinline__ float load_f(const __nv_bfloat16* p) { return __bfloat162float(__ldg(p)); }
+
+__device__ __forceinline__ void load_f4(const float* p, float (&v)[4]) {
+  const float4 t = __ldg((const float4*)p);
+  v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+}
+__device__ __forceinline__ void load_f4(const __half* p, float (&v)[4]) {
+  const uint2 t = __ldg((const uint2*)p);
+  const float2 a = __half22float2(*(const __half2*)&t.x), b = __half22float2(*(const __half2*)&t.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+__device__ __forceinline__ void load_f4(const __nv_bfloat16* p, float (&v)[4]) {
+  const uint2 t = __ldg((const uint2*)p);
+  const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&t.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&t.y);
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
+// acc[0..3] += x[0..K) W[:, 0..3], input channels ascending (the order of ffma_step).  XV / WV: four elements of the input /
+// filter row a load.
+template <typename T, bool XV, bool WV>
+__device__ __forceinline__ void add_pair(const T* __restrict__ x, const T* __restrict__ w, int K, int N, float (&acc)[4]) {
+  int k = 0;
+#pragma unroll 2
+  for (; k + 4 <= K; k += 4) {
+    float xv[4], wv[4][4];
+    if constexpr (XV) load_f4(x + k, xv);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if constexpr (!XV) xv[u] = load_f(x + k + u);
+      if constexpr (WV) {
+        load_f4(w + (k + u) * N, wv[u]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) wv[u][j] = load_f(w + (k + u) * N + j);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[j] = fmaf(xv[u], wv[u][j], acc[j]);
+  }
+#pragma unroll 1
+  for (; k < K; ++k) {
+    const float xv = load_f(x + k);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[j] = fmaf(xv, load_f(w + k * N + j), acc[j]);
+  }
+}
+
+template <typename T, bool XV, bool WV>
+__global__ void __launch_bounds__(kFewThreads, 2) conv_few_kernel(FfmaParams p) {
+  __shared__ unsigned s_present[kFewWords][kRows];   // bit k: the row has a neighbour at offset k
+  __shared__ int s_count[kFewThreads / 32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t r0 = (int64_t)blockIdx.x * kRows;
+  const int words = (p.kv + 31) / 32, first = min(kBatch, p.kv);
+  const int r = tid % kRows;
+  auto entry = [&](int k) {
+    const int v = r0 + r < p.n_out ? __ldg(p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - k : k) * p.n_out + r0 + r) : -1;
+    if (v < p.n_rows) return v;
+    if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
+    return -1;
+  };
+  int n = 0;
+#pragma unroll
+  for (int h = 0; h < (kBatch * kRows + kFewThreads - 1) / kFewThreads; ++h) {
+    const int k = tid / kRows + h * (kFewThreads / kRows);
+    n += k < first && entry(k) >= 0;
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  if (lane == 0) s_count[warp] = n;
+  for (int e = tid; e < words * kRows; e += kFewThreads) s_present[e / kRows][e % kRows] = 0;
+  __syncthreads();
+  n = 0;
+#pragma unroll
+  for (int w = 0; w < kFewThreads / 32; ++w) n += s_count[w];
+  if (n > p.few_first) return;
+  n = 0;
+#pragma unroll 7
+  for (int k = tid / kRows; k < p.kv; k += kFewThreads / kRows) {
+    if (entry(k) >= 0) {
+      atomicOr(&s_present[k / 32][r], 1u << (k & 31));
+      ++n;
+    }
+  }
+  n = __reduce_add_sync(0xffffffffu, n);
+  __syncthreads();                                   // the first count has been read
+  if (lane == 0) s_count[warp] = n;
+  __syncthreads();
+  n = 0;
+#pragma unroll
+  for (int w = 0; w < kFewThreads / 32; ++w) n += s_count[w];
+  if (n > p.few) return;
+  const int groups = (p.N + 3) / 4;
+  const int rows_here = (int)min((int64_t)kRows, p.n_out - r0);
+  const T* weight = (const T*)p.weight;
+  for (int e = tid; e < rows_here * groups; e += kFewThreads) {
+    const int row = e / groups, c = min(e % groups * 4, p.N - 4);   // the last two of an odd width share columns: the same values
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int w = 0; w < words; ++w) {
+      for (unsigned m = s_present[w][row]; m; m &= m - 1) {
+        const int k = w * 32 + __ffs(m) - 1;
+        const int i = __ldg(p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - k : k) * p.n_out + r0 + row);
+        add_pair<T, XV, WV>((const T*)p.rows + (int64_t)i * p.K, weight + (int64_t)k * p.K * p.N + c, p.K, p.N, acc);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float v = acc[j];
+      if (p.scale) v *= __ldg(p.scale + c + j);
+      if (p.bias) v += __ldg(p.bias + c + j);
+      store_one(p.out, p.out_dtype, (r0 + row) * p.N + c + j, p.relu ? fmaxf(v, 0.f) : v);
+    }
   }
 }
 
@@ -452,7 +622,23 @@ int launch_ffma(const FfmaParams& p, cudaStream_t st) {
 }
 
 template <typename T, int KC, bool VEC>
-int launch_ffma_cg(const FfmaParams& p, cudaStream_t st) {
+int launch_ffma_cg(FfmaParams p, cudaStream_t st) {
+  // Two pairs a row (odd widths, whose staging is dearer: 2.5), by a count of all offsets for the tiles that have few at the
+  // first ones.  (By the first ones alone the top row of a scan, which has no neighbours above it, would pass; by all of
+  // them alone every dense tile would pay for the count.)  A limit of three costs a 64 -> 64 training layer on 103 k rows
+  // 774 -> 984 us of convolution kernels.
+  // Rows of up to 16 channels and products of up to 8 are staged in any case: their steps are short.
+  const bool may_be_few = p.kv <= kFewWords * 32 && p.K > 16 && p.N > 8;
+  p.few = may_be_few ? (VEC ? kRows * 2 : kRows * 5 / 2) : -1;
+  p.few_first = p.kv <= kBatch ? p.few : kRows * 3 / 4;
+  p.w_vec = p.N % 4 == 0 && ((uintptr_t)p.weight & (4 * sizeof(T) - 1)) == 0;
+  if (p.few >= 0) {
+    const unsigned tiles = (unsigned)div_up64(p.n_out, kRows);
+    if (VEC) conv_few_kernel<T, VEC, VEC><<<tiles, kFewThreads, 0, st>>>(p);
+    else if (p.w_vec) conv_few_kernel<T, false, true><<<tiles, kFewThreads, 0, st>>>(p);
+    else conv_few_kernel<T, false, false><<<tiles, kFewThreads, 0, st>>>(p);
+    SPH_LAUNCH_CHECK();
+  }
   // the narrowest tile that holds the output channels; beyond 64 of them the grid repeats the rows per 64
   if (p.N <= 8) return launch_ffma<T, 1, KC, VEC>(p, st);
   if (p.N <= 16) return launch_ffma<T, 2, KC, VEC>(p, st);
@@ -461,7 +647,8 @@ int launch_ffma_cg(const FfmaParams& p, cudaStream_t st) {
 }
 
 // Narrow float32 rows take a step as wide as they are: the zeros that would fill it to 32 channels cost as many issue slots
-// as channels do, and the smaller buffers let more CTAs reside (sparse layers are bound by the latency of their steps).  Four buffers instead of two are slower (16 -> 32, 78 k rows: 46 -> 72 us).
+// as channels do, and the smaller buffers let more CTAs reside (sparse layers are bound by the latency of their
+// steps).  Four buffers instead of two are slower (16 -> 32, 78 k rows: 46 -> 72 us).
 template <bool VEC>
 int launch_ffma_f32(const FfmaParams& p, cudaStream_t st) {
   if (p.K <= 8) return launch_ffma_cg<float, 8, VEC>(p, st);

@@ -40,3 +40,13 @@ def test_narrow_float32_rows(iC, oC, dens):
     g = torch.as_tensor(rng.standard_normal((n_out, oC)), dtype=torch.float32).cuda()
     dw = ops.rule_conv_d_weight(feat, g, rules, rule_size)
     _close(dw, conv_np.conv_wgrad(f64, g.double().cpu().numpy(), pairs, 27), 1e-4)
+
+
+@pytest.mark.parametrize("iC,oC", [(17, 9), (20, 12), (32, 32), (33, 10), (37, 64), (40, 66)])
+@pytest.mark.parametrize("dens,ks", [(0.02, (3, 3, 3)), (0.07, (3, 3, 3)), (0.1, (3, 3, 3)), (0.15, (1, 3, 3)), (0.05, (5, 5, 5))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_sparse_and_dense_tiles(iC, oC, dens, ks, dtype):
+    """Around two pairs a row, tiles of one layer go to either kernel; each must take exactly what the other leaves."""
+    rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(2, [17, 23, 16], True, dens, 5, iC, oC, dtype, ks)
+    f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
+    _close(ops.rule_conv(feat, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[dtype])
