@@ -225,6 +225,8 @@ def kernel_of(lib, dcode, kind, k_ch, n_ch, esize, dtype_name):
     tc = bool(lib.sph_conv_uses_tensor_cores(dcode, k_ch, n_ch))
     if kind == "wgrad":
         which = lib.sph_conv_wgrad_kernel(dcode, k_ch, n_ch)
+        if esize == 2 and k_ch <= 64 and n_ch <= 64 and (k_ch * n_ch <= 2048 or which != 1):
+            return "conv_wgrad_strip_kernel", True
         if which == 1:
             return "conv_wgrad_tc_kernel<%d>" % (k_ch * esize // 16), True
         return ("conv_wgrad_pairs_kernel<%d,%d>" % (k_ch, n_ch)) if which == 2 else "conv_wgrad_ffma_kernel", False

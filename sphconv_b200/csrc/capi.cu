@@ -196,8 +196,8 @@ extern "C" int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype,
     return conv_wgrad_strip(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
   if (conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch))
     return conv_wgrad_tc(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
-  // narrow rows the tensor-core kernel does not take and small fp32 layers: the pair-compacting walk
-  if (conv_wgrad_pairs_supported(dtype, kv, k_ch, n_ch) && ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0))
+  // small fp32 layers: the pair-compacting walk
+  if (dtype == SPH_F32 && conv_wgrad_pairs_supported(dtype, kv, k_ch, n_ch) && ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0))
     return conv_wgrad_pairs(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
   return conv_wgrad_ffma(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
 }

@@ -628,7 +628,7 @@ bool conv_wgrad_pairs_supported(int dtype, int kv, int K, int N) {
 
 int conv_wgrad_pairs(const void* rows, const void* dout, int dtype, int64_t n_rows, const int* nbr, int64_t n_out,
                      int kv, int K, int N, float* dw, int* status, cudaStream_t st) {
-  if (!conv_wgrad_pairs_supported(dtype, kv, K, N)) {
+  if (dtype != SPH_F32 || !conv_wgrad_pairs_supported(dtype, kv, K, N)) {    // 16-bit rows: the strip kernel's
     set_error("conv_wgrad_pairs: unsupported dtype/shape");
     return SPH_ERR_UNSUPPORTED;
   }
@@ -640,12 +640,7 @@ int conv_wgrad_pairs(const void* rows, const void* dout, int dtype, int64_t n_ro
   p.rows = rows; p.dout = dout; p.nbr = nbr;
   p.n_rows = n_rows; p.n_out = n_out; p.n_chunks = div_up64(n_out, 32);
   p.kv = kv; p.dw = dw; p.status = status;
-  switch (dtype) {
-    case SPH_F32: return launch_wgrad_pairs_ic<float>(p, K, N, st);
-    case SPH_F16: return launch_wgrad_pairs_ic<__half>(p, K, N, st);
-    case SPH_BF16: return launch_wgrad_pairs_ic<__nv_bfloat16>(p, K, N, st);
-  }
-  return SPH_ERR_UNSUPPORTED;
+  return launch_wgrad_pairs_ic<float>(p, K, N, st);
 }
 
 }  // namespace sph
