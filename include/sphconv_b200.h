@@ -227,7 +227,10 @@ int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype, int64_t n_
  *                  copies every row to its voxel (the other voxels of d_dense are left as they are, as in the
  *                  reference: the caller zero-fills), backward = 1 copies the voxels' values back into d_rows.
  * sph_dense_channels_first  the same between rows [nnz, channels] of elem_bytes-byte elements and a channels-first dense
- *                  tensor [B,channels,s0,s1,s2] (s2 <= 2048), which backward = 0 writes in full, zeros included. */
+ *                  tensor [B,channels,s0,s1,s2] (s2 <= 2048), which backward = 0 writes in full, zeros included.  Of several
+ *                  rows at one depth of a column the last one is the voxel's value, and each gets the voxel's gradient;
+ *                  a row whose depth is out of range (status bit SPH_STATUS_BAD_INDEX) or that lies behind the last
+ *                  column's rows gets zeros. */
 int64_t sph_init_tensor_scratch_bytes(int32_t B, const int32_t shape[3]);
 int sph_init_tensor(const void* d_feature, int32_t row_bytes, int64_t nnz, const int32_t* d_indices, int32_t B,
                     const int32_t shape[3], void* d_scratch, void* d_out_feature, int32_t* d_z_idx,

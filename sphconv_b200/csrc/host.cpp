@@ -513,7 +513,7 @@ Tensor dense_channels_first(const Tensor& from, const Tensor& z_idx, const Tenso
   require_cuda(z_idx);
   require_cuda(z_ptr);
   const c10::cuda::CUDAGuard guard(from.device());
-  const int64_t nnz = z_idx.size(0);
+  const int64_t nnz = backward ? z_idx.size(0) : std::min(from.size(0), z_idx.size(0));
   const int32_t dims[3] = {(int32_t)shape.at(2), (int32_t)shape.at(3), (int32_t)shape.at(4)};
   Tensor out = backward ? empty({nnz, shape[1]}, from.scalar_type(), from) : empty(shape, from.scalar_type(), from);
   const Tensor& rows = backward ? out : from;

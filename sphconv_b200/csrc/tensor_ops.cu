@@ -102,6 +102,10 @@ dense_rows_kernel(V* __restrict__ rows, const int* __restrict__ z_idx, const int
 // tensor is written once; a fill, a channels-last scatter and a permuting copy moved its bytes four times.  [8,64,16,128,64]
 // fp16 (134 MB) with 30 % of the cells occupied: 58 us to dense and 53 us back against 350 and 325 us, half the copy rate
 // (the per-element reads of the staged rows).
+//
+// Rows need not own their cells: of several rows at one depth of a column the last is the cell's value and each gets the
+// cell's gradient; a row whose depth lies outside the grid has the status bit set and a gradient of zero.  A block can hence have
+// more rows than cells (`crowded`): shared memory then holds one row per cell, the one its value comes from.
 constexpr int kDenseCells = 256;         // cells of a block, when columns are shorter
 constexpr int kDenseMaxCells = 2048;     // columns up to this deep are staged
 
@@ -140,20 +144,32 @@ dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx,
   const int nc = (int)min((int64_t)cols_per_block, cols_per_b - col0);
   const int64_t gcol0 = (int64_t)blockIdx.y * cols_per_b + col0;
   const int cells = nc * D;
-  const int64_t r0 = min((int64_t)col_begin(z_ptr, gcol0), nnz);
+  const int64_t r0 = max((int64_t)0, min((int64_t)col_begin(z_ptr, gcol0), nnz));
   const int n_rows = (int)(min((int64_t)__ldg(z_ptr + gcol0 + nc - 1), nnz) - r0);
-  for (int i = tid; i < cells; i += kOpsThreads) s_map[i] = -1;
-  __syncthreads();
-  for (int i = tid; i < n_rows; i += kOpsThreads) {
+  const bool crowded = n_rows > cells;
+  auto cell_of = [&](int i) {              // of row r0 + i, or -1
     int lo = 0, hi = nc - 1;               // first column of the block whose inclusive prefix exceeds the row
     while (lo < hi) {
       const int mid = (lo + hi) >> 1;
       if (__ldg(z_ptr + gcol0 + mid) > r0 + i) hi = mid; else lo = mid + 1;
     }
     const int z = __ldg(z_idx + r0 + i);
-    if ((unsigned)z < (unsigned)D) s_map[lo * D + z] = i;
-    else if (status) atomicOr(status, SPH_STATUS_BAD_INDEX);
+    return (unsigned)z < (unsigned)D ? lo * D + z : -1;
+  };
+  for (int i = tid; i < cells; i += kOpsThreads) s_map[i] = -1;
+  __syncthreads();
+  bool others = false;                     // a row that does not own its cell
+  for (int i = tid; i < n_rows; i += kOpsThreads) {
+    const int cell = cell_of(i);
+    if (cell < 0) {
+      others = true;
+      if (status) atomicOr(status, SPH_STATUS_BAD_INDEX);
+    } else {
+      others |= atomicMax(s_map + cell, i) >= 0;
+    }
   }
+  if (BACK) others = __syncthreads_or(others);
+  else if (crowded) __syncthreads();
   const int64_t vol = cols_per_b * D;
   E* plane0 = dense + (int64_t)blockIdx.y * C * vol + col0 * D;
   struct alignas(V * sizeof(E)) Vec { E e[V]; };
@@ -161,8 +177,17 @@ dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx,
   for (int c0 = 0; c0 < C; c0 += chunk) {
     const int cn = min(chunk, C - c0);
     E* mem = rows + r0 * C + c0;
-    if (!BACK) move_rows_of<E, true>(mem, s_rows, n_rows, cn, C, stride);
-    __syncthreads();
+    if (!BACK) {
+      if (!crowded) {
+        move_rows_of<E, true>(mem, s_rows, n_rows, cn, C, stride);
+      } else {
+        for (int e = tid; e < cells * cn; e += kOpsThreads) {
+          const int cell = e / cn, c = e % cn, r = s_map[cell];
+          if (r >= 0) s_rows[cell * stride + c] = mem[(int64_t)r * C + c];
+        }
+      }
+      __syncthreads();
+    }
     // a thread keeps the staged rows of its V cells in registers and walks channels, two at a time for 2-byte elements
     // (one 4-byte access to shared memory per cell and pair)
     const int groups = cells / V;
@@ -173,7 +198,7 @@ dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx,
 #pragma unroll
       for (int j = 0; j < V; ++j) {
         const int r = s_map[g * V + j];
-        at[j] = r < 0 ? -1 : r * stride;
+        at[j] = r < 0 ? -1 : (crowded ? g * V + j : r) * stride;
       }
       Vec* cell = (Vec*)(plane0 + (int64_t)c0 * vol) + g;
       const int64_t plane = vol / V;
@@ -217,10 +242,20 @@ dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx,
     }
     __syncthreads();
     if (BACK) {
-      move_rows_of<E, false>(mem, s_rows, n_rows, cn, C, stride);
+      if (!others) {
+        move_rows_of<E, false>(mem, s_rows, n_rows, cn, C, stride);
+      } else {
+        for (int i = tid; i < n_rows; i += kOpsThreads) {
+          const int cell = cell_of(i);
+          const E* src = s_rows + (cell < 0 ? 0 : crowded ? cell : s_map[cell]) * stride;
+          for (int c = 0; c < cn; ++c) mem[(int64_t)i * C + c] = cell < 0 ? E(0) : src[c];
+        }
+      }
       __syncthreads();
     }
   }
+  if (BACK && blockIdx.x == gridDim.x - 1 && blockIdx.y == gridDim.y - 1)    // rows behind the last column's
+    for (int64_t e = (r0 + max(n_rows, 0)) * C + tid; e < nnz * C; e += kOpsThreads) rows[e] = E(0);
 }
 
 template <typename E, int V>

@@ -95,3 +95,49 @@ def test_dense_channels_first_matches_two_step(dtype, C, shape, dens):
     assert torch.equal(got, want.permute(0, 4, 1, 2, 3))
     assert torch.equal(ops.dense_channels_first_backward(got, z_idx, z_ptr), f)
     assert check_status() == 0
+
+
+@pytest.mark.parametrize("dtype,C", [(torch.float16, 64), (torch.float16, 3), (torch.float32, 5), (torch.int8, 6), (torch.bfloat16, 130)])
+@pytest.mark.parametrize("shape,per_column", [([5, 7, 16], 9), ([3, 9, 13], 40), ([2, 3, 300], 700), ([1, 2, 2048], 2500)])
+def test_dense_channels_first_rows_without_a_cell_of_their_own(dtype, C, shape, per_column):
+    """Repeated depths - some blocks with more rows than cells - against the oracle (the last row of a depth is the cell's value,
+    each of them gets its gradient), then with depths outside the grid (status bit, gradient zero) and with rows behind the
+    last column's (gradient zero)."""
+    rng = np.random.default_rng(C + per_column)
+    B, (H, W, D) = 2, shape
+    counts = rng.integers(0, per_column + 1, (B, H, W))
+    counts[0, 0, 0] = per_column
+    z_ptr = counts.reshape(-1).cumsum().astype(np.int32).reshape(B, H, W)
+    n = int(z_ptr[-1, -1, -1])
+    z_idx = rng.integers(0, D, n).astype(np.int32)
+    feat = torch.as_tensor(rng.integers(-100, 100, (n, C))).to(dtype)
+    grad = torch.as_tensor(rng.integers(-100, 100, (B, C, *shape))).to(dtype)
+    zi, zp = torch.as_tensor(z_idx, device=DEV), torch.as_tensor(z_ptr, device=DEV)
+
+    def dense(rows, depths, ptr):
+        return torch.as_tensor(tensor_np.to_dense(rows.double().numpy(), depths, ptr, B, shape)).permute(0, 4, 1, 2, 3)
+
+    def back(depths, ptr):
+        d = grad.double().permute(0, 2, 3, 4, 1).numpy()
+        return torch.as_tensor(tensor_np.to_dense_backward(d, depths, ptr))
+
+    got = ops.dense_channels_first(feat.to(DEV), zi, zp, [B, C, *shape])
+    assert torch.equal(got.cpu().double(), dense(feat, z_idx, z_ptr))
+    got = ops.dense_channels_first_backward(grad.to(DEV), zi, zp)
+    assert torch.equal(got.cpu().double(), back(z_idx, z_ptr))
+    longer = torch.cat([zi, torch.zeros(3, dtype=torch.int32, device=DEV)])
+    got = ops.dense_channels_first_backward(grad.to(DEV), longer, zp)
+    assert torch.equal(got[:n].cpu().double(), back(z_idx, z_ptr)) and not got[n:].any()
+    assert check_status() == 0
+
+    out = rng.random(n) < 0.1
+    out[0] = True
+    column = np.repeat(np.arange(B * H * W), counts.reshape(-1))[~out]
+    ptr = np.bincount(column, minlength=B * H * W).cumsum().astype(np.int32).reshape(B, H, W)
+    bad = torch.as_tensor(np.where(out, np.where(rng.random(n) < 0.5, D, -1), z_idx).astype(np.int32), device=DEV)
+    got = ops.dense_channels_first(feat.to(DEV), bad, zp, [B, C, *shape])
+    assert torch.equal(got.cpu().double(), dense(feat[torch.as_tensor(~out)], z_idx[~out], ptr))
+    got = ops.dense_channels_first_backward(grad.to(DEV), bad, zp)
+    assert torch.equal(got[~out].cpu().double(), back(z_idx[~out], ptr)) and not got[out].any()
+    with pytest.raises(RuntimeError):
+        check_status()
