@@ -355,6 +355,7 @@ py::tuple rules_to_nbr(const Tensor& rules, const Tensor& rule_size, int64_t n_i
 // ---- convolution ---------------------------------------------------------------------------------------------------
 // UMMA image of a [KV, K, N] weight, or None where a CUDA-core kernel runs.
 optional<Tensor> pack_weight(const Tensor& w) {
+  require_cuda(w);             // the image is made from the raw memory: of an expanded weight that is too short
   const int code = dtype_code(w, "weight");
   const int32_t kv = (int32_t)w.size(0), k = (int32_t)w.size(1), n = (int32_t)w.size(2);
   const int64_t bytes = abi.sph_packed_weight_bytes(code, kv, k, n);

@@ -214,3 +214,15 @@ def test_module_rules_written_beside_the_convolution():
             n_want, want = canon(wr, wn)
             assert (n_got == n_want).all() and got == want
     sphconv.check_status()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.int8])
+def test_weights_that_are_not_contiguous_are_refused(dtype):
+    """An expanded or transposed weight is refused before anything reads its memory as [KV, iC, oC]."""
+    from sphconv_b200 import sphconv_cuda as ops
+    x = torch.zeros(8, 16, device=DEV, dtype=dtype)
+    nbr = torch.full((27, 8), -1, dtype=torch.int32, device=DEV)
+    for w in (torch.zeros(1, 1, 16, device=DEV, dtype=dtype).expand(27, 16, 16),
+              torch.zeros(27, 16, 16, device=DEV, dtype=dtype).transpose(1, 2)):
+        with pytest.raises(RuntimeError, match="contiguous"):
+            ops._gather(x, w, nbr, 8, False, None, None, False, None)
