@@ -118,7 +118,7 @@ void check_index(const Tensor& z_idx, const Tensor& z_ptr) {
 }
 
 // ---- per-device state ----------------------------------------------------------------------------------------------
-// The int32 word the kernels OR error bits into.
+// The int32 word the kernels OR error bits into.  Looked up under the lock: autograd's threads come here without the GIL.
 std::mutex state_mutex;
 std::array<Tensor, 64> status_words;
 
@@ -126,14 +126,15 @@ Tensor status_tensor(int device) {
   if (device < 0 || device >= (int)status_words.size()) fail("device ordinal not supported");
   std::lock_guard<std::mutex> lock(state_mutex);
   Tensor& t = status_words[device];
-  if (!t.defined()) t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+  if (!t.defined()) {
+    t = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, device));
+    // kernels of other streams may be the next to write it
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
+      at::cuda::getCurrentCUDAStream(device).synchronize();
+  }
   return t;
 }
-int32_t* status_of(const Tensor& t) {
-  const int device = t.device().index();
-  Tensor& s = status_words.at(device);
-  return ints(s.defined() ? s : status_tensor(device));
-}
+int32_t* status_of(const Tensor& t) { return ints(status_tensor(t.device().index())); }
 
 // The stream pair lists are written on, beside the convolution that reads the table only.
 c10::cuda::CUDAStream side_stream(int device) {

@@ -226,3 +226,40 @@ def test_weights_that_are_not_contiguous_are_refused(dtype):
               torch.zeros(27, 16, 16, device=DEV, dtype=dtype).transpose(1, 2)):
         with pytest.raises(RuntimeError, match="contiguous"):
             ops._gather(x, w, nbr, 8, False, None, None, False, None)
+
+
+FIRST_USE = """
+import sys, threading
+import torch
+sys.path[:0] = sys.argv[1:]
+import sphconv_b200 as sphconv
+from sphconv_b200 import sphconv_cuda as ops
+x = torch.ones(300, 16, device="cuda", dtype=torch.float16)
+nbr = torch.arange(300, device="cuda", dtype=torch.int32).repeat(27, 1)
+nbr[3, 5] = 300                                   # no row: every call sets the status bit
+w = torch.ones(27, 16, 16, device="cuda", dtype=torch.float16)
+torch.cuda.synchronize()
+gate, out = threading.Barrier(8), [None] * 8
+def work(i):
+    with torch.cuda.stream(torch.cuda.Stream()):
+        gate.wait()
+        out[i] = (ops.C.host().conv_wgrad(x, x, nbr, None, False), ops.C.host().status_tensor(0).data_ptr())
+        torch.cuda.current_stream().synchronize()
+threads = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+[t.start() for t in threads]; [t.join() for t in threads]
+assert all(torch.equal(o[0], out[0][0]) and o[1] == out[0][1] for o in out)
+try:
+    sphconv.check_status()
+except RuntimeError:
+    print("status seen")
+"""
+
+
+def test_first_use_from_many_threads():
+    """The first operators of a process, issued by eight threads on eight streams: one status word, and none of its bits lost."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    got = subprocess.run([sys.executable, "-c", FIRST_USE, root], capture_output=True, text=True, timeout=300)
+    assert got.returncode == 0 and "status seen" in got.stdout, got.stderr[-2000:]
