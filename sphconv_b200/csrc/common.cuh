@@ -66,6 +66,14 @@ struct Geom {
   int tH, tW, tgH, tgW, nTile;
 };
 
+// Allows a kernel `limit` bytes of dynamic shared memory: what all its launches stay within, not what the launch at hand takes.
+// Threads launch one kernel with different sizes, and a bound lowered between another thread's call and its launch would
+// fail that launch.
+template <typename F>
+inline cudaError_t allow_smem(F* kernel, int limit) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
+}
+
 // Validates and converts; returns SPH_OK or an error code (message set).
 int make_geom(const sph_geom* g, Geom* out);
 

@@ -614,7 +614,7 @@ template <typename T, int CG, int KC, bool VEC>
 int launch_ffma(const FfmaParams& p, cudaStream_t st) {
   using S = FfmaShape<CG, KC>;
   auto kern = conv_ffma_kernel<T, CG, KC, VEC>;
-  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
+  SPH_CUDA(allow_smem(kern, S::BYTES));
   const dim3 grid((unsigned)div_up64(p.n_out, kRows), (unsigned)div_up(p.N, S::NP));
   kern<<<grid, S::T, S::BYTES, st>>>(p);
   SPH_LAUNCH_CHECK();
@@ -660,7 +660,7 @@ template <typename T, int KG, int NG, bool VEC>
 int launch_wg(const FfmaWgradParams& p, int kv, cudaStream_t st) {
   using S = WgShape<KG, NG>;
   auto kern = conv_wgrad_ffma_kernel<T, KG, NG, VEC>;
-  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::BYTES));
+  SPH_CUDA(allow_smem(kern, S::BYTES));
   kern<<<dim3((unsigned)div_up64(p.n_out, kWgSlice), (unsigned)kv), kThreads, S::BYTES, st>>>(p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;

@@ -29,6 +29,7 @@ namespace {
 constexpr int kSpWarps = 8;
 constexpr int kSpThreads = kSpWarps * 32;
 constexpr int kSpList = 64;          // an offset adds at most 32 items to fewer than 32 waiting ones
+constexpr int kSpSmem = 112 * 1024, kSpWgradSmem = 120 * 1024;   // shared memory of a CTA at most: two on an SM, or one
 
 struct SparseParams {
   const void* rows;
@@ -350,7 +351,7 @@ int launch_sparse(const SparseParams& p, cudaStream_t st) {
   using S = SparseShape<T, IC, OC>;
   const int smem = S::smem_bytes(p.kv);
   auto kern = conv_sparse_rows_kernel<T, IC, OC>;
-  if (smem > 48 * 1024) SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (smem > 48 * 1024) SPH_CUDA(allow_smem(kern, kSpSmem));
   int per_sm = 0;
   SPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSpThreads, smem));
   const int sms = current_sm_count();
@@ -539,7 +540,7 @@ int launch_wgrad_pairs(const WgradParams& p, cudaStream_t st) {
   using S = WgradShape<IC, OC>;
   const int smem = S::smem_bytes(p.kv);
   auto kern = conv_wgrad_pairs_kernel<T, IC, OC>;
-  if (smem > 48 * 1024) SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (smem > 48 * 1024) SPH_CUDA(allow_smem(kern, kSpWgradSmem));
   int per_sm = 0;
   SPH_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kSpThreads, smem));
   const int sms = current_sm_count();
@@ -589,7 +590,7 @@ bool conv_sparse_supported(int dtype, int kv, int K, int N) {
   const int w_size = (K * N > 256 && dtype != SPH_F32) ? 2 : 4;
   const int64_t smem = (int64_t)kv * (K * N + kSpWPad) * w_size + 2 * N * 4 +
                        (int64_t)kSpWarps * (32 * (K + 4) * 4 + 32 * (N + 4) * 4 + kSpList * 8);
-  return kv < (1 << 20) && smem <= 112 * 1024;
+  return kv < (1 << 20) && smem <= kSpSmem;
 }
 
 int conv_gather_sparse(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
@@ -623,7 +624,7 @@ bool conv_wgrad_pairs_supported(int dtype, int kv, int K, int N) {
   if (dtype != SPH_F32 && dtype != SPH_F16 && dtype != SPH_BF16) return false;
   if (!channels_ok(K) || !channels_ok(N) || K * N > 512) return false;
   const int64_t smem = (int64_t)kv * K * N * 4 + (int64_t)kSpWarps * (32 * (K + 4) * 4 + 32 * (N + 4) * 4 + kSpList * 8);
-  return kv < (1 << 20) && smem <= 120 * 1024;
+  return kv < (1 << 20) && smem <= kSpWgradSmem;
 }
 
 int conv_wgrad_pairs(const void* rows, const void* dout, int dtype, int64_t n_rows, const int* nbr, int64_t n_out,

@@ -450,7 +450,7 @@ int launch_strip_kernel(StripParams& p, cudaStream_t st) {
   }
   p.cap = cap < 3 * R ? cap : 3 * R;
   const int smem = fixed + 2 * ((p.cap * (pitch / 16) + 7) & ~7) * 16;
-  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SPH_CUDA(allow_smem(kern, kStripSmem));
   const int sms = current_sm_count();
   if (sms <= 0) return SPH_ERR_CUDA;
   const int grid = p.tiles < sms * per_sm ? p.tiles : sms * per_sm;

@@ -406,8 +406,7 @@ int conv_gather_tc(const void* rows, int dtype, int64_t n_rows, const void* pack
   if (grid < 1) return SPH_OK;
 #define SPH_TC_LAUNCH(KC_, I8_)                                                                                  \
   do {                                                                                                         \
-    SPH_CUDA(cudaFuncSetAttribute(conv_gather_tc_kernel<KC_, I8_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                  smem_bytes));                                                                \
+    SPH_CUDA(allow_smem(conv_gather_tc_kernel<KC_, I8_>, kSmemTotal));                                         \
     conv_gather_tc_kernel<KC_, I8_><<<grid, kTcThreads, smem_bytes, st>>>(p);                                  \
   } while (0)
   if (p.is_i8) {

@@ -294,7 +294,7 @@ int launch_wgrad_strip(WgradStripParams& p, cudaStream_t st) {
   }
   p.cap = (cap < 3 * kRows ? cap : 3 * kRows) & ~7;
   const int smem = fixed_bytes(NP) + 2 * ((p.cap * PX + 7) & ~7) * 16;
-  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SPH_CUDA(allow_smem(kern, kSmem));
   const int sms = current_sm_count();
   if (sms <= 0) return SPH_ERR_CUDA;
   int slices = sms * per_sm / (p.groups * p.halves);

@@ -327,7 +327,7 @@ int conv_wgrad_tc(const void* rows, const void* dout, int dtype, int64_t n_rows,
   const int smem_bytes = p.x_off + p.stages * p.x_bytes;
 #define SPH_WG_LAUNCH(KCX_)                                                                                        \
   do {                                                                                                           \
-    SPH_CUDA(cudaFuncSetAttribute(conv_wgrad_tc_kernel<KCX_>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes)); \
+    SPH_CUDA(allow_smem(conv_wgrad_tc_kernel<KCX_>, kSmemTotal));                                                \
     conv_wgrad_tc_kernel<KCX_><<<grid, kThreads, smem_bytes, st>>>(p);                                           \
   } while (0)
   switch (p.kc_x) {

@@ -108,6 +108,7 @@ dense_rows_kernel(V* __restrict__ rows, const int* __restrict__ z_idx, const int
 // more rows than cells (`crowded`): shared memory then holds one row per cell, the one its value comes from.
 constexpr int kDenseCells = 256;         // cells of a block, when columns are shorter
 constexpr int kDenseMaxCells = 2048;     // columns up to this deep are staged
+constexpr int kDenseSmem = 96 * 1024;    // the cells' map (8 KB), 64 KB of rows, and at most 8 bytes a row of padding
 
 // Rows of `words` pieces between memory (pitch words apart) and shared memory (s_pitch), a power of two of lanes per row.
 template <typename P, bool TO_SMEM>
@@ -272,7 +273,7 @@ int launch_dense_cf(void* rows, const int* z_idx, const int* z_ptr, int64_t nnz,
   const int stride = (div_up(chunk, per) | 1) * per;
   const int smem = (cells * (int)sizeof(int) + 15) / 16 * 16 + cells * stride * (int)sizeof(E);
   auto kern = backward ? dense_channels_first_kernel<E, V, true> : dense_channels_first_kernel<E, V, false>;
-  SPH_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SPH_CUDA(allow_smem(kern, kDenseSmem));
   kern<<<dim3((unsigned)div_up64(cols_per_b, cols), (unsigned)B), kOpsThreads, smem, st>>>(
       (E*)rows, z_idx, z_ptr, nnz, cols_per_b, cols, D, C, chunk, stride, (E*)dense, status);
   SPH_LAUNCH_CHECK();

@@ -141,3 +141,40 @@ def test_dense_channels_first_rows_without_a_cell_of_their_own(dtype, C, shape, 
     assert torch.equal(got[~out].cpu().double(), back(z_idx[~out], ptr)) and not got[out].any()
     with pytest.raises(RuntimeError):
         check_status()
+
+
+def test_one_kernel_with_two_sizes_from_two_threads():
+    """Launches of one kernel that take 8 and 70 KB of shared memory, through the C ABI from two threads at once: neither
+    lowers the bound the other one needs."""
+    import threading
+
+    from sphconv_b200 import _capi as C
+    lib, errors = C.lib(), []
+    gate = threading.Barrier(2)
+
+    def work(C_, D):
+        torch.cuda.set_device(0)
+        H, W = 2, 4
+        zi = torch.zeros(H * W, dtype=torch.int32, device=DEV)
+        zp = torch.arange(1, H * W + 1, dtype=torch.int32, device=DEV)
+        rows = torch.ones(H * W, C_, dtype=torch.float16, device=DEV)
+        dense = torch.empty(1, C_, H, W, D, dtype=torch.float16, device=DEV)
+        torch.cuda.synchronize()
+        shape = ops._shape3([H, W, D])
+        gate.wait()
+        for _ in range(3000):
+            rc = lib.sph_dense_channels_first(C.ptr(rows), 2, C_, H * W, C.ptr(zi), C.ptr(zp), 1, shape, C.ptr(dense), 0, None,
+                                              C.stream_ptr(zi.device))
+            if rc != 0:
+                errors.append(lib.sph_last_error().decode())
+                return
+        torch.cuda.synchronize()
+        if float(dense.sum()) != H * W * C_:
+            errors.append("wrong values")
+
+    threads = [threading.Thread(target=work, args=a) for a in ((4, 512), (64, 512))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
