@@ -84,10 +84,6 @@ int conv_gather_strip(const void* rows, int dtype, int64_t n_rows, const void* p
     set_error("conv_gather_strip: rows, filter image and output must be 16-byte aligned");
     return SPH_ERR_INVALID;
   }
-  if ((int64_t)kv * n_out >= (1LL << 32)) {
-    set_error("conv_gather_strip: more than 2^32 table entries");
-    return SPH_ERR_LIMIT;
-  }
   StripParams p;
   p.rows = (const uint8_t*)rows; p.filter = (const uint4*)packed; p.nbr = nbr;
   p.n_rows = n_rows; p.n_out = n_out;

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
   const int groups = (p.kv + kGroup - 1) / kGroup;
   const int my_tiles = (p.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
   const int total = my_tiles * groups;
-  const unsigned n_out = (unsigned)p.n_out;                // KV x n_out < 2^32: the launcher checks
+  const unsigned n_out = (unsigned)p.n_out;
   uint32_t bad = 0u;
 
   struct Place { int ti, g; };                             // tile (of this CTA) and group of a step
@@ -101,12 +101,12 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
 #pragma unroll
     for (int j = 0; j < EPL; ++j) ok[j] = q.ti < my_tiles && r + j * 32 < n_out;
     const int nk = p.kv - q.g * kGroup;
-    const unsigned step = p.flip_k ? 0u - n_out : n_out;
-    unsigned at = (unsigned)(p.flip_k ? p.kv - 1 - q.g * kGroup : q.g * kGroup) * n_out + r;
+    const int64_t step = p.flip_k ? -p.n_out : p.n_out;
+    const int* at = p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - q.g * kGroup : q.g * kGroup) * p.n_out + r;
 #pragma unroll
     for (int o = 0; o < kGroup; ++o) {
 #pragma unroll
-      for (int j = 0; j < EPL; ++j) raw[o][j] = (ok[j] && o < nk) ? __ldg(p.nbr + (at + j * 32)) : -1;
+      for (int j = 0; j < EPL; ++j) raw[o][j] = (ok[j] && o < nk) ? __ldg(at + j * 32) : -1;
       at += step;
     }
   };

@@ -96,3 +96,21 @@ def test_entries_that_are_no_rows():
     with pytest.raises(RuntimeError):
         check_status()
     assert check_status() == 0 and C.lib() is not None
+
+
+@pytest.mark.parametrize("flip", [False, True])
+def test_tables_of_more_than_2_to_the_32_entries(flip):
+    """Entries at both ends of the planes on either side of the 2^32nd; every other row has no neighbour."""
+    kv, n_out = 27, (1 << 32) // 27 + 300
+    if torch.cuda.mem_get_info()[0] < 40 << 30:
+        pytest.skip("needs 40 GB of device memory")
+    rng = np.random.default_rng(5)
+    x, w = _operands(rng, 100, kv, 16, 4, torch.float16)
+    at = torch.cat([torch.arange(300), torch.arange(n_out - 600, n_out)]).to(DEV)
+    some = torch.as_tensor(rng.integers(-1, 100, (kv, at.numel())).astype(np.int32), device=DEV)
+    nbr = torch.full((kv, n_out), -1, dtype=torch.int32, device=DEV)
+    nbr[:, at] = some
+    got = ops._gather(x, w, nbr, n_out, flip, None, None, False, torch.float32)
+    _close(got[at], _reference(x, w, some.flip(0) if flip else some), TOL[torch.float16])
+    assert int(torch.count_nonzero(got)) == int(torch.count_nonzero(got[at]))
+    assert check_status() == 0
