@@ -111,12 +111,13 @@ int sph_rules_subm_static(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_
  * ref: get_rules, src/sphconv/rules.cu:405-462 (prepareGridKernel + the cumsum/roll scans).
  *   d_scratch   sph_rules_strided_scratch_bytes(g, nnz) bytes; must be kept untouched until step 2 has run
  *   d_oz_ptr    int32 [B,oH,oW], inclusive prefix like z_ptr
- *   d_out_nnz   int32 [1] on the device (= oz_ptr[-1])
+ *   d_out_nnz   int32 [1] on the device (= oz_ptr[-1]), or pinned host memory the device can write
  *   h_out_nnz   optional host pointer: when non-null the call synchronises `stream` and stores the
  *               count there (the same device->host read the reference does at rules.cu:461).  The kernel
  *               hands the count over through a word of mapped pinned host memory, not a memcpy, so the read
- *               does not queue behind bulk copies on the copy engines; the first such call on a device
- *               allocates 1 KiB of pinned host memory that lives until the process ends. */
+ *               does not queue behind bulk copies on the copy engines.  Such words are mapped 1 KiB at a
+ *               time, live until the process ends and are shared with sph_voxelize_count: one or two per call
+ *               that is waiting. */
 int64_t sph_rules_strided_scratch_bytes(const sph_geom* g, int64_t nnz);
 int sph_rules_strided_count(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t nnz, const sph_geom* g,
                             void* d_scratch, int32_t* d_oz_ptr, int32_t* d_out_nnz, int32_t* h_out_nnz,
@@ -125,7 +126,8 @@ int sph_rules_strided_count(const int32_t* d_z_idx, const int32_t* d_z_ptr, int6
  * word the count will be written to; it may be read once work enqueued on `stream` up to this call has completed
  * (e.g. after cudaEventSynchronize on an event recorded right after the call).  Lets a caller enqueue other work
  * behind step 1 - the convolution of the layer before - so that the GPU is busy during the host's round trip.
- * At most 256 such words per device are in use at a time (a ring): read the count before 255 further calls. */
+ * At most 256 such words per device are in use at a time (a ring): read the count before 255 further calls of this
+ * function.  A caller that needs more passes pinned host memory as d_out_nnz of sph_rules_strided_count and no h_out_nnz. */
 int sph_rules_strided_count_async(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t nnz, const sph_geom* g,
                                   void* d_scratch, int32_t* d_oz_ptr, int32_t* d_out_nnz,
                                   const int32_t** h_count_word, void* stream);

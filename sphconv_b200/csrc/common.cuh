@@ -82,7 +82,12 @@ int make_geom(const sph_geom* g, Geom* out);
 int column_prefix_from_masks(const uint32_t* mask, int words, int64_t ncols, int* prefix, int* blocksum, int* total_dev,
                              int* total_host, cudaStream_t st);
 
-// rules.cu: the next word of the current device's ring of mapped pinned host words (see there).
-int count_slot(int32_t** host_word, int32_t** dev_word);
+// rules.cu: a word of mapped pinned host memory of the current device, for a call that waits for what its kernels write there
+// (see there), which then gives it back.
+struct HostWord {
+  int32_t *host, *dev;
+};
+int take_host_word(HostWord* w);
+void give_host_word(const HostWord& w);
 
 }  // namespace sph

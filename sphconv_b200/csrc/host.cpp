@@ -4,6 +4,7 @@
 // An operator of this path is a handful of launches of a few microseconds each; driven from Python (one ctypes call and one
 // torch.empty at a time, ~100 us a layer) a scan waited for the host, not for the GPU.  The library itself stays free of
 // torch: this module loads it and calls it through the same entry points as any other binding.
+#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -28,7 +29,7 @@ using Ints = std::vector<int64_t>;
 // ---- the C ABI -----------------------------------------------------------------------------------------------------
 #define SPH_ENTRY_POINTS(X)                                                                                          \
   X(sph_last_error) X(sph_num_tiles) X(sph_tile_n_max) X(sph_rules_subm_scratch_bytes) X(sph_rules_subm)             \
-  X(sph_rules_strided_scratch_bytes) X(sph_rules_strided_count_async) X(sph_rules_strided_fill) X(sph_rule_lists)    \
+  X(sph_rules_strided_scratch_bytes) X(sph_rules_strided_count) X(sph_rules_strided_fill) X(sph_rule_lists)    \
   X(sph_rules_to_nbr) X(sph_packed_weight_bytes) X(sph_pack_weight) X(sph_conv_gather) X(sph_conv_wgrad)             \
   X(sph_init_tensor_scratch_bytes) X(sph_init_tensor) X(sph_permute_rows) X(sph_dense_channels_first)                \
   X(sph_epilogue_backward) X(sph_voxel_transform) X(sph_voxel_feature_count) X(sph_voxelize_scratch_bytes)           \
@@ -249,12 +250,29 @@ py::tuple rules_subm(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, const 
   return py::make_tuple(or_none(l.rules), or_none(l.rule_size), nbr, or_none(ready));
 }
 
-// Step 1 of a strided rule set, enqueued; the row count is in the mapped host word once the step has run.
+// Step 1 of a strided rule set, enqueued; the row count is in the word, pinned host memory that the step's last kernel writes,
+// once the step has run.  The word is the handle's own: any number of them may be outstanding, for any time.
 struct Pending {
   sph_geom g;
-  Tensor z_idx, z_ptr, scratch, oz_ptr, d_count;
-  const int32_t* word = nullptr;
+  Tensor z_idx, z_ptr, scratch, oz_ptr, word;
+  c10::cuda::CUDAStream stream;
   at::cuda::CUDAEvent event;
+  bool read = false;
+
+  explicit Pending(c10::cuda::CUDAStream s) : stream(s) {}
+  Pending(const Pending&) = delete;
+  ~Pending() {                  // never completed: the word is not handed out again before the kernel has written it
+    if (!read && word.defined())
+      try {
+        at::getHostAllocator(at::kCUDA)->record_event(word.data_ptr(), word.storage().data_ptr().get_context(), stream.unwrap());
+      } catch (...) {
+      }
+  }
+  int64_t count() {
+    event.synchronize();
+    read = true;
+    return *static_cast<const volatile int32_t*>(word.data_ptr());
+  }
 
   bool matches(const Tensor& zi, const Tensor& zp, const sph_geom& o) const {
     return zi.is_same(z_idx) && zp.is_same(z_ptr) && std::memcmp(&g, &o, sizeof(g)) == 0;
@@ -265,17 +283,17 @@ std::shared_ptr<Pending> strided_begin(const Tensor& z_idx, const Tensor& z_ptr,
                                        const Ints& k, const Ints& s, const Ints& p, const Ints& d, const Ints& tile) {
   check_index(z_idx, z_ptr);
   const c10::cuda::CUDAGuard guard(z_idx.device());
-  auto r = std::make_shared<Pending>();
+  auto r = std::make_shared<Pending>(at::cuda::getCurrentCUDAStream(z_idx.device().index()));
   r->g = geometry(B, in, out, k, s, p, d, tile);
   r->z_idx = z_idx;
   r->z_ptr = z_ptr;
   const int64_t nnz = z_idx.size(0);
   r->scratch = empty({check(abi.sph_rules_strided_scratch_bytes(&r->g, nnz))}, at::kByte, z_idx);
   r->oz_ptr = empty({B, out[0], out[1]}, at::kInt, z_idx);
-  r->d_count = empty({1}, at::kInt, z_idx);
-  check(abi.sph_rules_strided_count_async(ints(z_idx), ints(z_ptr), nnz, &r->g, ptr(r->scratch), ints(r->oz_ptr),
-                                          ints(r->d_count), &r->word, stream_of(z_idx)));
-  r->event.record(at::cuda::getCurrentCUDAStream(z_idx.device().index()));
+  r->word = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  check(abi.sph_rules_strided_count(ints(z_idx), ints(z_ptr), nnz, &r->g, ptr(r->scratch), ints(r->oz_ptr), ints(r->word),
+                                    nullptr, r->stream.stream()));
+  r->event.record(r->stream);
   return r;
 }
 
@@ -291,11 +309,11 @@ py::tuple strided_rules(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, con
   Lists l = make_lists(g, nnz, z_idx, materialize);
   Padding padding(l.rules, fill);
   Tensor nbr_t = transposed ? empty({kv, nnz}, at::kInt, z_idx) : Tensor();
+  int64_t n_out;
   {
     py::gil_scoped_release release;
-    pending->event.synchronize();
+    n_out = pending->count();
   }
-  const int64_t n_out = *const_cast<volatile const int32_t*>(pending->word);
   defer = defer && materialize && n_out > 0;
   Tensor oz_idx = empty({n_out}, at::kInt, z_idx);
   Tensor nbr = empty({kv, n_out}, at::kInt, z_idx);

@@ -13,6 +13,8 @@
 //  * the same pass fills the neighbour tables nbr[k][out] / nbr_t[k][in] the convolution kernels read.
 #include <atomic>
 #include <mutex>
+#include <new>
+#include <vector>
 
 #include "common.cuh"
 
@@ -633,7 +635,7 @@ rule_lists_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int t
 // ---------------------------------------------------------------------------------------------
 // Strided conv: output sparsity pattern.
 // Per output column a depth bitmask (ceil(oD/32) words) = OR over the KH*KW input columns that reach it
-// of the shifted/strided depth bits; popcount = column count; a three-kernel scan gives oz_ptr.
+// of the shifted/strided depth bits; popcount = column count; a scan gives oz_ptr.
 // ---------------------------------------------------------------------------------------------
 constexpr int kScanThreads = 256;
 
@@ -1264,41 +1266,79 @@ ColMask strided_colmask(const Geom& g, int64_t nnz, const StridedScratch& l, con
 // The host needs the output row count before it can size the outputs.  A cudaMemcpyAsync of those 4 bytes
 // would queue on the device-to-host copy engine behind whatever bulk copy another stream has in flight there
 // (measured: a result read-back of 90 MB on a side stream delayed it by milliseconds); instead the scan kernel
-// writes the count to a word of mapped pinned host memory.  A small ring of words per device, allocated on first
-// use, keeps concurrent calls apart.
+// writes the count to a word of mapped pinned host memory.  A call that waits for its words takes them from a list per
+// device and gives them back; a call that hands its word to the caller takes it from a ring, which the waiting calls do not
+// turn.
 namespace {
 constexpr int kCountSlots = 256;
+constexpr int kMaxDevices = 64;
 struct CountRing {
-  int32_t* host = nullptr;
-  int32_t* dev = nullptr;
+  HostWord first = {nullptr, nullptr};
   unsigned next = 0;          // per device: a word is reused only after kCountSlots - 1 further calls on ITS device
 };
-}  // namespace
-namespace sph {
-int count_slot(int32_t** host_word, int32_t** dev_word) {
-  constexpr int kMaxDevices = 64;
-  static CountRing rings[kMaxDevices];
-  static std::mutex mu;
-  int dev = 0;
-  SPH_CUDA(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= kMaxDevices) {
-    set_error("device ordinal %d not supported", dev);
+std::mutex words_mutex;
+std::vector<HostWord> free_words[kMaxDevices];
+
+int device_index(int* dev) {
+  SPH_CUDA(cudaGetDevice(dev));
+  if (*dev < 0 || *dev >= kMaxDevices) {
+    set_error("device ordinal %d not supported", *dev);
     return SPH_ERR_LIMIT;
   }
-  std::lock_guard<std::mutex> lock(mu);
-  CountRing& r = rings[dev];
-  if (r.host == nullptr) {
-    void* h = nullptr;
-    SPH_CUDA(cudaHostAlloc(&h, kCountSlots * sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
-    void* d = nullptr;
-    SPH_CUDA(cudaHostGetDevicePointer(&d, h, 0));
-    r.host = (int32_t*)h;
-    r.dev = (int32_t*)d;
-  }
-  const unsigned slot = r.next++ % kCountSlots;
-  *host_word = r.host + slot;
-  *dev_word = r.dev + slot;
   return SPH_OK;
+}
+
+int map_words(HostWord* first) {           // kCountSlots of them
+  void *h = nullptr, *d = nullptr;
+  SPH_CUDA(cudaHostAlloc(&h, kCountSlots * sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+  SPH_CUDA(cudaHostGetDevicePointer(&d, h, 0));
+  *first = {(int32_t*)h, (int32_t*)d};
+  return SPH_OK;
+}
+
+int ring_word(HostWord* w) {
+  static CountRing rings[kMaxDevices];
+  int dev = 0;
+  int rc = device_index(&dev);
+  if (rc != SPH_OK) return rc;
+  std::lock_guard<std::mutex> lock(words_mutex);
+  CountRing& r = rings[dev];
+  if (r.first.host == nullptr && (rc = map_words(&r.first)) != SPH_OK) return rc;
+  const unsigned slot = r.next++ % kCountSlots;
+  *w = {r.first.host + slot, r.first.dev + slot};
+  return SPH_OK;
+}
+}  // namespace
+namespace sph {
+int take_host_word(HostWord* w) {
+  int dev = 0;
+  int rc = device_index(&dev);
+  if (rc != SPH_OK) return rc;
+  std::lock_guard<std::mutex> lock(words_mutex);
+  static size_t made[kMaxDevices];
+  std::vector<HostWord>& list = free_words[dev];
+  if (list.empty()) {
+    HostWord first;
+    if ((rc = map_words(&first)) != SPH_OK) return rc;
+    try {
+      list.reserve(made[dev] + kCountSlots);         // room for all there are: giving one back allocates nothing
+    } catch (const std::bad_alloc&) {
+      set_error("out of host memory");
+      return SPH_ERR_LIMIT;
+    }
+    made[dev] += kCountSlots;
+    for (int i = 0; i < kCountSlots; ++i) list.push_back({first.host + i, first.dev + i});
+  }
+  *w = list.back();
+  list.pop_back();
+  return SPH_OK;
+}
+
+void give_host_word(const HostWord& w) {
+  int dev = 0;
+  if (device_index(&dev) != SPH_OK) return;
+  std::lock_guard<std::mutex> lock(words_mutex);
+  free_words[dev].push_back(w);
 }
 }  // namespace sph
 
@@ -1312,11 +1352,9 @@ extern "C" int64_t sph_rules_strided_scratch_bytes(const sph_geom* s, int64_t nn
 
 namespace {
 
-// Launches the kernels of step 1.  With want_host_word the scan also writes the count to a word of mapped pinned
-// host memory whose address is returned (readable once the work enqueued so far has completed).
+// Launches the kernels of step 1; the scan also writes the count to dev_word (mapped pinned host memory) if there is one.
 int strided_count_impl(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t nnz, const sph_geom* s, void* d_scratch,
-                       int32_t* d_oz_ptr, int32_t* d_out_nnz, bool want_host_word, int32_t** host_word_out,
-                       cudaStream_t st) {
+                       int32_t* d_oz_ptr, int32_t* d_out_nnz, int32_t* dev_word, cudaStream_t st) {
   Geom g;
   int rc = make_geom(s, &g);
   if (rc != SPH_OK) return rc;
@@ -1338,16 +1376,9 @@ int strided_count_impl(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t n
         d_z_idx, d_z_ptr, g, l.words, l.ncols, cm, mask, d_oz_ptr, blocksum);
     SPH_LAUNCH_CHECK();
   }
-  int32_t* host_word = nullptr;
-  int32_t* dev_word = nullptr;
-  if (want_host_word) {
-    rc = count_slot(&host_word, &dev_word);
-    if (rc != SPH_OK) return rc;
-  }
   scan_columns_kernel<<<(unsigned)div_up64(l.ncols, kScanCols), kScanThreads, 0, st>>>(d_oz_ptr, l.ncols, blocksum, per,
                                                                                        d_out_nnz, dev_word);
   SPH_LAUNCH_CHECK();
-  if (host_word_out) *host_word_out = host_word;
   return SPH_OK;
 }
 
@@ -1357,27 +1388,28 @@ extern "C" int sph_rules_strided_count(const int32_t* d_z_idx, const int32_t* d_
                                        const sph_geom* s, void* d_scratch, int32_t* d_oz_ptr, int32_t* d_out_nnz,
                                        int32_t* h_out_nnz, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
-  int32_t* host_word = nullptr;
-  int rc = strided_count_impl(d_z_idx, d_z_ptr, nnz, s, d_scratch, d_oz_ptr, d_out_nnz, h_out_nnz != nullptr,
-                              &host_word, st);
+  HostWord word = {nullptr, nullptr};
+  int rc = h_out_nnz ? take_host_word(&word) : SPH_OK;
   if (rc != SPH_OK) return rc;
+  rc = strided_count_impl(d_z_idx, d_z_ptr, nnz, s, d_scratch, d_oz_ptr, d_out_nnz, word.dev, st);
   if (h_out_nnz) {
     SPH_CUDA(cudaStreamSynchronize(st));
-    *h_out_nnz = *(volatile int32_t*)host_word;
+    if (rc == SPH_OK) *h_out_nnz = *(volatile int32_t*)word.host;
+    give_host_word(word);
   }
-  return SPH_OK;
+  return rc;
 }
 
 extern "C" int sph_rules_strided_count_async(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t nnz,
                                              const sph_geom* s, void* d_scratch, int32_t* d_oz_ptr,
                                              int32_t* d_out_nnz, const int32_t** h_count_word, void* stream) {
   SPH_CHECK_ARG(h_count_word != nullptr, "null argument");
-  int32_t* host_word = nullptr;
-  int rc = strided_count_impl(d_z_idx, d_z_ptr, nnz, s, d_scratch, d_oz_ptr, d_out_nnz, true, &host_word,
-                              (cudaStream_t)stream);
+  HostWord word;
+  int rc = ring_word(&word);
   if (rc != SPH_OK) return rc;
-  *h_count_word = host_word;
-  return SPH_OK;
+  rc = strided_count_impl(d_z_idx, d_z_ptr, nnz, s, d_scratch, d_oz_ptr, d_out_nnz, word.dev, (cudaStream_t)stream);
+  if (rc == SPH_OK) *h_count_word = word.host;
+  return rc;
 }
 
 extern "C" int sph_rules_strided_fill(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t nnz,

@@ -364,22 +364,23 @@ extern "C" int sph_voxelize_count(const float* d_sys_points, const int32_t* d_sc
   cudaStream_t st = (cudaStream_t)stream;
   const VoxScratch l = vox_layout(g, n_points);
   char* scratch = (char*)d_scratch;
-  int32_t *rows_host = nullptr, *rows_dev = nullptr, *cut_host = nullptr, *cut_dev = nullptr;
-  rc = count_slot(&rows_host, &rows_dev);
-  if (rc == SPH_OK) rc = count_slot(&cut_host, &cut_dev);
+  HostWord rows, was_cut;
+  rc = take_host_word(&rows);
   if (rc != SPH_OK) return rc;
-  *(volatile int32_t*)cut_host = 0;
+  rc = take_host_word(&was_cut);
+  if (rc != SPH_OK) return rc;
+  *(volatile int32_t*)was_cut.host = 0;
   std::atomic_thread_fence(std::memory_order_seq_cst);
-  rc = run_passes((const float4*)d_sys_points, d_scan_ptr, n_points, g, l, scratch, d_z_ptr, rows_dev, cut_dev, st);
-  if (rc != SPH_OK) return rc;
+  rc = run_passes((const float4*)d_sys_points, d_scan_ptr, n_points, g, l, scratch, d_z_ptr, rows.dev, was_cut.dev, st);
   SPH_CUDA(cudaStreamSynchronize(st));
-  if (*(volatile int32_t*)cut_host) {                  // rare: repeat without the points behind the cuts
-    rc = run_passes((const float4*)d_sys_points, d_scan_ptr, n_points, g, l, scratch, d_z_ptr, rows_dev, nullptr, st);
-    if (rc != SPH_OK) return rc;
+  if (rc == SPH_OK && *(volatile int32_t*)was_cut.host) {       // rare: repeat without the points behind the cuts
+    rc = run_passes((const float4*)d_sys_points, d_scan_ptr, n_points, g, l, scratch, d_z_ptr, rows.dev, nullptr, st);
     SPH_CUDA(cudaStreamSynchronize(st));
   }
-  *h_nnz = *(volatile int32_t*)rows_host;
-  return SPH_OK;
+  if (rc == SPH_OK) *h_nnz = *(volatile int32_t*)rows.host;
+  give_host_word(rows);
+  give_host_word(was_cut);
+  return rc;
 }
 
 extern "C" int sph_voxelize_fill(const float* d_points, int32_t point_stride, const float* d_sys_points,

@@ -317,3 +317,53 @@ def test_more_runs_per_tile_than_one_staging_pass(subm):
     assert_rules_equal(res, oz_idx, oz_ptr, rules, rule_size)
     assert_tables_match(res, rules, z_idx.shape[0], oz_idx.shape[0])
     assert check_status() & 1 == 0
+
+
+def _small(n, seed):
+    rng = np.random.default_rng(seed)
+    zi, zp = synthetic.make_random_occupancy(rng, 1, [6, 8, 10], 0.1 + 0.8 * (n % 7) / 7)
+    return to_dev(zi, zp)
+
+
+GEOM = (1, [6, 8, 10], [3, 4, 5], [3, 3, 3], [2, 2, 2], [1, 1, 1], [1, 1, 1], [2, 2])
+
+
+def test_many_rule_sets_begun_before_the_first_is_completed():
+    """Handles outlive any number of further calls, whatever those write their counts to; dropped ones harm nobody."""
+    from sphconv_b200.voxelize import VoxelGenerator
+    inputs = [_small(n, n) for n in range(600)]
+    begun = [ops.get_rules_begin(zi, zp, *GEOM) for zi, zp in inputs]
+    gen = VoxelGenerator([0, -40, -3, 70.4, 40, 1], [0, -45, 87.5, 70.4, 45, 100], 2, 100, [10, 8, 6], "spherical")
+    pts = torch.rand(200, 4, device=inputs[0][0].device) * 40
+    for n in range(200):
+        gen.generate(pts[: 100 + n % 50])
+        ops.get_rules_begin(*inputs[n], *GEOM)          # dropped at once
+    for n in list(range(0, 600, 37)) + [599]:
+        got = ops.get_rules(*inputs[n], *GEOM, pending=begun[n])
+        want = ops.get_rules(*inputs[n], *GEOM)
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), n
+
+
+def test_counts_handed_to_the_caller_are_not_turned_by_calls_that_wait():
+    """C ABI: a count word stays its caller's while waiting calls come and go."""
+    import ctypes
+
+    from sphconv_b200 import _capi as C
+    lib = C.lib()
+    zi, zp = _small(3, 3)
+    g = C.make_geom(GEOM[0], GEOM[1], GEOM[2], GEOM[3], GEOM[4], GEOM[5], GEOM[7], GEOM[6])
+    bytes_ = lib.sph_rules_strided_scratch_bytes(ctypes.byref(g), zi.numel())
+    new = lambda *s: torch.empty(s, dtype=torch.int32, device=zi.device)  # noqa: E731
+    scratch, oz_ptr, count = new(bytes_ // 4), new(1, 3, 4), new(1)
+    word = ctypes.c_void_p(0)
+    C.check(lib.sph_rules_strided_count_async(C.ptr(zi), C.ptr(zp), zi.numel(), ctypes.byref(g), C.ptr(scratch), C.ptr(oz_ptr),
+                                              C.ptr(count), ctypes.byref(word), C.stream_ptr(zi.device)))
+    torch.cuda.synchronize()
+    want = int(count)
+    empty = torch.zeros_like(zp)
+    h = ctypes.c_int32(-1)
+    for _ in range(300):
+        C.check(lib.sph_rules_strided_count(C.ptr(zi), C.ptr(empty), zi.numel(), ctypes.byref(g), C.ptr(scratch), C.ptr(oz_ptr),
+                                            C.ptr(count), ctypes.byref(h), C.stream_ptr(zi.device)))
+        assert h.value == 0
+    assert want > 0 and ctypes.c_int32.from_address(word.value).value == want
