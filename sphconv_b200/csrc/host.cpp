@@ -304,6 +304,10 @@ py::tuple strided_rules(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, con
   const sph_geom g = geometry(B, in, out, k, s, p, d, tile);
   if (!pending || !pending->matches(z_idx, z_ptr, g)) pending = strided_begin(z_idx, z_ptr, B, in, out, k, s, p, d, tile);
   const c10::cuda::CUDAGuard guard(z_idx.device());
+  const auto current = at::cuda::getCurrentCUDAStream(z_idx.device().index());
+  if (current != pending->stream)        // begun on another stream, whose allocator must not reuse them under this one's kernels
+    for (const Tensor& t : {pending->scratch, pending->oz_ptr})
+      c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), current);
   const int64_t nnz = z_idx.size(0), kv = k[0] * k[1] * k[2];
   // everything that does not need the row count is made before the wait for it
   Lists l = make_lists(g, nnz, z_idx, materialize);

@@ -367,3 +367,26 @@ def test_counts_handed_to_the_caller_are_not_turned_by_calls_that_wait():
                                             C.ptr(count), ctypes.byref(h), C.stream_ptr(zi.device)))
         assert h.value == 0
     assert want > 0 and ctypes.c_int32.from_address(word.value).value == want
+
+
+def test_rule_set_begun_on_another_stream():
+    """What a handle holds is not reused on the stream it was begun on while the completing stream still reads it."""
+    rng = np.random.default_rng(8)
+    B, shape, out = 2, [64, 256, 64], [32, 128, 32]
+    zi, zp = to_dev(*synthetic.make_random_occupancy(rng, B, shape, 0.05))
+    args = (zi, zp, B, shape, out, [3, 3, 3], [2, 2, 2], [1, 1, 1], [1, 1, 1], [2, 2])
+    want = ops.get_rules(*args)
+    torch.cuda.synchronize()
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.stream(s1):
+        handle = ops.get_rules_begin(*args)
+    with torch.cuda.stream(s2):
+        a = torch.randn(4096, 4096, device=zi.device)
+        for _ in range(20):                     # the completing kernels wait behind these
+            a = a @ a * 1e-3
+        got = ops.get_rules(*args, pending=handle)
+    del handle
+    with torch.cuda.stream(s1):
+        spoil = [torch.full((1 << 16,), -1, dtype=torch.int32, device=zi.device) for _ in range(400)]
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, y) for x, y in zip(got, want)) and len(spoil) == 400
