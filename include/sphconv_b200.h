@@ -187,6 +187,8 @@ int sph_conv_uses_pair_kernel(int dtype, int32_t k_ch, int32_t n_ch);
  * the FFMA kernel).  No reference counterpart. */
 int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch);
 
+#define SPH_BIAS_IN_ROW_TYPE 0x10000
+
 /* out[r,:] = epilogue( sum_k rows[ nbr[k][r], : ] @ weight[k] )   for r in [0, n_out)
  * forward: ref rule_conv, src/sphconv/rule_conv.cu:286-336 (rows = feature, nbr = d_nbr, weight [KV,iC,oC]).
  * dgrad:   ref rule_conv_d_feature, src/sphconv/rule_conv.cu:520-575 (rows = d_out, nbr = d_nbr_t,
@@ -197,12 +199,13 @@ int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch);
  *   d_nbr       int32 [KV, n_out]
  *   flip_k      != 0: offset k reads table row KV-1-k (dgrad of an odd-kernel submanifold layer reuses the
  *               forward table this way)
- *   d_scale/d_bias  float [n_ch] or null; relu != 0 applies max(0,.) ; epilogue = relu(acc*scale + bias)
+ *   d_scale/d_bias  float [n_ch] or null; relu != 0 applies max(0,.) ; epilogue = relu(acc*scale + bias).  With
+ *               SPH_BIAS_IN_ROW_TYPE or-ed into relu, d_bias holds 16-bit values of the rows' dtype
  *   out_dtype   dtype of d_out [n_out, n_ch]; F32/F16/BF16 accumulate in fp32, I8 accumulates in int32
  *               and converts to float before the epilogue; I8 output rounds to nearest and saturates. */
 int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, const void* d_weight, const void* d_packed,
                     const int32_t* d_nbr, int64_t n_out, int32_t kv, int32_t k_ch, int32_t n_ch, int flip_k,
-                    const float* d_scale, const float* d_bias, int relu, void* d_out, int out_dtype,
+                    const float* d_scale, const void* d_bias, int relu, void* d_out, int out_dtype,
                     int32_t* d_status, void* stream);
 
 /* d_weight[k] (+)= rows[nbr[k][r], :]^T @ d_out[r, :] summed over r.

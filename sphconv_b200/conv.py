@@ -171,7 +171,10 @@ class Conv3d(Convolution):
             else:    # gradients into a caller's buffer, sections to time, or a transposed table still to be made
                 out_feature = ConvFunction.apply(feature, w, rules, rule_size, tile_grid_shape, n_out, bias, relu, master)
         else:
-            w, b = self._inference_weights(feature.dtype, bias)
+            w = self._inference_weight(feature.dtype)
+            b = None if bias is None else bias.detach()              # read in every call: a write through `.data` is seen
+            if b is not None and (b.dtype not in (torch.float32, feature.dtype) or not b.is_contiguous()):
+                b = b.float().contiguous()
             if profiling.is_active() or profiling.pair_counts is not None:
                 with profiling.section("conv:" + tag, iC=in_channels, oC=out_channels, n_in=feature.shape[0],
                                        n_out=oz_idx.shape[0], esize=feature.element_size()):
@@ -185,23 +188,22 @@ class Conv3d(Convolution):
         out_tensor.rule_cache = input.rule_cache
         return out_tensor
 
-    def _inference_weights(self, dtype, bias):
-        """Inference: the weight in the features' dtype (with its tensor-core image attached) and the float32 bias, kept
-        across calls while the parameters are unchanged."""
+    def _inference_weight(self, dtype):
+        """Inference: the weight in the features' dtype with its tensor-core image attached, kept across calls while the
+        parameter's version and storage are unchanged (a write through `.data` is not noticed).  The entry keeps the storage
+        it was made from, so that no other weight can come to lie at its address."""
         weight = self.weight
-        key = (weight._version, weight.data_ptr(), weight.dtype, dtype, None if bias is None else bias._version,
-               None if bias is None else bias.data_ptr())
+        key = (weight._version, weight.data_ptr(), weight.dtype, dtype)
         cached = getattr(self, "_w_cache", None)
         if cached is not None and cached[0] == key:
-            return cached[1], cached[2]
+            return cached[1]
         w = weight.detach().view((-1, self.in_channels, weight.shape[4]))
         if w.dtype != dtype and dtype != torch.int8:
             w = w.to(dtype)
         w = w.contiguous()
         ops._packed_weight(w)
-        b = None if bias is None else bias.detach().float()
-        self._w_cache = (key, w, b)
-        return w, b
+        self._w_cache = (key, w, weight.detach())
+        return w
 
 
 SparseConv3d = Conv3d

@@ -45,13 +45,13 @@ int conv_gather_generic(const void* rows, int64_t n_rows, const void* weight, co
                         int out_dtype, int* status, cudaStream_t st);
 // conv_ffma.cu
 int conv_gather_ffma(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
-                     int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                     int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                      int out_dtype, int* status, cudaStream_t st);
 int conv_wgrad_ffma(const void* rows, const void* dout, int dtype, int64_t n_rows, const int* nbr, int64_t n_out, int kv,
                     int K, int N, float* dw, int* status, cudaStream_t st);
 // conv_tc.cu
 int conv_gather_tc(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
-                   int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                   int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                    int out_dtype, int* status, cudaStream_t st);
 bool conv_tc_supported(int dtype, int kv, int K, int N);
 int64_t packed_weight_bytes(int dtype, int kv, int K, int N);
@@ -59,19 +59,19 @@ int pack_weight(const void* w, int dtype, int kv, int K, int N, void* packed, cu
 // conv_tc_rows.cu
 bool conv_tc_rows_supported(int dtype, int kv, int K, int N);
 int conv_gather_tc_rows(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
-                        int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                        int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                         int out_dtype, int* status, cudaStream_t st);
 // conv_strip.cu
 bool conv_strip_supported(int dtype, int kv, int K, int N);
 int64_t strip_filter_bytes(int dtype, int kv, int K, int N);
 int pack_strip_filter(const void* w, int dtype, int kv, int K, int N, void* packed, cudaStream_t st);
 int conv_gather_strip(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out, int kv,
-                    int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out, int out_dtype,
+                    int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out, int out_dtype,
                     int* status, cudaStream_t st);
 // conv_sparse.cu
 bool conv_sparse_supported(int dtype, int kv, int K, int N);
 int conv_gather_sparse(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
-                       int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                       int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                        int out_dtype, int* status, cudaStream_t st);
 
 bool conv_wgrad_pairs_supported(int dtype, int kv, int K, int N);
@@ -138,7 +138,7 @@ static bool out_dtype_ok(int dtype, int out_dtype) {
 
 extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, const void* d_weight,
                                const void* d_packed, const int32_t* d_nbr, int64_t n_out, int32_t kv, int32_t k_ch,
-                               int32_t n_ch, int flip_k, const float* d_scale, const float* d_bias, int relu,
+                               int32_t n_ch, int flip_k, const float* d_scale, const void* d_bias, int relu,
                                void* d_out, int out_dtype, int32_t* d_status, void* stream) {
   SPH_CHECK_ARG(n_rows >= 0 && n_out >= 0 && kv > 0 && k_ch > 0 && n_ch > 0, "bad sizes");
   SPH_CHECK_ARG(dtype >= SPH_F32 && dtype <= SPH_I8, "unknown dtype");
@@ -147,21 +147,25 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
   SPH_CHECK_ARG(d_nbr && d_out && (d_weight || d_packed), "null pointer");
   SPH_CHECK_ARG(n_rows == 0 || d_rows, "null rows");
   SPH_CHECK_ARG(n_rows < 0x7fffffffLL && n_out < 0x7fffffffLL, "row ids are 32-bit");
+  const bool bias_16 = relu & SPH_BIAS_IN_ROW_TYPE;
+  relu = (relu & ~SPH_BIAS_IN_ROW_TYPE) != 0;
+  SPH_CHECK_ARG(!bias_16 || dtype == SPH_F16 || dtype == SPH_BF16, "a bias in the rows' type needs 16-bit rows");
+  const Bias bias = {d_bias, bias_16 ? dtype : SPH_F32};
   cudaStream_t st = (cudaStream_t)stream;
   if (d_packed && runs_strip(dtype, kv, k_ch, n_ch)) {
     if ((((uintptr_t)d_rows | (uintptr_t)d_out) & 15u) == 0)
-      return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias, relu,
+      return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
                              d_out, out_dtype, d_status, st);
     d_packed = nullptr;      // its image is not the one the other tensor-core kernels read
   }
   // 64-byte rows: the form with the output row on the TMEM lane (absent neighbours masked, not copied) is the faster
   // of the two; wider rows are dense deep layers, where the transposed form issues half as many instructions
   if (d_packed && k_ch * dtype_bytes(dtype) == 64 && conv_tc_rows_supported(dtype, kv, k_ch, n_ch)) {
-    return conv_gather_tc_rows(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias,
+    return conv_gather_tc_rows(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias,
                                relu, d_out, out_dtype, d_status, st);
   }
   if (d_packed && conv_tc_supported(dtype, kv, k_ch, n_ch)) {
-    return conv_gather_tc(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias,
+    return conv_gather_tc(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias,
                           relu, d_out, out_dtype, d_status, st);
   }
   SPH_CHECK_ARG(d_weight, "the CUDA-core kernels need the unpacked weight");
@@ -169,13 +173,13 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
   // int8 rows of up to 16 channels) and small fp32 layers: the pair-compacting kernel (faster than the row-walking one from 1 to 22 neighbours per row)
   if (conv_sparse_supported(dtype, kv, k_ch, n_ch) &&
       ((((uintptr_t)d_rows | (uintptr_t)d_weight | (uintptr_t)d_out) & 15u) == 0)) {
-    return conv_gather_sparse(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias,
+    return conv_gather_sparse(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias,
                               relu, d_out, out_dtype, d_status, st);
   }
   if (dtype == SPH_I8)
-    return conv_gather_generic(d_rows, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias, relu,
+    return conv_gather_generic(d_rows, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, (const float*)d_bias, relu,
                                d_out, out_dtype, d_status, st);
-  return conv_gather_ffma(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, d_bias, relu,
+  return conv_gather_ffma(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
                           d_out, out_dtype, d_status, st);
 }
 

@@ -66,6 +66,24 @@ struct Geom {
   int tH, tW, tgH, tgW, nTile;
 };
 
+// Per-channel bias of a convolution's epilogue: float32, or 16-bit values as the parameter holds them (a float32 copy would have
+// to be made in every call, or would not see every write to the parameter).
+struct Bias {
+  const void* data;                 // or null: no bias
+  int dtype;                        // SPH_F32, SPH_F16 or SPH_BF16
+  // A kernel without 16-bit rows has no 16-bit bias.  The 16-bit load is the builtin one of an integer: that of a __half is
+  // an asm statement, which the compiler may move in front of the check for null.
+  template <bool MAY_BE_16_BIT>
+  __device__ __forceinline__ float at(int c) const {
+    if (data == nullptr) return 0.f;
+    if (MAY_BE_16_BIT && dtype != SPH_F32) {
+      const unsigned short bits = __ldg((const unsigned short*)data + c);
+      return dtype == SPH_F16 ? __half2float(__ushort_as_half(bits)) : __uint_as_float((unsigned)bits << 16);
+    }
+    return __ldg((const float*)data + c);
+  }
+};
+
 // Allows a kernel `limit` bytes of dynamic shared memory: what all its launches stay within, not what the launch at hand takes.
 // Threads launch one kernel with different sizes, and a bound lowered between another thread's call and its launch would
 // fail that launch.

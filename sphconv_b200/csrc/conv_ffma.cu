@@ -44,7 +44,7 @@ struct FfmaParams {
                                       // offsets; -1: it has none
   int w_vec;                          // filter rows can be read 4 elements at a time
   const float* scale;
-  const float* bias;
+  Bias bias;
   void* out;
   int* status;
 };
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
     const int r = e / nc, c = e % nc;
     float v = s_acc[r * (S::NP + 4) + c];
     if (p.scale) v *= __ldg(p.scale + n0 + c);
-    if (p.bias) v += __ldg(p.bias + n0 + c);
+    if (p.bias.data) v += p.bias.at<sizeof(T) == 2>(n0 + c);
     store_one(p.out, p.out_dtype, (r0 + r) * p.N + n0 + c, p.relu ? fmaxf(v, 0.f) : v);
   }
 }
@@ -427,7 +427,7 @@ __global__ void __launch_bounds__(kFewThreads, 2) conv_few_kernel(FfmaParams p) 
     for (int j = 0; j < 4; ++j) {
       float v = acc[j];
       if (p.scale) v *= __ldg(p.scale + c + j);
-      if (p.bias) v += __ldg(p.bias + c + j);
+      if (p.bias.data) v += p.bias.at<sizeof(T) == 2>(c + j);
       store_one(p.out, p.out_dtype, (r0 + row) * p.N + c + j, p.relu ? fmaxf(v, 0.f) : v);
     }
   }
@@ -685,7 +685,7 @@ int launch_wg_k(const FfmaWgradParams& p, int kv, cudaStream_t st) {
 }  // namespace
 
 int conv_gather_ffma(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
-                     int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                     int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                      int out_dtype, int* status, cudaStream_t st) {
   FfmaParams p;
   p.rows = rows; p.weight = weight; p.nbr = nbr;

@@ -38,7 +38,7 @@ struct SparseParams {
   int64_t n_rows, n_out, n_chunks;
   int kv, flip_k, relu, out_dtype;
   const float* scale;
-  const float* bias;
+  Bias bias;
   void* out;
   int* status;
 };
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kSpThreads, 4) conv_sparse_rows_kernel(SparseP
   }
   for (int c = threadIdx.x; c < OC; c += kSpThreads) {
     s_epi[c] = p.scale ? __ldg(p.scale + c) : 1.f;
-    s_epi[OC + c] = p.bias ? __ldg(p.bias + c) : 0.f;
+    s_epi[OC + c] = p.bias.at<sizeof(T) == 2>(c);
   }
   for (int e = lane; e < 32 * AS; e += 32) acc[e] = 0.f;
   __syncthreads();
@@ -594,7 +594,7 @@ bool conv_sparse_supported(int dtype, int kv, int K, int N) {
 }
 
 int conv_gather_sparse(const void* rows, int dtype, int64_t n_rows, const void* weight, const int* nbr, int64_t n_out,
-                       int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                       int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                        int out_dtype, int* status, cudaStream_t st) {
   if (!conv_sparse_supported(dtype, kv, K, N) || (out_dtype == SPH_I8 && dtype != SPH_I8)) {
     set_error("conv_gather_sparse: unsupported dtype/shape");

@@ -73,7 +73,7 @@ int pack_strip_filter(const void* w, int dtype, int kv, int K, int N, void* pack
 }
 
 int conv_gather_strip(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out, int kv,
-                      int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out, int out_dtype,
+                      int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out, int out_dtype,
                       int* status, cudaStream_t st) {
   Plan s;
   if (!plan(dtype, kv, K, N, &s)) {

@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
           for (int q = 0; q < 2; ++q) {
             const int c = (nn + i) * 8 + 2 * t + q;
             sc[i][q] = (p.scale && c < p.N) ? __ldg(p.scale + c) : 1.f;
-            bi[i][q] = (p.bias && c < p.N) ? __ldg(p.bias + c) : 0.f;
+            bi[i][q] = c < p.N ? p.bias.at<DT != SPH_I8>(c) : 0.f;
           }
 #pragma unroll
         for (int m = 0; m < MT; ++m)

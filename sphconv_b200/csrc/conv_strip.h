@@ -2,7 +2,7 @@
 #pragma once
 #include <stdint.h>
 
-#include <cuda_runtime.h>
+#include "common.cuh"
 
 namespace sph {
 
@@ -15,7 +15,7 @@ struct StripParams {
   int64_t n_rows, n_out;
   int kv, N, row_bytes, flip_k, relu, out_dtype;
   const float* scale;
-  const float* bias;
+  Bias bias;
   void* out;
   int* status;
   int filter_units;                       // 16-byte units of the image

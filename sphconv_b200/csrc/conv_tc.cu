@@ -56,7 +56,7 @@ struct TcParams {
   int flip_k;
   int is_i8, is_bf16;
   const float* scale;
-  const float* bias;
+  Bias bias;
   int relu;
   void* out;
   int out_dtype, out_esize;
@@ -251,7 +251,7 @@ __global__ void __maxnreg__(112) conv_gather_tc_kernel(TcParams p) {
     const int oc = p.MP == 64 ? (lane < 16 ? 16 * q + lane : -1) : 32 * q + lane;
     const bool has_oc = oc >= 0 && oc < p.N;
     const float sc = (has_oc && p.scale) ? __ldg(p.scale + oc) : 1.f;
-    const float bi = (has_oc && p.bias) ? __ldg(p.bias + oc) : 0.f;
+    const float bi = has_oc ? p.bias.at<!I8>(oc) : 0.f;
     const int row_pitch = p.N * p.out_esize;      // bytes of one output row
     for (int ti = 0; ti < my_tiles; ++ti) {
       const int buf = ti & 1;
@@ -374,7 +374,7 @@ int g_test_withhold = 0;
 }  // namespace
 
 int conv_gather_tc(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
-                   int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                   int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                    int out_dtype, int* status, cudaStream_t st) {
   if (!tc_shape_ok(dtype, kv, K, N)) {
     set_error("conv_gather_tc: unsupported dtype/shape");

@@ -55,7 +55,7 @@ struct RowsParams {
   int flip_k;
   int is_i8, is_bf16;
   const float* scale;
-  const float* bias;
+  Bias bias;
   int relu;
   void* out;
   int out_dtype, out_esize;
@@ -143,7 +143,7 @@ __global__ void __maxnreg__(112) conv_gather_rows_kernel(RowsParams p) {
 
   for (int c = tid; c < 128; c += kTcThreads) {
     s_epi[c] = (c < p.N && p.scale) ? __ldg(p.scale + c) : 1.f;
-    s_epi[128 + c] = (c < p.N && p.bias) ? __ldg(p.bias + c) : 0.f;
+    s_epi[128 + c] = c < p.N ? p.bias.at<!I8>(c) : 0.f;
   }
   if (tid == 0) {
     s_abort = 0;
@@ -369,7 +369,7 @@ bool shape_ok(int dtype, int kv, int K, int N) {
 bool conv_tc_rows_supported(int dtype, int kv, int K, int N) { return rowsform::shape_ok(dtype, kv, K, N); }
 
 int conv_gather_tc_rows(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
-                        int kv, int K, int N, int flip_k, const float* scale, const float* bias, int relu, void* out,
+                        int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
                         int out_dtype, int* status, cudaStream_t st) {
   using namespace rowsform;
   if (!shape_ok(dtype, kv, K, N)) {

@@ -404,15 +404,17 @@ Tensor conv_gather(const Tensor& rows, const Tensor& weight, const optional<Tens
   const int64_t kv = weight.size(0), k_ch = weight.size(1), n_ch = weight.size(2);
   if (rows.dim() != 2 || rows.size(1) != k_ch)
     fail("feature has " + std::to_string(rows.size(-1)) + " channels, weight expects " + std::to_string(k_ch));
+  const bool bias_16 = bias && rows.itemsize() == 2 && bias->scalar_type() == rows.scalar_type();
   for (const auto* v : {&scale, &bias})
-    if (*v && ((*v)->scalar_type() != at::kFloat || (*v)->numel() != n_ch)) fail("scale / bias must be float32 [out_channels]");
+    if (*v && (((*v)->scalar_type() != at::kFloat && !(v == &bias && bias_16)) || (*v)->numel() != n_ch))
+      fail("scale / bias must be float32 [out_channels] (the bias may have the features' 16-bit type)");
   Tensor out = empty({n_out, n_ch}, out_dtype.value_or(code == SPH_I8 ? at::kFloat : rows.scalar_type()), rows);
   if (n_out == 0) return out;
   const c10::cuda::CUDAGuard guard(rows.device());
   check(abi.sph_conv_gather(ptr(rows), code, rows.size(0), ptr(weight), ptr(packed), ints(nbr), n_out, (int32_t)kv,
-                            (int32_t)k_ch, (int32_t)n_ch, flip, static_cast<const float*>(ptr(scale)),
-                            static_cast<const float*>(ptr(bias)), relu, ptr(out), dtype_code(out, "output"), status_of(rows),
-                            stream_of(rows)));
+                            (int32_t)k_ch, (int32_t)n_ch, flip, static_cast<const float*>(ptr(scale)), ptr(bias),
+                            (relu ? 1 : 0) | (bias_16 ? SPH_BIAS_IN_ROW_TYPE : 0), ptr(out), dtype_code(out, "output"),
+                            status_of(rows), stream_of(rows)));
   return out;
 }
 

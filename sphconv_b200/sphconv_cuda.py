@@ -173,7 +173,8 @@ def rule_conv(feature: torch.Tensor, weight: torch.Tensor, rules, ruleSize, outN
               scale: Optional[torch.Tensor] = None, bias: Optional[torch.Tensor] = None, relu: bool = False,
               out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """ref: rule_conv, src/sphconv/rule_conv.cu:286-336.  feature [NNZ,iC], weight [KV,iC,oC] ->
-    [outNNZ,oC].  Keyword arguments are extensions (fused epilogue relu(acc*scale + bias), output dtype)."""
+    [outNNZ,oC].  Keyword arguments are extensions (fused epilogue relu(acc*scale + bias), output dtype); `scale` is
+    float32, `bias` float32 or of the features' 16-bit type."""
     tb = _tables_for(rules, ruleSize, feature.shape[0], int(outNNZ), need_t=False)
     out = _gather(feature, weight, tb.nbr, int(outNNZ), False, scale, bias, relu, out_dtype)
     if getattr(rules, "_sph_ready", None) is not None:

@@ -263,3 +263,41 @@ def test_first_use_from_many_threads():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     got = subprocess.run([sys.executable, "-c", FIRST_USE, root], capture_output=True, text=True, timeout=300)
     assert got.returncode == 0 and "status seen" in got.stdout, got.stderr[-2000:]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_bias_written_in_place_is_seen_at_inference(dtype):
+    """The bias is read in every call, also after a write that leaves the parameter's version as it was."""
+    rng = np.random.default_rng(4)
+    zi, zp = (torch.as_tensor(a, device=DEV) for a in synthetic.make_random_occupancy(rng, 1, [5, 6, 7], 0.4))
+    layer = sphconv.SubMConv3d(16, 32, 3, bias=True, apply_bias=True).to(DEV).to(dtype).eval()
+    x = torch.zeros(zi.numel(), 16, device=DEV, dtype=dtype)
+    with torch.no_grad():
+        for value in (0.25, -3.0):
+            layer.bias.data.fill_(value)
+            y = layer(sphconv.SparseConvTensor(x, [5, 6, 7], 1, z_idx=zi, z_ptr=zp))
+            assert torch.equal(y.feature, torch.full_like(y.feature, value))
+
+
+@pytest.mark.parametrize("K,N", [(4, 16), (16, 16), (32, 64), (64, 64), (128, 128), (24, 40), (5, 7), (48, 48), (100, 9), (33, 130)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_bias_in_the_type_of_the_rows(K, N, dtype):
+    """A 16-bit bias gives what its float32 values give, bit for bit, in each kernel that has an epilogue; other types of bias
+    are refused."""
+    from sphconv_b200 import sphconv_cuda as ops
+    g = torch.Generator(device=DEV).manual_seed(K * N)
+    n = 1000
+    nbr = torch.randint(0, n, (27, n), generator=g, device=DEV, dtype=torch.int32)
+    nbr[torch.rand(27, n, generator=g, device=DEV) < 0.9] = -1
+    w = torch.randn(27, K, N, generator=g, device=DEV).to(dtype)
+    x = torch.randn(n, K, generator=g, device=DEV).to(dtype)
+    bias = torch.randn(N, generator=g, device=DEV).to(dtype)
+    plain = ops._gather(x, w, nbr, n, False, None, None, False, None)
+    for relu in (False, True):
+        a, b = (ops._gather(x, w, nbr, n, False, None, v, relu, None) for v in (bias, bias.float()))
+        assert torch.equal(a, b) and not torch.equal(a, plain)
+    for other in (bias.double(), bias.to(torch.bfloat16 if dtype == torch.float16 else torch.float16)):
+        with pytest.raises(RuntimeError):
+            ops._gather(x, w, nbr, n, False, None, other, False, None)
+    with pytest.raises(RuntimeError):
+        ops._gather(x.float(), w.float(), nbr, n, False, None, bias, False, None)
