@@ -152,12 +152,11 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
   SPH_CHECK_ARG(!bias_16 || dtype == SPH_F16 || dtype == SPH_BF16, "a bias in the rows' type needs 16-bit rows");
   const Bias bias = {d_bias, bias_16 ? dtype : SPH_F32};
   cudaStream_t st = (cudaStream_t)stream;
-  if (d_packed && runs_strip(dtype, kv, k_ch, n_ch)) {
-    if ((((uintptr_t)d_rows | (uintptr_t)d_out) & 15u) == 0)
-      return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
+  // the tensor-core kernels copy 16 bytes at a time
+  if (((uintptr_t)d_rows | (uintptr_t)d_packed | (uintptr_t)d_out) & 15u) d_packed = nullptr;
+  if (d_packed && runs_strip(dtype, kv, k_ch, n_ch))
+    return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
                              d_out, out_dtype, d_status, st);
-    d_packed = nullptr;      // its image is not the one the other tensor-core kernels read
-  }
   // 64-byte rows: the form with the output row on the TMEM lane (absent neighbours masked, not copied) is the faster
   // of the two; wider rows are dense deep layers, where the transposed form issues half as many instructions
   if (d_packed && k_ch * dtype_bytes(dtype) == 64 && conv_tc_rows_supported(dtype, kv, k_ch, n_ch)) {
@@ -192,16 +191,17 @@ extern "C" int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype,
   if (zero_init) SPH_CUDA(cudaMemsetAsync(d_dweight, 0, (size_t)kv * k_ch * n_ch * sizeof(float), st));
   if (n_out == 0 || n_rows == 0) return SPH_OK;
   SPH_CHECK_ARG(d_rows && d_dout && d_nbr, "null pointer");
+  const bool aligned = (((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0;      // copies of 16 bytes
   // the pairs' kernel up to 2048 gradients an offset (1.1 to 3 times faster than the tcgen05 kernel from 1.5 to 12 pairs a row);
   // at 64 x 64, the deep and dense levels, the tcgen05 kernel (22 pairs of 27: 0.70 against 1.19 ms on 1.4 M rows)
   if (conv_wgrad_strip_supported(dtype, k_ch, n_ch) &&
-      (k_ch * n_ch <= 2048 || !conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch)) &&
+      (k_ch * n_ch <= 2048 || !aligned || !conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch)) &&
       ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 3u) == 0))
     return conv_wgrad_strip(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
-  if (conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch))
+  if (aligned && conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch))
     return conv_wgrad_tc(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
   // small fp32 layers: the pair-compacting walk
-  if (dtype == SPH_F32 && conv_wgrad_pairs_supported(dtype, kv, k_ch, n_ch) && ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0))
+  if (dtype == SPH_F32 && aligned && conv_wgrad_pairs_supported(dtype, kv, k_ch, n_ch))
     return conv_wgrad_pairs(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
   return conv_wgrad_ffma(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
 }

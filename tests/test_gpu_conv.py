@@ -181,3 +181,36 @@ def test_forward_many_blocks(dtype, iC, oC):
         ref = conv_np.conv_forward(feat.double().cpu().numpy(), w.double().cpu().numpy(), pairs, n)
         _close(out, ref, TOL[dtype])
     assert check_status() == 0
+
+
+@pytest.mark.parametrize("K,N", [(16, 16), (16, 32), (32, 64), (64, 64), (64, 32), (128, 64), (128, 128)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.int8])
+@pytest.mark.parametrize("shift", [1, 2, 4])
+def test_rows_off_a_16_byte_boundary(K, N, dtype, shift):
+    """Rows (and gradients) that start 1, 2 or 4 elements behind a 16-byte boundary, at the widths of the tensor-core kernels:
+    what the same rows give from a fresh allocation, or - 128 channels have one weight-gradient kernel - a refusal."""
+    g = torch.Generator(device=DEV).manual_seed(K + N)
+    n = 700
+    nbr = torch.randint(0, n, (27, n), generator=g, device=DEV, dtype=torch.int32)
+    nbr[torch.rand(27, n, generator=g, device=DEV) < 0.8] = -1
+
+    def rows(width):
+        v = torch.randn(n * width + shift, generator=g, device=DEV) * 8
+        return v.to(dtype)[shift:].view(n, width)
+
+    x, d = rows(K), rows(N)
+    w = (torch.randn(27, K, N, generator=g, device=DEV) * (8 if dtype == torch.int8 else 0.1)).to(dtype)
+    got, want = (ops._gather(v, w, nbr, n, False, None, None, False, torch.float32) for v in (x, x.clone()))
+    # other kernels, the same products: fp32 sums in another order
+    assert float((got - want).abs().max()) <= (0.0 if dtype == torch.int8 else 1e-4) * float(want.abs().max())
+    if dtype == torch.int8 or K * N > 128 * 64:        # no weight gradient
+        return
+    host = ops.C.host()
+    want = host.conv_wgrad(x.clone(), d.clone(), nbr, None, False)
+    try:
+        got = host.conv_wgrad(x, d, nbr, None, False)
+    except RuntimeError:
+        assert max(K, N) > 64
+        return
+    assert float((got - want).abs().max()) <= 1e-4 * float(want.abs().max())
+    assert check_status() == 0
