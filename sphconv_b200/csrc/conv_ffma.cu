@@ -315,9 +315,13 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
 constexpr int kFewThreads = 512;
 constexpr int kFewWords = 11;         // 32 offsets a word
 
+// 16-bit values by the builtin load of an integer: the one of a __half is an asm statement, which the compiler may move in
+// front of the check that guards it.
 __device__ __forceinline__ float load_f(const float* p) { return __ldg(p); }
-__device__ __forceinline__ float load_f(const __half* p) { return __half2float(__ldg(p)); }
-__device__ __forceinline__ float load_f(const __nv_bfloat16* p) { return __bfloat162float(__ldg(p)); }
+__device__ __forceinline__ float load_f(const __half* p) { return __half2float(__ushort_as_half(__ldg((const unsigned short*)p))); }
+__device__ __forceinline__ float load_f(const __nv_bfloat16* p) {
+  return __uint_as_float((uint32_t)__ldg((const unsigned short*)p) << 16);
+}
 
 __device__ __forceinline__ void load_f4(const float* p, float (&v)[4]) {
   const float4 t = __ldg((const float4*)p);
