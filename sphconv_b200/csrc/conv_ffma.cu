@@ -42,6 +42,7 @@ struct FfmaParams {
   int kv, K, N, flip_k, relu, out_dtype;
   int few, few_first;                 // conv_few_kernel's tiles: at most so many pairs, at most so many at the first kBatch
                                       // offsets; -1: it has none
+  int walk_all;                       // conv_few_kernel takes every tile
   int w_vec;                          // filter rows can be read 4 elements at a time
   const float* scale;
   Bias bias;
@@ -312,8 +313,10 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
 // Rules and forward of a layer on 78 k rows of 1.5 neighbours, row walks for all tiles -> staged only -> both: 64 -> 64
 // 200 -> 220 -> 155 us, with stride 2 717 -> 537 -> 390; 37 -> 64 fp16 with stride 2 514 -> 623 -> 260.  A training step of the
 // fp32 encoder, whose deeper levels are dense, takes 11.8 ms either way.
+// Layers of which no tile is better staged (launch_ffma_cg says which) are walked in one launch that counts nothing.
+// The tile's table entries are read once, into shared memory, with a bit per present offset.
 constexpr int kFewThreads = 512;
-constexpr int kFewWords = 11;         // 32 offsets a word
+constexpr int kFewSmem = 200 * 1024;  // entries and bits of a tile: up to 387 offsets
 
 // 16-bit values by the builtin load of an integer: the one of a __half is an asm statement, which the compiler may move in
 // front of the check that guards it.
@@ -372,48 +375,49 @@ __device__ __forceinline__ void add_pair(const T* __restrict__ x, const T* __res
 
 template <typename T, bool XV, bool WV>
 __global__ void __launch_bounds__(kFewThreads, 2) conv_few_kernel(FfmaParams p) {
-  __shared__ unsigned s_present[kFewWords][kRows];   // bit k: the row has a neighbour at offset k
+  extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_count[kFewThreads / 32];
+  const int words = (p.kv + 31) / 32;
+  int* s_entry = (int*)smem;                         // [kv][kRows]
+  unsigned* s_present = (unsigned*)(s_entry + p.kv * kRows);   // [words][kRows], bit k: the row has a neighbour at offset k
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t r0 = (int64_t)blockIdx.x * kRows;
-  const int words = (p.kv + 31) / 32, first = min(kBatch, p.kv);
   const int r = tid % kRows;
+  for (int e = tid; e < words * kRows; e += kFewThreads) s_present[e] = 0u;
+  __syncthreads();
+  int n = 0;
   auto entry = [&](int k) {
     const int v = r0 + r < p.n_out ? __ldg(p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - k : k) * p.n_out + r0 + r) : -1;
-    if (v < p.n_rows) return v;
-    if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
-    return -1;
-  };
-  int n = 0;
-#pragma unroll
-  for (int h = 0; h < (kBatch * kRows + kFewThreads - 1) / kFewThreads; ++h) {
-    const int k = tid / kRows + h * (kFewThreads / kRows);
-    n += k < first && entry(k) >= 0;
-  }
-  n = __reduce_add_sync(0xffffffffu, n);
-  if (lane == 0) s_count[warp] = n;
-  for (int e = tid; e < words * kRows; e += kFewThreads) s_present[e / kRows][e % kRows] = 0;
-  __syncthreads();
-  n = 0;
-#pragma unroll
-  for (int w = 0; w < kFewThreads / 32; ++w) n += s_count[w];
-  if (n > p.few_first) return;
-  n = 0;
-#pragma unroll 7
-  for (int k = tid / kRows; k < p.kv; k += kFewThreads / kRows) {
-    if (entry(k) >= 0) {
-      atomicOr(&s_present[k / 32][r], 1u << (k & 31));
+    if (v >= p.n_rows) {
+      if (p.status) atomicOr(p.status, SPH_STATUS_BAD_INDEX);
+    } else if (v >= 0) {
+      s_entry[k * kRows + r] = v;
+      atomicOr(s_present + k / 32 * kRows + r, 1u << (k & 31));
       ++n;
     }
-  }
-  n = __reduce_add_sync(0xffffffffu, n);
-  __syncthreads();                                   // the first count has been read
-  if (lane == 0) s_count[warp] = n;
-  __syncthreads();
-  n = 0;
+  };
+  auto pairs = [&]() {                               // the CTA's, so far
+    const int mine = __reduce_add_sync(0xffffffffu, n);
+    __syncthreads();                                 // the last sum has been read
+    if (lane == 0) s_count[warp] = mine;
+    __syncthreads();
+    int sum = 0;
 #pragma unroll
-  for (int w = 0; w < kFewThreads / 32; ++w) n += s_count[w];
-  if (n > p.few) return;
+    for (int w = 0; w < kFewThreads / 32; ++w) sum += s_count[w];
+    return sum;
+  };
+  constexpr int STEP = kFewThreads / kRows;
+  const int first = p.walk_all ? 0 : min(kBatch, p.kv);
+  if (!p.walk_all) {
+#pragma unroll
+    for (int h = 0; h < (kBatch + STEP - 1) / STEP; ++h)
+      if (tid / kRows + h * STEP < first) entry(tid / kRows + h * STEP);
+    if (pairs() > p.few_first) return;
+  }
+#pragma unroll 7
+  for (int k = first + tid / kRows; k < p.kv; k += STEP) entry(k);
+  if (p.walk_all) __syncthreads();
+  else if (pairs() > p.few) return;
   const int groups = (p.N + 3) / 4;
   const int rows_here = (int)min((int64_t)kRows, p.n_out - r0);
   const T* weight = (const T*)p.weight;
@@ -421,9 +425,9 @@ __global__ void __launch_bounds__(kFewThreads, 2) conv_few_kernel(FfmaParams p) 
     const int row = e / groups, c = min(e % groups * 4, p.N - 4);   // the last two of an odd width share columns: the same values
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
     for (int w = 0; w < words; ++w) {
-      for (unsigned m = s_present[w][row]; m; m &= m - 1) {
+      for (unsigned m = s_present[w * kRows + row]; m; m &= m - 1) {
         const int k = w * 32 + __ffs(m) - 1;
-        const int i = __ldg(p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - k : k) * p.n_out + r0 + row);
+        const int i = s_entry[k * kRows + row];
         add_pair<T, XV, WV>((const T*)p.rows + (int64_t)i * p.K, weight + (int64_t)k * p.K * p.N + c, p.K, p.N, acc);
       }
     }
@@ -625,23 +629,50 @@ int launch_ffma(const FfmaParams& p, cudaStream_t st) {
   return SPH_OK;
 }
 
+template <typename T, bool XV, bool WV>
+int launch_few(const FfmaParams& p, int smem, cudaStream_t st) {
+  auto kern = conv_few_kernel<T, XV, WV>;
+  SPH_CUDA(allow_smem(kern, kFewSmem));
+  kern<<<(unsigned)div_up64(p.n_out, kRows), kFewThreads, smem, st>>>(p);
+  SPH_LAUNCH_CHECK();
+  return SPH_OK;
+}
+
 template <typename T, int KC, bool VEC>
 int launch_ffma_cg(FfmaParams p, cudaStream_t st) {
-  // Two pairs a row (odd widths, whose staging is dearer: 2.5), by a count of all offsets for the tiles that have few at the
-  // first ones.  (By the first ones alone the top row of a scan, which has no neighbours above it, would pass; by all of
-  // them alone every dense tile would pay for the count.)  A limit of three costs a 64 -> 64 training layer on 103 k rows
-  // 774 -> 984 us of convolution kernels.
-  // Rows of up to 16 channels and products of up to 8 are staged in any case: their steps are short.
-  const bool may_be_few = p.kv <= kFewWords * 32 && p.K > 16 && p.N > 8;
-  p.few = may_be_few ? (VEC ? kRows * 2 : kRows * 5 / 2) : -1;
-  p.few_first = p.kv <= kBatch ? p.few : kRows * 3 / 4;
   p.w_vec = p.N % 4 == 0 && ((uintptr_t)p.weight & (4 * sizeof(T) - 1)) == 0;
-  if (p.few >= 0) {
-    const unsigned tiles = (unsigned)div_up64(p.n_out, kRows);
-    if (VEC) conv_few_kernel<T, VEC, VEC><<<tiles, kFewThreads, 0, st>>>(p);
-    else if (p.w_vec) conv_few_kernel<T, false, true><<<tiles, kFewThreads, 0, st>>>(p);
-    else conv_few_kernel<T, false, false><<<tiles, kFewThreads, 0, st>>>(p);
-    SPH_LAUNCH_CHECK();
+  const bool x_vec = p.K % 4 == 0 && ((uintptr_t)p.rows & (4 * sizeof(T) - 1)) == 0;
+  const int sms = current_sm_count();
+  if (sms <= 0) return SPH_ERR_CUDA;
+  const int smem = (p.kv + (p.kv + 31) / 32) * kRows * 4;
+  // What a staged tile multiplies beyond its channels: K in steps of KC, N in tiles of 8, 16, 32 or 64.
+  const int np = p.N <= 8 ? 8 : p.N <= 16 ? 16 : p.N <= 32 ? 32 : div_up(p.N, 64) * 64;
+  const double waste = (double)(div_up(p.K, KC) * KC) / p.K * np / p.N;
+  const bool small = div_up64(p.n_out, kRows) <= 4 * (int64_t)sms;     // few CTAs to hide a CTA's steps behind
+  // All tiles are walked where padding makes every staged step dear: 16-bit rows (a conversion each; 48 -> 40 at 1.3 to 15 neighbours a
+  // row 872 -> 313 to 4207 -> 3239 us), float32 rows of 9 to 16 channels staged element by element (9 -> 16: 139 -> 87, 565 -> 432),
+  // small float32 layers (3 -> 16 on 23 k rows 48 -> 19, 24 -> 40 on 67 k rows 183 -> 122; on 531 k rows 939 -> 1119).
+  const bool can = p.N >= 4 && smem <= kFewSmem;
+  const bool padded = waste >= 1.5;
+  p.walk_all = can && padded && (sizeof(T) == 2 || (!VEC && p.K > 8 && p.K <= 16) || (small && (p.kv > kBatch || p.K > 8)));
+  // Else two pairs a row for 27 offsets (in large layers as many for an offset of larger filters: 32 -> 32 at 45 offsets and 2.5
+  // pairs a row 548 -> 452 us), by a count of all offsets for the tiles that have few at the first ones.  (By the first ones alone
+  // the top row of a scan, which has no neighbours above it, would pass; by all of them alone every dense tile would pay for the
+  // count.)  A limit of three costs a 64 -> 64 training layer on 103 k rows 774 -> 984 us of convolution kernels.  Large layers of
+  // 16-bit rows, staged at a conversion an element: four (64 -> 64 at 45 offsets and 2.5 pairs a row 1424 -> 802 us).  Rows of
+  // up to 16 channels and products of up to 8 are staged in any case: their steps are short.
+  p.few = p.few_first = -1;
+  if (can && !p.walk_all && p.K > 16 && p.N > 8) {
+    const double more = p.kv > 27 && !small ? p.kv / 27.0 : 1.0;
+    p.few = (int)(kRows * (sizeof(T) == 2 && !small ? 4 : (VEC ? 2 : 2.5) * more));
+    p.few_first = p.kv <= kBatch ? p.few : sizeof(T) == 2 && !small ? kRows * 3 / 2 : kRows * 3 / 4;
+  }
+  if (p.walk_all || p.few >= 0) {
+    int rc;
+    if (x_vec && p.w_vec) rc = launch_few<T, true, true>(p, smem, st);
+    else if (p.w_vec) rc = launch_few<T, false, true>(p, smem, st);
+    else rc = launch_few<T, false, false>(p, smem, st);
+    if (rc != SPH_OK || p.walk_all) return rc;
   }
   // the narrowest tile that holds the output channels; beyond 64 of them the grid repeats the rows per 64
   if (p.N <= 8) return launch_ffma<T, 1, KC, VEC>(p, st);

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from oracle import conv_np
+from sphconv_b200 import check_status
 from sphconv_b200 import sphconv_cuda as ops
 from test_gpu_conv import TOL, _close, _setup
 
@@ -50,3 +51,22 @@ def test_sparse_and_dense_tiles(iC, oC, dens, ks, dtype):
     rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(2, [17, 23, 16], True, dens, 5, iC, oC, dtype, ks)
     f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
     _close(ops.rule_conv(feat, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[dtype])
+
+
+@pytest.mark.parametrize("iC,oC,dtype", [(9, 16, torch.float32), (3, 16, torch.float32), (12, 40, torch.float32), (24, 40, torch.float32),
+                                         (33, 64, torch.float16), (48, 40, torch.bfloat16), (40, 130, torch.float16)])
+@pytest.mark.parametrize("dens,ks", [(0.03, (3, 3, 3)), (1.0, (3, 3, 3)), (0.3, (5, 5, 3)), (0.3, (1, 1, 1)), (0.1, (7, 7, 7))])
+def test_layers_walked_whole(iC, oC, dtype, dens, ks):
+    """Layers whose padding makes staging dear are walked whatever their tiles hold: kernel volumes of one to many words of
+    offsets, and an entry that is no row."""
+    rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(1, [11, 13, 9], True, dens, 5, iC, oC, dtype, ks)
+    f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
+    x = torch.cat([feat.new_zeros(1), feat.flatten()])[1:].view_as(feat)         # off a 16-byte boundary: no other kernel
+    _close(ops.rule_conv(x, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[dtype])
+    nbr = rules._sph.nbr.clone()
+    nbr[0][nbr[0] < 0] = n_in
+    got = ops._gather(x, w, nbr, n_out, False, None, None, False, None)
+    assert torch.equal(got, ops._gather(x, w, rules._sph.nbr, n_out, False, None, None, False, None))
+    if bool((rules._sph.nbr[0] < 0).any()):
+        with pytest.raises(RuntimeError):
+            check_status()
