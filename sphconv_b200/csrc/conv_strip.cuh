@@ -15,7 +15,7 @@
 //    the offsets in groups of 9: table entries of the group after next in flight, the next group's run being copied
 //    (16-byte cp.async, consecutive rows on different banks), the present group multiplied; one barrier per group;
 //  * the runs are found from the table itself (smallest and largest entry of a warp's rows, merged to at most two windows):
-//    any table is right.  A group whose rows do not fit the buffer reads its operands from global memory;
+//    any table is right.  Of a group whose rows do not fit the buffer every warp fetches its own, offset by offset;
 //  * offsets that none of a warp's 16-row tiles has are skipped; a row without a neighbour reads a row of zeros;
 //  * the order of sums is that of the tcgen05 kernels - offsets ascending, 32 bytes of a row per instruction, fp32 / int32
 //    accumulators - and so are the results, bit for bit.
@@ -306,35 +306,57 @@ __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) c
         if (tiles) multiply(k0 + o, tiles, [&](int m, int s, uint32_t (&f)[4]) { fetch(at[m], s, f); });
       }
     } else {
-      // the rows of this group are too far apart for a buffer: operands from global memory
-      const unsigned r = tile_row(here.ti) + (lane >> 2);
-      for (int o = 0; o < kGroup && k0 + o < p.kv; ++o) {
-        const int* src = p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - k0 - o : k0 + o) * p.n_out + r;
-        uint32_t tiles = 0u;
-        int e[MT][2];
+      // The rows of this group are too far apart for a buffer (filters whose nine offsets span several lines of columns, input
+      // gradients of strided layers): every warp fetches the rows of its own 32 into its share of the buffer the group does not
+      // use, up to three offsets at a time, the next ones' entries in flight with them.  (Fragments straight from global memory,
+      // four bytes a load and one offset behind the other: 3 x 3 x 1 16 -> 16 on 547 k rows 88 -> 62 us, 5 -> 7 131 -> 88; the 16-channel
+      // gradient of a strided layer 99 -> 61.)
+      const int share = p.cap / kWarps, held = min(share / WR, 3);           // rows; at least 320 / 8
+      const int mine = kZeroUnits + (j & 1) * buf_units + warp * share * pitch;
+      const unsigned r = tile_row(here.ti) + lane;
+      const int nk = min(kGroup, p.kv - k0);
+      int e[3];
+      auto entries = [&](int o0) {
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            e[m][h] = r + m * 16 + h * 8 < n_out ? __ldg(src + m * 16 + h * 8) : -1;
-            if ((unsigned)e[m][h] >= (unsigned)p.n_rows) e[m][h] = -1;
-          }
-          tiles |= (__any_sync(0xffffffffu, e[m][0] >= 0 || e[m][1] >= 0) ? 1u : 0u) << m;
+        for (int q = 0; q < 3; ++q) {
+          const int k = k0 + o0 + q;
+          e[q] = q < held && o0 + q < nk && r < n_out ? __ldg(p.nbr + (int64_t)(p.flip_k ? p.kv - 1 - k : k) * p.n_out + r) : -1;
+          if ((unsigned)e[q] >= (unsigned)p.n_rows) e[q] = -1;
         }
-        multiply(k0 + o, tiles, [&](int m, int s, uint32_t (&f)[4]) {
+      };
+      entries(0);
+      for (int o0 = 0; o0 < nk; o0 += held) {
+        uint32_t have[3];
 #pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int row = e[m][q & 1], byte = s * 32 + (q >> 1) * 16 + (lane & 3) * 4;
-            const uint8_t* src = p.rows + (int64_t)row * p.row_bytes + byte;
-            if (row < 0) f[q] = 0u;
-            else if (WHOLE || ((p.row_bytes & 3) == 0 && byte < p.row_bytes)) f[q] = __ldg((const uint32_t*)src);
-            else {
-              f[q] = 0u;
-              for (int i = 0; i < 4; ++i)
-                if (byte + i < p.row_bytes) f[q] |= (uint32_t)__ldg(src + i) << (8 * i);
+        for (int q = 0; q < 3; ++q) {
+          have[q] = __ballot_sync(0xffffffffu, e[q] >= 0);
+          if (e[q] >= 0) {
+            const uint8_t* src = p.rows + (int64_t)e[q] * p.row_bytes;
+            const uint32_t dst = smem0 + (mine + (q * WR + lane) * pitch) * 16;
+            if (WHOLE) {
+#pragma unroll
+              for (int u = 0; u < 2 * KS; ++u) cp_async_16(dst + u * 16, src + u * 16, 16u);
+            } else {
+              copy_ragged_row(src, p.row_bytes, dst);
             }
           }
-        });
+        }
+        entries(o0 + held);
+        cp_async_wait_all();
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          if (have[q] == 0u) continue;
+          uint32_t at[MT];
+#pragma unroll
+          for (int m = 0; m < MT; ++m) {
+            const int row = 16 * m + (lane & 15);
+            at[m] = operand0 + (have[q] >> row & 1u ? (uint32_t)(mine + (q * WR + row) * pitch) * 16u : 0u);
+          }
+          const uint32_t tiles = ((have[q] & 0xffffu) ? 1u : 0u) | ((have[q] >> 16) ? 2u : 0u);
+          multiply(k0 + o0 + q, tiles, [&](int m, int s, uint32_t (&f)[4]) { fetch(at[m], s, f); });
+        }
+        __syncwarp();
       }
     }
 

@@ -154,5 +154,25 @@ __device__ __forceinline__ void copy_ragged_rows(const uint8_t* rows, int64_t n_
   }
 }
 
+// One row of any width, by one thread, in the widest pieces that both sides allow (rows of a multiple of 16 bytes are 16-byte
+// aligned, and so on down).
+__device__ __forceinline__ void copy_ragged_row(const uint8_t* src, int bytes, uint32_t dst) {
+  if ((bytes & 15) == 0) {
+    for (int b = 0; b < bytes; b += 16) cp_async_16(dst + b, src + b, 16u);
+  } else if ((bytes & 7) == 0) {
+    for (int b = 0; b < bytes; b += 8) cp_async_8(dst + b, src + b);
+  } else if ((bytes & 3) == 0) {
+    for (int b = 0; b < bytes; b += 4) cp_async_4(dst + b, src + b);
+  } else if ((bytes & 1) == 0) {
+#pragma unroll 4
+    for (int b = 0; b < bytes; b += 2)
+      asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + b), "h"(__ldg((const uint16_t*)(src + b))) : "memory");
+  } else {
+#pragma unroll 4
+    for (int b = 0; b < bytes; ++b)
+      asm volatile("{.reg .b16 t; cvt.u16.u32 t, %1; st.shared.u8 [%0], t;}" ::"r"(dst + b), "r"((uint32_t)__ldg(src + b)) : "memory");
+  }
+}
+
 }  // namespace strip
 }  // namespace sph

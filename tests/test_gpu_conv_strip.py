@@ -9,7 +9,8 @@ import torch
 from sphconv_b200 import _capi as C
 from sphconv_b200 import check_status
 from sphconv_b200 import sphconv_cuda as ops
-from test_gpu_conv import TOL, _close
+from oracle import conv_np
+from test_gpu_conv import TOL, _close, _setup
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -113,4 +114,22 @@ def test_tables_of_more_than_2_to_the_32_entries(flip):
     got = ops._gather(x, w, nbr, n_out, flip, None, None, False, torch.float32)
     _close(got[at], _reference(x, w, some.flip(0) if flip else some), TOL[torch.float16])
     assert int(torch.count_nonzero(got)) == int(torch.count_nonzero(got[at]))
+    assert check_status() == 0
+
+
+@pytest.mark.parametrize("iC,oC", [(16, 16), (4, 16), (24, 40), (5, 7), (32, 64)])
+@pytest.mark.parametrize("ks,subm", [((3, 3, 1), True), ((3, 1, 3), True), ((3, 1, 1), True), ((3, 3, 3), False)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_filters_whose_groups_span_lines_of_columns(iC, oC, ks, subm, dtype):
+    """Nine consecutive offsets in three lines of 1500 rows, and input gradients of strided layers, in both directions."""
+    rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(1, [5, 300, 16], subm, 0.3, 17, iC, oC, dtype, ks)
+    f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
+    _close(ops.rule_conv(feat, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[dtype])
+    g = torch.as_tensor(rng.standard_normal((n_out, oC)), dtype=torch.float32).to(dtype).to(DEV)
+    g64 = g.double().cpu().numpy()
+    dx = ops.rule_conv_d_feature(g, w.permute(0, 2, 1).contiguous(), rules, rule_size, [3, 150], n_in)
+    _close(dx, conv_np.conv_dgrad(g64, w64, pairs, n_in), TOL[dtype])
+    dw = ops.rule_conv_d_weight(feat, g, rules, rule_size)
+    want = conv_np.conv_wgrad(f64, g64, pairs, int(np.prod(ks)))
+    assert np.abs(dw.double().cpu().numpy() - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
     assert check_status() == 0
