@@ -193,9 +193,10 @@ extern "C" int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype,
   SPH_CHECK_ARG(d_rows && d_dout && d_nbr, "null pointer");
   const bool aligned = (((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0;      // copies of 16 bytes
   // the pairs' kernel up to 2048 gradients an offset (1.1 to 3 times faster than the tcgen05 kernel from 1.5 to 12 pairs a row);
-  // at 64 x 64, the deep and dense levels, the tcgen05 kernel (22 pairs of 27: 0.70 against 1.19 ms on 1.4 M rows)
+  // at 64 x 64, the deep and dense levels, the tcgen05 kernel (22 pairs of 27: 0.70 against 1.19 ms on 1.4 M rows), and where fewer
+  // than nine offsets leave the former's warps idle (3 x 1 x 1: 32 -> 32 on 525 k rows 46 against 107 us)
   if (conv_wgrad_strip_supported(dtype, k_ch, n_ch) &&
-      (k_ch * n_ch <= 2048 || !aligned || !conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch)) &&
+      ((k_ch * n_ch <= 2048 && kv >= 9) || !aligned || !conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch)) &&
       ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 3u) == 0))
     return conv_wgrad_strip(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
   if (aligned && conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch))

@@ -12,6 +12,7 @@
 //    after next in flight, the next tile's rows being copied, the present tile multiplied; one barrier per tile;
 //  * the centre offset of a submanifold layer has a pair for every row, the others for a fifth: three more warps (nine warps
 //    leave room for twelve) take three quarters of the longest list, found on the CTA's first tile;
+//  * of a tile whose input rows lie too far apart for a buffer every warp fetches those of its own pairs;
 //  * more than 32 input channels are two launches' worth of CTAs, 32 channels each: the accumulators of 64 x 64 would spill;
 //  * a warp keeps its K x N gradient in registers over all its tiles and adds it to the fp32 gradient once, at the end (the
 //    reference writes [NTile,KV,iC,oC] partials and sums them, src/sphconv/rule_conv.cu:483-484,517).
@@ -41,6 +42,7 @@ struct WgradStripParams {
   int kv, K, N;
   int groups, halves, slices, tiles;       // halves: parts of 32 input channels
   int cap;                                // input rows a buffer holds
+  int x_piece;                            // bytes of a row of X that may be copied at a time
   int pairs_of_floats;                    // the gradient may be added to two floats at a time
   int* status;
 };
@@ -75,6 +77,21 @@ __device__ __forceinline__ void copy_rows(const uint8_t* tensor, int64_t n_rows,
   }
 }
 
+// n channels of one row by one thread; piece: bytes at a time (16, 8, 4 or 2).
+__device__ __forceinline__ void copy_channels(const uint16_t* src, int n, int piece, uint32_t to) {
+  const int bytes = n * 2;
+  if (piece == 16) {
+    for (int b = 0; b < bytes; b += 16) cp_async_16(to + b, (const uint8_t*)src + b, 16u);
+  } else if (piece == 8) {
+    for (int b = 0; b < bytes; b += 8) cp_async_8(to + b, (const uint8_t*)src + b);
+  } else if (piece == 4) {
+    for (int b = 0; b < bytes; b += 4) cp_async_4(to + b, (const uint8_t*)src + b);
+  } else {
+#pragma unroll 4
+    for (int c = 0; c < n; ++c) asm volatile("st.shared.u16 [%0], %1;" ::"r"(to + c * 2), "h"(__ldg(src + c)) : "memory");
+  }
+}
+
 // KT: tiles of 16 input channels, NP: pairs of 8-channel tiles of the output.
 template <int KT, int NP, int DT>
 __global__ void __launch_bounds__(kThreads, KT * NP <= 2 ? 2 : 1) conv_wgrad_strip_kernel(WgradStripParams p) {
@@ -100,6 +117,7 @@ __global__ void __launch_bounds__(kThreads, KT * NP <= 2 ? 2 : 1) conv_wgrad_str
   auto first_row = [&](int ti) { return ((int64_t)slice + (int64_t)ti * p.slices) * kRows; };
   const int* plane = p.nbr + (int64_t)(owner ? k : 0) * p.n_out;
   const unsigned lower = (1u << lane) - 1u;
+  const int share = p.cap / (kThreads / 32);               // rows of a buffer per warp: 32 at least
   bool bad = false;
 
   int e[kChunks];
@@ -209,35 +227,7 @@ __global__ void __launch_bounds__(kThreads, KT * NP <= 2 ? 2 : 1) conv_wgrad_str
 
     const uint32_t* list = s_lists + (list_of * 2 + slot) * kRows;
     const int n = s_count[slot * kGroup + list_of];
-#pragma unroll 1
-    for (int c = part * 16; c < n; c += parts * 16) {
-      const uint32_t ea = list[c + a_pair], eb = list[c + b_pair];
-      const uint32_t b_at = b_base + (eb >> 16) * 16;
-      uint32_t a[KT][4];
-      if (fit) {
-        const uint32_t a_at = a_base + (ea & 0xffffu) * 16;
-#pragma unroll
-        for (int m = 0; m < KT; ++m) ldmatrix4_trans(a[m], a_at + m * 32);
-      } else {
-        // the input rows of this tile are too far apart for a buffer: fragments from global memory
-        int row[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int idx = (int)(list[c + (q >> 1) * 8 + (lane & 3) * 2 + (q & 1)] & 0xffffu) - 1;
-          row[q] = idx < 0 ? -1 : __ldg(p.nbr + (int64_t)k * p.n_out + first_row(ti) + idx);
-          if ((unsigned)row[q] >= (unsigned)p.n_rows) row[q] = -1;
-        }
-#pragma unroll
-        for (int m = 0; m < KT; ++m)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int ch = m * 16 + (q & 1) * 8 + (lane >> 2);
-            auto value = [&](int r) {
-              return r >= 0 && ch < kc ? (uint32_t)__ldg((const uint16_t*)p.rows + (int64_t)r * p.K + ch0 + ch) : 0u;
-            };
-            a[m][q] = value(row[q & 2]) | value(row[(q & 2) + 1]) << 16;
-          }
-      }
+    auto products = [&](const uint32_t (&a)[KT][4], uint32_t b_at) {          // 16 pairs
 #pragma unroll
       for (int j = 0; j < NP; ++j) {
         uint32_t b[4];
@@ -247,6 +237,44 @@ __global__ void __launch_bounds__(kThreads, KT * NP <= 2 ? 2 : 1) conv_wgrad_str
           mma_step<DT>(acc[m][2 * j], a[m], b[0], b[1]);
           mma_step<DT>(acc[m][2 * j + 1], a[m], b[2], b[3]);
         }
+      }
+    };
+    if (fit) {
+#pragma unroll 1
+      for (int c = part * 16; c < n; c += parts * 16) {
+        const uint32_t ea = list[c + a_pair], eb = list[c + b_pair];
+        const uint32_t b_at = b_base + (eb >> 16) * 16, a_at = a_base + (ea & 0xffffu) * 16;
+        uint32_t a[KT][4];
+#pragma unroll
+        for (int m = 0; m < KT; ++m) ldmatrix4_trans(a[m], a_at + m * 32);
+        products(a, b_at);
+      }
+    } else {
+      // The input rows of this tile are too far apart for a buffer: every warp fetches those of its pairs into its share of the
+      // one the tile does not use, two steps at a time.  (Fragments straight from global memory, an element a load: 3 x 3 x 1
+      // 32 -> 32 on 531 k rows 187 -> 107 us.)
+      const int mine = x0 + slot * x_units + warp * share * PX;
+#pragma unroll 1
+      for (int c = part * 32; c < n; c += parts * 32) {
+        const int idx = c + lane < n ? (int)(list[c + lane] & 0xffffu) - 1 : -1;
+        int row = idx < 0 ? -1 : __ldg(p.nbr + (int64_t)k * p.n_out + first_row(ti) + idx);
+        if ((unsigned)row >= (unsigned)p.n_rows) row = -1;
+        const uint32_t have = __ballot_sync(0xffffffffu, row >= 0);
+        if (row >= 0)
+          copy_channels((const uint16_t*)p.rows + (int64_t)row * p.K + ch0, kc, p.x_piece, smem0 + (mine + lane * PX) * 16);
+        cp_async_wait_all();
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (c + h * 16 >= n) break;
+          const int i = h * 16 + a_pair;
+          const uint32_t a_at = a_base + (have >> i & 1u ? (uint32_t)(mine + i * PX) * 16u : 0u);
+          uint32_t a[KT][4];
+#pragma unroll
+          for (int m = 0; m < KT; ++m) ldmatrix4_trans(a[m], a_at + m * 32);
+          products(a, b_base + (list[c + h * 16 + b_pair] >> 16) * 16);
+        }
+        __syncwarp();
       }
     }
     post_run(slot);
@@ -293,6 +321,8 @@ int launch_wgrad_strip(WgradStripParams& p, cudaStream_t st) {
     cap = (kSmem - fixed_bytes(NP)) / (2 * PX * 16);
   }
   p.cap = (cap < 3 * kRows ? cap : 3 * kRows) & ~7;
+  static_assert((kSmem - (kZeroUnits + 2 * ((kRows * (2 * 4 + 1) + 7) & ~7)) * 16 - kGroup * 2 * kRows * 4 - 2 * kGroup * 20) /
+                        (2 * 5 * 16) >= 32 * (kThreads / 32), "a warp's share of a buffer holds the rows of two steps");
   const int smem = fixed_bytes(NP) + 2 * ((p.cap * PX + 7) & ~7) * 16;
   SPH_CUDA(allow_smem(kern, kSmem));
   const int sms = current_sm_count();
@@ -334,6 +364,9 @@ int conv_wgrad_strip(const void* rows, const void* dout, int dtype, int64_t n_ro
   p.groups = div_up(kv, kGroup);
   p.halves = div_up(K, 32);
   p.tiles = (int)div_up64(n_out, kRows);
+  // rows, and the halves of them that start 32 channels in, as wide as their addresses and lengths allow (K odd: single elements)
+  const uintptr_t at = (uintptr_t)rows | (uintptr_t)(K * 2);
+  p.x_piece = at & 2 ? 2 : at & 4 ? 4 : at & 8 ? 8 : 16;
   p.pairs_of_floats = N % 2 == 0 && ((uintptr_t)dw & 7u) == 0;
   const int kt = K <= 16 ? 1 : 2, np = N <= 16 ? 1 : N <= 32 ? 2 : 4;
   return dtype == SPH_F16 ? launch_wgrad_shape<SPH_F16>(p, kt, np, st) : launch_wgrad_shape<SPH_BF16>(p, kt, np, st);
