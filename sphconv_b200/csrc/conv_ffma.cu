@@ -650,11 +650,12 @@ int launch_ffma_cg(FfmaParams p, cudaStream_t st) {
   const double waste = (double)(div_up(p.K, KC) * KC) / p.K * np / p.N;
   const bool small = div_up64(p.n_out, kRows) <= 4 * (int64_t)sms;     // few CTAs to hide a CTA's steps behind
   // All tiles are walked where padding makes every staged step dear: 16-bit rows (a conversion each; 48 -> 40 at 1.3 to 15 neighbours a
-  // row 872 -> 313 to 4207 -> 3239 us), float32 rows of 9 to 16 channels staged element by element (9 -> 16: 139 -> 87, 565 -> 432),
+  // row 872 -> 313 to 4207 -> 3239 us; not with filter rows read by the element: 64 -> 33 at 9.4 3063 -> 5883), float32 rows of 9 to 16 channels staged element by element (9 -> 16: 139 -> 87, 565 -> 432),
   // small float32 layers (3 -> 16 on 23 k rows 48 -> 19, 24 -> 40 on 67 k rows 183 -> 122; on 531 k rows 939 -> 1119).
   const bool can = p.N >= 4 && smem <= kFewSmem;
   const bool padded = waste >= 1.5;
-  p.walk_all = can && padded && (sizeof(T) == 2 || (!VEC && p.K > 8 && p.K <= 16) || (small && (p.kv > kBatch || p.K > 8)));
+  p.walk_all = can && padded && ((p.w_vec && (sizeof(T) == 2 || (!VEC && p.K > 8 && p.K <= 16))) ||
+                                 (sizeof(T) == 4 && small && (p.kv > kBatch || p.K > 8)));
   // Else two pairs a row for 27 offsets (in large layers as many for an offset of larger filters: 32 -> 32 at 45 offsets and 2.5
   // pairs a row 548 -> 452 us), by a count of all offsets for the tiles that have few at the first ones.  (By the first ones alone
   // the top row of a scan, which has no neighbours above it, would pass; by all of them alone every dense tile would pay for the
@@ -663,9 +664,10 @@ int launch_ffma_cg(FfmaParams p, cudaStream_t st) {
   // up to 16 channels and products of up to 8 are staged in any case: their steps are short.
   p.few = p.few_first = -1;
   if (can && !p.walk_all && p.K > 16 && p.N > 8) {
-    const double more = p.kv > 27 && !small ? p.kv / 27.0 : 1.0;
-    p.few = (int)(kRows * (sizeof(T) == 2 && !small ? 4 : (VEC ? 2 : 2.5) * more));
-    p.few_first = p.kv <= kBatch ? p.few : sizeof(T) == 2 && !small ? kRows * 3 / 2 : kRows * 3 / 4;
+    const double more = p.kv > 27 && !small && sizeof(T) == 4 ? p.kv / 27.0 : 1.0;
+    const bool dear = sizeof(T) == 2 && !small && p.w_vec;
+    p.few = (int)(kRows * (dear ? 4 : VEC ? 2 : 2.5) * more);
+    p.few_first = p.kv <= kBatch ? p.few : dear ? kRows * 3 / 2 : kRows * 3 / 4;
   }
   if (p.walk_all || p.few >= 0) {
     int rc;
