@@ -221,22 +221,19 @@ def run_reference(args):
 
 
 def kernel_of(lib, dcode, kind, k_ch, n_ch, esize, dtype_name):
-    """Name of the kernel instantiation a conv / dgrad / wgrad layer launches (for grouping layers by kernel)."""
-    tc = bool(lib.sph_conv_uses_tensor_cores(dcode, k_ch, n_ch))
-    if kind == "wgrad":
-        which = lib.sph_conv_wgrad_kernel(dcode, k_ch, n_ch)
-        if esize == 2 and k_ch <= 64 and n_ch <= 64 and (k_ch * n_ch <= 2048 or which != 1):
-            return "conv_wgrad_strip_kernel", True
-        if which == 1:
-            return "conv_wgrad_tc_kernel<%d>" % (k_ch * esize // 16), True
-        return ("conv_wgrad_pairs_kernel<%d,%d>" % (k_ch, n_ch)) if which == 2 else "conv_wgrad_ffma_kernel", False
-    if not tc:
-        if lib.sph_conv_uses_pair_kernel(dcode, k_ch, n_ch):
-            return "conv_sparse_rows_kernel<%d,%d>" % (k_ch, n_ch), tc
-        return "conv_gather_generic_kernel" if dtype_name == "int8" else "conv_ffma_kernel", tc
-    # 64-byte rows run the form with the output row on the TMEM lane (conv_tc_rows.cu), wider rows the transposed one
-    name = "conv_gather_rows_kernel" if k_ch * esize == 64 and n_ch % 16 == 0 else "conv_gather_tc_kernel"
-    return "%s<%d,%s>" % (name, k_ch * esize // 16, "i8" if dtype_name == "int8" else "f16"), tc
+    """(name, on the tensor pipe) of the kernel a 3 x 3 x 3 conv / dgrad / wgrad layer launches, for grouping layers by kernel:
+    what the library's own dispatch answers."""
+    wgrad = kind == "wgrad"
+    kernel = lib.sph_conv_kernel(dcode, 27, k_ch, n_ch, int(wgrad))
+    row = k_ch * esize // 16                      # 16-byte pieces of a gathered row
+    typ = "i8" if dtype_name == "int8" else "f16"
+    if wgrad:
+        return {0: "conv_wgrad_ffma_kernel", 1: "conv_wgrad_tc_kernel<%d>" % row, 3: "conv_wgrad_strip_kernel<%d,%d>" % (k_ch, n_ch),
+                4: "conv_wgrad_pairs_kernel<%d,%d>" % (k_ch, n_ch)}[kernel], kernel in (1, 3)
+    return {0: "conv_gather_generic_kernel" if dtype_name == "int8" else "conv_ffma_kernel",
+            1: "conv_gather_tc_kernel<%d,%s>" % (row, typ), 2: "conv_gather_rows_kernel<%d,%s>" % (row, typ),
+            3: "conv_strip_kernel<%d,%d,%s>" % (k_ch, n_ch, typ),
+            4: "conv_sparse_rows_kernel<%d,%d>" % (k_ch, n_ch)}[kernel], kernel in (1, 2, 3)
 
 
 class Workload:
@@ -724,11 +721,16 @@ TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per output r
 BUSIEST_UNIT = {
     "conv_gather_rows_kernel<4,f16>": "shared-memory data pipe 92 % busy (gather writes 64 % + tensor-core operand reads 28 %); DRAM 12 %, tensor pipe 11 %",
     "conv_gather_tc_kernel<8,f16>": "shared-memory data pipe 88 % busy (gather writes 58 % + operand reads 30 %); tensor pipe 47 %, DRAM 8 %",
-    "conv_gather_tc_kernel<2,f16>": "shared-memory data pipe 69-93 % busy (gather writes 52-72 % + operand reads 17-22 %); DRAM 9-13 %",
-    "conv_sparse_rows_kernel<4,16>": "instruction issue 68 % of the slots; DRAM 15 %",
+    "conv_gather_tc_kernel<2,f16>": "shared-memory data pipe 93 % busy (gather writes 72 % + operand reads 22 %); DRAM 13 %",
+    "conv_sparse_rows_kernel<4,16>": "instruction issue 64 % of the slots; DRAM 13 %",
+    "conv_strip_kernel<16,16,f16>": "instruction issue 51 % of the slots; shared-memory data pipe 24 %, DRAM 13 %, tensor pipe 8 %",
+    "conv_wgrad_strip_kernel<16,16>": "instruction issue 68 % of the slots; shared-memory data pipe 40 %, DRAM 13 %",
+    "conv_wgrad_strip_kernel<32,32>": "shared-memory data pipe 43 %, instruction issue 41 % of the slots; DRAM 12 %, tensor pipe 15 %",
+    "conv_ffma_kernel": "shared-memory data pipe 74 %, instruction issue 66 % of the slots; FMA pipe 46 %, DRAM 2 %",
+    "conv_wgrad_ffma_kernel": "instruction issue 76 % of the slots; FMA pipe 55 %, DRAM 27 %",
 }
 TRAFFIC_BYTES_PER_OUT_ROW = {
-    "fp16": {"L0": 116.2, "L1": 141.3, "L2": 146.5, "L3": 211.3, "L4": 208.9, "L5": 288.9, "L6": 280.6, "L7": 281.1},
+    "fp16": {"L0": 116.2, "L1": 140.3, "L2": 146.5, "L3": 211.3, "L4": 208.9, "L5": 288.9, "L6": 280.6, "L7": 281.1},
 }
 
 if __name__ == "__main__":

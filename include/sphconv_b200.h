@@ -187,6 +187,16 @@ int sph_conv_uses_pair_kernel(int dtype, int32_t k_ch, int32_t n_ch);
  * the FFMA kernel).  No reference counterpart. */
 int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch);
 
+/* The kernel that sph_conv_gather (wgrad = 0; with the packed filter) or sph_conv_wgrad (wgrad = 1) runs for a combination of
+ * sizes when all operands are 16-byte aligned.  The three functions above sort widths into classes instead.
+ * No reference counterpart. */
+#define SPH_KERNEL_GENERAL 0 /* CUDA cores, any width: FFMA (int8: row by row) */
+#define SPH_KERNEL_TC 1      /* tcgen05 */
+#define SPH_KERNEL_TC_ROWS 2 /* tcgen05 with the output row on the TMEM lane */
+#define SPH_KERNEL_STRIP 3   /* mma.sync over staged runs of input rows */
+#define SPH_KERNEL_PAIRS 4   /* CUDA cores, narrow rows over compacted pairs */
+int sph_conv_kernel(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch, int wgrad);
+
 #define SPH_BIAS_IN_ROW_TYPE 0x10000
 
 /* out[r,:] = epilogue( sum_k rows[ nbr[k][r], : ] @ weight[k] )   for r in [0, n_out)

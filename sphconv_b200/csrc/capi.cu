@@ -130,6 +130,38 @@ extern "C" int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch) {
   return conv_wgrad_pairs_supported(dtype, 27, k_ch, n_ch) ? 2 : 0;
 }
 
+// The kernels that run; sph_conv_gather and sph_conv_wgrad switch on these.  packed: the caller passes the filter's image and all
+// operands are 16-byte aligned; aligned: the operands the kernel reads are (words: 4-byte aligned).
+static int gather_kernel(int dtype, int kv, int K, int N, bool packed, bool aligned) {
+  if (packed && runs_strip(dtype, kv, K, N)) return SPH_KERNEL_STRIP;
+  // 64-byte rows: the form with the output row on the TMEM lane (absent neighbours masked, not copied) is the faster
+  // of the two; wider rows are dense deep layers, where the transposed form issues half as many instructions
+  if (packed && K * dtype_bytes(dtype) == 64 && conv_tc_rows_supported(dtype, kv, K, N)) return SPH_KERNEL_TC_ROWS;
+  if (packed && conv_tc_supported(dtype, kv, K, N)) return SPH_KERNEL_TC;
+  // narrow rows the tensor-core kernels do not take (the first layer of an encoder: 4 or 8 channels in, a sparse level;
+  // int8 rows of up to 16 channels) and small fp32 layers: the pair-compacting kernel (faster than the row-walking one from 1 to
+  // 22 neighbours per row)
+  if (aligned && conv_sparse_supported(dtype, kv, K, N)) return SPH_KERNEL_PAIRS;
+  return SPH_KERNEL_GENERAL;
+}
+
+static int wgrad_kernel(int dtype, int kv, int K, int N, bool aligned, bool words) {
+  // the pairs' kernel up to 2048 gradients an offset (1.1 to 3 times faster than the tcgen05 kernel from 1.5 to 12 pairs a row);
+  // at 64 x 64, the deep and dense levels, the tcgen05 kernel (22 pairs of 27: 0.70 against 1.19 ms on 1.4 M rows), and where fewer
+  // than nine offsets leave the former's warps idle (3 x 1 x 1: 32 -> 32 on 525 k rows 46 against 107 us)
+  const bool tc = aligned && conv_wgrad_tc_supported(dtype, kv, K, N);
+  if (words && conv_wgrad_strip_supported(dtype, K, N) && ((K * N <= 2048 && kv >= 9) || !tc)) return SPH_KERNEL_STRIP;
+  if (tc) return SPH_KERNEL_TC;
+  // small fp32 layers: the pair-compacting walk
+  if (dtype == SPH_F32 && aligned && conv_wgrad_pairs_supported(dtype, kv, K, N)) return SPH_KERNEL_PAIRS;
+  return SPH_KERNEL_GENERAL;
+}
+
+extern "C" int sph_conv_kernel(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch, int wgrad) {
+  SPH_CHECK_ARG(dtype >= SPH_F32 && dtype <= SPH_I8 && kv > 0 && k_ch > 0 && n_ch > 0, "bad sizes");
+  return wgrad ? wgrad_kernel(dtype, kv, k_ch, n_ch, true, true) : gather_kernel(dtype, kv, k_ch, n_ch, true, true);
+}
+
 static bool out_dtype_ok(int dtype, int out_dtype) {
   if (out_dtype < SPH_F32 || out_dtype > SPH_I8) return false;
   if (out_dtype == SPH_I8 && dtype != SPH_I8) return false;
@@ -153,27 +185,24 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
   const Bias bias = {d_bias, bias_16 ? dtype : SPH_F32};
   cudaStream_t st = (cudaStream_t)stream;
   // the tensor-core kernels copy 16 bytes at a time
-  if (((uintptr_t)d_rows | (uintptr_t)d_packed | (uintptr_t)d_out) & 15u) d_packed = nullptr;
-  if (d_packed && runs_strip(dtype, kv, k_ch, n_ch))
-    return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
-                             d_out, out_dtype, d_status, st);
-  // 64-byte rows: the form with the output row on the TMEM lane (absent neighbours masked, not copied) is the faster
-  // of the two; wider rows are dense deep layers, where the transposed form issues half as many instructions
-  if (d_packed && k_ch * dtype_bytes(dtype) == 64 && conv_tc_rows_supported(dtype, kv, k_ch, n_ch)) {
-    return conv_gather_tc_rows(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias,
-                               relu, d_out, out_dtype, d_status, st);
-  }
-  if (d_packed && conv_tc_supported(dtype, kv, k_ch, n_ch)) {
-    return conv_gather_tc(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias,
-                          relu, d_out, out_dtype, d_status, st);
-  }
-  SPH_CHECK_ARG(d_weight, "the CUDA-core kernels need the unpacked weight");
-  // narrow rows the tensor-core kernels do not take (the first layer of an encoder: 4 or 8 channels in, a sparse level;
-  // int8 rows of up to 16 channels) and small fp32 layers: the pair-compacting kernel (faster than the row-walking one from 1 to 22 neighbours per row)
-  if (conv_sparse_supported(dtype, kv, k_ch, n_ch) &&
-      ((((uintptr_t)d_rows | (uintptr_t)d_weight | (uintptr_t)d_out) & 15u) == 0)) {
-    return conv_gather_sparse(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias,
-                              relu, d_out, out_dtype, d_status, st);
+  const bool packed = d_packed && (((uintptr_t)d_rows | (uintptr_t)d_packed | (uintptr_t)d_out) & 15u) == 0;
+  const bool aligned = (((uintptr_t)d_rows | (uintptr_t)d_weight | (uintptr_t)d_out) & 15u) == 0;
+  const int kernel = gather_kernel(dtype, kv, k_ch, n_ch, packed, aligned);
+  SPH_CHECK_ARG(d_weight || (kernel != SPH_KERNEL_PAIRS && kernel != SPH_KERNEL_GENERAL),
+                "the CUDA-core kernels need the unpacked weight");
+  switch (kernel) {
+    case SPH_KERNEL_STRIP:
+      return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
+                               d_out, out_dtype, d_status, st);
+    case SPH_KERNEL_TC_ROWS:
+      return conv_gather_tc_rows(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
+                                 d_out, out_dtype, d_status, st);
+    case SPH_KERNEL_TC:
+      return conv_gather_tc(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu, d_out,
+                            out_dtype, d_status, st);
+    case SPH_KERNEL_PAIRS:
+      return conv_gather_sparse(d_rows, dtype, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
+                                d_out, out_dtype, d_status, st);
   }
   if (dtype == SPH_I8)
     return conv_gather_generic(d_rows, n_rows, d_weight, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, (const float*)d_bias, relu,
@@ -191,18 +220,14 @@ extern "C" int sph_conv_wgrad(const void* d_rows, const void* d_dout, int dtype,
   if (zero_init) SPH_CUDA(cudaMemsetAsync(d_dweight, 0, (size_t)kv * k_ch * n_ch * sizeof(float), st));
   if (n_out == 0 || n_rows == 0) return SPH_OK;
   SPH_CHECK_ARG(d_rows && d_dout && d_nbr, "null pointer");
-  const bool aligned = (((uintptr_t)d_rows | (uintptr_t)d_dout) & 15u) == 0;      // copies of 16 bytes
-  // the pairs' kernel up to 2048 gradients an offset (1.1 to 3 times faster than the tcgen05 kernel from 1.5 to 12 pairs a row);
-  // at 64 x 64, the deep and dense levels, the tcgen05 kernel (22 pairs of 27: 0.70 against 1.19 ms on 1.4 M rows), and where fewer
-  // than nine offsets leave the former's warps idle (3 x 1 x 1: 32 -> 32 on 525 k rows 46 against 107 us)
-  if (conv_wgrad_strip_supported(dtype, k_ch, n_ch) &&
-      ((k_ch * n_ch <= 2048 && kv >= 9) || !aligned || !conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch)) &&
-      ((((uintptr_t)d_rows | (uintptr_t)d_dout) & 3u) == 0))
-    return conv_wgrad_strip(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
-  if (aligned && conv_wgrad_tc_supported(dtype, kv, k_ch, n_ch))
-    return conv_wgrad_tc(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
-  // small fp32 layers: the pair-compacting walk
-  if (dtype == SPH_F32 && aligned && conv_wgrad_pairs_supported(dtype, kv, k_ch, n_ch))
-    return conv_wgrad_pairs(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
+  const uintptr_t at = (uintptr_t)d_rows | (uintptr_t)d_dout;
+  switch (wgrad_kernel(dtype, kv, k_ch, n_ch, (at & 15u) == 0, (at & 3u) == 0)) {
+    case SPH_KERNEL_STRIP:
+      return conv_wgrad_strip(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
+    case SPH_KERNEL_TC:
+      return conv_wgrad_tc(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
+    case SPH_KERNEL_PAIRS:
+      return conv_wgrad_pairs(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
+  }
   return conv_wgrad_ffma(d_rows, d_dout, dtype, n_rows, d_nbr, n_out, kv, k_ch, n_ch, d_dweight, d_status, st);
 }

@@ -98,3 +98,17 @@ def test_kernel_selection_predicates(lib):
     assert wk(C.SPH_BF16, 32, 32) == 1 and wk(C.SPH_F16, 16, 16) == 1 and wk(C.SPH_F16, 64, 64) == 1
     assert wk(C.SPH_BF16, 4, 16) == 2 and wk(C.SPH_F32, 16, 16) == 2 and wk(C.SPH_F32, 16, 32) == 2
     assert wk(C.SPH_F32, 64, 64) == 0 and wk(C.SPH_F16, 5, 16) == 0 and wk(C.SPH_I8, 16, 16) == 0
+
+
+def test_kernel_that_runs(lib):
+    """The dispatch's own answer, by offsets and width: 0 general, 1 tcgen05, 2 its rows form, 3 strip, 4 pairs."""
+    k = lib.sph_conv_kernel
+    for want, dt, kv, a, b in [(3, C.SPH_F16, 27, 16, 16), (1, C.SPH_F16, 27, 16, 32), (2, C.SPH_F16, 27, 32, 32), (1, C.SPH_BF16, 27, 64, 64),
+                               (3, C.SPH_F16, 27, 24, 40), (4, C.SPH_F16, 27, 4, 16), (3, C.SPH_F16, 27, 5, 7), (0, C.SPH_F16, 45, 64, 64),
+                               (3, C.SPH_I8, 27, 16, 32), (4, C.SPH_I8, 27, 4, 16), (2, C.SPH_I8, 27, 64, 64), (0, C.SPH_I8, 27, 300, 7),
+                               (4, C.SPH_F32, 27, 16, 16), (0, C.SPH_F32, 27, 64, 64)]:
+        assert k(dt, kv, a, b, 0) == want, (dt, kv, a, b)
+    for want, dt, kv, a, b in [(3, C.SPH_F16, 27, 16, 16), (3, C.SPH_BF16, 27, 32, 64), (1, C.SPH_BF16, 27, 64, 64), (3, C.SPH_F16, 27, 5, 7),
+                               (1, C.SPH_F16, 3, 32, 32), (3, C.SPH_F16, 3, 24, 40), (4, C.SPH_F32, 27, 16, 32), (0, C.SPH_F32, 27, 64, 64)]:
+        assert k(dt, kv, a, b, 1) == want, (dt, kv, a, b)
+    assert k(9, 27, 16, 16, 0) < 0
