@@ -138,6 +138,8 @@ def _tables_for(rules, rule_size, n_in: int, n_out: int, need_t: bool) -> _Table
     reference-format tensors (cached on `rules`)."""
     if isinstance(rules, _Tables):
         tb = rules
+        if tb.n_in != n_in or tb.n_out != n_out:
+            raise RuntimeError("this rule set has %d input and %d output rows, the call %d and %d" % (tb.n_in, tb.n_out, n_in, n_out))
     else:
         tb = getattr(rules, "_sph", None)
         if tb is not None and (tb.version != rules._version or tb.n_in != n_in or tb.n_out != n_out):

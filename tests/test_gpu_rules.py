@@ -390,3 +390,21 @@ def test_rule_set_begun_on_another_stream():
         spoil = [torch.full((1 << 16,), -1, dtype=torch.int32, device=zi.device) for _ in range(400)]
     torch.cuda.synchronize()
     assert all(torch.equal(x, y) for x, y in zip(got, want)) and len(spoil) == 400
+
+
+def test_tables_of_other_sizes_are_refused():
+    """A rule set without lists serves the row counts it was made for, and no others."""
+    ops.config.materialize_rules = False
+    try:
+        zi, zp = _small(4, 4)
+        n = zi.numel()
+        tables = ops.get_rules_subm(zi, zp, 1, [6, 8, 10], [6, 8, 10], [3] * 3, [1] * 3, [1] * 3, [1] * 3, [2, 2])[2]
+    finally:
+        ops.config.materialize_rules = True
+    w = torch.zeros(27, 16, 16, device=zi.device)
+    assert ops.rule_conv(torch.zeros(n, 16, device=zi.device), w, tables, None, n).shape == (n, 16)
+    for n_in, n_out in ((n - 1, n), (n, n + 1000)):
+        with pytest.raises(RuntimeError, match="rows"):
+            ops.rule_conv(torch.zeros(n_in, 16, device=zi.device), w, tables, None, n_out)
+        with pytest.raises(RuntimeError, match="rows"):
+            ops.rule_conv_d_weight(torch.zeros(n_in, 16, device=zi.device), torch.zeros(n_out, 16, device=zi.device), tables, None)
