@@ -172,9 +172,9 @@ class Conv3d(Convolution):
                 out_feature = ConvFunction.apply(feature, w, rules, rule_size, tile_grid_shape, n_out, bias, relu, master)
         else:
             w = self._inference_weight(feature.dtype)
-            b = None if bias is None else bias.detach()              # read in every call: a write through `.data` is seen
-            if b is not None and (b.dtype not in (torch.float32, feature.dtype) or not b.is_contiguous()):
-                b = b.float().contiguous()
+            b = bias                                                 # read in every call: a write through `.data` is seen
+            if b is not None and ((b.dtype is not torch.float32 and b.dtype is not feature.dtype) or not b.is_contiguous()):
+                b = b.detach().float().contiguous()
             if profiling.is_active() or profiling.pair_counts is not None:
                 with profiling.section("conv:" + tag, iC=in_channels, oC=out_channels, n_in=feature.shape[0],
                                        n_out=oz_idx.shape[0], esize=feature.element_size()):

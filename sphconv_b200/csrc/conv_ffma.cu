@@ -114,7 +114,7 @@ __device__ __noinline__ int pairs_from(int k0, const int* __restrict__ nbr, int 
 // same accumulator.
 // The CTA is small (64 or 128 threads) so that a thread has up to four rows: with one row per thread (256 threads a tile)
 // the shared-memory reads of the filter, not the FMAs, set the pace; with eight rows too few warps fit on an SM.
-// Bound by the issue slots (67 % busy, two thirds of them FMAs) and the shared-memory reads (60 %).  Measured: 64 -> 64 on
+// Bound by the shared-memory reads of the operands (74 % of that pipe) and the issue slots (66 %, two thirds of them FMAs).  Measured: 64 -> 64 on
 // 170 k rows of 22 neighbours 3.2 -> 0.94 ms, 32 -> 32 on 390 k rows of 12 neighbours 1.9 -> 0.5 ms against the kernel it
 // replaced (one thread group per row walking every slot of the table).
 // VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by

@@ -100,8 +100,8 @@ dense_rows_kernel(V* __restrict__ rows, const int* __restrict__ z_idx, const int
 // columns are consecutive rows AND consecutive dense cells of every channel), stages their rows in shared memory with a
 // cell -> row map, and moves every channel's cells in vectors of V elements; cells without a row are zeros.  The dense
 // tensor is written once; a fill, a channels-last scatter and a permuting copy moved its bytes four times.  [8,64,16,128,64]
-// fp16 (134 MB) with 30 % of the cells occupied: 58 us to dense and 53 us back against 350 and 325 us, half the copy rate
-// (the per-element reads of the staged rows).
+// fp16 (134 MB) with 30 % of the cells occupied: 58 us to dense and 53 us back against 350 and 325 us; DRAM is 22 and 40 % busy,
+// the rest is the per-element traffic of the staged rows.
 //
 // Rows need not own their cells: of several rows at one depth of a column the last is the cell's value and each gets the
 // cell's gradient; a row whose depth lies outside the grid has the status bit set and a gradient of zero.  A block can hence have
