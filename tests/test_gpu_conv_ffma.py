@@ -70,3 +70,33 @@ def test_layers_walked_whole(iC, oC, dtype, dens, ks):
     if bool((rules._sph.nbr[0] < 0).any()):
         with pytest.raises(RuntimeError):
             check_status()
+
+
+@pytest.mark.parametrize("iC,oC", [(64, 64), (62, 61), (31, 30), (48, 60)])
+@pytest.mark.parametrize("dens,ks", [(0.02, (3, 3, 3)), (0.07, (3, 3, 3)), (0.15, (5, 3, 3))])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16])
+def test_tiles_shared_at_widths_that_fill_their_tiles(iC, oC, dens, ks, dtype):
+    """Widths with little padding, whose tiles do go to either kernel (padded ones of this size are walked whole)."""
+    rng, feat, w, rules, rule_size, pairs, n_in, n_out = _setup(2, [17, 23, 16], True, dens, 5, iC, oC, dtype, ks)
+    f64, w64 = feat.double().cpu().numpy(), w.double().cpu().numpy()
+    _close(ops.rule_conv(feat, w, rules, rule_size, n_out), conv_np.conv_forward(f64, w64, pairs, n_out), TOL[dtype])
+
+
+@pytest.mark.parametrize("iC,oC,dtype", [(32, 32, torch.float32), (24, 40, torch.float32), (9, 16, torch.float32), (64, 64, torch.float16),
+                                         (48, 40, torch.float16), (64, 33, torch.bfloat16)])
+@pytest.mark.parametrize("kv", [27, 45])
+def test_layers_larger_than_the_machine(iC, oC, dtype, kv):
+    """80 k rows (the rules for large layers), tiles of half a pair to eight pairs a row side by side."""
+    g = torch.Generator(device="cuda").manual_seed(iC + kv)
+    n = 80123
+    share = torch.rand(kv, n // 128 + 1, generator=g, device="cuda").pow(3).repeat_interleave(128, 1)[:, :n] * 0.5
+    nbr = torch.randint(0, n, (kv, n), generator=g, device="cuda", dtype=torch.int32)
+    nbr[torch.rand(kv, n, generator=g, device="cuda") > share] = -1
+    x = torch.randn(n, iC, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(kv, iC, oC, generator=g, device="cuda") / (4 * iC) ** 0.5).to(dtype)
+    want = torch.zeros(n, oC, dtype=torch.float64, device="cuda")
+    for k in range(kv):
+        m = nbr[k] >= 0
+        want[m] += x.double()[nbr[k][m].long()] @ w[k].double()
+    _close(ops._gather(x, w, nbr, n, False, None, None, False, torch.float32), want.cpu().numpy(), TOL[dtype])
+    assert check_status() == 0
