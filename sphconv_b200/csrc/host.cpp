@@ -4,7 +4,6 @@
 // An operator of this path is a handful of launches of a few microseconds each; driven from Python (one ctypes call and one
 // torch.empty at a time, ~100 us a layer) a scan waited for the host, not for the GPU.  The library itself stays free of
 // torch: this module loads it and calls it through the same entry points as any other binding.
-#include <ATen/core/CachingHostAllocator.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDACachingAllocator.h>
@@ -12,6 +11,7 @@
 #include <dlfcn.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <array>
 #include <mutex>
 #include <stdexcept>
@@ -250,28 +250,69 @@ py::tuple rules_subm(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, const 
   return py::make_tuple(or_none(l.rules), or_none(l.rule_size), nbr, or_none(ready));
 }
 
-// Step 1 of a strided rule set, enqueued; the row count is in the word, pinned host memory that the step's last kernel writes,
-// once the step has run.  The word is the handle's own: any number of them may be outstanding, for any time.
+// Words of pinned host memory that kernels write row counts to, 1 KiB at a time; a word given back before the kernel that writes
+// it has run waits for that kernel's event.  (An allocation of torch's pinned memory for every count took 2 us longer.)
+class CountWords {
+ public:
+  int32_t* take() {
+    std::lock_guard<std::mutex> lock(mutex_);
+    if (free_.empty()) {
+      auto done = std::partition(busy_.begin(), busy_.end(), [](const auto& b) { return !b.first.query(); });
+      for (auto b = done; b != busy_.end(); ++b) free_.push_back(b->second);
+      busy_.erase(done, busy_.end());
+    }
+    if (free_.empty()) {
+      void* words = nullptr;
+      C10_CUDA_CHECK(cudaHostAlloc(&words, kWords * sizeof(int32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+      for (int i = 0; i < kWords; ++i) free_.push_back(static_cast<int32_t*>(words) + i);
+    }
+    int32_t* word = free_.back();
+    free_.pop_back();
+    return word;
+  }
+  void give(int32_t* word) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    free_.push_back(word);
+  }
+  void give(int32_t* word, at::cuda::CUDAEvent&& written) {
+    std::lock_guard<std::mutex> lock(mutex_);
+    busy_.emplace_back(std::move(written), word);
+  }
+
+ private:
+  static constexpr int kWords = 256;
+  std::mutex mutex_;
+  std::vector<int32_t*> free_;
+  std::vector<std::pair<at::cuda::CUDAEvent, int32_t*>> busy_;
+};
+CountWords& count_words() {
+  static CountWords* words = new CountWords;      // outlives the interpreter's last handles
+  return *words;
+}
+
+// Step 1 of a strided rule set, enqueued; the row count is in the word once the step has run.  The word is the handle's own: any
+// number of them may be outstanding, for any time.
 struct Pending {
   sph_geom g;
-  Tensor z_idx, z_ptr, scratch, oz_ptr, word;
+  Tensor z_idx, z_ptr, scratch, oz_ptr;
   c10::cuda::CUDAStream stream;
   at::cuda::CUDAEvent event;
-  bool read = false;
+  int32_t* word = count_words().take();
+  bool enqueued = false, read = false;
 
   explicit Pending(c10::cuda::CUDAStream s) : stream(s) {}
   Pending(const Pending&) = delete;
-  ~Pending() {                  // never completed: the word is not handed out again before the kernel has written it
-    if (!read && word.defined())
-      try {
-        at::getHostAllocator(at::kCUDA)->record_event(word.data_ptr(), word.storage().data_ptr().get_context(), stream.unwrap());
-      } catch (...) {
-      }
+  ~Pending() {
+    try {
+      if (!enqueued || read) count_words().give(word);
+      else count_words().give(word, std::move(event));
+    } catch (...) {                 // the word is lost
+    }
   }
   int64_t count() {
     event.synchronize();
     read = true;
-    return *static_cast<const volatile int32_t*>(word.data_ptr());
+    return *const_cast<const volatile int32_t*>(word);
   }
 
   bool matches(const Tensor& zi, const Tensor& zp, const sph_geom& o) const {
@@ -290,10 +331,10 @@ std::shared_ptr<Pending> strided_begin(const Tensor& z_idx, const Tensor& z_ptr,
   const int64_t nnz = z_idx.size(0);
   r->scratch = empty({check(abi.sph_rules_strided_scratch_bytes(&r->g, nnz))}, at::kByte, z_idx);
   r->oz_ptr = empty({B, out[0], out[1]}, at::kInt, z_idx);
-  r->word = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-  check(abi.sph_rules_strided_count(ints(z_idx), ints(z_ptr), nnz, &r->g, ptr(r->scratch), ints(r->oz_ptr), ints(r->word),
-                                    nullptr, r->stream.stream()));
+  check(abi.sph_rules_strided_count(ints(z_idx), ints(z_ptr), nnz, &r->g, ptr(r->scratch), ints(r->oz_ptr), r->word, nullptr,
+                                    r->stream.stream()));
   r->event.record(r->stream);
+  r->enqueued = true;
   return r;
 }
 
