@@ -233,7 +233,8 @@ def kernel_of(lib, dcode, kind, k_ch, n_ch, esize, dtype_name):
     return {0: "conv_gather_generic_kernel" if dtype_name == "int8" else "conv_ffma_kernel",
             1: "conv_gather_tc_kernel<%d,%s>" % (row, typ), 2: "conv_gather_rows_kernel<%d,%s>" % (row, typ),
             3: "conv_strip_kernel<%d,%d,%s>" % (k_ch, n_ch, typ),
-            4: "conv_sparse_rows_kernel<%d,%d>" % (k_ch, n_ch)}[kernel], kernel in (1, 2, 3)
+            4: "conv_sparse_rows_kernel<%d,%d>" % (k_ch, n_ch),
+            5: "conv_gather_tmem_kernel<%d,%s>" % (row, typ)}[kernel], kernel in (1, 2, 3, 5)
 
 
 class Workload:

@@ -195,6 +195,7 @@ int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch);
 #define SPH_KERNEL_TC_ROWS 2 /* tcgen05 with the output row on the TMEM lane */
 #define SPH_KERNEL_STRIP 3   /* mma.sync over staged runs of input rows */
 #define SPH_KERNEL_PAIRS 4   /* CUDA cores, narrow rows over compacted pairs */
+#define SPH_KERNEL_TC_TMEM 5 /* tcgen05 with the gathered rows in tensor memory */
 int sph_conv_kernel(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch, int wgrad);
 
 #define SPH_BIAS_IN_ROW_TYPE 0x10000

@@ -12,7 +12,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libsphconv_b200.so")
-SOURCES = ["rules.cu", "conv_generic.cu", "conv_ffma.cu", "conv_strip.cu", "conv_strip_f16.cu", "conv_strip_bf16.cu", "conv_strip_i8.cu", "conv_sparse.cu", "conv_tc.cu", "conv_tc_rows.cu", "conv_wgrad_tc.cu", "conv_wgrad_strip.cu", "tensor_ops.cu", "voxelize.cu", "capi.cu"]
+SOURCES = ["rules.cu", "conv_generic.cu", "conv_ffma.cu", "conv_strip.cu", "conv_strip_f16.cu", "conv_strip_bf16.cu", "conv_strip_i8.cu", "conv_sparse.cu", "conv_tc.cu", "conv_tc_rows.cu", "conv_tmem.cu", "conv_wgrad_tc.cu", "conv_wgrad_strip.cu", "tensor_ops.cu", "voxelize.cu", "capi.cu"]
 # the explicit -gencode pair is required: the sm_100a shorthand does not enable tcgen05 in ptxas
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17",
               "-Xcompiler", "-fPIC", "--use_fast_math=false"]
@@ -50,22 +50,23 @@ def _host_command():
             ["-l" + n for n in ("c10", "c10_cuda", "torch", "torch_cpu", "torch_cuda", "torch_python", "cudart", "dl")])
 
 
+HOOKED = ["conv_tc.cu", "conv_tmem.cu"]
 HOOKS_LIB = os.path.join(LIBDIR, "libsphconv_b200_hooks.so")
 
 
 def build_test_hooks(force=False):
-    """A second library for the test of the bounded waits only: the same sources, with conv_tc.cu compiled with
+    """A second library for the test of the bounded waits only: the same sources, with HOOKED compiled with
     -DSPH_TEST_HOOKS (a 10 ms wait limit and the entry point sph_test_withhold_arrival).  The shipped library holds
     none of it.  Returns the path."""
     build(force=force)
-    src = os.path.join(CSRC, "conv_tc.cu")
     if not force and os.path.exists(HOOKS_LIB) and os.path.getmtime(HOOKS_LIB) >= os.path.getmtime(LIB):
         return HOOKS_LIB
     flags = [f for f in NVCC_FLAGS if not f.startswith("--use_fast_math")]
-    obj = os.path.join(LIBDIR, "conv_tc_hooks.o")
-    subprocess.check_call([_nvcc(), *flags, "-DSPH_TEST_HOOKS", "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c", src,
-                           "-o", obj], stdout=subprocess.DEVNULL, stderr=subprocess.STDOUT)
-    objs = [os.path.join(LIBDIR, s_.replace(".cu", ".o")) for s_ in SOURCES if s_ != "conv_tc.cu"] + [obj]
+    objs = [os.path.join(LIBDIR, s_.replace(".cu", ".o")) for s_ in SOURCES if s_ not in HOOKED]
+    for src in HOOKED:
+        objs.append(os.path.join(LIBDIR, src.replace(".cu", "_hooks.o")))
+        subprocess.check_call([_nvcc(), *flags, "-DSPH_TEST_HOOKS", "-I", os.path.join(ROOT, "include"), "-I", CSRC, "-c",
+                               os.path.join(CSRC, src), "-o", objs[-1]], stdout=subprocess.DEVNULL, stderr=subprocess.STDOUT)
     subprocess.check_call([_nvcc(), "-shared", "-o", HOOKS_LIB, *objs, "-lcudart"])
     return HOOKS_LIB
 

@@ -367,11 +367,11 @@ bool tc_shape_ok(int dtype, int kv, int K, int N) {
   return plan_smem(&p, kv, &bytes);
 }
 
-#ifdef SPH_TEST_HOOKS
-int g_test_withhold = 0;
-#endif
-
 }  // namespace
+
+#ifdef SPH_TEST_HOOKS
+int g_test_withhold = 0;          // conv_tmem.cu reads it too
+#endif
 
 int conv_gather_tc(const void* rows, int dtype, int64_t n_rows, const void* packed, const int* nbr, int64_t n_out,
                    int kv, int K, int N, int flip_k, const float* scale, Bias bias, int relu, void* out,
