@@ -230,11 +230,12 @@ def kernel_of(lib, dcode, kind, k_ch, n_ch, esize, dtype_name):
     if wgrad:
         return {0: "conv_wgrad_ffma_kernel", 1: "conv_wgrad_tc_kernel<%d>" % row, 3: "conv_wgrad_strip_kernel<%d,%d>" % (k_ch, n_ch),
                 4: "conv_wgrad_pairs_kernel<%d,%d>" % (k_ch, n_ch)}[kernel], kernel in (1, 3)
+    if lib.sph_conv_uses_tmem(dcode, 27, k_ch, n_ch):
+        return "conv_gather_tmem_kernel<%d,%s>" % (row, typ), True
     return {0: "conv_gather_generic_kernel" if dtype_name == "int8" else "conv_ffma_kernel",
             1: "conv_gather_tc_kernel<%d,%s>" % (row, typ), 2: "conv_gather_rows_kernel<%d,%s>" % (row, typ),
             3: "conv_strip_kernel<%d,%d,%s>" % (k_ch, n_ch, typ),
-            4: "conv_sparse_rows_kernel<%d,%d>" % (k_ch, n_ch),
-            5: "conv_gather_tmem_kernel<%d,%s>" % (row, typ)}[kernel], kernel in (1, 2, 3, 5)
+            4: "conv_sparse_rows_kernel<%d,%d>" % (k_ch, n_ch)}[kernel], kernel in (1, 2, 3)
 
 
 class Workload:

@@ -191,12 +191,14 @@ int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch);
  * sizes when all operands are 16-byte aligned.  The three functions above sort widths into classes instead.
  * No reference counterpart. */
 #define SPH_KERNEL_GENERAL 0 /* CUDA cores, any width: FFMA (int8: row by row) */
-#define SPH_KERNEL_TC 1      /* tcgen05 */
-#define SPH_KERNEL_TC_ROWS 2 /* tcgen05 with the output row on the TMEM lane */
+#define SPH_KERNEL_TC 1      /* tcgen05, rows of 32, 128 or 256 bytes */
+#define SPH_KERNEL_TC_ROWS 2 /* tcgen05, rows of 64 bytes */
 #define SPH_KERNEL_STRIP 3   /* mma.sync over staged runs of input rows */
 #define SPH_KERNEL_PAIRS 4   /* CUDA cores, narrow rows over compacted pairs */
-#define SPH_KERNEL_TC_TMEM 5 /* tcgen05 with the gathered rows in tensor memory */
 int sph_conv_kernel(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch, int wgrad);
+/* 1 where the answer 1 or 2 of sph_conv_kernel (wgrad = 0) is the kernel with the gathered rows in tensor memory (9 or 27
+ * offsets, at most 64 channels out), 0 where it is one of the two that gather into shared memory.  No reference counterpart. */
+int sph_conv_uses_tmem(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch);
 
 #define SPH_BIAS_IN_ROW_TYPE 0x10000
 

@@ -139,9 +139,6 @@ extern "C" int sph_conv_wgrad_kernel(int dtype, int32_t k_ch, int32_t n_ch) {
 // operands are 16-byte aligned; aligned: the operands the kernel reads are (words: 4-byte aligned).
 static int gather_kernel(int dtype, int kv, int K, int N, bool packed, bool aligned) {
   if (packed && runs_strip(dtype, kv, K, N)) return SPH_KERNEL_STRIP;
-  // 9 or 27 offsets, rows of 32, 64 or 128 bytes, up to 64 channels out: the rows by way of tensor memory (1.2 to 1.6 times faster
-  // than the two forms below from 17 k rows to 12 M; conv_tmem.cu)
-  if (packed && conv_tmem_supported(dtype, kv, K, N)) return SPH_KERNEL_TC_TMEM;
   // 64-byte rows: the form with the output row on the TMEM lane (absent neighbours masked, not copied) is the faster
   // of the two; wider rows are dense deep layers, where the transposed form issues half as many instructions
   if (packed && K * dtype_bytes(dtype) == 64 && conv_tc_rows_supported(dtype, kv, K, N)) return SPH_KERNEL_TC_ROWS;
@@ -170,6 +167,11 @@ extern "C" int sph_conv_kernel(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch
   return wgrad ? wgrad_kernel(dtype, kv, k_ch, n_ch, true, true) : gather_kernel(dtype, kv, k_ch, n_ch, true, true);
 }
 
+extern "C" int sph_conv_uses_tmem(int dtype, int32_t kv, int32_t k_ch, int32_t n_ch) {
+  const int kernel = sph_conv_kernel(dtype, kv, k_ch, n_ch, 0);
+  return (kernel == SPH_KERNEL_TC || kernel == SPH_KERNEL_TC_ROWS) && conv_tmem_supported(dtype, kv, k_ch, n_ch) ? 1 : 0;
+}
+
 static bool out_dtype_ok(int dtype, int out_dtype) {
   if (out_dtype < SPH_F32 || out_dtype > SPH_I8) return false;
   if (out_dtype == SPH_I8 && dtype != SPH_I8) return false;
@@ -195,17 +197,18 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
   // the tensor-core kernels copy 16 bytes at a time
   const bool packed = d_packed && (((uintptr_t)d_rows | (uintptr_t)d_packed | (uintptr_t)d_out) & 15u) == 0;
   const bool aligned = (((uintptr_t)d_rows | (uintptr_t)d_weight | (uintptr_t)d_out) & 15u) == 0;
-  int kernel = gather_kernel(dtype, kv, k_ch, n_ch, packed, aligned);
-  if (kernel == SPH_KERNEL_TC_TMEM && n_rows == 0) kernel = SPH_KERNEL_TC;      // no rows to describe to TMA
+  const int kernel = gather_kernel(dtype, kv, k_ch, n_ch, packed, aligned);
   SPH_CHECK_ARG(d_weight || (kernel != SPH_KERNEL_PAIRS && kernel != SPH_KERNEL_GENERAL),
                 "the CUDA-core kernels need the unpacked weight");
+  // 9 or 27 offsets and up to 64 channels out: the rows by way of tensor memory (1.2 to 1.6 times faster than the two forms that
+  // gather into shared memory, from 17 k rows to 12 M; conv_tmem.cu).  Without rows there is nothing to describe to TMA.
+  if ((kernel == SPH_KERNEL_TC || kernel == SPH_KERNEL_TC_ROWS) && n_rows > 0 && conv_tmem_supported(dtype, kv, k_ch, n_ch))
+    return conv_gather_tmem(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu, d_out,
+                            out_dtype, d_status, st);
   switch (kernel) {
     case SPH_KERNEL_STRIP:
       return conv_gather_strip(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
                                d_out, out_dtype, d_status, st);
-    case SPH_KERNEL_TC_TMEM:
-      return conv_gather_tmem(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
-                              d_out, out_dtype, d_status, st);
     case SPH_KERNEL_TC_ROWS:
       return conv_gather_tc_rows(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu,
                                  d_out, out_dtype, d_status, st);

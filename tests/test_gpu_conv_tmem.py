@@ -48,7 +48,7 @@ def _table(kv, n_out, n_rows, spread, share, seed):
 def _check(rows, weight, nbr, flip=False, **more):
     kv, K, N = weight.shape
     code = CODE[rows.dtype]
-    assert C.lib().sph_conv_kernel(code, kv, K, N, 0) == 5 and C.lib().sph_conv_kernel(code, kv + 1, K, N, 0) in (1, 2)
+    assert C.lib().sph_conv_uses_tmem(code, kv, K, N) and not C.lib().sph_conv_uses_tmem(code, kv + 1, K, N)
     out, status = _gather(rows, weight, nbr, flip, **more)
     assert status == 0
     none = torch.full((1, nbr.shape[1]), -1, dtype=torch.int32, device=DEV)
