@@ -17,11 +17,12 @@
 //  * the operand is handed over by 4 arrivals of warps instead of 128 of threads.
 // The order of sums is that of the other tensor-core kernels (offsets ascending, 32 bytes of a row per instruction), and so are
 // the results, bit for bit.  Measured against them (us, L2 flushed; tables of 27 offsets, share of neighbours present):
-//   32 -> 32 fp16, 1.5 M rows, 0.42   324 -> 206      64 -> 64 fp16, 683 k rows, 0.82   257 -> 180
-//   16 -> 32 fp16, 1.5 M rows, 0.05   201 -> 163      64 -> 32 fp16, 1.5 M rows, 0.13   513 -> 336
-//   32 -> 32 int8, 1.5 M rows, 0.42   256 -> 171      64 -> 64 fp16,  17 k rows, 0.70  24.6 -> 20.5
+//   32 -> 32 fp16, 1.5 M rows, 0.42   324 -> 205      64 -> 64 fp16, 683 k rows, 0.82   257 -> 162
+//   16 -> 32 fp16, 1.5 M rows, 0.05   201 -> 164      64 -> 32 fp16, 1.5 M rows, 0.13   513 -> 287
+//   32 -> 32 int8, 1.5 M rows, 0.42   256 -> 172      64 -> 64 fp16,  17 k rows, 0.70  24.6 -> 18.4
 // Bound by the instructions of the gather and planning warps (issue slots 77 % busy at 32- and 64-byte rows) and by the TMEM
-// writes (without them 206 -> 141), at 128-byte rows by the hand-over of an operand per offset (without MMAs 180 -> 151).  Tried and
+// writes (without them 206 -> 141), at 128-byte rows by the shared-memory
+// data path (82 % busy).  Tried and
 // slower: entries kept in registers with the offsets unrolled (instruction fetch: 577); rows of zeros in shared memory for absent
 // neighbours (bank conflicts: 263); the instruction's disable-output-lane mask instead of zeros (its operands: 217).
 //
@@ -66,6 +67,7 @@ constexpr int kOperandCols = 32;      // TMEM columns of an operand: one batch o
 constexpr int kOperands = 4;          // operands of a half in TMEM
 constexpr int kWeightSlots = 8;       // streamed weight images in flight: one takes about 2000 cycles to come
 constexpr uint32_t kAbsent = 0xffffu;   // place of a neighbour that there is not
+constexpr int kStagePieces = 8;       // 16-byte pieces of the widest output row that is staged (the narrowest: half as many)
 constexpr int kSmemTotal = 227 * 1024 - 2048;   // dynamic shared memory available next to the static part
 
 struct Partial {                      // what a planning warp found, for the others
@@ -90,6 +92,7 @@ struct TmemParams {
   int w_bytes;
   int cap;                            // rows of a run that a slot holds, a multiple of kBox
   int plan_off, part_off, epi_off, place_off, w_off, run_off;   // from the 1024-byte-aligned base
+  int stage_off;                      // -1: output rows are not staged
   int is_bf16;
   const float* scale;
   Bias bias;
@@ -195,10 +198,10 @@ __device__ __forceinline__ Plan combine(const Partial* part, int lane) {
   return r;
 }
 
-// 16 accumulator values of one output row (channels c0 .. c0+15) -> the output row, with 16-byte stores.
+// 16 accumulator values of one output row (channels c0 .. c0+15) -> 16-byte pieces; returns how many.
 template <bool I8>
-__device__ __forceinline__ void store_row16(uint8_t* dst, int out_dtype, const uint32_t (&raw)[16], const float* sc,
-                                            const float* bi, int relu) {
+__device__ __forceinline__ int convert16(uint4 (&to)[4], int out_dtype, const uint32_t (&raw)[16], const float* sc, const float* bi,
+                                         int relu) {
   float x[16];
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
@@ -208,8 +211,11 @@ __device__ __forceinline__ void store_row16(uint8_t* dst, int out_dtype, const u
   }
   if (out_dtype == SPH_F32) {
 #pragma unroll
-    for (int j = 0; j < 16; j += 4) *(float4*)(dst + j * 4) = make_float4(x[j], x[j + 1], x[j + 2], x[j + 3]);
-  } else if (out_dtype == SPH_I8) {
+    for (int j = 0; j < 4; ++j)
+      to[j] = make_uint4(__float_as_uint(x[4 * j]), __float_as_uint(x[4 * j + 1]), __float_as_uint(x[4 * j + 2]), __float_as_uint(x[4 * j + 3]));
+    return 4;
+  }
+  if (out_dtype == SPH_I8) {
     uint32_t w[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -221,22 +227,23 @@ __device__ __forceinline__ void store_row16(uint8_t* dst, int out_dtype, const u
       }
       w[j] = acc;
     }
-    *(uint4*)dst = make_uint4(w[0], w[1], w[2], w[3]);
-  } else {
-    uint32_t h[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      if (out_dtype == SPH_F16) {
-        const __half2 v = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
-        h[j] = *(const uint32_t*)&v;
-      } else {
-        const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
-        h[j] = *(const uint32_t*)&v;
-      }
-    }
-    *(uint4*)dst = make_uint4(h[0], h[1], h[2], h[3]);
-    *(uint4*)(dst + 16) = make_uint4(h[4], h[5], h[6], h[7]);
+    to[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    return 1;
   }
+  uint32_t h[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (out_dtype == SPH_F16) {
+      const __half2 v = __floats2half2_rn(x[2 * j], x[2 * j + 1]);
+      h[j] = *(const uint32_t*)&v;
+    } else {
+      const __nv_bfloat162 v = __floats2bfloat162_rn(x[2 * j], x[2 * j + 1]);
+      h[j] = *(const uint32_t*)&v;
+    }
+  }
+  to[0] = make_uint4(h[0], h[1], h[2], h[3]);
+  to[1] = make_uint4(h[4], h[5], h[6], h[7]);
+  return 2;
 }
 
 // KC = 16-byte pieces of a row (2, 4, 8), I8 = int8 operands, L = offsets that share a run (9 of 27, 3 of 9).
@@ -439,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
       const uint32_t a0 = tmem_a + (uint32_t)(h * kOperands * kOperandCols);
       int ws = 0;
       uint32_t w_par = 0u, count = 0u;               // count: batches of this half so far
-      bool dead = false;
+      bool dead = false, seen = false;                // seen: the next offset's barriers are complete
       if (!STREAM) dead = !warp_wait(w_full0, 0u, abort_flag);
       for (int ti = 0; ti < my_tiles && !dead; ++ti) {
         const int buf = ti & 1;
@@ -452,19 +459,54 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)((buf * 2 + h) * 64);
         uint32_t acc = 0u;
-#pragma unroll 1
-        for (int l = 0; l < kLines && !dead; ++l) {
-          uint32_t todo = (walk >> (l * L)) & ((1u << L) - 1u);
+        if constexpr (STREAM) {
+          uint32_t todo = walk;
+          int k = __ffs((int)todo) - 1;
 #pragma unroll 1
           while (todo) {
-            int k[U];                                 // offsets of the batch in the line, -1: no more
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              k[u] = todo ? __ffs((int)todo) - 1 : -1;
-              todo &= todo - 1u;
+            const uint32_t op = count % kOperands;
+            const bool mine = own >> k & 1u;
+            if (!__all_sync(0xffffffffu, seen)) {
+              if (!warp_wait(w_full0 + 8u * ws, w_par, abort_flag)) { dead = true; break; }
+              if (mine && !warp_wait(a_full0 + 8u * op, count / kOperands & 1u, abort_flag)) { dead = true; break; }
             }
-            if (STREAM && !warp_wait(w_full0 + 8u * ws, w_par, abort_flag)) { dead = true; break; }
-            if (!STREAM || (own >> (l * L + k[0]) & 1u)) {
+            tc_fence_after();
+            if (one) {
+              if (mine) {
+                const uint32_t w_lo = w_lo0 + (uint32_t)ws * w_units;
+#pragma unroll
+                for (int j = 0; j < KC / 2; ++j)
+                  umma_ta<I8>(d_tmem, a0 + op * kOperandCols + (uint32_t)(j * 8), w_hi | (uint64_t)(w_lo + (uint32_t)j * w_step), idesc,
+                              j ? 1u : acc);
+                umma_commit(a_empty0 + 8u * op);
+                umma_commit(w_empty0 + 8u * ws);
+              } else {
+                mbar_arrive(w_empty0 + 8u * ws);
+              }
+            }
+            if (mine) {
+              acc = 1u;
+              ++count;
+            }
+            if (++ws == kWeightSlots) { ws = 0; w_par ^= 1u; }
+            todo &= todo - 1u;
+            k = __ffs((int)todo) - 1;
+            // looked at now, the barriers of the next offset are known to be complete without the 90 cycles a wait takes for each
+            seen = mbar_test_wait(a_full0 + 8u * (count % kOperands), count / kOperands & 1u) &
+                   mbar_test_wait(w_full0 + 8u * ws, w_par);
+          }
+        } else {
+#pragma unroll 1
+          for (int l = 0; l < kLines && !dead; ++l) {
+            uint32_t todo = (own >> (l * L)) & ((1u << L) - 1u);
+#pragma unroll 1
+            while (todo) {
+              int k[U];                               // offsets of the batch in the line, -1: no more
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                k[u] = todo ? __ffs((int)todo) - 1 : -1;
+                todo &= todo - 1u;
+              }
               const uint32_t op = count % kOperands;
               if (!warp_wait(a_full0 + 8u * op, count / kOperands & 1u, abort_flag)) { dead = true; break; }
               tc_fence_after();
@@ -472,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
                   if (u == 0 || k[u] >= 0) {
-                    const uint32_t w_lo = w_lo0 + (uint32_t)(STREAM ? ws : l * L + k[u]) * w_units;
+                    const uint32_t w_lo = w_lo0 + (uint32_t)(l * L + k[u]) * w_units;
 #pragma unroll
                     for (int j = 0; j < KC / 2; ++j)
                       umma_ta<I8>(d_tmem, a0 + op * kOperandCols + (uint32_t)(u * KC * 4 + j * 8),
@@ -480,14 +522,10 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
                   }
                 }
                 umma_commit(a_empty0 + 8u * op);
-                if (STREAM) umma_commit(w_empty0 + 8u * ws);
               }
               acc = 1u;
               ++count;
-            } else if (one) {
-              mbar_arrive(w_empty0 + 8u * ws);
             }
-            if (STREAM && ++ws == kWeightSlots) { ws = 0; w_par ^= 1u; }
           }
         }
         if (!dead && one) umma_commit(smem_u32(&s_acc_full[buf][h]));
@@ -496,8 +534,12 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
   } else if (warp < kRunWarp) {
     // ======================= epilogue =======================
     const int q = warp & 3;                       // TMEM lane quarter this warp may read: rows 32q .. 32q+31 of a half
-    const int row_pitch = p.N * p.out_esize;
-    const int chunk_bytes = 16 * p.out_esize;
+    // Rows of 80 to 128 bytes go through shared memory, an odd number of 16-byte pieces apart: stored by the lane that has them, a
+    // store instruction touches 32 lines and takes 37 turns of the data path that the gather waits for, staged 12 (64 -> 64
+    // channels of fp16: 177 -> 162 us).  Narrower rows do not repay the instructions (32 -> 32: 205 against 208).
+    const int pieces = p.N * p.out_esize / 16, pitch = pieces | 1;
+    const bool staged = p.stage_off >= 0;
+    uint4* stage = (uint4*)(base + (staged ? p.stage_off : 0)) + q * 32 * (kStagePieces + 1);
     const bool one = elect_one();
     bool dead = false;
     for (int ti = 0; ti < my_tiles && !dead; ++ti) {
@@ -506,18 +548,30 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
       for (int h = 0; h < halves; ++h) {
         if (!warp_wait(smem_u32(&s_acc_full[buf][h]), ((uint32_t)ti >> 1) & 1u, abort_flag)) { dead = true; break; }
         tc_fence_after();
-        const int64_t row = tile_row(ti) + h * kHalfRows + q * 32 + lane;
-        if (row - lane < p.n_out) {               // warp-uniform
-          const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((buf * 2 + h) * 64);
-          uint8_t* dst = (uint8_t*)p.out + row * row_pitch;
+        const int64_t row0 = tile_row(ti) + h * kHalfRows + q * 32;
+        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((buf * 2 + h) * 64);
+        const int rows = row0 < p.n_out ? (int)min((int64_t)32, p.n_out - row0) : 0;
+        uint4* dst = (uint4*)((uint8_t*)p.out + row0 * p.N * p.out_esize);
 #pragma unroll 1
-          for (int c0 = 0; c0 < p.N; c0 += 16) {
-            uint32_t raw[16];
-            tmem_ld16(taddr + (uint32_t)c0, raw);   // this thread's row, channels c0 .. c0+15
-            tmem_ld_wait();
-            if (row < p.n_out) store_row16<I8>(dst, p.out_dtype, raw, s_epi + c0, s_epi + 64 + c0, p.relu);
-            dst += chunk_bytes;
+        for (int c0 = 0, c = 0; c0 < p.N && rows > 0; c0 += 16) {
+          uint32_t raw[16];
+          tmem_ld16(taddr + (uint32_t)c0, raw);     // this thread's row, channels c0 .. c0+15
+          tmem_ld_wait();
+          uint4 piece[4];
+          const int n = convert16<I8>(piece, p.out_dtype, raw, s_epi + c0, s_epi + 64 + c0, p.relu);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            if (j >= n) break;
+            if (staged) stage[lane * pitch + c + j] = piece[j];
+            else if (lane < rows) dst[lane * pieces + c + j] = piece[j];
           }
+          c += n;
+        }
+        if (staged) {                               // the rows are consecutive: 512 bytes a store
+          __syncwarp();
+          const int n = rows * pieces;
+          for (int i = lane; i < n; i += 32) dst[i] = stage[i / pieces * pitch + i % pieces];
+          __syncwarp();
         }
         tc_fence_before();
         __syncwarp();
@@ -712,6 +766,12 @@ bool plan_smem(TmemParams* p, int kv, int row_bytes, int* smem_bytes) {
   p->plan_off = off; off += 2 * (int)sizeof(Plan);
   p->part_off = off; off += 2 * 8 * (int)sizeof(Partial);
   p->epi_off = off; off += 2 * 64 * (int)sizeof(float);
+  const int pieces = p->N * p->out_esize / 16;
+  p->stage_off = -1;
+  if (pieces > kStagePieces / 2 && pieces <= kStagePieces) {
+    p->stage_off = off;
+    off += 4 * 32 * (kStagePieces + 1) * 16;
+  }
   p->place_off = off; off += 2 * 8 * kLines * line * 32 * (int)sizeof(uint16_t);
   off = (off + 127) & ~127;
   p->w_off = off;
