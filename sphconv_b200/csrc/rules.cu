@@ -529,6 +529,103 @@ rule_lists_fixed_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz,
   if (overflow && status) atomicOr(status, SPH_STATUS_RULE_OVERFLOW);
 }
 
+// The same lists by a CTA per tile, for 27 offsets: nine warps of three offsets each.  The position -> row mapping of the tile is
+// written to shared memory once for all of them, and a warp has the entries of 4 x 32 positions and its three offsets in flight
+// while it compacts those before (rule_lists_fixed_kernel: nine entries, and its lanes walk the runs by themselves).
+constexpr int kTileWarps = 9;
+constexpr int kTileNK = 3;
+constexpr int kTileCH = 4;
+constexpr int kTilePositions = 2048;   // list positions whose rows are mapped at a time
+
+__global__ void __launch_bounds__(kTileWarps * 32)
+rule_lists_tile_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int tile_n_max, const int* __restrict__ nbr,
+                       int* __restrict__ rules, int* __restrict__ rule_size, int* __restrict__ status) {
+  __shared__ int s_rs[kListRanges];
+  __shared__ int s_off[kListRanges + 1];
+  __shared__ int s_row[kTilePositions];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = blockIdx.x, k0 = warp * kTileNK;
+  const int th = t / g.tgW, tw = t % g.tgW;
+  const int ox0 = th * g.tH, oy0 = tw * g.tW;
+  const int tHe = min(g.tH, g.oH - ox0), tWe = min(g.tW, g.oW - oy0);
+  const int R = g.B * tHe;
+  const unsigned lt = (1u << lane) - 1u;
+  const int* plane[kTileNK];
+  int* list[kTileNK];
+  int base[kTileNK];
+#pragma unroll
+  for (int j = 0; j < kTileNK; ++j) {
+    plane[j] = nbr + (int64_t)(k0 + j) * out_nnz;
+    list[j] = rules ? rules + ((int64_t)t * (kTileWarps * kTileNK) + k0 + j) * 2 * tile_n_max : nullptr;
+    base[j] = 0;
+  }
+  bool overflow = false;
+  for (int rg = 0; rg < R; rg += kListRanges) {
+    const int nr = min(kListRanges, R - rg);
+    if (warp == 0) stage_tile_runs(out_zp, g, ox0, oy0, tHe, tWe, rg, nr, s_rs, s_off, lane);
+    __syncthreads();
+    const int T = s_off[nr];
+    for (int w0 = 0; w0 < T; w0 += kTilePositions) {
+      const int n = min(kTilePositions, T - w0);
+      for (int i = warp; i < nr; i += kTileWarps) {
+        const int hi = min(s_off[i + 1] - w0, n), shift = s_rs[i] - s_off[i] + w0;
+        for (int p = max(s_off[i] - w0, 0) + lane; p < hi; p += 32) s_row[p] = shift + p;
+      }
+      __syncthreads();
+      auto fetch = [&](int p0, int (&row)[kTileCH], int (&v)[kTileCH][kTileNK]) {
+#pragma unroll
+        for (int u = 0; u < kTileCH; ++u) {
+          const int p = p0 + u * 32 + lane;
+          const bool ok = p < n;
+          row[u] = ok ? s_row[p] : 0;
+#pragma unroll
+          for (int j = 0; j < kTileNK; ++j) v[u][j] = ok ? __ldg(plane[j] + row[u]) : -1;
+        }
+      };
+      int row[kTileCH], v[kTileCH][kTileNK];
+      fetch(0, row, v);
+      for (int p0 = 0; p0 < n; p0 += 32 * kTileCH) {
+        int nrow[kTileCH], nv[kTileCH][kTileNK];
+        const bool more = p0 + 32 * kTileCH < n;
+        if (more) fetch(p0 + 32 * kTileCH, nrow, nv);
+#pragma unroll
+        for (int u = 0; u < kTileCH; ++u) {
+          if (p0 + u * 32 >= n) break;
+#pragma unroll
+          for (int j = 0; j < kTileNK; ++j) {
+            const unsigned m = __ballot_sync(0xffffffffu, v[u][j] >= 0);
+            if (list[j] && v[u][j] >= 0) {
+              const int slot = base[j] + __popc(m & lt);
+              if (slot < tile_n_max) {
+                list[j][slot] = v[u][j];
+                list[j][tile_n_max + slot] = row[u];
+              } else {
+                overflow = true;
+              }
+            }
+            base[j] += __popc(m);
+          }
+        }
+        if (more) {
+#pragma unroll
+          for (int u = 0; u < kTileCH; ++u) {
+            row[u] = nrow[u];
+#pragma unroll
+            for (int j = 0; j < kTileNK; ++j) v[u][j] = nv[u][j];
+          }
+        }
+      }
+      __syncthreads();   // the next positions overwrite the mapping, the next group of runs the runs
+    }
+  }
+  if (rule_size) {
+#pragma unroll
+    for (int j = 0; j < kTileNK; ++j)
+      if (lane == j) rule_size[(int64_t)t * (kTileWarps * kTileNK) + k0 + j] = base[j];
+  }
+  if (overflow && status) atomicOr(status, SPH_STATUS_RULE_OVERFLOW);
+}
+
 // kListChunks: 32-row chunks whose table reads are in flight together (8 for tiles of hundreds of rows; 1 or 2 for
 // tiles of a few dozen, where the chunks beyond the tile's rows would only cost instructions)
 template <int kListChunks>
@@ -981,6 +1078,13 @@ int* parked_columns(const Geom& g, int* nbr, int64_t out_nnz) {
 // Pair lists of every (tile, offset) from a finished neighbour table.
 int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm, const int* nbr, int* rules,
                       int* rule_size, int* status, cudaStream_t st) {
+  if (g.KV == kTileWarps * kTileNK && g.nTile >= 1024 && out_nnz >= 256 * (int64_t)g.nTile) {
+    // Large tiles, and enough of them: 1.5 M rows in 2048 tiles of 745, 1.9 M / 18.3 M pairs 107 -> 82 / 133 -> 98 us.  A CTA's
+    // start takes too long where tiles are small (567 k rows in 8192 tiles of 69: 53 -> 86) or few (683 k in 512: 51 -> 61).
+    rule_lists_tile_kernel<<<(unsigned)g.nTile, kTileWarps * 32, 0, st>>>(out_zp, g, out_nnz, tnm, nbr, rules, rule_size, status);
+    SPH_LAUNCH_CHECK();
+    return SPH_OK;
+  }
   if (g.KV == 27 && (int64_t)tnm * 54 < (1LL << 32)) {
     // the usual 3 x 3 x 3 filter: the kernel with the offsets' running counts in registers
     // nine offsets per warp where that gives the machine enough warps, else three (small tile grids have long tiles:

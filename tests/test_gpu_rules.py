@@ -11,7 +11,7 @@ from oracle import rules_np
 from sphconv_b200 import check_status, synthetic
 from sphconv_b200 import sphconv_cuda as ops
 
-from gpu_util import assert_rules_equal, assert_tables_match, gpu_rules, oracle_rules, to_dev
+from gpu_util import DEV, assert_rules_equal, assert_tables_match, gpu_rules, oracle_rules, to_dev
 from test_oracle import CASES
 
 pytestmark = pytest.mark.gpu
@@ -408,3 +408,31 @@ def test_tables_of_other_sizes_are_refused():
             ops.rule_conv(torch.zeros(n_in, 16, device=zi.device), w, tables, None, n_out)
         with pytest.raises(RuntimeError, match="rows"):
             ops.rule_conv_d_weight(torch.zeros(n_in, 16, device=zi.device), torch.zeros(n_out, 16, device=zi.device), tables, None)
+
+
+@pytest.mark.parametrize("B,H,W,D,occ,nmax,subm", [(1, 64, 66, 96, 1.0, 96, True),       # tiles of 290 rows, columns of up to 96
+                                                   (6, 64, 64, 128, 0.95, 128, True),    # more than 2048 positions in a tile
+                                                   (70, 64, 64, 16, 0.9, 3, True),       # more than 128 runs in a tile
+                                                   (3, 130, 126, 64, 0.9, 12, False)])
+def test_lists_of_large_tiles_in_order(B, H, W, D, occ, nmax, subm):
+    """Lists that a CTA per tile writes (27 offsets, 1024 tiles of 256 rows and more): every pair of the table, by tile and
+    offset, in the order (batch, tile row, row)."""
+    rng = np.random.default_rng(B)
+    want = np.where(rng.random((B, H, W)) < occ, rng.integers(nmax // 2 + 1, nmax + 1, (B, H, W)), 0)
+    cells = rng.random((B, H, W, D)).argsort(-1).argsort(-1) < want[..., None]
+    z_idx, z_ptr = np.nonzero(cells)[3].astype(np.int32), want.reshape(-1).cumsum().reshape(B, H, W).astype(np.int32)
+    zi, zp, osh, oz_idx, oz_ptr, rules, rule_size = gpu_rules(z_idx, z_ptr, B, (H, W, D), (3, 3, 3), (1, 1, 1) if subm else (2, 2, 2),
+                                                              (1, 1, 1), (2, 2), subm)
+    n, tiles = oz_idx.numel(), rules.shape[0]
+    assert tiles >= 1024 and n >= 256 * tiles
+    column = torch.repeat_interleave(torch.arange(oz_ptr.numel(), device=DEV), torch.diff(oz_ptr.view(-1), prepend=oz_ptr.new_zeros(1)).long())
+    oy, ox, b = column % osh[1], column // osh[1] % osh[0], column // (osh[0] * osh[1])
+    tile = ox // 2 * ((osh[1] + 1) // 2) + oy // 2
+    order = (((tile * B + b) * 2 + ox % 2) * n + torch.arange(n, device=DEV)).argsort()      # rows in list order
+    nbr = rules._sph.nbr[:, order]
+    for k in range(27):
+        has = nbr[k] >= 0
+        size = torch.bincount(tile[order][has], minlength=tiles)
+        assert torch.equal(rule_size[:, k].long(), size)
+        used = torch.arange(rules.shape[3], device=DEV) < size[:, None]
+        assert torch.equal(rules[:, k, 0][used], nbr[k][has]) and torch.equal(rules[:, k, 1][used].long(), order[has])
