@@ -41,6 +41,36 @@ void note_launch();  // counts kernels launched by this library (sph_kernel_laun
     ::sph::note_launch();                                                                \
   } while (0)
 
+// A kernel of this library may be launched before the one in front of it in the stream has ended (programmatic dependent launch):
+// its blocks take their places when the last ones of that kernel have ended, or earlier where that kernel allows it, and
+// after_previous(), the first statement of every kernel, holds them until all of it is complete and its writes are visible.
+// A chain of small kernels then costs about a microsecond a kernel less (both rule sets of a batch of 3 small scans 117 -> 100 us).
+// The wait is in every kernel, also in those that nothing of the library precedes: a kernel that skipped it could complete before
+// its predecessor, and its successor would run too early.
+template <typename... Params, typename... Args>
+inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  cudaLaunchAttribute early;
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = st;
+  c.attrs = &early;
+  c.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);      // SPH_LAUNCH_CHECK() reads the error
+}
+// EARLY: a grid of at most two blocks per SM lets its successor in at once, which finds room beside it on every SM.  Blocks let in
+// beside a large grid, or at the end of a persistent one, would all go to the SMs that are free first: 16 blocks behind a
+// convolution took 57 us instead of 9.
+constexpr unsigned kEarlyBlocks = 2 * 148;
+template <bool EARLY = true>
+__device__ __forceinline__ void after_previous() {
+  if (EARLY && gridDim.x * gridDim.y <= kEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __host__ __device__ inline int div_up(int a, int b) { return (a + b - 1) / b; }
 __host__ __device__ inline int64_t div_up64(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

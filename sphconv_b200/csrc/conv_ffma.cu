@@ -121,6 +121,7 @@ __device__ __noinline__ int pairs_from(int k0, const int* __restrict__ nbr, int 
 // element.
 template <typename T, int CG, int KC, bool VEC>
 __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaParams p) {
+  after_previous<false>();
   using S = FfmaShape<CG, KC>;
   extern __shared__ __align__(16) unsigned char smem[];
   float* s_acc = (float*)smem;                       // [kRows][NP + 4]
@@ -375,6 +376,7 @@ __device__ __forceinline__ void add_pair(const T* __restrict__ x, const T* __res
 
 template <typename T, bool XV, bool WV>
 __global__ void __launch_bounds__(kFewThreads, 2) conv_few_kernel(FfmaParams p) {
+  after_previous<false>();
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_count[kFewThreads / 32];
   const int words = (p.kv + 31) / 32;
@@ -490,6 +492,7 @@ __device__ __forceinline__ int fold_copies(float (&v)[64], int lane) {
 
 template <typename T, int KG, int NG, bool VEC>
 __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradParams p) {
+  after_previous<false>();
   using S = WgShape<KG, NG>;
   extern __shared__ __align__(16) unsigned char smem[];
   float* s_st = (float*)smem;                                // [2]{x [PAIRS][XS], dy [PAIRS][DS]}, later the sum
@@ -624,7 +627,7 @@ int launch_ffma(const FfmaParams& p, cudaStream_t st) {
   auto kern = conv_ffma_kernel<T, CG, KC, VEC>;
   SPH_CUDA(allow_smem(kern, S::BYTES));
   const dim3 grid((unsigned)div_up64(p.n_out, kRows), (unsigned)div_up(p.N, S::NP));
-  kern<<<grid, S::T, S::BYTES, st>>>(p);
+  launch(kern, grid, S::T, S::BYTES, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -633,7 +636,7 @@ template <typename T, bool XV, bool WV>
 int launch_few(const FfmaParams& p, int smem, cudaStream_t st) {
   auto kern = conv_few_kernel<T, XV, WV>;
   SPH_CUDA(allow_smem(kern, kFewSmem));
-  kern<<<(unsigned)div_up64(p.n_out, kRows), kFewThreads, smem, st>>>(p);
+  launch(kern, (unsigned)div_up64(p.n_out, kRows), kFewThreads, smem, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -698,7 +701,7 @@ int launch_wg(const FfmaWgradParams& p, int kv, cudaStream_t st) {
   using S = WgShape<KG, NG>;
   auto kern = conv_wgrad_ffma_kernel<T, KG, NG, VEC>;
   SPH_CUDA(allow_smem(kern, S::BYTES));
-  kern<<<dim3((unsigned)div_up64(p.n_out, kWgSlice), (unsigned)kv), kThreads, S::BYTES, st>>>(p);
+  launch(kern, dim3((unsigned)div_up64(p.n_out, kWgSlice), (unsigned)kv), kThreads, S::BYTES, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }

@@ -28,6 +28,7 @@ conv_gather_generic_kernel(const int8_t* __restrict__ rows, int64_t n_rows, cons
                            const int* __restrict__ nbr, int64_t n_out, int kv, int K, int N, int tpr, int flip_k,
                            const float* __restrict__ scale, const float* __restrict__ bias, int relu,
                            void* __restrict__ out, int out_dtype, int* __restrict__ status) {
+  after_previous();
   const int rows_per_block = kGenThreads / tpr;
   const int sub = threadIdx.x % tpr;
   const int64_t r = (int64_t)blockIdx.x * rows_per_block + threadIdx.x / tpr;
@@ -76,8 +77,7 @@ int conv_gather_generic(const void* rows, int64_t n_rows, const void* weight, co
   }
   const int rows_per_block = kGenThreads / tpr;
   const int64_t blocks = div_up64(n_out, rows_per_block);
-  conv_gather_generic_kernel<<<(unsigned)blocks, kGenThreads, 0, st>>>(
-      (const int8_t*)rows, n_rows, (const int8_t*)weight, nbr, n_out, kv, K, N, tpr, flip_k, scale, bias, relu, out,
+  launch(conv_gather_generic_kernel, (unsigned)blocks, kGenThreads, 0, st, (const int8_t*)rows, n_rows, (const int8_t*)weight, nbr, n_out, kv, K, N, tpr, flip_k, scale, bias, relu, out,
       out_dtype, status);
   SPH_LAUNCH_CHECK();
   return SPH_OK;

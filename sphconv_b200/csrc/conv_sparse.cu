@@ -240,6 +240,7 @@ __device__ __noinline__ void sparse_flush(const T* __restrict__ rows, const type
 
 template <typename T, int IC, int OC>
 __global__ void __launch_bounds__(kSpThreads, 4) conv_sparse_rows_kernel(SparseParams p) {
+  after_previous<false>();
   extern __shared__ __align__(16) unsigned char smem[];
   using S = SparseShape<T, IC, OC>;
   constexpr int AS = S::AS;
@@ -361,7 +362,7 @@ int launch_sparse(const SparseParams& p, cudaStream_t st) {
   }
   const int64_t want = div_up64(p.n_chunks, kSpWarps);
   const int64_t grid = want < (int64_t)sms * per_sm ? want : (int64_t)sms * per_sm;
-  kern<<<(unsigned)grid, kSpThreads, smem, st>>>(p);
+  launch(kern, (unsigned)grid, kSpThreads, smem, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -417,6 +418,7 @@ template <int IC, int OC> struct WgradShape {
 
 template <typename T, int IC, int OC>
 __global__ void __launch_bounds__(kSpThreads, 3) conv_wgrad_pairs_kernel(WgradParams p) {
+  after_previous<false>();
   extern __shared__ __align__(16) unsigned char smem[];
   using S = WgradShape<IC, OC>;
   constexpr int E = S::E, EPL = S::EPL, XS = S::XS, DS = S::DS;
@@ -550,7 +552,7 @@ int launch_wgrad_pairs(const WgradParams& p, cudaStream_t st) {
   }
   const int64_t want = div_up64(p.n_chunks, kSpWarps);
   const int64_t grid = want < (int64_t)sms * per_sm ? want : (int64_t)sms * per_sm;
-  kern<<<(unsigned)grid, kSpThreads, smem, st>>>(p);
+  launch(kern, (unsigned)grid, kSpThreads, smem, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }

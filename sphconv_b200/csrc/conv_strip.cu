@@ -11,6 +11,7 @@ namespace {
 // (t = lane % 4): the B fragments of two instructions.  Zeros beyond K and N.
 template <typename T>
 __global__ void pack_strip_kernel(const T* __restrict__ w, int kv, int K, int N, int ks, int nt, uint4* __restrict__ image) {
+  after_previous();
   const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int per_k = ks * (nt / 2) * 32;
   if (u >= (int64_t)kv * per_k) return;
@@ -66,8 +67,8 @@ int pack_strip_filter(const void* w, int dtype, int kv, int K, int N, void* pack
     return SPH_ERR_UNSUPPORTED;
   }
   const unsigned blocks = (unsigned)div_up(s.units, 256);
-  if (dtype == SPH_I8) pack_strip_kernel<int8_t><<<blocks, 256, 0, st>>>((const int8_t*)w, kv, K, N, s.ks, s.nt, (uint4*)packed);
-  else pack_strip_kernel<uint16_t><<<blocks, 256, 0, st>>>((const uint16_t*)w, kv, K, N, s.ks, s.nt, (uint4*)packed);
+  if (dtype == SPH_I8) launch(pack_strip_kernel<int8_t>, blocks, 256, 0, st, (const int8_t*)w, kv, K, N, s.ks, s.nt, (uint4*)packed);
+  else launch(pack_strip_kernel<uint16_t>, blocks, 256, 0, st, (const uint16_t*)w, kv, K, N, s.ks, s.nt, (uint4*)packed);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }

@@ -64,6 +64,7 @@ __device__ __forceinline__ void quad_transpose(uint32_t (&v)[4], int t) {
 // KS: 32-byte steps of a row, NT: 8-channel tiles of the output, WHOLE: rows are 32 * KS bytes.
 template <int KS, int NT, bool WHOLE, int DT>
 __global__ void __launch_bounds__(kStripThreads, (NT <= 4 && KS <= 2) ? 2 : 1) conv_strip_kernel(StripParams p) {
+  after_previous<false>();
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int EPL = MT / 2;                              // table entries per lane and offset
   constexpr int WR = MT * 16;                              // rows of a warp
@@ -476,7 +477,7 @@ int launch_strip_kernel(StripParams& p, cudaStream_t st) {
   const int sms = current_sm_count();
   if (sms <= 0) return SPH_ERR_CUDA;
   const int grid = p.tiles < sms * per_sm ? p.tiles : sms * per_sm;
-  kern<<<grid, kStripThreads, smem, st>>>(p);
+  launch(kern, grid, kStripThreads, smem, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }

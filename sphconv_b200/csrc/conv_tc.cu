@@ -118,6 +118,7 @@ __device__ __forceinline__ void store_rows64_any(uint8_t* dst, int row_pitch, in
 // streams, not the tensor pipe or the memory system, set the pace once the data path is asynchronous.
 template <int KC, bool I8>
 __global__ void __maxnreg__(112) conv_gather_tc_kernel(TcParams p) {
+  after_previous<false>();
   constexpr int GK = RowShape<KC>::GK, NMMA = RowShape<KC>::NMMA;
   constexpr uint32_t X_BYTES = RowShape<KC>::X_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -299,6 +300,7 @@ __global__ void __maxnreg__(112) conv_gather_tc_kernel(TcParams p) {
 // [KV][K][N] row-major weights -> per-offset UMMA image of W[k]^T ([N x K], K-major, no swizzle).
 template <typename T>
 __global__ void pack_weight_kernel(const T* __restrict__ w, int kv, int K, int N, T* __restrict__ packed) {
+  after_previous();
   const int64_t total = (int64_t)kv * K * N;
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= total) return;
@@ -407,7 +409,7 @@ int conv_gather_tc(const void* rows, int dtype, int64_t n_rows, const void* pack
 #define SPH_TC_LAUNCH(KC_, I8_)                                                                                  \
   do {                                                                                                         \
     SPH_CUDA(allow_smem(conv_gather_tc_kernel<KC_, I8_>, kSmemTotal));                                         \
-    conv_gather_tc_kernel<KC_, I8_><<<grid, kTcThreads, smem_bytes, st>>>(p);                                  \
+    launch(conv_gather_tc_kernel<KC_, I8_>, grid, kTcThreads, smem_bytes, st, p);                                  \
   } while (0)
   if (p.is_i8) {
     switch (p.kc) {
@@ -444,9 +446,9 @@ int pack_weight(const void* w, int dtype, int kv, int K, int N, void* packed, cu
   const int threads = 256;
   const unsigned blocks = (unsigned)div_up64(total, threads);
   if (dtype == SPH_I8)
-    pack_weight_kernel<int8_t><<<blocks, threads, 0, st>>>((const int8_t*)w, kv, K, N, (int8_t*)packed);
+    launch(pack_weight_kernel<int8_t>, blocks, threads, 0, st, (const int8_t*)w, kv, K, N, (int8_t*)packed);
   else
-    pack_weight_kernel<uint16_t><<<blocks, threads, 0, st>>>((const uint16_t*)w, kv, K, N, (uint16_t*)packed);
+    launch(pack_weight_kernel<uint16_t>, blocks, threads, 0, st, (const uint16_t*)w, kv, K, N, (uint16_t*)packed);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }

@@ -118,6 +118,7 @@ __device__ __forceinline__ void store_row16(uint8_t* dst, int out_dtype, const u
 // streams, not the tensor pipe or the memory system, set the pace once the data path is asynchronous.
 template <int KC, bool I8>
 __global__ void __maxnreg__(112) conv_gather_rows_kernel(RowsParams p) {
+  after_previous<false>();
   constexpr int GK = RowShape<KC>::GK, NMMA = RowShape<KC>::NMMA;
   constexpr uint32_t X_BYTES = RowShape<KC>::X_BYTES;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -400,7 +401,7 @@ int conv_gather_tc_rows(const void* rows, int dtype, int64_t n_rows, const void*
 #define SPH_TC_LAUNCH(KC_, I8_)                                                                                    \
   do {                                                                                                           \
     SPH_CUDA(allow_smem(conv_gather_rows_kernel<KC_, I8_>, kSmemTotal));                                         \
-    conv_gather_rows_kernel<KC_, I8_><<<grid, kTcThreads, smem_bytes, st>>>(p);                                  \
+    launch(conv_gather_rows_kernel<KC_, I8_>, grid, kTcThreads, smem_bytes, st, p);                                  \
   } while (0)
   if (p.is_i8) {
     switch (p.kc) {

@@ -274,10 +274,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
   uint16_t* s_place = (uint16_t*)(base + p.place_off);  // [2][8 warps][kLines * LP][32]: of neighbours, in 16 bytes from the start of the run
   const int halves = p.halves;
 
-  if (tid < 64) {
-    s_epi[tid] = (tid < p.N && p.scale) ? __ldg(p.scale + tid) : 1.f;
-    s_epi[64 + tid] = tid < p.N ? p.bias.at<!I8>(tid) : 0.f;
-  }
   const uint32_t cap = (uint32_t)p.cap;
   const uint32_t slot_bytes = cap * ROW;
   if (tid < 16) {
@@ -314,6 +310,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
   if (warp == kMmaWarp) {
     tmem_alloc(smem_u32(&s_tmem_base), 512u);
     tmem_relinquish();
+  }
+  after_previous<false>();                     // nothing before this reads what another kernel writes
+  if (tid < 64) {
+    s_epi[tid] = (tid < p.N && p.scale) ? __ldg(p.scale + tid) : 1.f;
+    s_epi[64 + tid] = tid < p.N ? p.bias.at<!I8>(tid) : 0.f;
   }
   tc_fence_before();
   __syncthreads();
@@ -863,7 +864,7 @@ int conv_gather_tmem(const void* rows, int dtype, int64_t n_rows, const void* pa
 #define SPH_TMEM_LAUNCH(KC_, I8_, L_)                                                                    \
   do {                                                                                                   \
     SPH_CUDA(allow_smem(conv_gather_tmem_kernel<KC_, I8_, L_>, kSmemTotal));                             \
-    conv_gather_tmem_kernel<KC_, I8_, L_><<<grid, kThreads, smem_bytes, st>>>(map, p);                   \
+    launch(conv_gather_tmem_kernel<KC_, I8_, L_>, grid, kThreads, smem_bytes, st, map, p);                   \
   } while (0)
 #define SPH_TMEM_ROWS(I8_, L_)                        \
   switch (row_bytes) {                                \

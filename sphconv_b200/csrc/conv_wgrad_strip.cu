@@ -95,6 +95,7 @@ __device__ __forceinline__ void copy_channels(const uint16_t* src, int n, int pi
 // KT: tiles of 16 input channels, NP: pairs of 8-channel tiles of the output.
 template <int KT, int NP, int DT>
 __global__ void __launch_bounds__(kThreads, KT * NP <= 2 ? 2 : 1) conv_wgrad_strip_kernel(WgradStripParams p) {
+  after_previous<false>();
   extern __shared__ __align__(128) unsigned char smem[];
   constexpr int PX = 2 * KT + 1, PY = 2 * NP + 1;          // 16-byte units between rows (odd: other banks)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -330,7 +331,7 @@ int launch_wgrad_strip(WgradStripParams& p, cudaStream_t st) {
   int slices = sms * per_sm / (p.groups * p.halves);
   if (slices > p.tiles) slices = p.tiles;
   p.slices = slices < 1 ? 1 : slices;
-  kern<<<p.slices * p.groups * p.halves, kThreads, smem, st>>>(p);
+  launch(kern, p.slices * p.groups * p.halves, kThreads, smem, st, p);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }

@@ -58,6 +58,7 @@ struct WgParams {
 // KCX = 16-byte chunks per gathered X row (2, 4, 8, 16); compile-time so that the gather of a batch is straight-line code.
 template <int KCX>
 __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) {
+  after_previous<false>();
   constexpr int OB = 16 / KCX;                   // offsets per batch (= p.ob)
   constexpr int LPR = KCX < 8 ? KCX : 8;         // lanes per row = consecutive rows per lane
   constexpr int PASSES = KCX / LPR;              // 2 only for 256-byte rows
@@ -328,7 +329,7 @@ int conv_wgrad_tc(const void* rows, const void* dout, int dtype, int64_t n_rows,
 #define SPH_WG_LAUNCH(KCX_)                                                                                        \
   do {                                                                                                           \
     SPH_CUDA(allow_smem(conv_wgrad_tc_kernel<KCX_>, kSmemTotal));                                                \
-    conv_wgrad_tc_kernel<KCX_><<<grid, kThreads, smem_bytes, st>>>(p);                                           \
+    launch(conv_wgrad_tc_kernel<KCX_>, grid, kThreads, smem_bytes, st, p);                                           \
   } while (0)
   switch (p.kc_x) {
     case 2: SPH_WG_LAUNCH(2); break;

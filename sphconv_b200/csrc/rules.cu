@@ -53,6 +53,7 @@ struct ColMask {
 __global__ void __launch_bounds__(256)
 build_colmask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, int64_t ncols, int words, int D,
                      uint2* __restrict__ table, int* __restrict__ row_col) {
+  after_previous();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ncols * words) return;
   const int64_t c = t / words;
@@ -82,6 +83,7 @@ template <int WORDS>
 __global__ void __launch_bounds__(256)
 build_colmask_cols_kernel(const int* __restrict__ zi, const int* __restrict__ zp, int64_t ncols, int D,
                           uint2* __restrict__ table, int* __restrict__ row_col) {
+  after_previous();
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncols) return;
   const int s = col_start(zp, c), e = __ldg(zp + c);
@@ -120,6 +122,7 @@ build_colmask_cols_kernel(const int* __restrict__ zi, const int* __restrict__ zp
 // Column id of every row, for grids without the index.
 __global__ void __launch_bounds__(256)
 park_columns_kernel(const int* __restrict__ zp, int64_t ncols, int* __restrict__ row_col) {
+  after_previous();
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncols) return;
   const int e = __ldg(zp + c);
@@ -132,6 +135,7 @@ __global__ void __launch_bounds__(kEmitThreads)
 emit_rules_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
                   const int* __restrict__ out_zp, Geom g, int64_t in_nnz, int tile_n_max, int* __restrict__ rules,
                   int* __restrict__ rule_size, int* __restrict__ nbr_t, int* __restrict__ status) {
+  after_previous();
   __shared__ int s_cnt[kMaxKV];
   __shared__ int s_rstart[kEmitMaxRanges];
   __shared__ int s_roff[kEmitMaxRanges + 1];
@@ -311,6 +315,7 @@ __global__ void __launch_bounds__(256)
 nbr_search_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, const int* __restrict__ out_zi,
                   Geom g,
                   int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, int* __restrict__ status) {
+  after_previous();
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= out_nnz) return;
   const int c = parked_column(g, out_nnz, r, nbr, status);
@@ -325,6 +330,7 @@ nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, co
                 Geom g,
                 int64_t in_nnz, int64_t out_nnz, int* nbr, int* __restrict__ nbr_t, ColMask cm,
                 int* __restrict__ status) {
+  after_previous();
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= out_nnz) return;
   const int c = parked_column(g, out_nnz, r, nbr, status);
@@ -430,6 +436,7 @@ __global__ void __launch_bounds__(kFixWarps * 32)
 rule_lists_fixed_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int tile_n_max, int n_kg,
                         const int* __restrict__ nbr, int* __restrict__ rules, int* __restrict__ rule_size,
                         int* __restrict__ status) {
+  after_previous();
   __shared__ int s_rs[kFixWarps][kListRanges];
   __shared__ int s_off[kFixWarps][kListRanges + 1];
   const int lane = threadIdx.x & 31;
@@ -540,6 +547,7 @@ constexpr int kTilePositions = 2048;   // list positions whose rows are mapped a
 __global__ void __launch_bounds__(kTileWarps * 32)
 rule_lists_tile_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int tile_n_max, const int* __restrict__ nbr,
                        int* __restrict__ rules, int* __restrict__ rule_size, int* __restrict__ status) {
+  after_previous();
   __shared__ int s_rs[kListRanges];
   __shared__ int s_off[kListRanges + 1];
   __shared__ int s_row[kTilePositions];
@@ -633,6 +641,7 @@ __global__ void __launch_bounds__(kListWarps * 32)
 rule_lists_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, int tile_n_max, int kg, int n_kg,
                   const int* __restrict__ nbr, int* __restrict__ rules, int* __restrict__ rule_size,
                   int* __restrict__ status) {
+  after_previous();
   __shared__ int s_rs[kListWarps][kListRanges];
   __shared__ int s_off[kListWarps][kListRanges + 1];
   const int lane = threadIdx.x & 31;
@@ -764,6 +773,7 @@ __device__ __forceinline__ int block_inclusive_scan(int v, int* s_warp /*[8]*/, 
 __global__ void __launch_bounds__(kScanThreads)
 strided_mask_kernel(const int* __restrict__ zi, const int* __restrict__ zp, Geom g, int words, int64_t ncols,
                     ColMask cm, uint32_t* __restrict__ mask, int* __restrict__ counts, int* __restrict__ blocksum) {
+  after_previous();
   __shared__ int s_warp[kScanThreads / 32];
   const int64_t c = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
   int count = 0;
@@ -839,6 +849,7 @@ __host__ __device__ inline bool strided_bits_ok(const Geom& g) {
 __global__ void __launch_bounds__(256)
 strided_bits_kernel(Geom g, int words_out, int cols_per_block, int64_t ncols_out, ColMask cm, uint32_t* __restrict__ mask,
                     int* __restrict__ counts, int* __restrict__ blocksum) {
+  after_previous();
   __shared__ int s_pop[256];
   __shared__ int s_warp[kScanThreads / 32];
   const int64_t c0 = (int64_t)blockIdx.x * cols_per_block;
@@ -928,6 +939,7 @@ strided_bits_kernel(Geom g, int words_out, int cols_per_block, int64_t ncols_out
 __global__ void __launch_bounds__(kScanThreads)
 count_columns_kernel(const uint32_t* __restrict__ mask, int words, int64_t ncols, int* __restrict__ counts,
                      int* __restrict__ blocksum) {
+  after_previous();
   __shared__ int s_warp[kScanThreads / 32];
   const int64_t c = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
   int count = 0;
@@ -950,6 +962,7 @@ constexpr int kScanCols = 4 * kScanThreads;
 __global__ void __launch_bounds__(kScanThreads)
 scan_columns_kernel(int* __restrict__ counts, int64_t ncols, const int* __restrict__ blocksum, int per,
                     int* __restrict__ out_total, int* out_total_host) {
+  after_previous();
   __shared__ int s_warp[kScanThreads / 32];
   const int tid = threadIdx.x;
   int before = 0;
@@ -982,6 +995,7 @@ scan_columns_kernel(int* __restrict__ counts, int64_t ncols, const int* __restri
 __global__ void __launch_bounds__(kScanThreads)
 write_oz_idx_kernel(const uint32_t* __restrict__ mask, const int* __restrict__ oz_ptr, int words, int64_t ncols,
                     int* __restrict__ oz_idx, int* __restrict__ row_col) {
+  after_previous();
   // one thread per (column, 32-bin word): its first row is the column's start plus the bins of the words before it
   const int64_t t = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
   if (t >= ncols * words) return;
@@ -1003,6 +1017,7 @@ write_oz_idx_kernel(const uint32_t* __restrict__ mask, const int* __restrict__ o
 __global__ void rules_to_nbr_kernel(const int* __restrict__ rules, const int* __restrict__ rule_size, int n_lists,
                                     int kv, int tnm, int64_t in_rows, int64_t out_rows, int* __restrict__ nbr,
                                     int* __restrict__ nbr_t, int* __restrict__ status) {
+  after_previous();
   const int lane = threadIdx.x & 31;
   const int64_t lst = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (lst >= n_lists) return;
@@ -1046,7 +1061,7 @@ int build_colmask(const int* zi, const int* zp, const Geom& g, int64_t in_nnz, v
   const int64_t ncols = (int64_t)g.B * g.H * g.W;
   if (!want_colmask(g, in_nnz) || scratch == nullptr) {
     if (row_col == nullptr || in_nnz == 0) return SPH_OK;
-    park_columns_kernel<<<(unsigned)div_up64(ncols, 256), 256, 0, st>>>(zp, ncols, row_col);
+    launch(park_columns_kernel, (unsigned)div_up64(ncols, 256), 256, 0, st, zp, ncols, row_col);
     SPH_LAUNCH_CHECK();
     return SPH_OK;
   }
@@ -1058,12 +1073,12 @@ int build_colmask(const int* zi, const int* zp, const Geom& g, int64_t in_nnz, v
   // one thread per column pays off on large grids; a small grid (a few hundred CTAs of the other form) is launch-bound
   // either way and has more threads in flight with one thread per column and word
   switch (ncols >= 100000 ? words : 0) {
-    case 1: build_colmask_cols_kernel<1><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
-    case 2: build_colmask_cols_kernel<2><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
-    case 4: build_colmask_cols_kernel<4><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
-    case 8: build_colmask_cols_kernel<8><<<col_grid, 256, 0, st>>>(zi, zp, ncols, g.D, table, row_col); break;
+    case 1: launch(build_colmask_cols_kernel<1>, col_grid, 256, 0, st, zi, zp, ncols, g.D, table, row_col); break;
+    case 2: launch(build_colmask_cols_kernel<2>, col_grid, 256, 0, st, zi, zp, ncols, g.D, table, row_col); break;
+    case 4: launch(build_colmask_cols_kernel<4>, col_grid, 256, 0, st, zi, zp, ncols, g.D, table, row_col); break;
+    case 8: launch(build_colmask_cols_kernel<8>, col_grid, 256, 0, st, zi, zp, ncols, g.D, table, row_col); break;
     default:
-      build_colmask_kernel<<<(unsigned)div_up64(ncols * words, 256), 256, 0, st>>>(zi, zp, ncols, words, g.D, table,
+      launch(build_colmask_kernel, (unsigned)div_up64(ncols * words, 256), 256, 0, st, zi, zp, ncols, words, g.D, table,
                                                                                             row_col);
   }
   SPH_LAUNCH_CHECK();
@@ -1081,7 +1096,7 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
   if (g.KV == kTileWarps * kTileNK && g.nTile >= 1024 && out_nnz >= 256 * (int64_t)g.nTile) {
     // Large tiles, and enough of them: 1.5 M rows in 2048 tiles of 745, 1.9 M / 18.3 M pairs 107 -> 82 / 133 -> 98 us.  A CTA's
     // start takes too long where tiles are small (567 k rows in 8192 tiles of 69: 53 -> 86) or few (683 k in 512: 51 -> 61).
-    rule_lists_tile_kernel<<<(unsigned)g.nTile, kTileWarps * 32, 0, st>>>(out_zp, g, out_nnz, tnm, nbr, rules, rule_size, status);
+    launch(rule_lists_tile_kernel, (unsigned)g.nTile, kTileWarps * 32, 0, st, out_zp, g, out_nnz, tnm, nbr, rules, rule_size, status);
     SPH_LAUNCH_CHECK();
     return SPH_OK;
   }
@@ -1092,8 +1107,8 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
     // positions per step beats 2, 4 or 8 (more registers per thread = fewer list warps resident beside the persistent
     // convolution CTA), and 27 offsets per warp leaves too few warps.
 #define SPH_LISTS_FIXED(NK)                                                                                           \
-  rule_lists_fixed_kernel<NK, 1><<<(unsigned)div_up64((int64_t)g.nTile * (27 / NK), kFixWarps), kFixWarps * 32, 0,     \
-                                   st>>>(out_zp, g, out_nnz, tnm, 27 / NK, nbr, rules, rule_size, status)
+  launch(rule_lists_fixed_kernel<NK, 1>, (unsigned)div_up64((int64_t)g.nTile * (27 / NK), kFixWarps), kFixWarps * 32, 0,     \
+                                   st, out_zp, g, out_nnz, tnm, 27 / NK, nbr, rules, rule_size, status)
     if ((int64_t)g.nTile * 3 >= 6000) SPH_LISTS_FIXED(9);
     else SPH_LISTS_FIXED(3);
 #undef SPH_LISTS_FIXED
@@ -1111,7 +1126,7 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
   // chunks per step: the smallest that holds 1.25 x the average tile (larger tiles take more steps)
   const int64_t want = (out_nnz / (g.nTile > 0 ? g.nTile : 1)) * 5 / 4;
 #define SPH_LISTS(CH)                                                                                             \
-  rule_lists_kernel<CH><<<grid, kListWarps * 32, 0, st>>>(out_zp, g, out_nnz, tnm, kg, n_kg, nbr, rules, rule_size, \
+  launch(rule_lists_kernel<CH>, grid, kListWarps * 32, 0, st, out_zp, g, out_nnz, tnm, kg, n_kg, nbr, rules, rule_size, \
                                                           status)
   if (want <= 32) SPH_LISTS(1);
   else if (want <= 64) SPH_LISTS(2);
@@ -1134,7 +1149,7 @@ int launch_emit(const int* in_zi, const int* in_zp, const int* out_zi, const int
     SPH_CUDA(cudaMemsetAsync(nbr_t, 0xFF, (size_t)g.KV * (size_t)in_nnz * sizeof(int), st));
   }
   if (nbr == nullptr && out_nnz > 0) {
-    emit_rules_kernel<<<g.nTile, kEmitThreads, 0, st>>>(in_zi, in_zp, out_zi, out_zp, g, in_nnz, tnm, rules, rule_size,
+    launch(emit_rules_kernel, g.nTile, kEmitThreads, 0, st, in_zi, in_zp, out_zi, out_zp, g, in_nnz, tnm, rules, rule_size,
                                                         nbr_t, status);
     SPH_LAUNCH_CHECK();
     return SPH_OK;
@@ -1142,9 +1157,9 @@ int launch_emit(const int* in_zi, const int* in_zp, const int* out_zi, const int
   if (out_nnz > 0) {
     const unsigned grid = (unsigned)div_up64(out_nnz, 256);
 #define SPH_NBR_ROWS(KD, T) \
-  nbr_rows_kernel<KD, T><<<grid, 256, 0, st>>>(in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, cm, status)
+  launch(nbr_rows_kernel<KD, T>, grid, 256, 0, st, in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, cm, status)
     if (cm.table == nullptr) {
-      nbr_search_kernel<<<grid, 256, 0, st>>>(in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, status);
+      launch(nbr_search_kernel, grid, 256, 0, st, in_zi, in_zp, out_zi, g, in_nnz, out_nnz, nbr, nbr_t, status);
     } else if (g.KD == 3 && g.KW == 3) {
       if (nbr_t) SPH_NBR_ROWS(3, true); else SPH_NBR_ROWS(3, false);
     } else {
@@ -1164,10 +1179,9 @@ int launch_emit(const int* in_zi, const int* in_zp, const int* out_zi, const int
 // needs ceil(ncols / 256) ints.
 int column_prefix_from_masks(const uint32_t* mask, int words, int64_t ncols, int* prefix, int* blocksum, int* total_dev,
                              int* total_host, cudaStream_t st) {
-  count_columns_kernel<<<(unsigned)div_up64(ncols, kScanThreads), kScanThreads, 0, st>>>(mask, words, ncols, prefix, blocksum);
+  launch(count_columns_kernel, (unsigned)div_up64(ncols, kScanThreads), kScanThreads, 0, st, mask, words, ncols, prefix, blocksum);
   SPH_LAUNCH_CHECK();
-  scan_columns_kernel<<<(unsigned)div_up64(ncols, kScanCols), kScanThreads, 0, st>>>(
-      prefix, ncols, blocksum, kScanCols / kScanThreads, total_dev, total_host);
+  launch(scan_columns_kernel, (unsigned)div_up64(ncols, kScanCols), kScanThreads, 0, st, prefix, ncols, blocksum, kScanCols / kScanThreads, total_dev, total_host);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -1474,15 +1488,14 @@ int strided_count_impl(const int32_t* d_z_idx, const int32_t* d_z_ptr, int64_t n
   if (rc != SPH_OK) return rc;
   int per = kScanCols / kScanThreads;              // block sums per kScanCols columns
   if (cm.table != nullptr && strided_bits_ok(g) && l.words <= 64) {
-    strided_bits_kernel<<<l.nblk, 256, 0, st>>>(g, l.words, l.cols_per_block, l.ncols, cm, mask, d_oz_ptr, blocksum);
+    launch(strided_bits_kernel, l.nblk, 256, 0, st, g, l.words, l.cols_per_block, l.ncols, cm, mask, d_oz_ptr, blocksum);
     SPH_LAUNCH_CHECK();
     per = kScanCols / l.cols_per_block;
   } else {
-    strided_mask_kernel<<<(unsigned)div_up64(l.ncols, kScanThreads), kScanThreads, 0, st>>>(
-        d_z_idx, d_z_ptr, g, l.words, l.ncols, cm, mask, d_oz_ptr, blocksum);
+    launch(strided_mask_kernel, (unsigned)div_up64(l.ncols, kScanThreads), kScanThreads, 0, st, d_z_idx, d_z_ptr, g, l.words, l.ncols, cm, mask, d_oz_ptr, blocksum);
     SPH_LAUNCH_CHECK();
   }
-  scan_columns_kernel<<<(unsigned)div_up64(l.ncols, kScanCols), kScanThreads, 0, st>>>(d_oz_ptr, l.ncols, blocksum, per,
+  launch(scan_columns_kernel, (unsigned)div_up64(l.ncols, kScanCols), kScanThreads, 0, st, d_oz_ptr, l.ncols, blocksum, per,
                                                                                        d_out_nnz, dev_word);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
@@ -1534,8 +1547,7 @@ extern "C" int sph_rules_strided_fill(const int32_t* d_z_idx, const int32_t* d_z
   StridedScratch l = strided_layout(g, nnz);
   const uint32_t* mask = (const uint32_t*)d_scratch;
   if (out_nnz > 0) {
-    write_oz_idx_kernel<<<(unsigned)div_up64(l.ncols * l.words, kScanThreads), kScanThreads, 0, st>>>(
-        mask, d_oz_ptr, l.words, l.ncols, d_oz_idx, parked_columns(g, d_nbr, out_nnz));
+    launch(write_oz_idx_kernel, (unsigned)div_up64(l.ncols * l.words, kScanThreads), kScanThreads, 0, st, mask, d_oz_ptr, l.words, l.ncols, d_oz_idx, parked_columns(g, d_nbr, out_nnz));
     SPH_LAUNCH_CHECK();
   }
   return launch_emit(d_z_idx, d_z_ptr, d_oz_idx, d_oz_ptr, g, nnz, out_nnz, tile_n_max, d_rules, d_rule_size,
@@ -1553,7 +1565,7 @@ extern "C" int sph_rules_to_nbr(const int32_t* d_rules, const int32_t* d_rule_si
   int64_t n_lists = (int64_t)n_tile * kv;
   int threads = 256;
   int64_t blocks = div_up64(n_lists * 32, threads);
-  rules_to_nbr_kernel<<<(unsigned)blocks, threads, 0, st>>>(d_rules, d_rule_size, (int)n_lists, kv, tile_n_max,
+  launch(rules_to_nbr_kernel, (unsigned)blocks, threads, 0, st, d_rules, d_rule_size, (int)n_lists, kv, tile_n_max,
                                                             in_rows, out_rows, d_nbr, d_nbr_t, d_status);
   SPH_LAUNCH_CHECK();
   return SPH_OK;

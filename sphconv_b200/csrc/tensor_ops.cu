@@ -20,6 +20,7 @@ __device__ __forceinline__ int col_begin(const int* __restrict__ zp, int64_t c) 
 __global__ void __launch_bounds__(kOpsThreads)
 mark_voxels_kernel(const int* __restrict__ idx, int64_t nnz, int B, int H, int W, int D, int words,
                    uint32_t* __restrict__ mask, int* __restrict__ status) {
+  after_previous();
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnz) return;
   const int4 v = __ldg((const int4*)idx + n);
@@ -37,6 +38,7 @@ __global__ void __launch_bounds__(kOpsThreads)
 place_voxels_kernel(const int* __restrict__ idx, int64_t nnz, int B, int H, int W, int D, int words,
                     const uint32_t* __restrict__ mask, const int* __restrict__ z_ptr, int* __restrict__ z_idx,
                     int* __restrict__ permutation) {
+  after_previous();
   const int64_t n = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (n >= nnz) return;
   const int4 v = __ldg((const int4*)idx + n);
@@ -62,6 +64,7 @@ template <typename V>
 __global__ void __launch_bounds__(kOpsThreads)
 permute_rows_kernel(const V* __restrict__ src, V* __restrict__ dst, const int* __restrict__ perm, int64_t n_rows,
                     int pieces, int gather) {
+  after_previous();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t n = t / pieces;
   const int c = (int)(t % pieces);
@@ -77,6 +80,7 @@ template <typename V>
 __global__ void __launch_bounds__(kOpsThreads)
 dense_rows_kernel(V* __restrict__ rows, const int* __restrict__ z_idx, const int* __restrict__ z_ptr, int64_t nnz,
                   int64_t ncols, int D, int pieces, V* __restrict__ dense, int backward, int* __restrict__ status) {
+  after_previous();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t n = t / pieces;
   const int c = (int)(t % pieces);
@@ -137,6 +141,7 @@ __global__ void __launch_bounds__(kOpsThreads)
 dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx, const int* __restrict__ z_ptr,
                             int64_t nnz, int64_t cols_per_b, int cols_per_block, int D, int C, int chunk, int stride,
                             E* __restrict__ dense, int* __restrict__ status) {
+  after_previous<false>();
   extern __shared__ __align__(16) unsigned char smem[];
   int* s_map = (int*)smem;                                        // [cells] staged row of the cell or -1
   E* s_rows = (E*)(smem + ((size_t)cols_per_block * D * sizeof(int) + 15) / 16 * 16);   // [rows][stride]
@@ -274,8 +279,7 @@ int launch_dense_cf(void* rows, const int* z_idx, const int* z_ptr, int64_t nnz,
   const int smem = (cells * (int)sizeof(int) + 15) / 16 * 16 + cells * stride * (int)sizeof(E);
   auto kern = backward ? dense_channels_first_kernel<E, V, true> : dense_channels_first_kernel<E, V, false>;
   SPH_CUDA(allow_smem(kern, kDenseSmem));
-  kern<<<dim3((unsigned)div_up64(cols_per_b, cols), (unsigned)B), kOpsThreads, smem, st>>>(
-      (E*)rows, z_idx, z_ptr, nnz, cols_per_b, cols, D, C, chunk, stride, (E*)dense, status);
+  launch(kern, dim3((unsigned)div_up64(cols_per_b, cols), (unsigned)B), kOpsThreads, smem, st, (E*)rows, z_idx, z_ptr, nnz, cols_per_b, cols, D, C, chunk, stride, (E*)dense, status);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -343,14 +347,14 @@ extern "C" int sph_init_tensor(const void* d_feature, int32_t row_bytes, int64_t
   SPH_CUDA(cudaMemsetAsync(d_scratch, 0, 256 + l.mask_bytes, st));
   const int H = shape[0], W = shape[1], D = shape[2];
   if (nnz > 0) {
-    mark_voxels_kernel<<<(unsigned)div_up64(nnz, kOpsThreads), kOpsThreads, 0, st>>>(d_indices, nnz, B, H, W, D, l.words,
+    launch(mark_voxels_kernel, (unsigned)div_up64(nnz, kOpsThreads), kOpsThreads, 0, st, d_indices, nnz, B, H, W, D, l.words,
                                                                                       mask, d_status);
     SPH_LAUNCH_CHECK();
   }
   int rc = column_prefix_from_masks(mask, l.words, l.ncols, d_z_ptr, blocksum, header, nullptr, st);
   if (rc != SPH_OK) return rc;
   if (nnz > 0) {
-    place_voxels_kernel<<<(unsigned)div_up64(nnz, kOpsThreads), kOpsThreads, 0, st>>>(d_indices, nnz, B, H, W, D, l.words,
+    launch(place_voxels_kernel, (unsigned)div_up64(nnz, kOpsThreads), kOpsThreads, 0, st, d_indices, nnz, B, H, W, D, l.words,
                                                                                        mask, d_z_ptr, d_z_idx,
                                                                                        d_permutation);
     SPH_LAUNCH_CHECK();
@@ -372,10 +376,10 @@ extern "C" int sph_permute_rows(const void* d_src, int32_t row_bytes, int64_t n_
   const int pieces = row_bytes / pb;
   const unsigned blocks = (unsigned)div_up64(n_rows * pieces, kOpsThreads);
   switch (pb) {
-    case 16: permute_rows_kernel<uint4><<<blocks, kOpsThreads, 0, st>>>((const uint4*)d_src, (uint4*)d_dst, d_permutation, n_rows, pieces, gather); break;
-    case 4: permute_rows_kernel<uint32_t><<<blocks, kOpsThreads, 0, st>>>((const uint32_t*)d_src, (uint32_t*)d_dst, d_permutation, n_rows, pieces, gather); break;
-    case 2: permute_rows_kernel<uint16_t><<<blocks, kOpsThreads, 0, st>>>((const uint16_t*)d_src, (uint16_t*)d_dst, d_permutation, n_rows, pieces, gather); break;
-    default: permute_rows_kernel<uint8_t><<<blocks, kOpsThreads, 0, st>>>((const uint8_t*)d_src, (uint8_t*)d_dst, d_permutation, n_rows, pieces, gather); break;
+    case 16: launch(permute_rows_kernel<uint4>, blocks, kOpsThreads, 0, st, (const uint4*)d_src, (uint4*)d_dst, d_permutation, n_rows, pieces, gather); break;
+    case 4: launch(permute_rows_kernel<uint32_t>, blocks, kOpsThreads, 0, st, (const uint32_t*)d_src, (uint32_t*)d_dst, d_permutation, n_rows, pieces, gather); break;
+    case 2: launch(permute_rows_kernel<uint16_t>, blocks, kOpsThreads, 0, st, (const uint16_t*)d_src, (uint16_t*)d_dst, d_permutation, n_rows, pieces, gather); break;
+    default: launch(permute_rows_kernel<uint8_t>, blocks, kOpsThreads, 0, st, (const uint8_t*)d_src, (uint8_t*)d_dst, d_permutation, n_rows, pieces, gather); break;
   }
   SPH_LAUNCH_CHECK();
   return SPH_OK;
@@ -394,10 +398,10 @@ extern "C" int sph_to_dense(void* d_rows, int32_t row_bytes, int64_t nnz, const 
   const int pieces = row_bytes / pb;
   const unsigned blocks = (unsigned)div_up64(nnz * pieces, kOpsThreads);
   switch (pb) {
-    case 16: dense_rows_kernel<uint4><<<blocks, kOpsThreads, 0, st>>>((uint4*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint4*)d_dense, backward, d_status); break;
-    case 4: dense_rows_kernel<uint32_t><<<blocks, kOpsThreads, 0, st>>>((uint32_t*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint32_t*)d_dense, backward, d_status); break;
-    case 2: dense_rows_kernel<uint16_t><<<blocks, kOpsThreads, 0, st>>>((uint16_t*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint16_t*)d_dense, backward, d_status); break;
-    default: dense_rows_kernel<uint8_t><<<blocks, kOpsThreads, 0, st>>>((uint8_t*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint8_t*)d_dense, backward, d_status); break;
+    case 16: launch(dense_rows_kernel<uint4>, blocks, kOpsThreads, 0, st, (uint4*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint4*)d_dense, backward, d_status); break;
+    case 4: launch(dense_rows_kernel<uint32_t>, blocks, kOpsThreads, 0, st, (uint32_t*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint32_t*)d_dense, backward, d_status); break;
+    case 2: launch(dense_rows_kernel<uint16_t>, blocks, kOpsThreads, 0, st, (uint16_t*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint16_t*)d_dense, backward, d_status); break;
+    default: launch(dense_rows_kernel<uint8_t>, blocks, kOpsThreads, 0, st, (uint8_t*)d_rows, d_z_idx, d_z_ptr, nnz, ncols, shape[2], pieces, (uint8_t*)d_dense, backward, d_status); break;
   }
   SPH_LAUNCH_CHECK();
   return SPH_OK;
@@ -447,6 +451,7 @@ template <typename T>
 __global__ void __launch_bounds__(kEpiThreads)
 epilogue_backward_kernel(const T* __restrict__ d_out, const T* __restrict__ out, int64_t n, int C, int relu,
                          T* __restrict__ d_pre, float* __restrict__ d_bias) {
+  after_previous();
   __shared__ float s_sum[kEpiThreads];
   const int c = threadIdx.x % C;
   const int rows_per_block = kEpiThreads / C;
@@ -480,6 +485,7 @@ template <typename T>
 __global__ void __launch_bounds__(kEpiThreads)
 epilogue_backward_vec_kernel(const T* __restrict__ d_out, const T* __restrict__ out, int64_t n, int C, int relu,
                              T* __restrict__ d_pre, float* __restrict__ d_bias) {
+  after_previous();
   constexpr int V = 16 / (int)sizeof(T);
   struct alignas(16) Vec { T e[V]; };
   __shared__ float s_sum[kEpiThreads];                 // [C], C <= 256
@@ -540,7 +546,7 @@ bool launch_epilogue_vec(const void* d_out, const void* out, int64_t n, int C, i
   int64_t blocks = div_up64(n, (int64_t)rows_per_block * kVecRows);
   const int sms = current_sm_count();
   if (blocks > (int64_t)sms * 8) blocks = (int64_t)sms * 8;
-  epilogue_backward_vec_kernel<T><<<(unsigned)blocks, kEpiThreads, 0, st>>>((const T*)d_out, (const T*)out, n, C, relu, (T*)d_pre, d_bias);
+  launch(epilogue_backward_vec_kernel<T>, (unsigned)blocks, kEpiThreads, 0, st, (const T*)d_out, (const T*)out, n, C, relu, (T*)d_pre, d_bias);
   return true;
 }
 
@@ -568,9 +574,9 @@ extern "C" int sph_epilogue_backward(const void* d_dout, const void* d_out, int 
   if (blocks > 148 * 16) blocks = 148 * 16;
   if (blocks < 1) blocks = 1;
   switch (dtype) {
-    case SPH_F32: epilogue_backward_kernel<float><<<(unsigned)blocks, kEpiThreads, 0, st>>>((const float*)d_dout, (const float*)d_out, n, channels, relu, (float*)d_dpre, d_dbias); break;
-    case SPH_F16: epilogue_backward_kernel<__half><<<(unsigned)blocks, kEpiThreads, 0, st>>>((const __half*)d_dout, (const __half*)d_out, n, channels, relu, (__half*)d_dpre, d_dbias); break;
-    default: epilogue_backward_kernel<__nv_bfloat16><<<(unsigned)blocks, kEpiThreads, 0, st>>>((const __nv_bfloat16*)d_dout, (const __nv_bfloat16*)d_out, n, channels, relu, (__nv_bfloat16*)d_dpre, d_dbias); break;
+    case SPH_F32: launch(epilogue_backward_kernel<float>, (unsigned)blocks, kEpiThreads, 0, st, (const float*)d_dout, (const float*)d_out, n, channels, relu, (float*)d_dpre, d_dbias); break;
+    case SPH_F16: launch(epilogue_backward_kernel<__half>, (unsigned)blocks, kEpiThreads, 0, st, (const __half*)d_dout, (const __half*)d_out, n, channels, relu, (__half*)d_dpre, d_dbias); break;
+    default: launch(epilogue_backward_kernel<__nv_bfloat16>, (unsigned)blocks, kEpiThreads, 0, st, (const __nv_bfloat16*)d_dout, (const __nv_bfloat16*)d_out, n, channels, relu, (__nv_bfloat16*)d_dpre, d_dbias); break;
   }
   SPH_LAUNCH_CHECK();
   return SPH_OK;

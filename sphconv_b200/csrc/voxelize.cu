@@ -99,6 +99,7 @@ __device__ __forceinline__ int cell_of(float v, float lo, float hi, int cells) {
 // sys [n][4] = (first, second, third coordinate, intensity) of every point.
 __global__ void __launch_bounds__(kVoxThreads)
 voxel_transform_kernel(const float* __restrict__ pts, int stride, int64_t n, int system, float4* __restrict__ sys) {
+  after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float* p = pts + i * stride;
@@ -124,6 +125,7 @@ voxel_transform_kernel(const float* __restrict__ pts, int stride, int64_t n, int
 __global__ void __launch_bounds__(kVoxThreads)
 voxel_bin_kernel(const float4* __restrict__ sys, int64_t n, const int* __restrict__ scan_ptr, VoxGrid g,
                  const int* __restrict__ cut, uint32_t* __restrict__ mask, int2* __restrict__ cell) {
+  after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int b = scan_of(scan_ptr, g.B, i);
@@ -147,6 +149,7 @@ voxel_bin_kernel(const float4* __restrict__ sys, int64_t n, const int* __restric
 __global__ void __launch_bounds__(kVoxThreads)
 voxel_rows_kernel(const int2* __restrict__ cell, int64_t n, int words, const uint32_t* __restrict__ mask,
                   const int* __restrict__ z_ptr, int* __restrict__ row, int* __restrict__ sel0) {
+  after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int2 c = cell[i];
@@ -166,6 +169,7 @@ voxel_rows_kernel(const int2* __restrict__ cell, int64_t n, int words, const uin
 // Next smallest point index of every row: the smallest one above the previous round's.
 __global__ void __launch_bounds__(kVoxThreads)
 voxel_next_kernel(const int* __restrict__ row, int64_t n, const int* __restrict__ sel_prev, int* __restrict__ sel_cur) {
+  after_previous();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int r = __ldg(row + i);
@@ -178,6 +182,7 @@ __global__ void __launch_bounds__(kCutThreads)
 voxel_cut_kernel(const int* __restrict__ scan_ptr, VoxGrid g, const int* __restrict__ z_ptr,
                  const int* __restrict__ row, const int* __restrict__ sel0, int64_t n, int* __restrict__ cut,
                  int* any_cut_host) {
+  after_previous();
   __shared__ int s_warp[kCutThreads / 32];
   __shared__ int s_running;
   const int b = blockIdx.x;
@@ -223,6 +228,7 @@ voxel_mean_kernel(const float* __restrict__ pts, int stride, const float4* __res
                   const int* __restrict__ scan_ptr, VoxGrid g, const int2* __restrict__ cell,
                   const int* __restrict__ sel, int64_t sel_stride, int64_t nnz, int C, float* __restrict__ feature,
                   int* __restrict__ z_idx, int4* __restrict__ coords, int* __restrict__ num_points) {
+  after_previous();
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t r = t / C;
   const int c = (int)(t % C);
@@ -262,6 +268,7 @@ __global__ void __launch_bounds__(kVoxThreads)
 voxel_mean4_kernel(const float4* __restrict__ pts, VoxGrid g, const int2* __restrict__ cell, const int* __restrict__ sel,
                    int64_t sel_stride, int64_t nnz, float4* __restrict__ feature, int* __restrict__ z_idx,
                    int4* __restrict__ coords, int* __restrict__ num_points) {
+  after_previous();
   const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nnz) return;
   const int first = __ldg(sel + r);
@@ -303,20 +310,20 @@ int run_passes(const float4* sys, const int* scan_ptr, int64_t n, const VoxGrid&
   const unsigned blocks = (unsigned)div_up64(n, kVoxThreads);
   if (n > 0) {
     SPH_CUDA(cudaMemsetAsync(sel, 0x7f, (size_t)n * sizeof(int) * g.max_points, st));
-    voxel_bin_kernel<<<blocks, kVoxThreads, 0, st>>>(sys, n, scan_ptr, g, cut, mask, cell);
+    launch(voxel_bin_kernel, blocks, kVoxThreads, 0, st, sys, n, scan_ptr, g, cut, mask, cell);
     SPH_LAUNCH_CHECK();
   }
   int rc = column_prefix_from_masks(mask, g.words, g.ncols, z_ptr, blocksum, header + 1, rows_word, st);
   if (rc != SPH_OK) return rc;
   if (n > 0) {
-    voxel_rows_kernel<<<blocks, kVoxThreads, 0, st>>>(cell, n, g.words, mask, z_ptr, row, sel);
+    launch(voxel_rows_kernel, blocks, kVoxThreads, 0, st, cell, n, g.words, mask, z_ptr, row, sel);
     SPH_LAUNCH_CHECK();
     for (int j = 1; j < g.max_points; ++j) {
-      voxel_next_kernel<<<blocks, kVoxThreads, 0, st>>>(row, n, sel + (int64_t)(j - 1) * n, sel + (int64_t)j * n);
+      launch(voxel_next_kernel, blocks, kVoxThreads, 0, st, row, n, sel + (int64_t)(j - 1) * n, sel + (int64_t)j * n);
       SPH_LAUNCH_CHECK();
     }
     if (cut_word) {
-      voxel_cut_kernel<<<g.B, kCutThreads, 0, st>>>(scan_ptr, g, z_ptr, row, sel, n, cut, cut_word);
+      launch(voxel_cut_kernel, g.B, kCutThreads, 0, st, scan_ptr, g, z_ptr, row, sel, n, cut, cut_word);
       SPH_LAUNCH_CHECK();
     }
   }
@@ -337,8 +344,7 @@ extern "C" int sph_voxel_transform(const float* d_points, int32_t point_stride, 
   if (n_points == 0) return SPH_OK;
   SPH_CHECK_ARG(d_points && d_sys_points, "null pointer");
   SPH_CHECK_ARG(((uintptr_t)d_sys_points & 15) == 0, "system points must be 16-byte aligned");
-  voxel_transform_kernel<<<(unsigned)div_up64(n_points, kVoxThreads), kVoxThreads, 0, (cudaStream_t)stream>>>(
-      d_points, point_stride, n_points, system, (float4*)d_sys_points);
+  launch(voxel_transform_kernel, (unsigned)div_up64(n_points, kVoxThreads), kVoxThreads, 0, (cudaStream_t)stream, d_points, point_stride, n_points, system, (float4*)d_sys_points);
   SPH_LAUNCH_CHECK();
   return SPH_OK;
 }
@@ -399,14 +405,12 @@ extern "C" int sph_voxelize_fill(const float* d_points, int32_t point_stride, co
   const char* scratch = (const char*)d_scratch;
   const int C = sph_voxel_feature_count(point_stride, g.append_mode);
   if (point_stride == 4 && g.append_mode == 0 && (((uintptr_t)d_points | (uintptr_t)d_feature) & 15) == 0) {
-    voxel_mean4_kernel<<<(unsigned)div_up64(nnz, kVoxThreads), kVoxThreads, 0, (cudaStream_t)stream>>>(
-        (const float4*)d_points, g, (const int2*)(scratch + l.cell), (const int*)(scratch + l.sel), n_points, nnz,
+    launch(voxel_mean4_kernel, (unsigned)div_up64(nnz, kVoxThreads), kVoxThreads, 0, (cudaStream_t)stream, (const float4*)d_points, g, (const int2*)(scratch + l.cell), (const int*)(scratch + l.sel), n_points, nnz,
         (float4*)d_feature, d_z_idx, (int4*)d_coordinates, d_num_points);
     SPH_LAUNCH_CHECK();
     return SPH_OK;
   }
-  voxel_mean_kernel<<<(unsigned)div_up64(nnz * C, kVoxThreads), kVoxThreads, 0, (cudaStream_t)stream>>>(
-      d_points, point_stride, (const float4*)d_sys_points, d_scan_ptr, g, (const int2*)(scratch + l.cell),
+  launch(voxel_mean_kernel, (unsigned)div_up64(nnz * C, kVoxThreads), kVoxThreads, 0, (cudaStream_t)stream, d_points, point_stride, (const float4*)d_sys_points, d_scan_ptr, g, (const int2*)(scratch + l.cell),
       (const int*)(scratch + l.sel), n_points, nnz, C, d_feature, d_z_idx, (int4*)d_coordinates, d_num_points);
   SPH_LAUNCH_CHECK();
   return SPH_OK;

@@ -1,0 +1,74 @@
+"""Kernels are launched before the ones in front of them have ended and wait inside: chains that follow one another without a
+synchronisation, on two streams, and chains captured in a graph give what single steps with a synchronisation in between give."""
+import numpy as np
+import pytest
+import torch
+
+import sphconv_b200 as sphconv
+from sphconv_b200 import sphconv_cuda as ops
+from sphconv_b200.encoder import build_encoder8
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _scan(seed, shape, B):
+    rng = np.random.default_rng(seed)
+    cells = rng.random((B, *shape)) < 0.06 + 0.02 * seed
+    z_idx, per = np.nonzero(cells)[3], cells.sum(-1).reshape(-1)
+    return (torch.as_tensor(z_idx, dtype=torch.int32, device=DEV), torch.as_tensor(per.cumsum(), dtype=torch.int32, device=DEV).view(B, *shape[:2]),
+            torch.as_tensor(rng.standard_normal((z_idx.size, 4)), device=DEV).half())
+
+
+def test_passes_without_synchronisation_on_two_streams():
+    shape, B = [16, 48, 32], 2
+    scans = [_scan(s, shape, B) for s in range(4)]
+    net = build_encoder8(dtype=torch.float16, device=DEV).eval()
+
+    def run(scan):
+        z_idx, z_ptr, feature = scan
+        with torch.no_grad():
+            y = net(sphconv.SparseConvTensor(feature, shape, B, z_idx=z_idx, z_ptr=z_ptr))
+        return y.feature, y.z_idx, y.z_ptr
+
+    want = []
+    for scan in scans:
+        want.append(run(scan))
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    got = []
+    for i in range(24):
+        with torch.cuda.stream(streams[i % 2]):
+            got.append(run(scans[i % 4]))
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(g, want[i % 4]))
+
+
+@pytest.mark.parametrize("K,N", [(4, 16), (16, 16), (32, 32), (64, 64)])
+def test_rules_and_layers_in_a_graph(K, N):
+    """A submanifold rule set with its lists and two layers, captured once and replayed on other inputs."""
+    shape, B = [24, 40, 32], 2
+    z_idx, z_ptr, _ = _scan(2, shape, B)
+    n = z_idx.numel()
+    feature = torch.randn(n, K, device=DEV).half()
+    w1, w2 = (torch.randn(27, K, N, device=DEV) * 0.1).half(), (torch.randn(27, N, N, device=DEV) * 0.1).half()
+
+    def chain():
+        _, _, rules, size = ops.get_rules_subm(z_idx, z_ptr, B, shape, shape, [3] * 3, [1] * 3, [1] * 3, [1] * 3, [2, 2])
+        y = ops.rule_conv(feature, w1, rules, size, n)
+        return ops.rule_conv(y, w2, rules, size, n), size
+
+    chain()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out, size = chain()
+    for _ in range(3):
+        feature.copy_(torch.randn(n, K, device=DEV))
+        want, want_size = (t.clone() for t in chain())
+        torch.cuda.synchronize()
+        for _ in range(5):
+            graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want) and torch.equal(size, want_size)
