@@ -154,22 +154,6 @@ __device__ __forceinline__ uint32_t row_at(uint32_t i) {
   return i * (KC * 16u) + (x << 4);
 }
 
-// Waits of whole warps, in converged code; bounded (tc_common.cuh).
-__device__ __noinline__ bool wait_slowly(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  const bool ok = mbar_wait(bar, parity, abort_flag);
-  return __all_sync(0xffffffffu, ok);
-}
-__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return wait_slowly(bar, parity, abort_flag);
-}
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));
-  return p != 0u;
-}
-__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
-
 // The runs of a tile and the offsets its halves have, from what the planning warps found; called by whole warps.
 __device__ __forceinline__ Plan combine(const Partial* part, int lane) {
   uint32_t lo = ~0u, bits = 0u;

@@ -7,8 +7,10 @@
 //       one operand of 16 planes), K = 256 output rows
 //   B = dY     : N = oC, K = the same 256 output rows (a plain contiguous copy, not a gather)
 //   D          : fp32 in TMEM, rows o*iC .. o*iC+iC-1 of a batch's accumulator are dW of its o-th offset.
-// An instruction costs the same ~60 cycles whether M is 32 or 128, and a tile needs 16 of them (K = 16 rows each)
-// per operand pair, so batching the offsets divides the instruction count by 128/iC.
+// An instruction costs the same whether M is 32 or 128, and a tile needs 16 of them (K = 16 rows each) per operand pair, so
+// batching the offsets divides the instruction count by 128/iC.  Bound by the gather's cp.async (an instruction of 32 x 16 bytes
+// takes 10 to 14 cycles); waits by whole warps and MMAs issued from converged code: 64 x 64 on 171 k rows of 22 neighbours
+// 173 -> 152 us.
 // TMEM holds 512 columns, i.e. floor(512/oC) batch accumulators; if the offsets need more they are split into groups
 // and the grid into (row-tile slice) x (offset group): a CTA keeps its accumulators in TMEM across ALL of its tiles
 // and adds them to the fp32 gradient once at the end with red.global.add.f32 (the reference writes a partial per
@@ -71,7 +73,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) 
   __shared__ uint32_t s_tmem_base;
   __shared__ int s_abort;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = (int)uniform((uint32_t)tid >> 5);
   const int S = p.stages;
   const int grp = (int)blockIdx.x % p.groups;       // which offsets
   const int slice = (int)blockIdx.x / p.groups;     // which tiles: slice, slice + slices, ...
@@ -102,7 +105,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = s_tmem_base;
+  const uint32_t tmem_base = uniform(s_tmem_base);
   volatile int* abort_flag = &s_abort;
 
   if (warp < kCopyWarps) {
@@ -126,9 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) 
       const int64_t r = (int64_t)tile * kTileRows + warp * kRowsPerWarp + lane;
       const int yb = ti & 1;
       // ---- dY tile (contiguous rows)
-      bool ok = true;
-      if (lane == 0) ok = mbar_wait(smem_u32(&s_yempty[yb]), (((uint32_t)ti >> 1) & 1u) ^ 1u, abort_flag);
-      if (__any_sync(0xffffffffu, !ok)) { dead = true; break; }
+      if (!warp_wait(smem_u32(&s_yempty[yb]), (((uint32_t)ti >> 1) & 1u) ^ 1u, abort_flag)) { dead = true; break; }
       {
         // the warp's 32 dY rows are one contiguous piece of memory: lanes walk it in 16-byte steps (coalesced) and
         // drop each piece into its chunk plane
@@ -152,8 +153,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) 
         for (int o = 0; o < 8; ++o) nb[o] = nb_next[o];
         if (kb + p.ob < k_end) load_ids(ti, kb + p.ob, nb_next);
         else load_ids(ti + 1, k_begin, nb_next);
-        if (lane == 0) ok = mbar_wait(smem_u32(&s_empty[s]), par, abort_flag);
-        if (__any_sync(0xffffffffu, !ok)) { dead = true; break; }
+        if (!warp_wait(smem_u32(&s_empty[s]), par, abort_flag)) { dead = true; break; }
         const uint32_t stage = smem_u32(x_smem + (size_t)s * p.x_bytes);
         __syncwarp();   // every lane has finished reading the previous batch's ids
 #pragma unroll
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) 
       }
     }
     cp_async_wait_all();
-  } else if (lane == 0) {
+  } else {
     // ======================= MMA issuer =======================
     // both operands MN-major: SBO = stride between 8-element blocks along M/N (= chunk planes),
     // LBO = stride between 8-row groups along K (= 128 bytes); one instruction consumes 16 rows = 2 groups
@@ -208,31 +208,36 @@ __global__ void __launch_bounds__(kThreads, 1) conv_wgrad_tc_kernel(WgParams p) 
     const uint64_t d0 = make_smem_desc(0u, 128u, kPlane);
     const uint64_t hi = d0 & 0xffffffff00000000ull;
     const uint32_t lo0 = (uint32_t)d0;
+    const bool one = elect_one();
     int s = 0;
     uint32_t par = 0u;
     bool dead = false;
     for (int ti = 0; ti < my_tiles && !dead; ++ti) {
       const int yb = ti & 1;
-      if (!mbar_wait(smem_u32(&s_yfull[yb]), ((uint32_t)ti >> 1) & 1u, abort_flag)) break;
+      if (!warp_wait(smem_u32(&s_yfull[yb]), ((uint32_t)ti >> 1) & 1u, abort_flag)) break;
       const uint32_t y_lo = lo0 + (smem_u32(y_smem + (size_t)yb * p.y_bytes) >> 4);
       for (int k = 0; k < nbatch; ++k) {
-        if (!mbar_wait(smem_u32(&s_full[s]), par, abort_flag)) { dead = true; break; }
+        if (!warp_wait(smem_u32(&s_full[s]), par, abort_flag)) { dead = true; break; }
         fence_proxy_async();
         tc_fence_after();
         const uint32_t x_lo = lo0 + (smem_u32(x_smem + (size_t)s * p.x_bytes) >> 4);
         const uint32_t d_tmem = tmem_base + (uint32_t)(k * p.N);
-#pragma unroll 4
-        for (int j = 0; j < kTileRows / 16; ++j) {
-          const uint32_t step = (uint32_t)j * ((2u * 128u) >> 4);
-          umma_f16(d_tmem, hi | (uint64_t)(x_lo + step), hi | (uint64_t)(y_lo + step), idesc, (ti | j) ? 1u : 0u);
+        const uint32_t first = ti ? 1u : 0u;
+        if (one) {
+#pragma unroll
+          for (int j = 0; j < kTileRows / 16; ++j) {
+            const uint32_t step = (uint32_t)j * ((2u * 128u) >> 4);
+            umma_f16(d_tmem, hi | (uint64_t)(x_lo + step), hi | (uint64_t)(y_lo + step), idesc, j ? 1u : first);
+          }
+          umma_commit(smem_u32(&s_empty[s]));
         }
-        umma_commit(smem_u32(&s_empty[s]));
         if (++s == S) { s = 0; par ^= 1u; }
       }
-      if (!dead) umma_commit(smem_u32(&s_yempty[yb]));
+      if (!dead && one) umma_commit(smem_u32(&s_yempty[yb]));
     }
-    umma_commit(smem_u32(&s_done));
-    mbar_wait(smem_u32(&s_done), 0u, abort_flag);
+    if (one) umma_commit(smem_u32(&s_done));
+    __syncwarp();
+    warp_wait(smem_u32(&s_done), 0u, abort_flag);
   }
 
   tc_fence_before();
