@@ -178,3 +178,24 @@ def test_one_kernel_with_two_sizes_from_two_threads():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("dtype,C", [(torch.float16, 2), (torch.float16, 33), (torch.float16, 64), (torch.float32, 1), (torch.int8, 12),
+                                     (torch.float16, 400)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_dense_rows_copied_ahead(dtype, C, shift):
+    """Rows that are whole 4-byte words (copied while the map of the cells is made) and rows that are not, or do not start on
+    one; more channels than a block stages at a time."""
+    g = torch.Generator(device="cuda").manual_seed(C)
+    B, H, W, D = 2, 5, 9, 48
+    m = torch.rand(B, H, W, D, device="cuda", generator=g) < 0.3
+    at = m.nonzero()
+    z_idx, z_ptr = at[:, 3].int().contiguous(), m.sum(-1).view(-1).cumsum(0).int().view(B, H, W)
+    n = at.shape[0]
+    memory = torch.randint(-100, 100, (n * C + 1,), device="cuda", generator=g).to(dtype)
+    rows = memory[shift:shift + n * C].view(n, C)
+    dense = ops.dense_channels_first(rows, z_idx, z_ptr, [B, C, H, W, D])
+    want = torch.zeros(B, C, H, W, D, dtype=dtype, device="cuda")
+    want.permute(0, 2, 3, 4, 1)[m] = rows
+    assert torch.equal(dense, want)
+    assert torch.equal(ops.dense_channels_first_backward(dense, z_idx, z_ptr), rows)
