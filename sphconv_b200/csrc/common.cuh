@@ -61,10 +61,10 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
   c.numAttrs = 1;
   (void)cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);      // SPH_LAUNCH_CHECK() reads the error
 }
-// EARLY: a grid of at most two blocks per SM lets its successor in at once, which finds room beside it on every SM.  Blocks let in
+// EARLY: a grid of at most four blocks per SM lets its successor in at once, which finds room beside it on every SM.  Blocks let in
 // beside a large grid, or at the end of a persistent one, would all go to the SMs that are free first: 16 blocks behind a
 // convolution took 57 us instead of 9.
-constexpr unsigned kEarlyBlocks = 2 * 148;
+constexpr unsigned kEarlyBlocks = 4 * 148;
 template <bool EARLY = true>
 __device__ __forceinline__ void after_previous() {
   if (EARLY && gridDim.x * gridDim.y <= kEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;");

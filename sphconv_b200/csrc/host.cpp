@@ -187,6 +187,12 @@ class Padding {
   int device_ = -1;
 };
 
+// Rule sets from this size on have their lists written on the side stream where the caller allows it, beside the convolution
+// (626 k rows 507 -> 500 us for a layer's training step, 8 scans of an encoder 1809 -> 1794).  The two events, the waits and the
+// allocator's records of a smaller one cost the host more than its lists cost the GPU: one layer on 6 k rows 58 -> 46 us with the
+// lists on the caller's stream, a training step on 45 k rows 217 -> 208.
+constexpr int64_t kListsBesideRows = 100000;
+
 // The lists of a rule set whose table has been enqueued on the current stream, on the side stream.
 std::shared_ptr<ListsReady> lists_beside(const sph_geom& g, const Tensor& oz_ptr, const Tensor& nbr, int32_t tnm,
                                          const Tensor& rules, const Tensor& rule_size, bool fill) {
@@ -230,7 +236,7 @@ py::tuple rules_subm(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, const 
   const int64_t nnz = z_idx.size(0), kv = k[0] * k[1] * k[2];
   Lists l = make_lists(g, nnz, z_idx, materialize);
   Padding padding(l.rules, fill && nnz > 0);
-  defer = defer && materialize && nnz > 0;
+  defer = defer && materialize && nnz >= kListsBesideRows;
   Tensor nbr = empty({kv, nnz}, at::kInt, z_idx);
   const int64_t bytes = check(abi.sph_rules_subm_scratch_bytes(&g, nnz));
   Tensor scratch = bytes ? empty({bytes}, at::kByte, z_idx) : Tensor();
@@ -359,7 +365,7 @@ py::tuple strided_rules(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, con
     py::gil_scoped_release release;
     n_out = pending->count();
   }
-  defer = defer && materialize && n_out > 0;
+  defer = defer && materialize && n_out >= kListsBesideRows;
   Tensor oz_idx = empty({n_out}, at::kInt, z_idx);
   Tensor nbr = empty({kv, n_out}, at::kInt, z_idx);
   const bool here = materialize && !defer && !padding.begun();
@@ -503,8 +509,8 @@ struct ConvLayer : public torch::autograd::Function<ConvLayer> {
   static Tensor forward(torch::autograd::AutogradContext* ctx, const Tensor& feature, const Tensor& weight,
                         const optional<Tensor>& bias, const Tensor& nbr, const optional<Tensor>& nbr_t, int64_t n_out, bool relu) {
     at::AutoDispatchBelowADInplaceOrView guard;
-    optional<Tensor> b;
-    if (bias) b = bias->detach().to(at::kFloat);
+    optional<Tensor> b;                  // float32, or the features' 16-bit type as it is
+    if (bias) b = (feature.itemsize() == 2 && bias->scalar_type() == feature.scalar_type() ? bias->detach() : bias->detach().to(at::kFloat)).contiguous();
     Tensor out = conv_gather(feature, weight, pack_weight(weight), nbr, n_out, false, std::nullopt, b, relu, std::nullopt);
     ctx->save_for_backward({feature, weight, relu ? out : Tensor(), nbr, nbr_t.value_or(Tensor())});
     ctx->saved_data["relu"] = relu;
