@@ -63,11 +63,21 @@ template <int CG, int KC> struct FfmaShape {
   static constexpr int BYTES = (ACC + 2 * A + 2 * W) * 4 + kBatch * kRows * 5 + kBatch * 4;
 };
 
+// Two fused multiply-adds an instruction, each rounded as fmaf rounds.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+
 // One step (offset, KC input channels) of RP rows x 8 output channels per thread.  The two 4-channel groups of a thread are
 // NP/2 apart, so the lanes of a row read consecutive 16-byte pieces of the filter row.
 template <int CG, int KC, int RP>
 __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const float* __restrict__ w, int kn, int rl, int cg,
-                                          float (&acc)[FfmaShape<CG, KC>::RP][8]) {
+                                          float2 (&acc)[FfmaShape<CG, KC>::RP][4]) {
   using S = FfmaShape<CG, KC>;
 #pragma unroll 2
   for (int k4 = 0; k4 < kn; k4 += 4) {
@@ -83,10 +93,11 @@ __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const flo
       const float4 w1 = *(const float4*)(w + (k4 + q) * S::NP + S::NP / 2 + cg * 4);
 #pragma unroll
       for (int j = 0; j < RP; ++j) {
-        acc[j][0] = fmaf(av[j][q], w0.x, acc[j][0]); acc[j][1] = fmaf(av[j][q], w0.y, acc[j][1]);
-        acc[j][2] = fmaf(av[j][q], w0.z, acc[j][2]); acc[j][3] = fmaf(av[j][q], w0.w, acc[j][3]);
-        acc[j][4] = fmaf(av[j][q], w1.x, acc[j][4]); acc[j][5] = fmaf(av[j][q], w1.y, acc[j][5]);
-        acc[j][6] = fmaf(av[j][q], w1.z, acc[j][6]); acc[j][7] = fmaf(av[j][q], w1.w, acc[j][7]);
+        const float2 x = make_float2(av[j][q], av[j][q]);
+        acc[j][0] = fma2(x, make_float2(w0.x, w0.y), acc[j][0]);
+        acc[j][1] = fma2(x, make_float2(w0.z, w0.w), acc[j][1]);
+        acc[j][2] = fma2(x, make_float2(w1.x, w1.y), acc[j][2]);
+        acc[j][3] = fma2(x, make_float2(w1.z, w1.w), acc[j][3]);
       }
     }
   }
@@ -114,9 +125,10 @@ __device__ __noinline__ int pairs_from(int k0, const int* __restrict__ nbr, int 
 // same accumulator.
 // The CTA is small (64 or 128 threads) so that a thread has up to four rows: with one row per thread (256 threads a tile)
 // the shared-memory reads of the filter, not the FMAs, set the pace; with eight rows too few warps fit on an SM.
-// Bound by the shared-memory reads of the operands (74 % of that pipe) and the issue slots (66 %, two thirds of them FMAs).  Measured: 64 -> 64 on
-// 170 k rows of 22 neighbours 3.2 -> 0.94 ms, 32 -> 32 on 390 k rows of 12 neighbours 1.9 -> 0.5 ms against the kernel it
-// replaced (one thread group per row walking every slot of the table).
+// Bound by the shared-memory reads of the operands (74 % of that pipe).  Measured: 64 -> 64 on 170 k rows of 22 neighbours 3.2 ->
+// 0.94 ms, 32 -> 32 on 390 k rows of 12 neighbours 1.9 -> 0.5 ms against the kernel it replaced (one thread group per row
+// walking every slot of the table).  Two FMAs an instruction (fma2; the same bits) take the issue slots off its limits: 64 -> 64
+// on 171 k rows 1070 -> 975 us, 32 -> 64 314 -> 292, 32 -> 32 545 -> 538; the weight gradient 845 -> 763, 228 -> 212, 511 -> 499.
 // VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by
 // element.
 template <typename T, int CG, int KC, bool VEC>
@@ -240,7 +252,7 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
     while (kk < nk && s_m[kk] == 0) ++kk;
     if (kk < nk) stage(0, kb, kk, 0, 0);
     cp_async_commit();
-    float acc[S::RP][8];
+    float2 acc[S::RP][4];
     for (int buf = 0; kk < nk; buf ^= 1) {
       int nkk = kk, np0 = p0, nkc = kc + 1;
       if (nkc == k_chunks) {
@@ -265,8 +277,8 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
           if (rl + j * S::RL < m) {
             const float* d = tile_row(rl + j * S::RL);
             const float4 t0 = *(const float4*)d, t1 = *(const float4*)(d + S::NP / 2);
-            acc[j][0] = t0.x; acc[j][1] = t0.y; acc[j][2] = t0.z; acc[j][3] = t0.w;
-            acc[j][4] = t1.x; acc[j][5] = t1.y; acc[j][6] = t1.z; acc[j][7] = t1.w;
+            acc[j][0] = make_float2(t0.x, t0.y); acc[j][1] = make_float2(t0.z, t0.w);
+            acc[j][2] = make_float2(t1.x, t1.y); acc[j][3] = make_float2(t1.z, t1.w);
           }
         }
       }
@@ -287,8 +299,8 @@ __global__ void __launch_bounds__(FfmaShape<CG, KC>::T) conv_ffma_kernel(FfmaPar
         for (int j = 0; j < S::RP; ++j) {
           if (rl + j * S::RL < m) {
             float* d = tile_row(rl + j * S::RL);
-            *(float4*)d = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
-            *(float4*)(d + S::NP / 2) = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
+            *(float4*)d = make_float4(acc[j][0].x, acc[j][0].y, acc[j][1].x, acc[j][1].y);
+            *(float4*)(d + S::NP / 2) = make_float4(acc[j][2].x, acc[j][2].y, acc[j][3].x, acc[j][3].y);
           }
         }
       }
@@ -571,9 +583,9 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
 
   const int copy = tid / (KG * NG), in_copy = tid % (KG * NG);
   const int ig = in_copy / NG, og = in_copy % NG;
-  float acc[64];                                             // [8 input][8 output channels]
+  float2 pairs[32];                                          // [8 input][4 x 2 output channels]
 #pragma unroll
-  for (int i = 0; i < 64; ++i) acc[i] = 0.f;
+  for (int i = 0; i < 32; ++i) pairs[i] = make_float2(0.f, 0.f);
   stage(0, 0);
   cp_async_commit();
   int buf = 0;
@@ -591,12 +603,18 @@ __global__ void __launch_bounds__(kThreads, 2) conv_wgrad_ffma_kernel(FfmaWgradP
       // the thread's output channels: 4 og .. 4 og + 3 of either half, so that the lanes read consecutive pieces
       const float4 d0 = *(const float4*)(d + r * S::DS), d1 = *(const float4*)(d + r * S::DS + NG * 4);
       const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
-      const float dv[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+      const float2 dv[4] = {make_float2(d0.x, d0.y), make_float2(d0.z, d0.w), make_float2(d1.x, d1.y), make_float2(d1.z, d1.w)};
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i * 8 + j] = fmaf(xv[i], dv[j], acc[i * 8 + j]);
+        for (int j = 0; j < 4; ++j) pairs[i * 4 + j] = fma2(make_float2(xv[i], xv[i]), dv[j], pairs[i * 4 + j]);
     }
+  }
+  float acc[64];                                             // [8 input][8 output channels]
+#pragma unroll
+  for (int i = 0; i < 32; ++i) {
+    acc[2 * i] = pairs[i].x;
+    acc[2 * i + 1] = pairs[i].y;
   }
   // Sum of the copies: those of a warp in its registers, then the warps' (or the wider copies') one after the other.
   constexpr int kLanes = KG * NG < 32 ? KG * NG : 32;        // lanes of a warp that hold one copy
