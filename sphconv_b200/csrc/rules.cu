@@ -343,6 +343,44 @@ nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, co
   int* dst = nbr + r;
   int* dst_t = nbr_t;
   uint32_t order = 0u;                       // the second half-words read: kUnsorted of any column
+  // Three consecutive depths: one look-up and one popcount serve a column, word and bit are the same for all columns, and the
+  // word behind is read by the rows that reach into it only.  1.5 M rows 60 -> 48 and 57 -> 42 us; with a second path for rows
+  // that reach into two words, over which the lanes of a warp split, 92 and 81.
+  if (KD_CT == 3 && g.dD == 1 && g.pD < 32) {
+    const int low = max(iz0, 0), w = low >> 5, sh = low & 31, outside = low - iz0;
+    const uint32_t below = (1u << sh) - 1u;
+    const bool inside = low < g.D, behind = sh > 29 && w + 1 < cm.words;
+    for (int kh = 0; kh < g.KH; ++kh) {
+      const int ix = ox * g.sH - g.pH + kh * g.dH;
+      const bool line_ok = ix >= 0 && ix < g.H;
+      const int64_t line = ((int64_t)b * g.H + ix) * g.W;
+#pragma unroll
+      for (int kw = 0; kw < KD_CT; ++kw) {
+        const int iy = oy * g.sW - g.pW + kw * g.dW;
+        uint32_t bits = 0u;
+        int at = 0;
+        if (line_ok && inside && iy >= 0 && iy < g.W) {
+          const int64_t ci = line + iy;
+          const uint2* word = cm.table + ci * cm.words + w;
+          const uint2 e = __ldg(word);
+          order |= e.y;
+          bits = __funnelshift_r(e.x, behind ? __ldg(&word[1].x) : 0u, sh) << outside;      // depths from D on are clear
+          at = col_start(in_zp, ci) + (int)(e.y & ~kUnsorted) + __popc(e.x & below);
+        }
+#pragma unroll
+        for (int kd = 0; kd < KD_CT; ++kd) {
+          const bool has = bits >> kd & 1u;
+          *dst = has ? at : -1;
+          dst += out_nnz;
+          if (HAS_T) {
+            if (has && !(order & kUnsorted)) dst_t[at] = (int)r;
+            dst_t += in_nnz;
+          }
+          at += has;
+        }
+      }
+    }
+  } else {
   for (int kh = 0; kh < g.KH; ++kh) {
     const int ix = ox * g.sH - g.pH + kh * g.dH;
     const int KW = KD_CT ? KD_CT : g.KW;   // the unrolled form is the cubic 3 x 3 x 3 filter
@@ -382,6 +420,7 @@ nbr_rows_kernel(const int* __restrict__ in_zi, const int* __restrict__ in_zp, co
         }
       }
     }
+  }
   }
   if (order & kUnsorted) search_row(in_zi, in_zp, __ldg(out_zi + r), g, in_nnz, out_nnz, r, c, nbr, HAS_T ? nbr_t : nullptr);
 }

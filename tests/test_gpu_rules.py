@@ -436,3 +436,20 @@ def test_lists_of_large_tiles_in_order(B, H, W, D, occ, nmax, subm):
         assert torch.equal(rule_size[:, k].long(), size)
         used = torch.arange(rules.shape[3], device=DEV) < size[:, None]
         assert torch.equal(rules[:, k, 0][used], nbr[k][has]) and torch.equal(rules[:, k, 1][used].long(), order[has])
+
+
+@pytest.mark.parametrize("D", [1, 2, 31, 32, 33, 64, 95])
+@pytest.mark.parametrize("sD,pD", [(1, 0), (1, 1), (1, 4), (2, 1), (3, 2), (2, 31), (1, 33)])
+def test_three_deep_filters_across_words_of_the_index(D, sD, pD):
+    """Depths whose three neighbours lie in two words of the column index, in front of the first depth and behind the last."""
+    if (D + 2 * pD - 3) // sD + 1 < 1:
+        pytest.skip("no output")
+    rng = np.random.default_rng(D * 100 + pD)
+    B, H, W = 2, 3, 5
+    cells = rng.random((B, H, W, D)) < 0.6
+    z_idx, z_ptr = np.nonzero(cells)[3].astype(np.int32), cells.sum(-1).reshape(-1).cumsum().reshape(B, H, W).astype(np.int32)
+    args = (z_idx, z_ptr, B, [H, W, D], [3, 3, 3], [1, 1, sD], [1, 1, pD], [2, 2], False)
+    zi, zp, osh, oz_idx, oz_ptr, rules, rule_size = gpu_rules(*args)
+    res = oracle_rules(*args)
+    assert (oz_idx.cpu().numpy() == res["oz_idx"]).all() and (rule_size.cpu().numpy() == res["rule_size"]).all()
+    assert_tables_match(res, rules, z_idx.size, oz_idx.numel())
