@@ -721,18 +721,18 @@ TRAFFIC_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum per output r
 # What limits each instantiation according to the same capture (neither HBM nor the tensor pipe: the bench line's `bound`
 # is the roofline the work is reported against, this is the unit that was busiest).
 BUSIEST_UNIT = {
-    "conv_gather_rows_kernel<4,f16>": "shared-memory data pipe 92 % busy (gather writes 64 % + tensor-core operand reads 28 %); DRAM 12 %, tensor pipe 11 %",
-    "conv_gather_tc_kernel<8,f16>": "shared-memory data pipe 88 % busy (gather writes 58 % + operand reads 30 %); tensor pipe 47 %, DRAM 8 %",
-    "conv_gather_tc_kernel<2,f16>": "shared-memory data pipe 93 % busy (gather writes 72 % + operand reads 22 %); DRAM 13 %",
+    "conv_gather_tmem_kernel<4,f16>": "instruction issue 74 % of the slots; shared-memory data path 68 %, tensor pipe 17 %, DRAM 17 %",
+    "conv_gather_tmem_kernel<8,f16>": "shared-memory data path 68 %; instruction issue 60 % of the slots, tensor pipe 35 %, DRAM 11 %",
+    "conv_gather_tmem_kernel<2,f16>": "instruction issue 75 % of the slots; shared-memory data path 34 %, DRAM 12 %, tensor pipe 8 %",
     "conv_sparse_rows_kernel<4,16>": "instruction issue 64 % of the slots; DRAM 13 %",
     "conv_strip_kernel<16,16,f16>": "instruction issue 51 % of the slots; shared-memory data pipe 24 %, DRAM 13 %, tensor pipe 8 %",
     "conv_wgrad_strip_kernel<16,16>": "instruction issue 68 % of the slots; shared-memory data pipe 40 %, DRAM 13 %",
     "conv_wgrad_strip_kernel<32,32>": "shared-memory data pipe 43 %, instruction issue 41 % of the slots; DRAM 12 %, tensor pipe 15 %",
-    "conv_ffma_kernel": "shared-memory data pipe 74 %, instruction issue 66 % of the slots; FMA pipe 46 %, DRAM 2 %",
-    "conv_wgrad_ffma_kernel": "instruction issue 76 % of the slots; FMA pipe 55 %, DRAM 27 %",
+    "conv_ffma_kernel": "shared-memory data pipe 74 %; with one FMA an instruction: issue 66 % of the slots, FMA pipe 46 %, DRAM 2 %",
+    "conv_wgrad_ffma_kernel": "with one FMA an instruction: issue 76 % of the slots, FMA pipe 55 %, DRAM 27 %",
 }
 TRAFFIC_BYTES_PER_OUT_ROW = {
-    "fp16": {"L0": 116.2, "L1": 140.3, "L2": 146.5, "L3": 211.3, "L4": 208.9, "L5": 288.9, "L6": 280.6, "L7": 281.1},
+    "fp16": {"L0": 116.2, "L1": 140.3, "L2": 146.1, "L3": 204.5, "L4": 202.8, "L5": 279.0, "L6": 259.9, "L7": 258.1},
 }
 
 if __name__ == "__main__":
