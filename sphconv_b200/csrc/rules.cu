@@ -1031,24 +1031,56 @@ scan_columns_kernel(int* __restrict__ counts, int64_t ncols, const int* __restri
   }
 }
 
+// A warp takes 32 consecutive (column, 32-bin word) items, whose rows are one run: a lane looks up which item and which set bit a row
+// is, so that the stores are consecutive.  626 k rows of 19 a column 22 -> 12 us, 1.5 M of 23 16 -> 9
+// against a thread per item that writes its rows one after the other.
 __global__ void __launch_bounds__(kScanThreads)
 write_oz_idx_kernel(const uint32_t* __restrict__ mask, const int* __restrict__ oz_ptr, int words, int64_t ncols,
                     int* __restrict__ oz_idx, int* __restrict__ row_col) {
   after_previous();
-  // one thread per (column, 32-bin word): its first row is the column's start plus the bins of the words before it
   const int64_t t = (int64_t)blockIdx.x * kScanThreads + threadIdx.x;
-  if (t >= ncols * words) return;
+  const int lane = threadIdx.x & 31;
+  if (t - lane >= ncols * words) return;
   const int64_t c = t / words;
   const int w = (int)(t - c * words);
-  uint32_t m = mask[t];
-  if (m == 0u) return;
-  int pos = c == 0 ? 0 : oz_ptr[c - 1];
-  for (int j = 0; j < w; ++j) pos += __popc(mask[c * words + j]);
-  while (m) {
-    const int bit = __ffs(m) - 1;
-    if (row_col) row_col[pos] = (int)c;   // column id of the row, for nbr_rows_kernel
-    oz_idx[pos++] = w * 32 + bit;
-    m &= m - 1;
+  const uint32_t m = t < ncols * words ? mask[t] : 0u;
+  int64_t first = 0;                          // row of the warp's first set bit
+  if (lane == 0) {
+    first = c == 0 ? 0 : oz_ptr[c - 1];
+    for (int j = 0; j < w; ++j) first += __popc(mask[c * words + j]);
+  }
+  first = __shfl_sync(0xffffffffu, first, 0);
+  int before = __popc(m);                     // set bits of the items in front of the lane's
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int n = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += n;
+  }
+  const int total = __shfl_sync(0xffffffffu, before, 31);
+  before -= __popc(m);
+  for (int o0 = 0; o0 < total; o0 += 32) {
+    const int o = min(o0 + lane, total - 1);
+    int item = 0;                             // the last one with no more than o bits in front of it
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+      if (__shfl_sync(0xffffffffu, before, item + s) <= o) item += s;
+    int rank = o - __shfl_sync(0xffffffffu, before, item), bit = 0;
+    uint32_t bits = __shfl_sync(0xffffffffu, m, item);
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      const int below = __popc(bits & ((1u << s) - 1u));
+      if (rank >= below) {
+        rank -= below;
+        bits >>= s;
+        bit += s;
+      }
+    }
+    const int z = __shfl_sync(0xffffffffu, w, item) * 32 + bit;
+    const int column = (int)__shfl_sync(0xffffffffu, (int)c, item);
+    if (o0 + lane < total) {
+      if (row_col) row_col[first + o] = column;   // column id of the row, for nbr_rows_kernel
+      oz_idx[first + o] = z;
+    }
   }
 }
 
