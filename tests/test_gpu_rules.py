@@ -453,3 +453,31 @@ def test_three_deep_filters_across_words_of_the_index(D, sD, pD):
     res = oracle_rules(*args)
     assert (oz_idx.cpu().numpy() == res["oz_idx"]).all() and (rule_size.cpu().numpy() == res["rule_size"]).all()
     assert_tables_match(res, rules, z_idx.size, oz_idx.numel())
+
+
+def test_lists_of_large_tiles_beyond_their_capacity():
+    """The kernel of large tiles with lists too short for some tiles: sizes in full, the status bit, no write behind a list; and
+    sizes alone."""
+    import ctypes
+    from sphconv_b200 import _capi as C
+    B, H, W, D = 2, 64, 64, 64
+    rng = np.random.default_rng(5)
+    cells = rng.random((B, H, W, D)) < 0.6
+    z_idx, z_ptr = np.nonzero(cells)[3].astype(np.int32), cells.sum(-1).reshape(-1).cumsum().reshape(B, H, W).astype(np.int32)
+    zi, zp, osh, oz_idx, oz_ptr, rules, rule_size = gpu_rules(z_idx, z_ptr, B, (H, W, D), (3, 3, 3), (1, 1, 1), (1, 1, 1), (2, 2), True)
+    assert rules.shape[0] >= 1024 and oz_idx.numel() >= 256 * rules.shape[0]
+    three, two = ctypes.c_int32 * 3, ctypes.c_int32 * 2
+    g = C.Geom(B=B, in_shape=three(H, W, D), out_shape=three(H, W, D), ksize=three(3, 3, 3), stride=three(1, 1, 1), padding=three(1, 1, 1),
+               tile=two(2, 2), dilation=three(1, 1, 1))
+    lib, st, nbr = C.lib(), C.stream_ptr(torch.device(DEV)), rules._sph.nbr
+    assert lib.sph_num_tiles(ctypes.byref(g)) == rules.shape[0]
+    capacity = int(rule_size.max()) - 20
+    short = torch.full((rules.shape[0], 27, 2, capacity), -7, dtype=torch.int32, device=DEV)
+    size, status = torch.zeros_like(rule_size), torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert lib.sph_rule_lists(C.ptr(oz_ptr), ctypes.byref(g), nbr.shape[1], C.ptr(nbr), capacity, C.ptr(short), C.ptr(size), 0, C.ptr(status), st) == 0
+    assert int(status) == C.STATUS_RULE_OVERFLOW and torch.equal(size, rule_size)
+    used = (torch.arange(capacity, device=DEV) < rule_size[..., None]).unsqueeze(2).expand_as(short)
+    assert torch.equal(short[used], rules[..., :capacity][used]) and (short[~used] == -7).all()
+    size.zero_()
+    assert lib.sph_rule_lists(C.ptr(oz_ptr), ctypes.byref(g), nbr.shape[1], C.ptr(nbr), 0, None, C.ptr(size), 0, C.ptr(status), st) == 0
+    assert torch.equal(size, rule_size)
