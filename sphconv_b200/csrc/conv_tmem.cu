@@ -65,7 +65,7 @@ __host__ __device__ constexpr int run_slots(int row_bytes) { return row_bytes ==
 constexpr int kBox = 32;              // rows a TMA load brings
 constexpr int kOperandCols = 32;      // TMEM columns of an operand: one batch of one to four offsets
 constexpr int kOperands = 4;          // operands of a half in TMEM
-constexpr int kWeightSlots = 8;       // streamed weight images in flight: one takes about 2000 cycles to come
+constexpr int kWeightSlots = 8;       // streamed weight images in flight (4: no slower, but their 32 KB hold no longer run)
 constexpr uint32_t kAbsent = 0xffffu;   // place of a neighbour that there is not
 constexpr int kStagePieces = 8;       // 16-byte pieces of the widest output row that is staged (the narrowest: half as many)
 constexpr int kSmemTotal = 227 * 1024 - 2048;   // dynamic shared memory available next to the static part
