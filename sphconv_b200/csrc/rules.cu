@@ -662,8 +662,9 @@ rule_lists_tile_kernel(const int* __restrict__ out_zp, Geom g, int64_t out_nnz, 
           }
         }
       }
-      __syncthreads();   // the next positions overwrite the mapping, the next group of runs the runs
+      __syncthreads();   // the next positions overwrite the mapping
     }
+    __syncthreads();     // every warp has read T: the next group overwrites the runs, also behind a group without rows
   }
   if (rule_size) {
 #pragma unroll

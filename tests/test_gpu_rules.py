@@ -421,8 +421,11 @@ def test_lists_of_large_tiles_in_order(B, H, W, D, occ, nmax, subm):
     want = np.where(rng.random((B, H, W)) < occ, rng.integers(nmax // 2 + 1, nmax + 1, (B, H, W)), 0)
     cells = rng.random((B, H, W, D)).argsort(-1).argsort(-1) < want[..., None]
     z_idx, z_ptr = np.nonzero(cells)[3].astype(np.int32), want.reshape(-1).cumsum().reshape(B, H, W).astype(np.int32)
-    zi, zp, osh, oz_idx, oz_ptr, rules, rule_size = gpu_rules(z_idx, z_ptr, B, (H, W, D), (3, 3, 3), (1, 1, 1) if subm else (2, 2, 2),
-                                                              (1, 1, 1), (2, 2), subm)
+    _check_lists_of_large_tiles(z_idx, z_ptr, B, (H, W, D), (1, 1, 1) if subm else (2, 2, 2), subm)
+
+
+def _check_lists_of_large_tiles(z_idx, z_ptr, B, shape, stride, subm):
+    zi, zp, osh, oz_idx, oz_ptr, rules, rule_size = gpu_rules(z_idx, z_ptr, B, shape, (3, 3, 3), stride, (1, 1, 1), (2, 2), subm)
     n, tiles = oz_idx.numel(), rules.shape[0]
     assert tiles >= 1024 and n >= 256 * tiles
     column = torch.repeat_interleave(torch.arange(oz_ptr.numel(), device=DEV), torch.diff(oz_ptr.view(-1), prepend=oz_ptr.new_zeros(1)).long())
@@ -436,6 +439,18 @@ def test_lists_of_large_tiles_in_order(B, H, W, D, occ, nmax, subm):
         assert torch.equal(rule_size[:, k].long(), size)
         used = torch.arange(rules.shape[3], device=DEV) < size[:, None]
         assert torch.equal(rules[:, k, 0][used], nbr[k][has]) and torch.equal(rules[:, k, 1][used].long(), order[has])
+
+
+@pytest.mark.parametrize("B,empty", [(70, (0, 64)), (140, (0, 64)), (200, (64, 128)), (200, (0, 128)), (140, (64, 140))])
+def test_lists_of_large_tiles_with_groups_of_empty_runs(B, empty):
+    """More than 128 runs in a tile (two a scan), of which whole groups of 128 have no row in a quarter of the tiles."""
+    rng = np.random.default_rng(B)
+    H, W, D = 64, 64, 16
+    want = rng.integers(2, 7, (B, H, W))
+    want[empty[0]:empty[1], :H // 2, W // 2:] = 0
+    cells = rng.random((B, H, W, D)).argsort(-1).argsort(-1) < want[..., None]
+    z_idx, z_ptr = np.nonzero(cells)[3].astype(np.int32), want.reshape(-1).cumsum().reshape(B, H, W).astype(np.int32)
+    _check_lists_of_large_tiles(z_idx, z_ptr, B, (H, W, D), (1, 1, 1), True)
 
 
 @pytest.mark.parametrize("D", [1, 2, 31, 32, 33, 64, 95])
