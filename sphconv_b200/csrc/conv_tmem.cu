@@ -20,11 +20,18 @@
 //   32 -> 32 fp16, 1.5 M rows, 0.42   324 -> 205      64 -> 64 fp16, 683 k rows, 0.82   257 -> 162
 //   16 -> 32 fp16, 1.5 M rows, 0.05   201 -> 164      64 -> 32 fp16, 1.5 M rows, 0.13   513 -> 287
 //   32 -> 32 int8, 1.5 M rows, 0.42   256 -> 172      64 -> 64 fp16,  17 k rows, 0.70  24.6 -> 18.4
-// Bound by the instructions of the gather and planning warps (issue slots 77 % busy at 32- and 64-byte rows) and by the TMEM
-// writes (without them 206 -> 141), at 128-byte rows by the shared-memory
-// data path (82 % busy).  Tried and
+// Bound by no single unit: issue slots 74 % busy at 32- and 64-byte rows and 60 % at 128-byte rows, the shared-memory data path
+// 34, 68 and 68 % (786 k rows of 16 -> 32 and 32 -> 32, 347 k of 64 -> 64); without the TMEM writes and the loads in front of them a
+// 32 -> 32 layer takes 141 instead of 206 us.  Tried and
 // slower: entries kept in registers with the offsets unrolled (instruction fetch: 577); rows of zeros in shared memory for absent
 // neighbours (bank conflicts: 263); the instruction's disable-output-lane mask instead of zeros (its operands: 217).
+//
+// A run longer than its buffer (tiles that pass from one line of columns into the next, dense or deep columns, strides that thin
+// the output, tables without locality) is read around it: the gather takes the table's entries a batch ahead, rows inside the
+// buffer from there and the others straight into registers, 32 bytes a load.  Against asking the table offset by offset when a
+// row was found missing: 32 -> 64 strided, 146 k rows of surfaces, every line too long, 68 -> 49 us; 16 -> 32 strided, 61 k rows,
+// 6 % of the lines too long, 24.6 -> 21.5; 32 -> 32 without locality, 300 k rows, 131 -> 95.  Bound there by the latency of L2: a warp
+// has one batch in flight.
 //
 // A CTA owns 256 consecutive output rows at a time (two halves of M = 128; one half where the tiles would not fill the SMs)
 // and is persistent over such tiles.  Warp roles: 0-15 gather (warp w: TMEM lanes 32 (w % 4) of half w / 4 % 2, and the batches
@@ -32,8 +39,7 @@
 // runs, 23 those of the weight images, 24-31 plan.
 //  * The planning warps run up to two tiles ahead: they read the table entries of their 32 rows, find the run of each line and
 //    the offsets that occur in each half, and leave for the gather warps where in its run the neighbour of each row lies (16
-//    bits), offset after offset that occurs.  Any table is right: entries beyond the part of a run that the buffer holds are
-//    read from global memory.
+//    bits), offset after offset that occurs.  Any table is right, also one whose runs the buffers do not hold.
 //  * Offsets that no row of a half has are skipped (half of them in the input gradient of a strided layer); a row without a
 //    neighbour at an offset that others have brings zeros, without an access to shared memory.
 //  * Every wait is made by a whole warp and MMAs are issued by an elected lane in converged code: an MMA from a divergent
@@ -61,11 +67,12 @@ constexpr int kHalfRows = 128;
 constexpr int kMmaWarp = 16, kEpiWarp = 18, kRunWarp = 22, kWeightWarp = 23, kPlanWarp = 24;
 constexpr int kTeams = 2;             // gather warps of a TMEM lane quarter: they take alternate batches
 constexpr int kLines = 3;             // groups of offsets that share a run
-__host__ __device__ constexpr int run_slots(int row_bytes) { return row_bytes == 128 ? 2 : 3; }     // runs in shared memory
+constexpr int kRunSlots = 3;          // most runs in shared memory (plan_smem)
 constexpr int kBox = 32;              // rows a TMA load brings
 constexpr int kOperandCols = 32;      // TMEM columns of an operand: one batch of one to four offsets
 constexpr int kOperands = 4;          // operands of a half in TMEM
-constexpr int kWeightSlots = 8;       // streamed weight images in flight (4: no slower, but their 32 KB hold no longer run)
+constexpr int kWeightSlots = 8;       // streamed weight images in flight
+constexpr uint32_t kScattered = 64;   // a run of this many times the rows that a slot holds is not brought (8: 200 instead of 192 us)
 constexpr uint32_t kAbsent = 0xffffu;   // place of a neighbour that there is not
 constexpr int kStagePieces = 8;       // 16-byte pieces of the widest output row that is staged (the narrowest: half as many)
 constexpr int kSmemTotal = 227 * 1024 - 2048;   // dynamic shared memory available next to the static part
@@ -90,6 +97,7 @@ struct TmemParams {
   int N, flip_k;
   int halves, num_tiles;
   int w_bytes;
+  int run_slots;                      // runs in shared memory
   int cap;                            // rows of a run that a slot holds, a multiple of kBox
   int plan_off, part_off, epi_off, place_off, w_off, run_off;   // from the 1024-byte-aligned base
   int stage_off;                      // -1: output rows are not staged
@@ -147,6 +155,20 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr, bool present) {
   return v;
 }
 
+// 32 bytes of global memory (as two pieces where the address is no multiple of 32) where `present`, else what a and b hold.
+__device__ __forceinline__ void ldg256(uint4& a, uint4& b, const void* at, bool present, bool whole) {
+  if (whole)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %9, 0;\n\t@p ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t}"
+                 : "+r"(a.x), "+r"(a.y), "+r"(a.z), "+r"(a.w), "+r"(b.x), "+r"(b.y), "+r"(b.z), "+r"(b.w)
+                 : "l"(at), "r"((int)present));
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %9, 0;\n\t@p ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%8];\n\t"
+        "@p ld.global.nc.v4.b32 {%4,%5,%6,%7}, [%8 + 16];\n\t}"
+        : "+r"(a.x), "+r"(a.y), "+r"(a.z), "+r"(a.w), "+r"(b.x), "+r"(b.y), "+r"(b.z), "+r"(b.w)
+        : "l"(at), "r"((int)present));
+}
+
 // Byte offset of 16-byte piece 0 of row i in a run of KC-piece rows as TMA swizzles it (piece c: xor with 16 c).
 template <int KC>
 __device__ __forceinline__ uint32_t row_at(uint32_t i) {
@@ -180,6 +202,12 @@ __device__ __forceinline__ Plan combine(const Partial* part, int lane) {
     r.hi[0] = 0;
   }
   return r;
+}
+
+// Rows of a run longer than `cap` that are brought to shared memory: its first ones, or none where the entries are scattered so
+// widely that few of them would be among these.
+__device__ __forceinline__ uint32_t held_of_split(uint32_t lo, int hi, uint32_t cap) {
+  return ((uint32_t)hi - lo) / kScattered >= cap ? 0u : cap;
 }
 
 // 16 accumulator values of one output row (channels c0 .. c0+15) -> 16-byte pieces; returns how many.
@@ -237,7 +265,6 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
   constexpr int U = 8 / KC;                         // offsets of a batch
   constexpr int LP = (L + U - 1) / U * U;           // a line's list of places, in whole batches
   constexpr int ROW = KC * 16;
-  constexpr int kRunSlots = run_slots(ROW);
   constexpr bool STREAM = KC == 8;                  // weight images come offset by offset (else all stay in shared memory)
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t s_run_full[kRunSlots], s_run_empty[kRunSlots];
@@ -266,7 +293,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
   }
   if (tid == 0) {
     s_abort = 0;
-    for (int s = 0; s < kRunSlots; ++s) {
+    for (int s = 0; s < p.run_slots; ++s) {
       mbar_init(smem_u32(&s_run_full[s]), 1);
       mbar_init(smem_u32(&s_run_empty[s]), 4 * kTeams * halves);
     }
@@ -355,6 +382,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
             if (!warp_wait(run_full0 + 8u * slot, run_par, abort_flag)) { dead = true; break; }
           }
           const bool split = any && (uint32_t)hi - lo >= cap;
+          const uint32_t held = split ? held_of_split(lo, hi, cap) : cap;   // rows from lo on that the buffer holds
           const uint32_t run = run0 + (uint32_t)slot * slot_bytes;
           const uint32_t line_offsets = (offsets >> (l * L)) & ((1u << L) - 1u);
           const int n = __popc(line_offsets);
@@ -362,37 +390,59 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
           int j = (int)((count ^ (uint32_t)team) & 1u) * U;            // first place of this team's next batch
           uint32_t c = count + (uint32_t)(j / U);
           count += (uint32_t)((n + U - 1) / U);
-          uint32_t next[U];
+          // A batch ahead, what says where its rows are: their places, or (a run that the buffer does not hold) the table's entries.
+          uint32_t next[U], todo = line_offsets;
+          const bool whole = ((uintptr_t)p.rows & 31u) == 0;
+          auto drop = [&]() {                         // the other team's batch
 #pragma unroll
-          for (int u = 0; u < U; ++u) next[u] = place[(j + u) * 32];        // behind the line: something unused
+            for (int u = 0; u < U; ++u) todo &= todo - 1u;
+          };
+          auto entries = [&]() {
+            const int64_t r = tile_row(ti) + rows_of * 32 + lane;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+              const int k = l * L + __ffs((int)todo) - 1;
+              const bool some = todo != 0u && r < p.n_out;
+              next[u] = some ? (uint32_t)__ldg(p.nbr + (int64_t)(p.flip_k ? KV - 1 - k : k) * p.n_out + r) : ~0u;
+              if (next[u] >= (uint32_t)p.n_rows) next[u] = ~0u;
+              todo &= todo - 1u;
+            }
+            drop();
+          };
+          if (!split) {
+#pragma unroll
+            for (int u = 0; u < U; ++u) next[u] = place[(j + u) * 32];        // behind the line: something unused
+          } else {
+            if (j) drop();
+            entries();
+          }
 #pragma unroll 1
           for (; j < n; j += kTeams * U, c += kTeams) {
             uint4 v[8];                               // U rows of KC pieces
+            if (!split) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const uint32_t at = run + next[u] * 16u;
+              for (int u = 0; u < U; ++u) {
+                const uint32_t at = run + next[u] * 16u;
 #pragma unroll
-              for (int q = 0; q < KC; ++q) v[u * KC + q] = lds128(at ^ (uint32_t)(q << 4), next[u] != kAbsent);
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) next[u] = place[(j + kTeams * U + u) * 32];
-            if (split) {                              // entries beyond the buffer
-#pragma unroll 1
-              for (int u = 0; u < U && j + u < n; ++u) {
-                const int k = l * L + (int)__fns(line_offsets, 0, j + u + 1);
-                const int64_t r = tile_row(ti) + rows_of * 32 + lane;
-                const int e = r < p.n_out ? __ldg(p.nbr + (int64_t)(p.flip_k ? KV - 1 - k : k) * p.n_out + r) : -1;
-                if ((uint32_t)e < (uint32_t)p.n_rows && (uint32_t)e - lo >= cap) {
-                  const uint4* src = (const uint4*)((const uint8_t*)p.rows + (size_t)(uint32_t)e * ROW);
-#pragma unroll
-                  for (int w = 0; w < U; ++w)
-                    if (w == u) {
-#pragma unroll
-                      for (int q = 0; q < KC; ++q) v[w * KC + q] = __ldg(src + q);
-                    }
-                }
+                for (int q = 0; q < KC; ++q) v[u * KC + q] = lds128(at ^ (uint32_t)(q << 4), next[u] != kAbsent);
               }
-              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < U; ++u) next[u] = place[(j + kTeams * U + u) * 32];
+            } else {
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const uint32_t i = next[u] - lo, at = run + row_at<KC>(i);
+#pragma unroll
+                for (int q = 0; q < KC; ++q) v[u * KC + q] = lds128(at ^ (uint32_t)(q << 4), i < held);
+              }
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const bool beyond = next[u] != ~0u && next[u] - lo >= held;
+                const uint8_t* src = (const uint8_t*)p.rows + (size_t)next[u] * ROW;
+#pragma unroll
+                for (int q = 0; q < KC; q += 2) ldg256(v[u * KC + q], v[u * KC + q + 1], src + q * 16, beyond, whole);
+              }
+              entries();
             }
             if (sent) report();                       // behind this batch's loads
             const uint32_t op = c % kOperands;
@@ -405,7 +455,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
           if (any) {
             __syncwarp();
             if (one) mbar_arrive(run_empty0 + 8u * slot);
-            if (++slot == kRunSlots) { slot = 0; run_par ^= 1u; }
+            if (++slot == p.run_slots) { slot = 0; run_par ^= 1u; }
           }
         }
         if (dead) break;
@@ -579,15 +629,17 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
         if (hi < 0 || dead) continue;
         if (!warp_wait(smem_u32(&s_run_empty[0]) + 8u * slot, par, abort_flag)) { dead = true; continue; }
         if (one) {
-          const uint32_t len = min((uint32_t)hi - lo + 1u, (uint32_t)p.cap);
+          const uint32_t span = (uint32_t)hi - lo + 1u;
+          const uint32_t len = span <= cap ? span : held_of_split(lo, hi, cap);
           const uint32_t boxes = (len + kBox - 1) / kBox;
           const uint32_t full = smem_u32(&s_run_full[0]) + 8u * slot;
           uint32_t dst = base_u + (uint32_t)p.run_off + (uint32_t)slot * slot_bytes;
-          mbar_arrive_expect_tx(full, boxes * (kBox * ROW));
+          if (boxes == 0) mbar_arrive(full);
+          else mbar_arrive_expect_tx(full, boxes * (kBox * ROW));
           for (uint32_t b = 0; b < boxes; ++b, dst += kBox * ROW) tma_rows(dst, &map, (int)(lo + b * kBox), full);
         }
         __syncwarp();
-        if (++slot == kRunSlots) { slot = 0; par ^= 1u; }
+        if (++slot == p.run_slots) { slot = 0; par ^= 1u; }
       }
     }
   } else if (warp == kWeightWarp) {
@@ -704,14 +756,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
 #pragma unroll
         for (int l = 0; l < kLines; ++l) {
           uint16_t* place = s_place + ((pb * 8 + w) * kLines + l) * (LP * 32) + lane;
-          const bool split = plan.hi[l] >= 0 && (uint32_t)plan.hi[l] - plan.lo[l] >= cap;
+          // the gather reads the table itself for a run that the buffer does not hold
+          if (plan.hi[l] >= 0 && (uint32_t)plan.hi[l] - plan.lo[l] >= cap) continue;
 #pragma unroll
           for (int o = 0; o < L; ++o) {
             if (offsets >> (l * L + o) & 1u) {
               const int v = entry[l * L + o];
-              const uint32_t i = (uint32_t)v - plan.lo[l];
-              // of an entry beyond the buffer, too: the gather reads it from global memory
-              *place = (uint16_t)(v < 0 || (split && i >= cap) ? kAbsent : row_at<KC>(i) >> 4);
+              *place = (uint16_t)(v < 0 ? kAbsent : row_at<KC>((uint32_t)v - plan.lo[l]) >> 4);
               place += 32;
             }
           }
@@ -762,9 +813,11 @@ bool plan_smem(TmemParams* p, int kv, int row_bytes, int* smem_bytes) {
   p->w_off = off;
   off += (row_bytes == 128 ? kWeightSlots : kv) * p->w_bytes;
   p->run_off = (off + 1023) & ~1023;
-  const int rows = (kSmemTotal - 1024 - p->run_off) / run_slots(row_bytes) / row_bytes / kBox * kBox;
+  const int bytes = kSmemTotal - 1024 - p->run_off;
+  p->run_slots = row_bytes == 128 ? 2 : kRunSlots;
+  const int rows = bytes / (p->run_slots * row_bytes) / kBox * kBox;
   p->cap = rows > 1024 ? 1024 : rows;
-  *smem_bytes = 1024 + p->run_off + run_slots(row_bytes) * p->cap * row_bytes;
+  *smem_bytes = 1024 + p->run_off + p->run_slots * p->cap * row_bytes;
   return p->cap >= 256;               // runs of 256 output rows are 260 to 450 rows long
 }
 

@@ -88,6 +88,29 @@ def test_runs_longer_than_their_buffer(K, N, dtype, spread):
     _check(rows, weight, _table(27, 30000, 40000, spread, 0.5, 2))
 
 
+@pytest.mark.parametrize("K,N,dtype", [(16, 32, torch.float16), (32, 64, torch.bfloat16), (64, 64, torch.float16), (32, 32, torch.int8)])
+@pytest.mark.parametrize("n_out,kv", [(5000, 27), (20001, 27), (20001, 9)])
+@pytest.mark.parametrize("shift", [0, 16])
+def test_tables_without_locality(K, N, dtype, n_out, kv, shift):
+    """Runs that are not brought to shared memory at all; rows that start on a multiple of 16 bytes, but not of 32; more input rows
+    than output rows and fewer; entries that are no rows among those that the gather reads itself."""
+    for n_rows in (200000, n_out // 2):
+        rows, weight = _operands(K, N, dtype, n_rows, kv, 11)
+        memory = torch.empty(rows.numel() + 16, dtype=dtype, device=DEV)
+        off = shift // rows.element_size()
+        rows = memory[off:off + rows.numel()].view_as(rows).copy_(rows)
+        assert rows.data_ptr() % 32 == shift
+        nbr = _table(kv, n_out, n_rows, n_rows, 0.5, 12)
+        nbr[:, n_out // 2:] = _table(kv, n_out - n_out // 2, n_rows, 700, 0.5, 13)      # every second row's runs a little too long
+        _check(rows, weight, nbr, flip=kv == 9)
+        bad = nbr.clone()
+        bad[1, ::7], bad[kv - 1, 5::9], bad[kv // 2, 3::8] = n_rows, n_rows + 100, -5
+        nbr[1, ::7], nbr[kv - 1, 5::9], nbr[kv // 2, 3::8] = -1, -1, -1
+        out, status = _gather(rows, weight, bad)
+        assert status & C.STATUS_BAD_INDEX
+        assert torch.equal(out, _gather(rows, weight, nbr)[0])
+
+
 @pytest.mark.parametrize("K,N,dtype", [(16, 32, torch.float16), (32, 32, torch.float16), (64, 64, torch.float16), (64, 64, torch.int8)])
 def test_offsets_and_tiles_without_pairs(K, N, dtype):
     """Offsets that tiles, or halves of tiles, do not have; tiles and whole tables without any pair."""
