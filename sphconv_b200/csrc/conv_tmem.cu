@@ -71,7 +71,7 @@ constexpr int kRunSlots = 3;          // most runs in shared memory (plan_smem)
 constexpr int kBox = 32;              // rows a TMA load brings
 constexpr int kOperandCols = 32;      // TMEM columns of an operand: one batch of one to four offsets
 constexpr int kOperands = 4;          // operands of a half in TMEM
-constexpr int kWeightSlots = 8;       // streamed weight images in flight
+constexpr int kWeightSlots = 8;       // most streamed weight images in flight (plan_smem)
 constexpr uint32_t kScattered = 64;   // a run of this many times the rows that a slot holds is not brought (8: 200 instead of 192 us)
 constexpr uint32_t kAbsent = 0xffffu;   // place of a neighbour that there is not
 constexpr int kStagePieces = 8;       // 16-byte pieces of the widest output row that is staged (the narrowest: half as many)
@@ -97,6 +97,7 @@ struct TmemParams {
   int N, flip_k;
   int halves, num_tiles;
   int w_bytes;
+  int weight_slots;                   // streamed weight images in flight
   int run_slots;                      // runs in shared memory
   int cap;                            // rows of a run that a slot holds, a multiple of kBox
   int plan_off, part_off, epi_off, place_off, w_off, run_off;   // from the 1024-byte-aligned base
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
               acc = 1u;
               ++count;
             }
-            if (++ws == kWeightSlots) { ws = 0; w_par ^= 1u; }
+            if (++ws == p.weight_slots) { ws = 0; w_par ^= 1u; }
             todo &= todo - 1u;
             k = __ffs((int)todo) - 1;
             // looked at now, the barriers of the next offset are known to be complete without the 90 cycles a wait takes for each
@@ -673,7 +674,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
                      w_full0 + 8u * ws);
           }
           __syncwarp();
-          if (++ws == kWeightSlots) { ws = 0; par ^= 1u; }
+          if (++ws == p.weight_slots) { ws = 0; par ^= 1u; }
         }
       }
     }
@@ -811,10 +812,15 @@ bool plan_smem(TmemParams* p, int kv, int row_bytes, int* smem_bytes) {
   p->place_off = off; off += 2 * 8 * kLines * line * 32 * (int)sizeof(uint16_t);
   off = (off + 127) & ~127;
   p->w_off = off;
-  off += (row_bytes == 128 ? kWeightSlots : kv) * p->w_bytes;
+  // Where there are more input rows than output rows the runs are longer: room for them rather than for weights or a third run.
+  // 128-byte rows, four images instead of eight (448 -> 576 rows at 64 channels of fp16): input gradients of strides (1,1,4) and (1,1,2)
+  // 83 -> 70 and 106 -> 102 us; but 64 -> 64 on 683 k rows whose runs fit 166 -> 173.  Two runs of 512 rows instead of three of
+  // 352 (32 -> 64): strided, 683 k rows, 131 -> 122 us, surfaces, 146 k rows, 44 -> 40; with fewer input rows than output rows 456 -> 488.
+  p->weight_slots = p->n_rows > p->n_out ? kWeightSlots / 2 : kWeightSlots;
+  off += (row_bytes == 128 ? p->weight_slots : kv) * p->w_bytes;
   p->run_off = (off + 1023) & ~1023;
   const int bytes = kSmemTotal - 1024 - p->run_off;
-  p->run_slots = row_bytes == 128 ? 2 : kRunSlots;
+  p->run_slots = row_bytes == 128 || (p->n_rows > p->n_out && bytes / (kRunSlots * row_bytes) < 512) ? 2 : kRunSlots;
   const int rows = bytes / (p->run_slots * row_bytes) / kBox * kBox;
   p->cap = rows > 1024 ? 1024 : rows;
   *smem_bytes = 1024 + p->run_off + p->run_slots * p->cap * row_bytes;
