@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import sphconv_b200 as sphconv
-from oracle import dense_ref
+from oracle import dense_ref, rules_np
 from sphconv_b200 import synthetic
 
 from gpu_util import DEV
@@ -213,6 +213,63 @@ def test_module_rules_written_beside_the_convolution():
             n_got, got = canon(r, n)
             n_want, want = canon(wr, wn)
             assert (n_got == n_want).all() and got == want
+    sphconv.check_status()
+
+
+@pytest.mark.parametrize("fill", [True, False])
+def test_module_rules_of_large_sets_written_beside_the_convolution(fill):
+    """The same with rule sets that are large enough for the side stream (100 k rows), submanifold and strided: the plain ops hand
+    out lists that are still to be joined, and behind a layer, on whichever stream it runs, they are complete."""
+    from sphconv_b200 import sphconv_cuda as ops
+    rng = np.random.default_rng(18)
+    B, shape, small = 3, [64, 100, 64], [32, 50, 32]
+    z_idx, z_ptr = synthetic.make_random_occupancy(rng, B, shape, 0.3, False)
+    zi, zp = torch.as_tensor(z_idx, device=DEV), torch.as_tensor(z_ptr, device=DEV)
+    feat = torch.as_tensor(rng.standard_normal((z_idx.shape[0], 16)), dtype=torch.float16, device=DEV)
+    sub = sphconv.SubMConv3d(16, 16, 3, indice_key="k").to(DEV).half().eval()
+    down = sphconv.SparseConv3d(16, 32, 3, stride=2, padding=1, indice_key="d").to(DEV).half().eval()
+    geom_s = (zi, zp, B, shape, shape, [3] * 3, [1] * 3, [1] * 3, [1] * 3, [2, 2])
+    geom_d = (zi, zp, B, shape, small, [3] * 3, [2] * 3, [1] * 3, [1] * 3, [2, 2])
+    ops.config.fill_unused_rules = fill
+
+    def used(rules, size):
+        return torch.arange(rules.shape[3], device=DEV) < size[:, :, None, None]
+
+    def same(got, want):
+        (rules, size), (want_rules, want_size) = got, want
+        assert torch.equal(size, want_size)
+        mask = torch.ones_like(rules, dtype=torch.bool) if fill else used(rules, size).expand_as(rules)
+        assert torch.equal(rules[mask], want_rules[mask])
+
+    try:
+        want_s, want_d = ops.get_rules_subm(*geom_s)[2:], ops.get_rules(*geom_d)[2:]
+        res = rules_np.get_rules_subm(z_idx, z_ptr, B, shape, shape, [3] * 3, [1] * 3, [1] * 3, [1] * 3, [2, 2])
+        assert (want_s[1].cpu().numpy() == res["rule_size"]).all()
+        assert (rules_np.canonical_pairs(want_s[0].cpu().numpy(), res["rule_size"]) == rules_np.canonical_from_table(res)).all()
+        torch.cuda.synchronize()
+        for fn, geom, want, n_out in ((ops.get_rules_subm, geom_s, want_s, zi.numel()), (ops.get_rules, geom_d, want_d, None)):
+            oz_idx, _, rules, size = fn(*geom, defer_lists=True)
+            assert oz_idx.numel() >= 100000 and rules._sph_ready is not None
+            ops.rule_conv(feat, torch.zeros(27, 16, 16, dtype=torch.float16, device=DEV), rules, size, oz_idx.numel())
+            snap = rules.clone(), size.clone()
+            assert rules._sph_ready is None
+            same(snap, want)
+        for i in range(6):
+            ops.config.overlap_rule_lists = i < 5
+            stream = torch.cuda.Stream() if i % 2 else torch.cuda.current_stream()
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream), torch.no_grad():
+                x = sphconv.SparseConvTensor(feat, shape, B, z_idx=zi, z_ptr=zp)
+                y = down(sub(x))
+                _, _, rules_s, size_s, _ = x.rule_cache["k"]
+                _, _, rules_d, size_d, _ = y.rule_cache["d"]
+                snap = rules_s.clone(), size_s.clone(), rules_d.clone(), size_d.clone()
+            del x, y, rules_s, rules_d         # their memory is taken again by the next pass
+            torch.cuda.current_stream().wait_stream(stream)
+            same(snap[:2], want_s)
+            same(snap[2:], want_d)
+    finally:
+        ops.config.overlap_rule_lists, ops.config.fill_unused_rules = True, True
     sphconv.check_status()
 
 

@@ -20,8 +20,8 @@ def _scan(seed, shape, B):
             torch.as_tensor(rng.standard_normal((z_idx.size, 4)), device=DEV).half())
 
 
-def test_passes_without_synchronisation_on_two_streams():
-    shape, B = [16, 48, 32], 2
+@pytest.mark.parametrize("shape,B", [([16, 48, 32], 2), ([64, 128, 64], 4)])      # the larger ones' lists: on the side stream
+def test_passes_without_synchronisation_on_two_streams(shape, B):
     scans = [_scan(s, shape, B) for s in range(4)]
     net = build_encoder8(dtype=torch.float16, device=DEV).eval()
 
@@ -29,7 +29,9 @@ def test_passes_without_synchronisation_on_two_streams():
         z_idx, z_ptr, feature = scan
         with torch.no_grad():
             y = net(sphconv.SparseConvTensor(feature, shape, B, z_idx=z_idx, z_ptr=z_ptr))
-        return y.feature, y.z_idx, y.z_ptr
+        rules = [r[2:4] for r in y.rule_cache.values()]
+        assert len(rules) == 3                 # of the submanifold levels
+        return [y.feature, y.z_idx, y.z_ptr] + [t.clone() for pair in rules for t in pair]
 
     want = []
     for scan in scans:
