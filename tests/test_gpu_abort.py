@@ -1,10 +1,11 @@
-"""The bounded waits of the tensor-core convolution kernel: when a pipeline stage never becomes full, every role
-leaves its loop, copies in flight are drained, tensor memory is freed, the launch returns and the status word carries
-SPH_STATUS_TIMEOUT; the context stays usable and the next launch is correct.
+"""The bounded waits of the tensor-core convolution kernels: when a pipeline stage (conv_tc.cu) or an operand in tensor memory
+(conv_tmem.cu) never becomes full, every role leaves its loop, copies in flight are drained, tensor memory is freed, the launch
+returns and the status word carries SPH_STATUS_TIMEOUT; the context stays usable and the next launch is correct.
 
 The failure is made on purpose only in a test-only build of the library (`libsphconv_b200_hooks.so`,
-sphconv_b200/build.py: conv_tc.cu compiled with -DSPH_TEST_HOOKS): there the wait limit is about 10 ms and
-`sph_test_withhold_arrival(1)` makes one gather thread skip its arrival for the second stage.  Nothing faults, traps or
+sphconv_b200/build.py: conv_tc.cu and conv_tmem.cu compiled with -DSPH_TEST_HOOKS): there the wait limit is about 10 ms and
+`sph_test_withhold_arrival(1)` makes one gather thread (conv_tc.cu) skip its arrival for the second stage, one gather warp
+(conv_tmem.cu) the report of its second operand.  Nothing faults, traps or
 spins without a bound."""
 import ctypes
 import os
@@ -32,11 +33,16 @@ def _hooks_lib():
     return h
 
 
-def test_withheld_arrival_times_out_cleanly():
+@pytest.mark.parametrize("kv,K,N,n,tmem", [
+    (28, 64, 64, 4096, 0), (28, 16, 32, 4096, 0), (27, 128, 64, 4096, 0),        # gathered into shared memory; 256-byte rows
+    (27, 64, 64, 4096, 1), (27, 32, 32, 4096, 1),                                # tiles of one half
+    (27, 64, 64, 20000, 1), (27, 32, 64, 20000, 1), (27, 16, 32, 20000, 1), (9, 64, 64, 20000, 1)])   # of two; streamed and resident weights
+def test_withheld_arrival_times_out_cleanly(kv, K, N, n, tmem):
     h = _hooks_lib()
+    assert C.lib().sph_conv_uses_tmem(C.SPH_F16, kv, K, N) == tmem
+    assert tmem or C.lib().sph_conv_kernel(C.SPH_F16, kv, K, N, 0) == 1          # SPH_KERNEL_TC
     dev = torch.device(DEV)
     rng = np.random.default_rng(3)
-    n, K, N, kv = 4096, 64, 64, 27                 # 16 tiles of 256 rows, 27 stages each
     rows = torch.as_tensor(rng.standard_normal((n, K)), dtype=torch.float32, device=DEV).half()
     w = torch.as_tensor(rng.uniform(-.1, .1, (kv, K, N)), dtype=torch.float32, device=DEV).half()
     nbr = torch.as_tensor(rng.integers(-1, n, size=(kv, n)), dtype=torch.int32, device=DEV)
