@@ -43,10 +43,13 @@ void note_launch();  // counts kernels launched by this library (sph_kernel_laun
 
 // A kernel of this library may be launched before the one in front of it in the stream has ended (programmatic dependent launch):
 // its blocks take their places when the last ones of that kernel have ended, or earlier where that kernel allows it, and
-// after_previous(), the first statement of every kernel, holds them until all of it is complete and its writes are visible.
+// after_previous(), in front of every access to global memory, holds them until all of it is complete and its writes are visible.
 // A chain of small kernels then costs about a microsecond a kernel less (both rule sets of a batch of 3 small scans 117 -> 100 us).
 // The wait is in every kernel, also in those that nothing of the library precedes: a kernel that skipped it could complete before
 // its predecessor, and its successor would run too early.
+// What the kernel in front writes is read behind the wait by __ldg and through const __restrict__ pointers as well: the data does not
+// change from there on, but it may have since the block began, so this relies on the compiler leaving read-only loads behind the
+// wait, a volatile statement that clobbers memory.  tests/test_gpu_overlap.py has the chains that would show it doing otherwise.
 template <typename... Params, typename... Args>
 inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchAttribute early;

@@ -20,10 +20,12 @@ def _scan(seed, shape, B):
             torch.as_tensor(rng.standard_normal((z_idx.size, 4)), device=DEV).half())
 
 
-@pytest.mark.parametrize("shape,B", [([16, 48, 32], 2), ([64, 128, 64], 4)])      # the larger ones' lists: on the side stream
-def test_passes_without_synchronisation_on_two_streams(shape, B):
+@pytest.mark.parametrize("shape,B,dtype", [([16, 48, 32], 2, torch.float16), ([64, 128, 64], 4, torch.float16),
+                                           ([64, 128, 64], 4, torch.float32)])       # the last one's lists: on the side stream
+def test_passes_without_synchronisation_on_two_streams(shape, B, dtype):
     scans = [_scan(s, shape, B) for s in range(4)]
-    net = build_encoder8(dtype=torch.float16, device=DEV).eval()
+    scans = [(z_idx, z_ptr, feature.to(dtype)) for z_idx, z_ptr, feature in scans]
+    net = build_encoder8(dtype=dtype, device=DEV).eval()
 
     def run(scan):
         z_idx, z_ptr, feature = scan
@@ -74,3 +76,45 @@ def test_rules_and_layers_in_a_graph(K, N):
             graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want) and torch.equal(size, want_size)
+
+
+@pytest.mark.parametrize("K,N,kv,dtype", [(16, 16, 27, torch.float32), (64, 64, 27, torch.float32), (20, 12, 27, torch.int8),
+                                          (4, 16, 27, torch.float16), (16, 16, 27, torch.float16), (24, 40, 27, torch.bfloat16),
+                                          (16, 32, 27, torch.float16), (32, 32, 9, torch.bfloat16), (64, 64, 27, torch.float16),
+                                          (32, 64, 27, torch.int8), (32, 32, 28, torch.float16), (128, 64, 27, torch.float16)])
+def test_rows_written_by_the_kernel_in_front(K, N, kv, dtype):
+    """Convolutions and weight gradients whose input rows the kernel in front of them in the stream, a small one that lets them in at
+    once, writes over the rows of the pass before."""
+    from sphconv_b200 import _capi as C
+    g = torch.Generator(device=DEV).manual_seed(K * N)
+    n = 4001
+    table = torch.arange(n, device=DEV) + torch.randint(-60, 61, (kv, n), device=DEV, generator=g)
+    table = torch.where((table < 0) | (table >= n) | (torch.rand(kv, n, device=DEV, generator=g) < 0.5), -1, table).int().contiguous()
+    rules = ops._Tables(table, None, n, n, 0, False)
+
+    def values(*shape):
+        if dtype == torch.int8:
+            return torch.randint(-100, 101, shape, device=DEV, generator=g, dtype=dtype)
+        return torch.randn(*shape, device=DEV, generator=g).to(dtype)
+
+    sources, weight, d_out = [values(n, K), values(n, K)], values(kv, K, N), None if dtype == torch.int8 else values(n, N)
+    order = torch.randperm(n, device=DEV, generator=g).int()
+
+    def step(i, wait=lambda: None):
+        x = C.host().gather_rows(sources[i % 2], order)
+        wait()
+        y = ops.rule_conv(x, weight, rules, None, n)
+        if d_out is None:
+            return y, None
+        x = C.host().gather_rows(sources[(i + 1) % 2], order)
+        wait()
+        return y, ops.rule_conv_d_weight(x, d_out, rules, None)
+
+    want = [step(i, torch.cuda.synchronize) for i in range(2)]
+    got = [step(i) for i in range(40)]
+    torch.cuda.synchronize()
+    for i, (y, dw) in enumerate(got):
+        assert torch.equal(y, want[i % 2][0])
+        if dw is not None:                 # sums of up to 4001 products in another order: 2^-24 sqrt(4001) of about 45, and 16 bits of result
+            w = want[i % 2][1].double()
+            assert (dw.double() - w).norm() <= (2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11) * w.norm()
