@@ -617,7 +617,7 @@ def main():
                 q = chunks * 4.0 * 27 * cm["n_out"] + 8.0 * pairs          # table read, pairs written
                 row.update({"bytes": int(q), "gbs": round(q / (ms * 1e-3) / 1e9, 1),
                             "frac_hbm": round(q / (ms * 1e-3) / h_peak, 4),
-                            "what": "reference-format pair lists from the table, on a side stream beside the convolution"})
+                            "what": "reference-format pair lists from the table (fp32 layers of more than 16 channels: on a side stream beside the convolution)"})
             layer_rows.append(row)
         else:
             layer_rows.append({"layer": name, "ms": round(ms, 4)})
@@ -650,7 +650,7 @@ def main():
                      "what": "the kernel instantiation with the largest share of the step's convolution time; achieved = "
                              "algorithmic work of its launches / their CUDA-event time inside the timed steps",
                      "all_tensor_core_layers_tflops": round(all_tc, 2), "conv_ms_per_step": round(conv_ms, 4),
-                     "rules_ms_per_step": round(rules_ms, 4), "lists_ms_per_step_side_stream": round(lists_ms, 4),
+                     "rules_ms_per_step": round(rules_ms, 4), "lists_ms_per_step": round(lists_ms, 4),
                      "by_kernel": by_kernel})
 
     cpu = None

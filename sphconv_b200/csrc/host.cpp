@@ -187,10 +187,10 @@ class Padding {
   int device_ = -1;
 };
 
-// Rule sets from this size on have their lists written on the side stream where the caller allows it, beside the convolution
-// (626 k rows 507 -> 500 us for a layer's training step, 8 scans of an encoder 1809 -> 1794).  The two events, the waits and the
-// allocator's records of a smaller one cost the host more than its lists cost the GPU: one layer on 6 k rows 58 -> 46 us with the
-// lists on the caller's stream, a training step on 45 k rows 217 -> 208.
+// Rule sets from this size on have their lists written on the side stream where the caller asks for it, beside the convolution.  The two
+// events, the waits and the allocator's records of a smaller one cost the host more than its lists cost the GPU (us, lists on the side /
+// the caller's stream): one layer on 6 k rows 58 / 46, on 16 k 66 / 39, a strided layer's training step on 16 k to 71 k rows 228 / 206.
+// From here on it is the layer that decides (Conv3d._rules).
 constexpr int64_t kListsBesideRows = 100000;
 
 // The lists of a rule set whose table has been enqueued on the current stream, on the side stream.
@@ -384,13 +384,19 @@ py::tuple strided_rules(const Tensor& z_idx, const Tensor& z_ptr, int64_t B, con
   return py::make_tuple(oz_idx, pending->oz_ptr, or_none(l.rules), or_none(l.rule_size), nbr, or_none(nbr_t), or_none(ready));
 }
 
-// The lists of a finished table on the side stream, as a step of its own (the caller times it).  -> (rules, rule_size, ready)
-py::tuple deferred_lists(const Tensor& oz_ptr, const Tensor& nbr, int64_t nnz, int64_t B, const Ints& in, const Ints& out,
-                         const Ints& k, const Ints& s, const Ints& p, const Ints& d, const Ints& tile, bool fill) {
+// The lists of a finished table as a step of its own (the caller times it), on the side stream or the current one.
+// -> (rules, rule_size, ready)
+py::tuple lists_of_table(const Tensor& oz_ptr, const Tensor& nbr, int64_t nnz, int64_t B, const Ints& in, const Ints& out,
+                         const Ints& k, const Ints& s, const Ints& p, const Ints& d, const Ints& tile, bool fill, bool beside) {
   const c10::cuda::CUDAGuard guard(nbr.device());
   const sph_geom g = geometry(B, in, out, k, s, p, d, tile);
   const Lists l = make_lists(g, nnz, nbr, true);
-  return py::make_tuple(l.rules, l.rule_size, lists_beside(g, oz_ptr, nbr, l.tnm, l.rules, l.rule_size, fill));
+  std::shared_ptr<ListsReady> ready;
+  if (beside) ready = lists_beside(g, oz_ptr, nbr, l.tnm, l.rules, l.rule_size, fill);
+  else
+    check(abi.sph_rule_lists(ints(oz_ptr), &g, nbr.size(1), ints(nbr), l.tnm, ints(l.rules), ints(l.rule_size), fill,
+                             status_of(nbr), stream_of(nbr)));
+  return py::make_tuple(l.rules, l.rule_size, or_none(ready));
 }
 
 // rules / rule_size with a capacity of exactly the longest list: count, read the maximum, allocate, fill.
@@ -672,7 +678,7 @@ PYBIND11_MODULE(sph_host, m) {
   m.def("rules_subm", &rules_subm);
   m.def("strided_begin", &strided_begin);
   m.def("strided_rules", &strided_rules);
-  m.def("deferred_lists", &deferred_lists);
+  m.def("lists_of_table", &lists_of_table);
   m.def("exact_lists", &exact_lists);
   m.def("rules_to_nbr", &rules_to_nbr);
   m.def("pack_weight", &pack_weight);

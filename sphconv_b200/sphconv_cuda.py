@@ -48,12 +48,15 @@ def _want_transposed():
     return bool(config.transposed_table)
 
 
-def _deferred_lists(dev, oz_ptr, nbr, nnz, geom):
-    """The pair lists on the side stream as a timed section of their own -> (rules, rule_size, ready)."""
+def _timed_lists(dev, oz_ptr, nbr, nnz, geom, beside):
+    """The pair lists as a timed section of their own, on the side stream (`beside`) or behind the table, where the section of the
+    rules ends -> (rules, rule_size, ready)."""
     h = C.host()
-    side = torch.cuda.ExternalStream(h.side_stream(dev.index), device=dev)
+    side = torch.cuda.ExternalStream(h.side_stream(dev.index), device=dev) if beside else None
+    if not beside:
+        profiling.mark_stop()
     with profiling.section("lists:" + profiling.current_rule_tag, stream=side):
-        return h.deferred_lists(oz_ptr, nbr, nnz, *geom, config.fill_unused_rules)
+        return h.lists_of_table(oz_ptr, nbr, nnz, *geom, config.fill_unused_rules, beside)
 
 
 def _join_lists(rules):
@@ -80,20 +83,20 @@ def _attach(rules, rule_size, ready, nbr, nbr_t, n_in, n_out, symmetric):
 
 def get_rules_subm(zIndices: torch.Tensor, zPtr: torch.Tensor, batchSize: int, spatialShape: List[int],
                    outSpatialShape: List[int], kernelSize: List[int], stride: List[int], padding: List[int],
-                   dilation: List[int], tileSize: List[int], defer_lists: bool = False):
+                   dilation: List[int], tileSize: List[int], defer_lists: bool = False, lists_beside: bool = True):
     """ref: get_rules_subm, src/sphconv/rules.cu:326-390.  Returns [zIndices, zPtr, rules, ruleSize]
     (the first two are the input objects, as in the reference).  `defer_lists` (extension, used by the modules):
-    rules / ruleSize are written on a side stream and are complete on the current stream only after one of the
-    rule_conv* ops has been called with them."""
+    rules / ruleSize of large rule sets are written on a side stream and are complete on the current stream only after one of the
+    rule_conv* ops has been called with them; not so with `lists_beside` off, for layers that gain nothing from it."""
     geom = (batchSize, spatialShape, outSpatialShape, kernelSize, stride, padding, dilation, tileSize)
     lists = config.materialize_rules
     exact = lists and config.exact_rule_capacity
     defer = defer_lists and config.overlap_rule_lists and lists and not exact
     timed = defer and profiling.is_active() and zIndices.shape[0] > 0
     rules, rule_size, nbr, ready = C.host().rules_subm(zIndices, zPtr, *geom, config.fill_unused_rules,
-                                                       lists and not exact and not timed, defer)
+                                                       lists and not exact and not timed, defer and lists_beside)
     if timed:
-        rules, rule_size, ready = _deferred_lists(zIndices.device, zPtr, nbr, zIndices.shape[0], geom)
+        rules, rule_size, ready = _timed_lists(zIndices.device, zPtr, nbr, zIndices.shape[0], geom, lists_beside)
     if exact:
         rules, rule_size = C.host().exact_lists(zPtr, nbr, *geom, config.fill_unused_rules)
     symmetric = all(k % 2 == 1 and p == d * (k // 2) and s == 1 for k, p, s, d in zip(kernelSize, padding, stride, dilation))
@@ -113,10 +116,10 @@ def get_rules_begin(zIndices: torch.Tensor, zPtr: torch.Tensor, batchSize: int, 
 
 def get_rules(zIndices: torch.Tensor, zPtr: torch.Tensor, batchSize: int, spatialShape: List[int],
               outSpatialShape: List[int], kernelSize: List[int], stride: List[int], padding: List[int],
-              dilation: List[int], tileSize: List[int], pending=None, defer_lists: bool = False):
+              dilation: List[int], tileSize: List[int], pending=None, defer_lists: bool = False, lists_beside: bool = True):
     """ref: get_rules, src/sphconv/rules.cu:405-486.  Returns [ozIndices, ozPtr, rules, ruleSize].
     `pending` (extension): the result of get_rules_begin on the same arguments; step 1 is then not run again (a handle of
-    other arguments is ignored).  `defer_lists` (extension): as for get_rules_subm."""
+    other arguments is ignored).  `defer_lists`, `lists_beside` (extensions): as for get_rules_subm."""
     geom = (batchSize, spatialShape, outSpatialShape, kernelSize, stride, padding, dilation, tileSize)
     lists = config.materialize_rules
     exact = lists and config.exact_rule_capacity
@@ -125,9 +128,10 @@ def get_rules(zIndices: torch.Tensor, zPtr: torch.Tensor, batchSize: int, spatia
     if pending is None:
         pending = get_rules_begin(zIndices, zPtr, *geom)
     oz_idx, oz_ptr, rules, rule_size, nbr, nbr_t, ready = C.host().strided_rules(
-        zIndices, zPtr, *geom, pending, config.fill_unused_rules, lists and not exact and not timed, _want_transposed(), defer)
+        zIndices, zPtr, *geom, pending, config.fill_unused_rules, lists and not exact and not timed, _want_transposed(),
+        defer and lists_beside)
     if timed:
-        rules, rule_size, ready = _deferred_lists(zIndices.device, oz_ptr, nbr, zIndices.shape[0], geom)
+        rules, rule_size, ready = _timed_lists(zIndices.device, oz_ptr, nbr, zIndices.shape[0], geom, lists_beside)
     if exact:
         rules, rule_size = C.host().exact_lists(oz_ptr, nbr, *geom, config.fill_unused_rules)
     return [oz_idx, oz_ptr, *_attach(rules, rule_size, ready, nbr, nbr_t, zIndices.shape[0], oz_idx.shape[0], False)]

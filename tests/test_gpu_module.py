@@ -225,9 +225,9 @@ def test_module_rules_of_large_sets_written_beside_the_convolution(fill):
     B, shape, small = 3, [64, 100, 64], [32, 50, 32]
     z_idx, z_ptr = synthetic.make_random_occupancy(rng, B, shape, 0.3, False)
     zi, zp = torch.as_tensor(z_idx, device=DEV), torch.as_tensor(z_ptr, device=DEV)
-    feat = torch.as_tensor(rng.standard_normal((z_idx.shape[0], 16)), dtype=torch.float16, device=DEV)
-    sub = sphconv.SubMConv3d(16, 16, 3, indice_key="k").to(DEV).half().eval()
-    down = sphconv.SparseConv3d(16, 32, 3, stride=2, padding=1, indice_key="d").to(DEV).half().eval()
+    feat = torch.as_tensor(rng.standard_normal((z_idx.shape[0], 16)), dtype=torch.float32, device=DEV)
+    sub = sphconv.SubMConv3d(16, 32, 3, indice_key="k").to(DEV).eval()
+    down = sphconv.SparseConv3d(32, 32, 3, stride=2, padding=1, indice_key="d").to(DEV).eval()
     geom_s = (zi, zp, B, shape, shape, [3] * 3, [1] * 3, [1] * 3, [1] * 3, [2, 2])
     geom_d = (zi, zp, B, shape, small, [3] * 3, [2] * 3, [1] * 3, [1] * 3, [2, 2])
     ops.config.fill_unused_rules = fill
@@ -250,7 +250,8 @@ def test_module_rules_of_large_sets_written_beside_the_convolution(fill):
         for fn, geom, want, n_out in ((ops.get_rules_subm, geom_s, want_s, zi.numel()), (ops.get_rules, geom_d, want_d, None)):
             oz_idx, _, rules, size = fn(*geom, defer_lists=True)
             assert oz_idx.numel() >= 100000 and rules._sph_ready is not None
-            ops.rule_conv(feat, torch.zeros(27, 16, 16, dtype=torch.float16, device=DEV), rules, size, oz_idx.numel())
+            assert getattr(fn(*geom, defer_lists=True, lists_beside=False)[2], "_sph_ready", None) is None
+            ops.rule_conv(feat, torch.zeros(27, 16, 16, device=DEV), rules, size, oz_idx.numel())
             snap = rules.clone(), size.clone()
             assert rules._sph_ready is None
             same(snap, want)
