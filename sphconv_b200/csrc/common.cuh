@@ -64,13 +64,14 @@ inline void launch(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem
   c.numAttrs = 1;
   (void)cudaLaunchKernelEx(&c, kernel, static_cast<Params>(args)...);      // SPH_LAUNCH_CHECK() reads the error
 }
-// EARLY: a grid of at most four blocks per SM lets its successor in at once, which finds room beside it on every SM.  Blocks let in
-// beside a large grid, or at the end of a persistent one, would all go to the SMs that are free first: 16 blocks behind a
-// convolution took 57 us instead of 9.
-constexpr unsigned kEarlyBlocks = 4 * 148;
+// EARLY: a grid of at most one block per SM lets its successor in at once, which finds room beside it on every SM.  Blocks let in
+// beside a larger grid, or at the end of a persistent one, all go to the SMs that are free first: 16 blocks behind a convolution
+// took 57 us instead of 9, and behind grids of up to four blocks per SM tables and lists took (us, such grids too / only these) 43 / 27 on 93 k
+// rows of 70 scans, 121 / 75 for their strided set, 199 / 132 on 128 k rows 2000 deep.
+constexpr unsigned kEarlyBlocks = 148;
 template <bool EARLY = true>
-__device__ __forceinline__ void after_previous() {
-  if (EARLY && gridDim.x * gridDim.y <= kEarlyBlocks) asm volatile("griddepcontrol.launch_dependents;");
+__device__ __forceinline__ void after_previous(unsigned most = kEarlyBlocks) {
+  if (EARLY && gridDim.x * gridDim.y <= most) asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
