@@ -110,8 +110,13 @@ dense_rows_kernel(V* __restrict__ rows, const int* __restrict__ z_idx, const int
 // Rows need not own their cells: of several rows at one depth of a column the last is the cell's value and each gets the
 // cell's gradient; a row whose depth lies outside the grid has the status bit set and a gradient of zero.  A block can hence have
 // more rows than cells (`crowded`): shared memory then holds one row per cell, the one its value comes from.
-constexpr int kDenseCells = 256;         // cells of a block, when columns are shorter
+constexpr int kDenseCells = 256;         // cells of a block, when columns are shorter and rows not narrow
 constexpr int kDenseMaxCells = 2048;     // columns up to this deep are staged
+// Narrow rows on large grids: more cells a block, up to this many bytes if all are occupied and while this many blocks are left.  Blocks
+// of 256 cells with a few words for each are bound by the two round trips to memory of every block: 33.5 M cells, 284 k rows, one
+// float32 channel 324 -> 56 us and 333 -> 61 back, 12 int8 channels 686 -> 293 and 659 -> 249.
+constexpr int64_t kDenseBytes = 16384;
+constexpr int64_t kDenseBlocks = 16 * 148;
 constexpr int kDenseSmem = 96 * 1024;    // the cells' map (8 KB), 64 KB of rows, and at most 8 bytes a row of padding
 
 // Rows of `words` pieces between memory (pitch words apart) and shared memory (s_pitch), a power of two of lanes per row.
@@ -292,7 +297,10 @@ dense_channels_first_kernel(E* __restrict__ rows, const int* __restrict__ z_idx,
 template <typename E, int V>
 int launch_dense_cf(void* rows, const int* z_idx, const int* z_ptr, int64_t nnz, int B, int64_t cols_per_b, int D, int C,
                     void* dense, int backward, int* status, cudaStream_t st) {
-  int cols = D >= kDenseCells ? 1 : kDenseCells / D;
+  int most = kDenseCells;
+  while (most < kDenseMaxCells && (int64_t)2 * most * C * (int64_t)sizeof(E) <= kDenseBytes && B * cols_per_b * D >= 2 * most * kDenseBlocks)
+    most *= 2;
+  int cols = D >= most ? 1 : most / D;
   while (cols > 1 && (int64_t)cols * D % V) --cols;
   const int cells = cols * D;
   // as many channels at a time as fit in 64 KB when every cell holds a row; an odd number of 4-byte words per row, so that

@@ -199,3 +199,20 @@ def test_dense_rows_copied_ahead(dtype, C, shift):
     want.permute(0, 2, 3, 4, 1)[m] = rows
     assert torch.equal(dense, want)
     assert torch.equal(ops.dense_channels_first_backward(dense, z_idx, z_ptr), rows)
+
+
+@pytest.mark.parametrize("dtype,C", [(torch.float32, 1), (torch.int8, 12), (torch.float16, 3), (torch.float32, 4), (torch.int8, 1)])
+@pytest.mark.parametrize("B,H,W,D", [(2, 40, 1001, 64), (1, 50, 1003, 100), (3, 7, 300, 900), (1, 3, 1100, 2000)])
+def test_dense_of_narrow_rows_on_large_grids(dtype, C, B, H, W, D):
+    """Blocks of up to 2048 cells: several columns, a last block with fewer, columns of more than half a block."""
+    g = torch.Generator(device="cuda").manual_seed(D)
+    at = torch.rand(B, H, W, D, device="cuda", generator=g)
+    m = (at < 0.03) & (torch.rand(B, H, W, 1, device="cuda", generator=g) < 0.7)
+    z_idx, z_ptr = m.nonzero()[:, 3].int().contiguous(), m.sum(-1).view(-1).cumsum(0).int().view(B, H, W)
+    rows = torch.randint(-100, 100, (z_idx.numel(), C), device="cuda", generator=g).to(dtype)
+    dense = ops.dense_channels_first(rows, z_idx, z_ptr, [B, C, H, W, D])
+    want = torch.zeros(B, C, H, W, D, dtype=dtype, device="cuda")
+    want.permute(0, 2, 3, 4, 1)[m] = rows
+    assert torch.equal(dense, want)
+    grad = torch.randint(-100, 100, (B, C, H, W, D), device="cuda", generator=g).to(dtype)
+    assert torch.equal(ops.dense_channels_first_backward(grad, z_idx, z_ptr), grad.permute(0, 2, 3, 4, 1)[m])
