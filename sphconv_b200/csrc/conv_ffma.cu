@@ -61,10 +61,13 @@ template <int CG, int KC> struct FfmaShape {
   static constexpr int A = kItem * AS;
   static constexpr int W = KC * NP;
   static constexpr int BYTES = (ACC + 2 * A + 2 * W) * 4 + kBatch * kRows * 5 + kBatch * 4;
+  static constexpr bool PACKED = CG != 4;            // fma2
 };
 
-// Two fused multiply-adds an instruction, each rounded as fmaf rounds.
+// Two fused multiply-adds, in one instruction (PACKED) or two; each is rounded as fmaf rounds.
+template <bool PACKED = true>
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  if (!PACKED) return make_float2(fmaf(a.x, b.x, c.x), fmaf(a.y, b.y, c.y));
   float2 d;
   asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
       "fma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
@@ -94,10 +97,10 @@ __device__ __forceinline__ void ffma_step(const float* __restrict__ a, const flo
 #pragma unroll
       for (int j = 0; j < RP; ++j) {
         const float2 x = make_float2(av[j][q], av[j][q]);
-        acc[j][0] = fma2(x, make_float2(w0.x, w0.y), acc[j][0]);
-        acc[j][1] = fma2(x, make_float2(w0.z, w0.w), acc[j][1]);
-        acc[j][2] = fma2(x, make_float2(w1.x, w1.y), acc[j][2]);
-        acc[j][3] = fma2(x, make_float2(w1.z, w1.w), acc[j][3]);
+        acc[j][0] = fma2<S::PACKED>(x, make_float2(w0.x, w0.y), acc[j][0]);
+        acc[j][1] = fma2<S::PACKED>(x, make_float2(w0.z, w0.w), acc[j][1]);
+        acc[j][2] = fma2<S::PACKED>(x, make_float2(w1.x, w1.y), acc[j][2]);
+        acc[j][3] = fma2<S::PACKED>(x, make_float2(w1.z, w1.w), acc[j][3]);
       }
     }
   }
@@ -128,7 +131,9 @@ __device__ __noinline__ int pairs_from(int k0, const int* __restrict__ nbr, int 
 // Bound by the shared-memory reads of the operands (74 % of that pipe).  Measured: 64 -> 64 on 170 k rows of 22 neighbours 3.2 ->
 // 0.94 ms, 32 -> 32 on 390 k rows of 12 neighbours 1.9 -> 0.5 ms against the kernel it replaced (one thread group per row
 // walking every slot of the table).  Two FMAs an instruction (fma2; the same bits) take the issue slots off its limits: 64 -> 64
-// on 171 k rows 1070 -> 975 us, 32 -> 64 314 -> 292, 32 -> 32 545 -> 538; the weight gradient 845 -> 763, 228 -> 212, 511 -> 499.
+// on 171 k rows 1070 -> 975 us, 32 -> 64 314 -> 292, 64 -> 16 on 472 k dense rows 1290 -> 1217; the weight gradient 845 -> 763, 228 -> 212,
+// 511 -> 499.  Not in tiles of 32 output channels, which they make slower: 32 -> 32 on 5.4 k / 228 k rows 60 -> 65 / 265 -> 273 us,
+// 16 -> 32 43 -> 47 / 165 -> 168, 128 -> 24 159 -> 173 / 733 -> 755.
 // VEC: float32 rows of a multiple of 4 channels in and out, staged by 16-byte cp.async; else element by
 // element.
 template <typename T, int CG, int KC, bool VEC>
