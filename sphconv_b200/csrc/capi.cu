@@ -202,14 +202,14 @@ extern "C" int sph_conv_gather(const void* d_rows, int dtype, int64_t n_rows, co
                 "the CUDA-core kernels need the unpacked weight");
   // 9 or 27 offsets and up to 64 channels out: the rows by way of tensor memory (conv_tmem.cu), against the two forms that gather into
   // shared memory (us, launches one behind the other, 16-bit rows):
-  //   submanifold 32 -> 32, 61 k / 1.5 M rows 23 -> 17 / 324 -> 201, 64 -> 64, 22 k / 683 k rows 21 -> 17 / 248 -> 165;
-  //   input gradients of strided layers 64 -> 32, 1.5 M rows 510 -> 188, 32 -> 16, 567 k rows 113 -> 91;
-  //   strided 16 -> 32, 61 k / 1.5 M rows 19 -> 16 / 197 -> 171, 32 -> 64, 22 k / 683 k rows 17.0 -> 17.8 / 179 -> 122;
-  //   9 x 3 x 1 filters, whose lines span three heights, 32 -> 32, 228 k rows 57 -> 57.
-  // It does not win where most rows lie beyond the runs' buffers: 64 -> 64 on volumes 95 % full at 256 depths, submanifold 190 -> 215,
-  // strided 36 -> 45; tables without locality, 300 k rows, 16 -> 32 56 -> 61, 32 -> 32 71 -> 83, 64 -> 64 112 -> 137.  The sizes that
-  // the call knows do not tell these from the others, and the rows of this library's own tables are numbered along the grid.
-  // Without rows there is nothing to describe to TMA.
+  //   submanifold 32 -> 32, 61 k / 1.5 M rows 23 -> 16 / 324 -> 194, 64 -> 64, 22 k / 683 k rows 21 -> 17 / 248 -> 165;
+  //   input gradients of strided layers 64 -> 32, 1.5 M rows 510 -> 185, 32 -> 16, 567 k rows 113 -> 83;
+  //   strided 16 -> 32, 61 k / 1.5 M rows 19 -> 16 / 197 -> 164, 32 -> 64, 22 k / 683 k rows 17.0 -> 16.6 / 179 -> 118;
+  //   9 x 3 x 1 filters, whose lines span three heights, 32 -> 32, 228 k rows 57 -> 51.
+  // It does not win where most rows lie beyond the runs' buffers: 64 -> 64 on volumes 95 % full at 256 depths, submanifold 190 -> 202,
+  // strided 36 -> 44; tables without locality, 300 k rows, 16 -> 32 56 -> 58, 32 -> 32 71 -> 78, 64 -> 64 112 -> 132, 1.5 M rows 575 -> 763.
+  // The sizes that the call knows do not tell these from the others, and the rows of this library's own tables are numbered along the
+  // grid.  Without rows there is nothing to describe to TMA.
   if ((kernel == SPH_KERNEL_TC || kernel == SPH_KERNEL_TC_ROWS) && n_rows > 0 && conv_tmem_supported(dtype, kv, k_ch, n_ch))
     return conv_gather_tmem(d_rows, dtype, n_rows, d_packed, d_nbr, n_out, kv, k_ch, n_ch, flip_k, d_scale, bias, relu, d_out,
                             out_dtype, d_status, st);

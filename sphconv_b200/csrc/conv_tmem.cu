@@ -17,9 +17,9 @@
 //  * the operand is handed over by 4 arrivals of warps instead of 128 of threads.
 // The order of sums is that of the other tensor-core kernels (offsets ascending, 32 bytes of a row per instruction), and so are
 // the results, bit for bit.  Measured against them (us, L2 flushed; tables of 27 offsets, share of neighbours present):
-//   32 -> 32 fp16, 1.5 M rows, 0.42   324 -> 205      64 -> 64 fp16, 683 k rows, 0.82   257 -> 162
-//   16 -> 32 fp16, 1.5 M rows, 0.05   201 -> 164      64 -> 32 fp16, 1.5 M rows, 0.13   513 -> 287
-//   32 -> 32 int8, 1.5 M rows, 0.42   256 -> 172      64 -> 64 fp16,  17 k rows, 0.70  24.6 -> 18.4
+//   32 -> 32 fp16, 1.5 M rows, 0.44   328 -> 201      64 -> 64 fp16, 683 k rows, 0.82   253 -> 172
+//   16 -> 32 fp16, 1.5 M rows, 0.05   200 -> 170      64 -> 32 fp16, 1.5 M rows, 0.12   515 -> 195
+//   32 -> 32 int8, 1.5 M rows, 0.44   255 -> 168      64 -> 64 fp16,  22 k rows, 0.69  25.6 -> 22.5
 // Bound by no single unit: issue slots 74 % busy at 32- and 64-byte rows and 60 % at 128-byte rows, the shared-memory data path
 // 34, 68 and 68 % (786 k rows of 16 -> 32 and 32 -> 32, 347 k of 64 -> 64); without the TMEM writes and the loads in front of them a
 // 32 -> 32 layer takes 141 instead of 206 us.  Tried and
@@ -29,9 +29,10 @@
 // A run longer than its buffer (tiles that pass from one line of columns into the next, dense or deep columns, strides that thin
 // the output, tables without locality) is read around it: the gather takes the table's entries a batch ahead, rows inside the
 // buffer from there and the others straight into registers, 32 bytes a load.  Against asking the table offset by offset when a
-// row was found missing: 32 -> 64 strided, 146 k rows of surfaces, every line too long, 68 -> 49 us; 16 -> 32 strided, 61 k rows,
-// 6 % of the lines too long, 24.6 -> 21.5; 32 -> 32 without locality, 300 k rows, 131 -> 95.  Bound there by the latency of L2: a warp
-// has one batch in flight.
+// row was found missing (us, launches one behind the other): 32 -> 64 strided, 146 k rows of surfaces, 91 % of the lines too long,
+// 59 -> 38; 16 -> 32 strided, 111 k rows, 9 % too long, 30 -> 22; input gradient 32 -> 16, 284 k rows, 77 % too long, 82 -> 51;
+// 32 -> 32 without locality, 300 k rows, 119 -> 78.  Bound there by the latency of L2: a warp has one batch in flight.  Both kinds
+// of line in one loop are slower (the state of one costs the other: 3 % over 130 tables, 32 -> 32 on 1.5 M rows 201 against 194).
 //
 // A CTA owns 256 consecutive output rows at a time (two halves of M = 128; one half where the tiles would not fill the SMs)
 // and is persistent over such tiles.  Warp roles: 0-15 gather (warp w: TMEM lanes 32 (w % 4) of half w / 4 % 2, and the batches
@@ -383,44 +384,31 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
             if (!warp_wait(run_full0 + 8u * slot, run_par, abort_flag)) { dead = true; break; }
           }
           const bool split = any && (uint32_t)hi - lo >= cap;
-          const uint32_t held = split ? held_of_split(lo, hi, cap) : cap;   // rows from lo on that the buffer holds
           const uint32_t run = run0 + (uint32_t)slot * slot_bytes;
           const uint32_t line_offsets = (offsets >> (l * L)) & ((1u << L) - 1u);
           const int n = __popc(line_offsets);
-          const uint16_t* place = s_place + ((pb * 8 + rows_of) * kLines + l) * (LP * 32) + lane;
           int j = (int)((count ^ (uint32_t)team) & 1u) * U;            // first place of this team's next batch
           uint32_t c = count + (uint32_t)(j / U);
           count += (uint32_t)((n + U - 1) / U);
-          // A batch ahead, what says where its rows are: their places, or (a run that the buffer does not hold) the table's entries.
-          uint32_t next[U], todo = line_offsets;
-          const bool whole = ((uintptr_t)p.rows & 31u) == 0;
-          auto drop = [&]() {                         // the other team's batch
-#pragma unroll
-            for (int u = 0; u < U; ++u) todo &= todo - 1u;
+          uint32_t next[U];                           // a batch ahead, what says where its rows are
+          auto hand_over = [&](const uint4 (&v)[8]) {
+            if (sent) report();                       // behind this batch's loads
+            const uint32_t op = c % kOperands;
+            if (!warp_wait(a_empty0 + 8u * op, (c / kOperands & 1u) ^ 1u, abort_flag)) return false;
+            tc_fence_after();
+            tmem_st_batch(a_lane + op * kOperandCols, v);
+            sent = op + 1u;
+            j += kTeams * U;
+            c += kTeams;
+            return true;
           };
-          auto entries = [&]() {
-            const int64_t r = tile_row(ti) + rows_of * 32 + lane;
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-              const int k = l * L + __ffs((int)todo) - 1;
-              const bool some = todo != 0u && r < p.n_out;
-              next[u] = some ? (uint32_t)__ldg(p.nbr + (int64_t)(p.flip_k ? KV - 1 - k : k) * p.n_out + r) : ~0u;
-              if (next[u] >= (uint32_t)p.n_rows) next[u] = ~0u;
-              todo &= todo - 1u;
-            }
-            drop();
-          };
-          if (!split) {
+          if (!split) {                               // their places
+            const uint16_t* place = s_place + ((pb * 8 + rows_of) * kLines + l) * (LP * 32) + lane;
 #pragma unroll
             for (int u = 0; u < U; ++u) next[u] = place[(j + u) * 32];        // behind the line: something unused
-          } else {
-            if (j) drop();
-            entries();
-          }
 #pragma unroll 1
-          for (; j < n; j += kTeams * U, c += kTeams) {
-            uint4 v[8];                               // U rows of KC pieces
-            if (!split) {
+            while (j < n) {
+              uint4 v[8];                             // U rows of KC pieces
 #pragma unroll
               for (int u = 0; u < U; ++u) {
                 const uint32_t at = run + next[u] * 16u;
@@ -429,7 +417,33 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
               }
 #pragma unroll
               for (int u = 0; u < U; ++u) next[u] = place[(j + kTeams * U + u) * 32];
-            } else {
+              if (!hand_over(v)) { dead = true; break; }
+            }
+          } else {                                    // the buffer does not hold the run: the table's entries
+            const uint32_t held = held_of_split(lo, hi, cap);          // rows from lo on that it holds
+            const bool whole = ((uintptr_t)p.rows & 31u) == 0;
+            const int64_t r = tile_row(ti) + rows_of * 32 + lane;
+            uint32_t todo = line_offsets;
+            auto drop = [&]() {                       // the other team's batch
+#pragma unroll
+              for (int u = 0; u < U; ++u) todo &= todo - 1u;
+            };
+            auto entries = [&]() {
+#pragma unroll
+              for (int u = 0; u < U; ++u) {
+                const int k = l * L + __ffs((int)todo) - 1;
+                const bool some = todo != 0u && r < p.n_out;
+                next[u] = some ? (uint32_t)__ldg(p.nbr + (int64_t)(p.flip_k ? KV - 1 - k : k) * p.n_out + r) : ~0u;
+                if (next[u] >= (uint32_t)p.n_rows) next[u] = ~0u;
+                todo &= todo - 1u;
+              }
+              drop();
+            };
+            if (j) drop();
+            entries();
+#pragma unroll 1
+            while (j < n) {
+              uint4 v[8];
 #pragma unroll
               for (int u = 0; u < U; ++u) {
                 const uint32_t i = next[u] - lo, at = run + row_at<KC>(i);
@@ -444,13 +458,8 @@ __global__ void __launch_bounds__(kThreads, 1) conv_gather_tmem_kernel(const __g
                 for (int q = 0; q < KC; q += 2) ldg256(v[u * KC + q], v[u * KC + q + 1], src + q * 16, beyond, whole);
               }
               entries();
+              if (!hand_over(v)) { dead = true; break; }
             }
-            if (sent) report();                       // behind this batch's loads
-            const uint32_t op = c % kOperands;
-            if (!warp_wait(a_empty0 + 8u * op, (c / kOperands & 1u) ^ 1u, abort_flag)) { dead = true; break; }
-            tc_fence_after();
-            tmem_st_batch(a_lane + op * kOperandCols, v);
-            sent = op + 1u;
           }
           if (dead) break;
           if (any) {
