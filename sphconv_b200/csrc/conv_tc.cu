@@ -2,8 +2,9 @@
 //
 //   out[r,:] = epilogue( sum_k rows[nbr[k][r], :] @ W[k] )          r in [0, n_out)
 //
-// A tcgen05.mma takes 55-128 SM cycles whatever its shape below M = 128, N = 256 (measured on B200), so the
-// instruction has to be as large as the problem allows.  The channel counts here are small (<= 128) and
+// Issued in a branch of one lane, as here, a tcgen05.mma takes 55-128 SM cycles whatever its shape below M = 128, N = 256
+// (its operands are moved to uniform registers one by one; from converged code it takes 16-64, which conv_tmem.cu is made for),
+// so the instruction has to be as large as the problem allows.  The channel counts here are small (<= 128) and
 // the row count is huge, so the product is computed
 // transposed:  D^T[oC x 256 rows] += W[k]^T[oC x iC] * X_k^T[iC x 256 rows]
 //   A operand = W[k]^T, M = oC padded to 64 or 128, K-major, pre-packed once per weight;

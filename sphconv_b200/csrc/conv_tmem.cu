@@ -20,8 +20,8 @@
 //   32 -> 32 fp16, 1.5 M rows, 0.44   328 -> 201      64 -> 64 fp16, 683 k rows, 0.82   253 -> 172
 //   16 -> 32 fp16, 1.5 M rows, 0.05   200 -> 170      64 -> 32 fp16, 1.5 M rows, 0.12   515 -> 195
 //   32 -> 32 int8, 1.5 M rows, 0.44   255 -> 168      64 -> 64 fp16,  22 k rows, 0.69  25.6 -> 22.5
-// Bound by no single unit: issue slots 74 % busy at 32- and 64-byte rows and 60 % at 128-byte rows, the shared-memory data path
-// 34, 68 and 68 % (786 k rows of 16 -> 32 and 32 -> 32, 347 k of 64 -> 64); without the TMEM writes and the loads in front of them a
+// Bound by no single unit: issue slots 75, 71 and 61 % busy at 32-, 64- and 128-byte rows, the shared-memory data path
+// 41, 71 and 68 % (786 k rows of 16 -> 32 and 32 -> 32, 347 k of 64 -> 64); without the TMEM writes and the loads in front of them a
 // 32 -> 32 layer takes 141 instead of 206 us.  Tried and
 // slower: entries kept in registers with the offsets unrolled (instruction fetch: 577); rows of zeros in shared memory for absent
 // neighbours (bank conflicts: 263); the instruction's disable-output-lane mask instead of zeros (its operands: 217).

@@ -1177,9 +1177,8 @@ int launch_rule_lists(const int* out_zp, const Geom& g, int64_t out_nnz, int tnm
   if (g.KV == 27 && (int64_t)tnm * 54 < (1LL << 32)) {
     // the usual 3 x 3 x 3 filter: the kernel with the offsets' running counts in registers
     // nine offsets per warp where that gives the machine enough warps, else three (small tile grids have long tiles:
-    // more warps per tile also evens out their lengths).  Measured beside the convolution kernels: one chunk of 32
-    // positions per step beats 2, 4 or 8 (more registers per thread = fewer list warps resident beside the persistent
-    // convolution CTA), and 27 offsets per warp leaves too few warps.
+    // more warps per tile also evens out their lengths).  One chunk of 32 positions per step beats 2, 4 or 8, and 27 offsets per
+    // warp leaves too few warps: measured beside convolutions that left registers of an SM for few list warps, within 20 % alone.
 #define SPH_LISTS_FIXED(NK)                                                                                           \
   launch(rule_lists_fixed_kernel<NK, 1>, (unsigned)div_up64((int64_t)g.nTile * (27 / NK), kFixWarps), kFixWarps * 32, 0,     \
                                    st, out_zp, g, out_nnz, tnm, 27 / NK, nbr, rules, rule_size, status)
