@@ -618,7 +618,7 @@ def main():
                 q = chunks * 4.0 * 27 * cm["n_out"] + 8.0 * pairs          # table read, pairs written
                 row.update({"bytes": int(q), "gbs": round(q / (ms * 1e-3) / 1e9, 1),
                             "frac_hbm": round(q / (ms * 1e-3) / h_peak, 4),
-                            "what": "reference-format pair lists from the table (fp32 layers of more than 16 channels: on a side stream beside the convolution)"})
+                            "what": "reference-format pair lists from the table (beside the convolution, on a side stream, where that gains)"})
             layer_rows.append(row)
         else:
             layer_rows.append({"layer": name, "ms": round(ms, 4)})

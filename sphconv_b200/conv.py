@@ -87,13 +87,9 @@ class Conv3d(Convolution):
         args = (input.z_idx, input.z_ptr, input.B, in_shape, out_shape, self.kernel_size, self.stride, self.padding,
                 self.dilation, self.tile_size)
         # defer_lists: the reference-format pair lists may be written on a side stream while this layer's convolution, which reads
-        # the neighbour table only, runs; rule_conv orders the stream behind them again.  Only the float32 layers of more than 16
-        # channels gain from it: the other kernels fill the SMs, and the lists beside them make their blocks start one after the
-        # other.  us, lists on the side / the caller's stream, submanifold layers: fp32 32 -> 32 on 284 k / 567 k rows 238 / 260 and
-        # 495 / 534, 64 -> 64 500 / 538 and 977 / 1028 (strided 16 -> 32 497 / 503 and 940 / 950), 16 -> 16 94 / 91 and 171 / 150;
-        # fp16 32 -> 32 99 / 88 and 180 / 147, 64 -> 64 127 / 112 and 225 / 191, 16 -> 16 on 567 k rows 138 / 134, 4 -> 16 123 / 119;
-        # encoders of 8 layers: fp16 8 scans 1728 / 1706, bf16 training 16 scans 10340 / 10270, int8 wide 11819 / 11830.
-        beside = input.feature.dtype == torch.float32 and max(self.in_channels, self.out_channels) > 16
+        # the neighbour table only, runs; rule_conv orders the stream behind them again
+        beside = ops.lists_beside(input.feature.dtype, math.prod(self.kernel_size), self.in_channels, self.out_channels,
+                                  ops.config.fill_unused_rules)
         if self.subm:
             oz_idx, oz_ptr, rules, rule_size = ops.get_rules_subm(*args, defer_lists=True, lists_beside=beside)
         else:

@@ -190,7 +190,7 @@ class Padding {
 // Rule sets from this size on have their lists written on the side stream where the caller asks for it, beside the convolution.  The two
 // events, the waits and the allocator's records of a smaller one cost the host more than its lists cost the GPU (us, lists on the side /
 // the caller's stream): one layer on 6 k rows 58 / 46, on 16 k 66 / 39, a strided layer's training step on 16 k to 71 k rows 228 / 206.
-// From here on it is the layer that decides (Conv3d._rules).
+// From here on it is the layer that decides (lists_beside in sphconv_cuda.py).
 constexpr int64_t kListsBesideRows = 100000;
 
 // The lists of a rule set whose table has been enqueued on the current stream, on the side stream.

@@ -16,6 +16,7 @@ tensor (attribute ``_sph``).  Rules without it - cloned, loaded from disk, made 
 converted on first use and the result is cached on the tensor until it is modified in place.
 """
 import ctypes
+import functools
 from typing import List, Optional
 
 import torch
@@ -46,6 +47,26 @@ def _want_transposed():
     if config.transposed_table is None:
         return torch.is_grad_enabled()
     return bool(config.transposed_table)
+
+
+@functools.lru_cache(maxsize=256)
+def lists_beside(dtype, kv, in_channels, out_channels, padded):
+    """Whether a layer gains from pair lists written on a side stream beside its convolution (us, lists on the side / the caller's
+    stream; submanifold layers where not said otherwise).
+    The CUDA-core kernels of more than 16 channels do: fp32 32 -> 32 on 284 k / 567 k rows 238 / 260 and 495 / 534, 64 -> 64 500 / 538
+    and 977 / 1028, strided 16 -> 32 497 / 503 and 940 / 950, bf16 48 -> 40 on 205 k rows 567 / 591; but fp32 16 -> 16 94 / 91 and 171 / 150.
+    The tensor-memory kernel fills the SMs and its blocks start one after the other behind lists beside it: fp16 32 -> 32 99 / 88 and
+    180 / 147, 64 -> 64 127 / 112 and 225 / 191, padded lists 191 / 178 and 333 / 298; encoders of 8 layers: fp16 8 scans 1728 / 1706, bf16 training
+    16 scans 10340 / 10270, int8 wide 11819 / 11830.
+    The other 16-bit kernels gain where the lists are padded, because those wait for the padding: bf16 on 205 k rows 24 -> 40 255 / 260,
+    4 -> 16 181 / 186 (16 -> 16 176 / 174), strided on 756 k rows 16 -> 16 451 / 462, 24 -> 40 1016 / 1033; without padding it goes
+    either way by 3 %, and by up to 14 % for the caller's stream below 150 k rows (fp16 4 -> 16 on 142 k rows 52 / 44)."""
+    if dtype not in C.DTYPE_CODE:
+        return False
+    layer = (C.DTYPE_CODE[dtype], kv, in_channels, out_channels)
+    if C.lib().sph_conv_kernel(*layer, 0) == 0:                  # SPH_KERNEL_GENERAL
+        return max(in_channels, out_channels) > 16
+    return padded and dtype is not torch.float32 and not C.lib().sph_conv_uses_tmem(*layer)
 
 
 def _timed_lists(dev, oz_ptr, nbr, nnz, geom, beside):

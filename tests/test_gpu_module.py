@@ -286,6 +286,15 @@ def test_weights_that_are_not_contiguous_are_refused(dtype):
             ops._gather(x, w, nbr, 8, False, None, None, False, None)
 
 
+def test_layers_whose_lists_are_written_beside_them():
+    from sphconv_b200 import sphconv_cuda as ops
+    f32, f16, i8 = torch.float32, torch.float16, torch.int8
+    for dtype, iC, oC, padded, want in ((f32, 16, 32, False, True), (f32, 64, 64, True, True), (f32, 16, 16, True, False), (f16, 32, 32, True, False),
+                                        (f16, 48, 40, False, True), (f16, 16, 16, True, True), (f16, 16, 16, False, False), (i8, 64, 64, True, False),
+                                        (torch.float64, 64, 64, True, False)):
+        assert ops.lists_beside(dtype, 27, iC, oC, padded) is want
+
+
 FIRST_USE = """
 import sys, threading
 import torch
